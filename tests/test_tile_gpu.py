@@ -1,0 +1,77 @@
+"""Edges of the tensor-memory tile kernel behind batched products: token tiles, row tiles, shared tiles, both f16 forms of
+lattice weights."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from oracle import mfq_oracle as O  # noqa: E402
+from tyloquant_b200 import QuantWeight, encode  # noqa: E402
+from test_gemm_gpu import _status  # noqa: E402
+from test_nint_gpu import bf16_tensor, REL_L2  # noqa: E402
+
+SHAPES = [(1, 24), (127, 200), (129, 1001), (272, 4104), (1000, 776)]   # rows around 16 and 128, one chunk to many, ragged columns
+TOKENS = [5, 16, 17, 33, 128, 129, 255, 257, 520]
+
+
+@pytest.mark.parametrize("profile", [(2, 16, 5), (3, 24, 5), (4, 24, 6), (4, 48, 6), (5, 28, 7), (6, 24, 7), (8, 22, 7), (8, 64, 7)])
+def test_scalar_weights(profile):
+    bits, gs, sb = profile
+    for n, k in SHAPES:
+        blob = encode.random_nint_blob(n, k, bits, gs, sb, seed=n + k + gs, device="cuda")
+        ref = O.dequant_nint(O.unpack_nint(blob))
+        w = QuantWeight.from_blob(f"NINT{bits}", blob)
+        for m in TOKENS:
+            x = encode.bf16_round(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32))
+            x[0] *= np.float32(2.0 ** 100)   # every row has its own scale
+            x[-1] *= np.float32(2.0 ** -66)
+            y = w.matmul(bf16_tensor(x), out_dtype=torch.float32).cpu().numpy()
+            assert _status() == 0
+            # against what the products add up to without cancellation (a single output can cancel to nearly nothing)
+            err = y.astype(np.float64) - x.astype(np.float64) @ ref.astype(np.float64).T
+            size = np.sqrt(np.square(x, dtype=np.float64) @ np.square(ref, dtype=np.float64).T)
+            for rows in (slice(0, 1), slice(1, m - 1), slice(m - 1, m)):
+                assert np.linalg.norm(err[rows]) <= REL_L2 * np.linalg.norm(size[rows]), (profile, n, k, m, rows)
+        w.free()
+
+
+@pytest.mark.parametrize("form", ["plain", "joint, exact scales", "joint, two terms"])
+def test_lattice_weights(form):
+    jsc = form != "plain"
+    banks = encode.synthetic_d4_banks(512, 2, seed=5) if jsc else O.d4_256_codebook()[None]
+    for n, k in SHAPES:
+        wt = encode.bf16_round(np.random.default_rng(n + k).standard_normal((n, k), dtype=np.float32) * np.float32(0.02))
+        blob = encode.nvq_blob(encode.quantize_nvq3(wt, banks, jsc=jsc, device="cuda"))
+        if form.endswith("two terms"):   # state scales with eleven significant bits: their products with the codes are no f16 numbers
+            at = blob.index(bytes([1, 2, 16, 1]), 36) + 4   # the metadata header: version, banks, states, mode, then the scales
+            lut = (np.frombuffer(blob[at:at + 32], dtype="<f2").astype(np.float32) * np.float32(1.2373)).astype("<f2")
+            blob = blob[:at] + lut.tobytes() + blob[at + 32:]
+        ref = O.dequant_nvq(O.unpack_nvq(blob))
+        w = QuantWeight.from_blob("NVQ3J-512" if jsc else "NVQ3", blob)
+        for m in [2, 3] + TOKENS:
+            x = encode.bf16_round(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32))
+            y = w.matmul(bf16_tensor(x), out_dtype=torch.float32).cpu().numpy()
+            assert _status() == 0
+            err = y.astype(np.float64) - x.astype(np.float64) @ ref.astype(np.float64).T
+            size = np.sqrt(np.square(x, dtype=np.float64) @ np.square(ref, dtype=np.float64).T)
+            assert np.linalg.norm(err) <= 1e-5 * np.linalg.norm(size), (form, n, k, m)   # exact weights and activations: float32 sums
+        w.free()
+
+
+def test_shared_tiles_are_left_clean():
+    """Tiles that several CTAs share are summed in a buffer that has to be zero again after every call, whatever the shapes."""
+    ws = {}
+    for n, k in ((200, 4200), (4096, 1536), (512, 9000)):
+        blob = encode.random_nint_blob(n, k, 4, 24, 6, seed=n, device="cuda")
+        ws[n] = (QuantWeight.from_blob("NINT4", blob), k, torch.from_numpy(O.dequant_nint(O.unpack_nint(blob))).cuda())
+    gen = torch.Generator("cuda").manual_seed(1)
+    for i in range(30):
+        n = (200, 4096, 512)[i % 3]
+        w, k, ref = ws[n]
+        x = torch.randn((7, 300, 21, 130)[i % 4], k, device="cuda", generator=gen).to(torch.bfloat16)
+        y_ref = x.double() @ ref.double().T
+        assert ((w.matmul(x, out_dtype=torch.float32).double() - y_ref).norm() / y_ref.norm()).item() <= REL_L2, i
+    assert _status() == 0

@@ -10,6 +10,7 @@
 #include "cuda_util.h"
 #include "nvq.h"
 #include "nvq_blayout.h"
+#include "tile_tc.h"
 
 namespace mfqb {
 
@@ -44,6 +45,7 @@ NvqDevicePtr make_nvq_device(const HostNvq& t, int device, mfqb_weight_info* inf
     w->anchors.upload(p.anchors.data(), p.anchors.size() * 4);
     w->table.upload(p.table.data(), p.table.size() * 4);
     w->d = p.d;
+    w->d.tile_terms = t.jsc ? lattice_terms(p.d.lut, t.codebooks.data(), t.codebooks.size()) : 1;
     w->d.items = static_cast<const uint32_t*>(w->items.p);
     w->d.anchors = static_cast<const uint32_t*>(w->anchors.p);
     w->d.table = static_cast<const uint32_t*>(w->table.p);
@@ -106,6 +108,7 @@ void nvq_dequant(const NvqDevice& w, void* out, int out_dtype, cudaStream_t stre
 }
 
 void nvq_mul_mat(const NvqDevice& w, const void* x_bf16, int m, void* y, int y_dtype, cudaStream_t stream) {
+    if (m >= 2 && launch_tile_product(w.d, x_bf16, m, y, y_dtype, w.device, stream)) return;
     const size_t ysz = y_dtype == MFQB_F32 ? 4 : 2;
     for (int m0 = 0; m0 < m; m0 += 8) {   // batch rows one launch covers
         const int mm = std::min(8, m - m0);

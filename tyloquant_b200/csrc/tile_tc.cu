@@ -1,0 +1,310 @@
+// Host side of the tensor-memory tile kernel (tile_tc.cuh): activation tiles, shared-memory plan, launches.
+#include <algorithm>
+#include <cmath>
+
+#include "cuda_util.h"
+#include "tile_tc.h"
+#include "tile_tc_launch.cuh"
+
+namespace mfqb {
+
+int* device_status_word(int device);
+
+// ---- activations ---------------------------------------------------------------------------------------------------------
+struct XTilesArgs {
+    const void* x;
+    int kind;              // TileX
+    int k, x_rows;
+    size_t row_bytes;
+    unsigned char* out;
+    float* down;
+    // experts: a block row is a position of the route plan, its source row the pair (src_div = 1), the pair's token (src_div =
+    // routes), or the position itself (src_div = 0)
+    const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool;
+    int n_experts, src_div, m;
+    int t8[kTileMaxPools], gs[kTileMaxPools], nchunks[kTileMaxPools];
+};
+
+// (2^e, 2^-e) with 2^e * max in [2^14, 2^15); (1, 1) for a zero, subnormal or non-finite maximum.
+__device__ __forceinline__ float2 x_row_scale(uint32_t absmax_bits) {
+    int eb = (int)(absmax_bits >> 23);
+    if (eb == 0 || eb == 255) return make_float2(1.f, 1.f);
+    eb = max(eb, 15);   // below 2^-112 rows keep fewer bits
+    return make_float2(__uint_as_float((uint32_t)(268 - eb) << 23), __uint_as_float((uint32_t)(eb - 14) << 23));
+}
+
+template <int KIND>
+__device__ __forceinline__ float x_value(const void* row, int k, int j) {
+    if constexpr (KIND == kTileXBf16) return __bfloat162float(__ldcg(static_cast<const __nv_bfloat16*>(row) + j));
+    const float v = __ldcg(static_cast<const float*>(row) + j);
+    if constexpr (KIND == kTileXSwiglu) return __ldcg(static_cast<const float*>(row) + k + j) * v / (1.0f + expf(-v));
+    return v;
+}
+// Four consecutive values from column j on, zero past the row.
+template <int KIND>
+__device__ __forceinline__ float4 x_quad(const void* row, int k, int j, bool aligned) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (aligned && j + 3 < k) {
+        if constexpr (KIND == kTileXBf16) {
+            const uint2 r = __ldcg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(row) + j));
+            v = make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
+        } else {
+            v = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + j));
+            if constexpr (KIND == kTileXSwiglu) {
+                const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k + j));
+                v = make_float4(u.x * v.x / (1.0f + expf(-v.x)), u.y * v.y / (1.0f + expf(-v.y)), u.z * v.z / (1.0f + expf(-v.z)), u.w * v.w / (1.0f + expf(-v.w)));
+            }
+        }
+    } else {
+        if (j < k) v.x = x_value<KIND>(row, k, j);
+        if (j + 1 < k) v.y = x_value<KIND>(row, k, j + 1);
+        if (j + 2 < k) v.z = x_value<KIND>(row, k, j + 2);
+        if (j + 3 < k) v.w = x_value<KIND>(row, k, j + 3);
+    }
+    return v;
+}
+__device__ __forceinline__ uint32_t x_pack(float a, float b) {   // non-finite -> NaN, which poisons the token's outputs
+    const __half ha = isfinite(a) ? __float2half_rn(a) : __ushort_as_half((unsigned short)0x7E00);
+    const __half hb = isfinite(b) ? __float2half_rn(b) : __ushort_as_half((unsigned short)0x7E00);
+    return (uint32_t)__half_as_ushort(ha) | ((uint32_t)__half_as_ushort(hb) << 16);
+}
+
+// Scales a row to the top of the f16 range and writes it as B operand: per 64-column slab the tile's rows of 128 bytes with
+// the 128-byte swizzle, columns in the decoders' order (slab of 16 columns (f, t, h): octet t of groups 4f + 2h, + 1; quads
+// c = 0..3 of these 16 slots, their slots 0 and 2 in columns 2c, 2c + 1, slots 1 and 3 in columns 8 + 2c, + 1).  Slots past
+// the group size, groups and columns past the row are zero.  Grid (splits, rows): every CTA takes the row's maximum for
+// itself (from L2; a second launch for the maxima costs more for the rows of a decoding batch) and writes its share.
+template <int KIND>
+__global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XTilesArgs a) {
+    __shared__ uint32_t red[8];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int p = blockIdx.y;
+    int pool = 0, src = p, tile_begin = p / a.x_rows * a.x_rows, ncols = min(a.x_rows, a.m - tile_begin), base = tile_begin;
+    if (a.tile_bounds != nullptr) {
+        if (p >= a.expert_bounds[a.n_experts]) return;
+        int lo = 0, hi = a.n_experts - 1;   // expert with expert_bounds[e] <= p < expert_bounds[e + 1]
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (a.expert_bounds[mid] <= p) lo = mid;
+            else hi = mid - 1;
+        }
+        pool = a.expert_pool[lo];
+        if (pool < 0) return;
+        const int eb = a.expert_bounds[lo], local = (p - eb) / a.x_rows * a.x_rows;
+        tile_begin = eb + local;
+        ncols = min(a.x_rows, a.expert_bounds[lo + 1] - tile_begin);
+        base = tile_x_row(eb, lo, local);
+        if (a.src_div > 0) src = a.pair_order[p] / a.src_div;
+    }
+    const int T = a.t8[pool], gs = a.gs[pool], nslabs = a.nchunks[pool] * 4 * T, k = a.k, tid = threadIdx.x;
+    constexpr int ESZ = KIND == kTileXBf16 ? 2 : 4;
+    const unsigned char* row = static_cast<const unsigned char*>(a.x) + (size_t)src * k * (KIND == kTileXSwiglu ? 2 : 1) * ESZ;
+    const bool row_al = (reinterpret_cast<uintptr_t>(row) & (4 * ESZ - 1)) == 0 && (KIND != kTileXSwiglu || (k & 3) == 0);
+    // largest magnitude as float bits (they order like the values, NaN and infinity largest).  Eight loads in flight per
+    // thread, out-of-range ones predicated off: a plain unrolled loop runs its few iterations one after the other.
+    uint32_t ab = 0u;
+    if (KIND == kTileXBf16 && (reinterpret_cast<uintptr_t>(row) & 15) == 0 && (k & 7) == 0) {
+        for (int j0 = tid; j0 < (k >> 3); j0 += 2048) {
+            uint4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) v[u] = j0 + 256 * u < (k >> 3) ? __ldcg(reinterpret_cast<const uint4*>(row) + j0 + 256 * u) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const uint32_t w4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) ab = max(ab, max(w4[i] & 0x7FFF0000u, (w4[i] << 16) & 0x7FFF0000u));
+            }
+        }
+    } else {
+        for (int j0 = 4 * tid; j0 < k; j0 += 4096) {
+            float4 v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = j0 + 1024 * u < k ? x_quad<KIND>(row, k, j0 + 1024 * u, row_al) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                ab = max(max(ab, __float_as_uint(fabsf(v[u].x))), max(__float_as_uint(fabsf(v[u].y)), max(__float_as_uint(fabsf(v[u].z)), __float_as_uint(fabsf(v[u].w)))));
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) ab = max(ab, __shfl_xor_sync(0xffffffffu, ab, o));
+    if ((tid & 31) == 0) red[tid >> 5] = ab;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) ab = max(ab, red[i]);
+    const float2 sc = x_row_scale(ab);
+    if (blockIdx.x == 0 && tid == 0) a.down[p] = sc.y;
+    const int r = p - tile_begin, pitch = ((ncols + 7) & ~7) * 128;
+    unsigned char* dst = a.out + (size_t)base * a.row_bytes + (size_t)r * 128;
+    const bool quad_al = row_al && (gs & 3) == 0;
+    for (int js = blockIdx.x * 256 + tid; js < nslabs; js += gridDim.x * 256) {
+        const int ch = js / (4 * T), jj = js - ch * 4 * T, h = jj & 1, ft = jj >> 1, f = ft / T, t = ft - f * T;
+        const int g = ch * kChunkGroupsB + 4 * f + 2 * h;
+        uint32_t w[8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int slot = 8 * t + 4 * (c & 1), k0 = (g + (c >> 1)) * gs + slot;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (slot + 3 < gs) {
+                v = x_quad<KIND>(row, k, k0, quad_al);
+            } else {
+                if (slot < gs && k0 < k) v.x = x_value<KIND>(row, k, k0);
+                if (slot + 1 < gs && k0 + 1 < k) v.y = x_value<KIND>(row, k, k0 + 1);
+                if (slot + 2 < gs && k0 + 2 < k) v.z = x_value<KIND>(row, k, k0 + 2);
+            }
+            w[c] = x_pack(v.x * sc.x, v.z * sc.x);
+            w[4 + c] = x_pack(v.y * sc.x, v.w * sc.x);
+        }
+        const int slab = js & 3;
+        unsigned char* at = dst + (size_t)(js >> 2) * pitch;
+        *reinterpret_cast<uint4*>(at + (((2 * slab) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(at + (((2 * slab + 1) ^ (r & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+
+static void launch_x_tiles(const XTilesArgs& a, int kind, int rows, int nslabs, int sms, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    // one CTA per row fills the chip from a few hundred rows on; fewer rows are shared out
+    const int splits = std::max(1, std::min((nslabs + 255) / 256, 2 * sms / std::max(rows, 1)));
+    cfg.gridDim = dim3((unsigned)splits, (unsigned)rows);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    switch (kind) {
+        case kTileXBf16: MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<kTileXBf16>, a)); break;
+        case kTileXF32: MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<kTileXF32>, a)); break;
+        default: MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<kTileXSwiglu>, a)); break;
+    }
+}
+
+// ---- plans ---------------------------------------------------------------------------------------------------------------
+static size_t x_row_bytes(const NintDevB& w) { return (size_t)w.nchunks * w.t8 * 128; }
+
+// Rings for tokens tiles of `n` columns: records first (two stages, then up to 64 KB of them, which is what keeps HBM busy),
+// activation slabs in the rest.  False when the codec's tables and two stages of each do not fit.
+static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8, int terms, size_t ctx_bytes) {
+    const size_t budget = kTileDynSmem - 1024, ctx = (ctx_bytes + 15) / 16 * 16;
+    a.n_mma = n;
+    a.d_bufs = n <= 128 ? 2 : 1;
+    a.d_cols = n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256));
+    const int a_total = 512 - a.d_bufs * a.d_cols;
+    // Small N: every barrier round trip costs more than the tensor work between two of them, so a step takes two chunks and an
+    // activation stage all of a step.  Large N: one chunk a step, activations in 64-column slabs.
+    for (int step = 2; step >= 0; --step) {
+        a.x_whole = step > 0;
+        a.step = std::max(step, 1);
+        a.a_cols = 16 * t8 * terms * a.step;
+        a.a_stages = std::min(kTileAStages, a_total / a.a_cols);
+        const size_t rec_stage = 8 * rec_bytes * a.step, x_stage = (size_t)n * 128 * (a.x_whole ? a.step * t8 : 1);
+        if (a.a_stages < 2 || ctx + 2 * rec_stage + 2 * x_stage > budget || (a.x_whole && x_stage > 24 * 1024)) continue;
+        size_t left = budget - ctx - 2 * rec_stage - 2 * x_stage;
+        int rs = 2, xs = 2;
+        for (bool grown = true; grown;) {
+            grown = false;
+            if (xs < 4 && left >= x_stage) { ++xs; left -= x_stage; grown = true; }
+            if (rs < kTileRecStages && (size_t)rs * rec_stage < 64 * 1024 && left >= rec_stage) { ++rs; left -= rec_stage; grown = true; }
+        }
+        while (xs < kTileXStages && !a.x_whole && left >= x_stage) { ++xs; left -= x_stage; }
+        a.rec_stages = rs;
+        a.rec_stage_bytes = (int)rec_stage;
+        a.x_stages = xs;
+        a.x_stage_bytes = (int)x_stage;
+        p.smem = 1024 + std::max((size_t)xs * x_stage + (size_t)rs * rec_stage + ctx, (size_t)n * kTileRows * 4);   // a shared tile is finished there
+        return true;
+    }
+    return false;
+}
+
+static cudaError_t launch_one(const TileArgs& a, const TilePlan& p, int terms, cudaStream_t s) {
+    switch (a.pools[0].table ? 0 : a.pools[0].bits) {
+        case 0: return launch_tile_nvq(a, p, terms, s);
+        case 2: return launch_tile_bits<2>(a, p, s);
+        case 3: return launch_tile_bits<3>(a, p, s);
+        case 4: return launch_tile_bits<4>(a, p, s);
+        case 5: return launch_tile_bits<5>(a, p, s);
+        case 6: return launch_tile_bits<6>(a, p, s);
+        case 8: return launch_tile_bits<8>(a, p, s);
+        default: return cudaErrorNotSupported;
+    }
+}
+
+// f16 state scales of a lattice record, normalised so that code x scale stays below 2^15.
+static void lattice_scales(const NintDevB& w, TileArgs& a) {
+    float top = 0.f;
+    for (int i = 0; i < 16; ++i) top = std::max(top, std::fabs(w.jsc ? w.lut[i] : (float)i));
+    int e = 0;
+    if (w.jsc && top > 0.f && std::isfinite(top)) std::frexp(top, &e);   // top = m 2^e, m in [0.5, 1)
+    const int shift = w.jsc ? 8 - e : 0;                                 // codes reach 127
+    for (int i = 0; i < 16; ++i) a.lut16[i] = __half_as_ushort(__float2half(std::ldexp(w.jsc ? w.lut[i] : (float)i, shift)));
+    a.lut_undo = std::ldexp(1.f, -shift);
+}
+int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes) {
+    bool used[128] = {};
+    for (size_t i = 0; i < n_codes; ++i) used[codes[i] & 127] = true;
+    for (int s = 0; s < 16; ++s)
+        for (int c = 0; c < 128; ++c) {
+            if (!used[c] || lut[s] == 0.f) continue;
+            int e;
+            const float m = std::frexp(lut[s] * (float)c, &e) * 2048.f;   // 11 significant bits are an f16
+            if (c && m != std::floor(m)) return 2;
+        }
+    return 1;
+}
+
+// y [m, n] = x [m, k] W^T.  False when this weight has no tile kernel.
+bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s) {
+    TileArgs a{};
+    TilePlan p;
+    const int terms = w.table ? w.tile_terms : 1;
+    // token tiles: as few as 256 columns allow, of equal size
+    const int ntok = (m + 255) / 256, n = std::max(16, ((m + ntok - 1) / ntok + 15) / 16 * 16);
+    if (!tile_plan(a, p, n, (size_t)w.rec_words * 4, w.t8, terms, w.table ? (size_t)w.table_words * 4 + 64 : 0)) return false;
+    const int row_tiles = (w.n + kTileRows - 1) / kTileRows, sms = device_sm_count(device);
+    const long long tiles = (long long)row_tiles * ((m + n - 1) / n), units = tiles * w.nchunks;
+    if (units * (sms + 1) >= (1ll << 31) * 1ll * sms || units >= (1ll << 31)) return false;
+    a.pools[0] = w;
+    if (w.table) lattice_scales(w, a);
+    a.m = m;
+    a.ntok = (m + n - 1) / n;
+    a.x_rows = n;
+    a.x_row_bytes = x_row_bytes(w);
+    a.y = y;
+    a.y_dtype = y_dtype;
+    a.ldy = w.n;
+    a.units = (int)units;
+    a.only_pool = -1;
+    a.error = device_status_word(device);
+    // no more CTAs than two chunks each, nor than a dozen per tile: the last one adds the others' partial tiles
+    p.grid = (int)std::max<long long>(1, std::min<long long>(sms, std::min((units + 1) / 2, tiles * 12)));
+    static GrowOnlyScratch xs[2], parts, counts;   // activations: decoding batches keep a small block of their own beside the prefill's
+    const size_t xb = ((size_t)(m + 7) / 8 * 8 * a.x_row_bytes + 255) / 256 * 256;
+    unsigned char* buf = static_cast<unsigned char*>(xs[m > 16].get(device, xb + (size_t)m * 4, s, "mfqb_mul_mat (f16 activation tiles)"));
+    a.x = buf;
+    a.x_down = reinterpret_cast<const float*>(buf + xb);
+    a.partial = static_cast<float*>(parts.get(device, (size_t)p.grid * n * kTileRows * 4, s, "mfqb_mul_mat (partial tiles)"));
+    a.counters = static_cast<unsigned*>(counts.get(device, (size_t)p.grid * 4, s, "mfqb_mul_mat (tile counters)"));
+    XTilesArgs xa{};
+    xa.x = x;
+    xa.kind = kTileXBf16;
+    xa.k = w.k;
+    xa.m = m;
+    xa.x_rows = n;
+    xa.row_bytes = a.x_row_bytes;
+    xa.out = buf;
+    xa.down = reinterpret_cast<float*>(buf + xb);
+    xa.t8[0] = w.t8;
+    xa.gs[0] = w.gs;
+    xa.nchunks[0] = w.nchunks;
+    launch_x_tiles(xa, kTileXBf16, m, w.nchunks * 4 * w.t8, sms, s);
+    const cudaError_t e = launch_one(a, p, terms, s);
+    if (e == cudaErrorNotSupported) return false;
+    if (e != cudaSuccess)
+        fail(MFQB_ERR_CUDA, "%s%d gs=%d tile product launch (m = %d, %zu bytes of shared memory): %s", w.table ? "NVQ index bits " : "NINT", w.table ? w.index_bits : w.bits,
+             w.gs, m, p.smem, cudaGetErrorString(e));
+    return true;
+}
+
+}  // namespace mfqb

@@ -1,0 +1,724 @@
+// Batched products of packed weights on tcgen05 tensor cores, weights decoded straight into tensor memory.
+//
+//   y[token, n] = sum_k x[token, k] * W[n, k]
+//
+// A CTA works on tiles of 128 weight rows x N tokens (N <= 256), one chunk (8 groups) of K at a time, and every warp has one
+// role for the whole kernel:
+//   * record loader: bulk copies of the chunk's eight packed records (one per 16-row block) into a ring in shared memory; the
+//     weights are constants, so it starts before the kernel waits for its predecessor in the stream;
+//   * activation loader: bulk copies of 64-column slabs of the scaled f16 activations, which x_tiles_kernel has already
+//     written in the order, padding and 128-byte swizzle the tensor core reads (no tensor map);
+//   * 16 decoders: warp (row-block, half of the chunk) turns codes into f16 pairs in registers -- in byte-lane fragment order
+//     these ARE rows q, q + 8 of a 16 x 16 A operand -- and stores them with tcgen05.st into the A ring in tensor memory.
+//     The A operand never touches shared memory, whose bandwidth the B operand needs (8 KB in and 8 KB out per 128 cycles
+//     for N = 256);
+//   * mma issuer: one thread, tcgen05.mma with A from tensor memory, B from shared memory, D in tensor memory;
+//   * 4 epilogue warps: tcgen05.ld, scaling by row and token factors, stores.
+//
+// Arithmetic.  A row of W is factored as F * (a ss (q - mid) + (mid a ss - b sm)) with F = max(|ns|, |nm| 2^-(BITS+1)),
+// a = ns / F, b = nm / F: F is applied to the finished sums in float32, and since F = ns for every ordinary row the step
+// a ss is an integer and exact in f16.  The offset is formed with two fused multiply-adds (b as high and low f16 part), so a
+// weight is rounded twice in f16, about 2e-4 relative L2 on the product.  Lattice weights are integers ss * code <= 225,
+// exact in f16; the scales of a joint-codebook record are f16 numbers, and where some product with a code has more than 11
+// bits the weight is fed as two f16 terms whose sum is exact.  Activations: one power-of-two scale per token
+// (largest magnitude next to 2^15), exact for bf16 values within 2^-28 of the row's largest.
+//
+// Work split.  Plain products: the (tile, chunk) units are cut into equal contiguous ranges, one per CTA; a tile that
+// straddles CTAs is summed with float32 reductions in L2, and the last CTA to arrive finishes it (no CTA ever waits for
+// another; a first form in which it added up the others' partial tiles spent 25,000 cycles on the loads).  Expert products (route plan): item = (row tile, token tile of one expert), strided over the CTAs.
+//
+// Every mbarrier wait is bounded: on expiry the CTA raises the device's status word, waits (bounded) for its own copies and
+// leaves through the common exit, which frees the tensor memory.
+#pragma once
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <type_traits>
+
+#include "common.h"
+#include "lane_unit.h"
+#include "nint_blayout.h"
+#include "tc05.cuh"
+
+namespace mfqb {
+
+constexpr int kTileRows = 128, kTileDecoders = 16, kTileEpilogue = 4;
+constexpr int kTileWarpMma = kTileDecoders + kTileEpilogue, kTileWarpRec = kTileWarpMma + 1, kTileWarpX = kTileWarpMma + 2;
+constexpr int kTileThreads = (kTileDecoders + kTileEpilogue + 3) * 32;
+constexpr size_t kTileDynSmem = 221 * 1024;   // beside 5 KB of barriers and tables
+constexpr int kTileMaxPools = 8, kTileRecStages = 8, kTileXStages = 8, kTileAStages = 8;
+constexpr float kTileWeightScale = 0.25f;   // of the f16 weights: 8-bit codes x 8-bit sub-scales x offset head-room stay below 65504
+
+struct TileArgs {
+    NintDevB pools[kTileMaxPools];   // the weight (entry 0), or the cohorts of an expert record
+    // lattice records: f16 state scales normalised by a power of two, and its inverse
+    uint16_t lut16[16];
+    float lut_undo;
+    const unsigned char* x;          // activation tiles (x_tiles_kernel)
+    size_t x_row_bytes;              // bytes of one row in the tiles' buffer (2 x the padded K, the largest among the cohorts)
+    int x_rows;                      // most rows of a tile; a tile of c rows is stored with (c + 7) / 8 * 8 rows per 64-column slab
+    const float* x_down;             // inverse scale per token, or per position of the route plan
+    void* y;
+    int y_dtype, ldy;
+    int m, ntok;                     // plain product: tokens, token tiles
+    int units;                       // plain product: (tile, chunk) units
+    float* partial;                  // [grid][N][128] float32 sums of tiles that several CTAs share, by the tile's first CTA; zero between calls
+    unsigned* counters;              // [grid], zero between calls
+    // expert product over a route plan with tiles of x_rows pairs; tile_bounds == nullptr: plain product
+    const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool, *expert_local;
+    int n_experts, rb_per_expert, rows_per_expert, only_pool /* -1: every cohort */, scatter /* rows go to pair_order[p], else to p */;
+    // shared- and tensor-memory plan
+    int n_mma;                       // N of the instruction
+    int rec_stages, rec_stage_bytes, x_stages, x_stage_bytes, x_whole /* 0: an activation stage is one 64-column slab; 1: the slabs of a step */, step /* chunks per step */, a_stages, a_cols, d_bufs, d_cols;
+    int* error;
+};
+
+// One stretch of work: chunks [ch0, ch1) of a tile.
+struct TileSeg {
+    int pool, rb0, nrb, row0, row_limit, ch0, ch1, nchunks;
+    int tok0, ncols;
+    size_t x_off;
+    int tile, part, parts, slot0;   // slot0: CTA index of the tile's first part
+};
+
+// Unit range of CTA b, and the CTA that owns a unit.
+__device__ __forceinline__ int tile_unit_begin(int b, int units, int grid) { return (int)((long long)b * units / grid); }
+__device__ __forceinline__ int tile_unit_owner(int u, int units, int grid) { return (int)((((long long)u + 1) * grid - 1) / units); }
+
+// First row of an expert's tile in the tiles' buffer: every tile starts on a multiple of eight rows, and experts do not overlap.
+__host__ __device__ __forceinline__ int tile_x_row(int expert_begin, int expert, int row_in_expert) { return (expert_begin + 7) / 8 * 8 + 8 * expert + row_in_expert; }
+
+// Next stretch of this CTA; `cursor` starts at the CTA's first unit (plain) or item (experts).
+__device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSeg& s) {
+    if (a.tile_bounds == nullptr) {
+        const int end = tile_unit_begin(blockIdx.x + 1, a.units, gridDim.x);
+        if (cursor >= end) return false;
+        const NintDevB& w = a.pools[0];
+        const int tile = cursor / w.nchunks, rt = tile / a.ntok, tt = tile - rt * a.ntok;
+        s.pool = 0;
+        s.tile = tile;
+        s.ch0 = cursor - tile * w.nchunks;
+        s.ch1 = min(w.nchunks, s.ch0 + end - cursor);
+        s.nchunks = w.nchunks;
+        s.rb0 = rt * 8;
+        s.nrb = min(8, w.nrb - s.rb0);
+        s.row0 = rt * kTileRows;
+        s.row_limit = w.n;
+        s.tok0 = tt * a.x_rows;
+        s.ncols = min(a.x_rows, a.m - s.tok0);
+        s.x_off = (size_t)s.tok0 * a.x_row_bytes;
+        s.slot0 = tile_unit_owner(tile * w.nchunks, a.units, gridDim.x);
+        s.parts = tile_unit_owner((tile + 1) * w.nchunks - 1, a.units, gridDim.x) - s.slot0 + 1;
+        s.part = blockIdx.x - s.slot0;
+        cursor += s.ch1 - s.ch0;
+        return true;
+    }
+    const int row_tiles = (a.rows_per_expert + kTileRows - 1) / kTileRows, items = a.tile_bounds[a.n_experts] * row_tiles;
+    for (; cursor < items; cursor += gridDim.x) {
+        const int t = cursor / row_tiles, rt = cursor - t * row_tiles;
+        int lo = 0, hi = a.n_experts - 1;   // expert e with tile_bounds[e] <= t < tile_bounds[e + 1]
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (a.tile_bounds[mid] <= t) lo = mid;
+            else hi = mid - 1;
+        }
+        const int pool = a.expert_pool[lo];
+        if (pool < 0 || (a.only_pool >= 0 && pool != a.only_pool)) continue;
+        s.pool = a.only_pool >= 0 ? 0 : pool;
+        s.nchunks = a.pools[s.pool].nchunks;
+        s.ch0 = 0;
+        s.ch1 = s.nchunks;
+        s.rb0 = a.expert_local[lo] * a.rb_per_expert + rt * 8;
+        s.nrb = min(8, a.rb_per_expert - rt * 8);
+        s.row0 = rt * kTileRows;
+        s.row_limit = a.rows_per_expert;
+        s.tok0 = a.expert_bounds[lo] + (t - a.tile_bounds[lo]) * a.x_rows;
+        s.ncols = min(a.x_rows, a.expert_bounds[lo + 1] - s.tok0);
+        s.x_off = (size_t)tile_x_row(a.expert_bounds[lo], lo, (t - a.tile_bounds[lo]) * a.x_rows) * a.x_row_bytes;
+        s.tile = t;
+        s.part = s.slot0 = 0;
+        s.parts = 1;
+        cursor += gridDim.x;
+        return true;
+    }
+    return false;
+}
+__device__ __forceinline__ int tile_first(const TileArgs& a) { return a.tile_bounds == nullptr ? tile_unit_begin(blockIdx.x, a.units, gridDim.x) : (int)blockIdx.x; }
+
+// F of a row and its (a, b): see the head of the file.
+__device__ __forceinline__ float tile_row_factor(uint32_t anchor, int bits, float& a, float& b) {
+    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&anchor));   // (ns, nm)
+    float f = fmaxf(fabsf(v.x), fabsf(v.y) * __uint_as_float((uint32_t)(126 - bits) << 23));
+    if (f == 0.f) f = 1.f;
+    a = v.x / f;
+    b = v.y / f;
+    return f;
+}
+
+__device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
+__device__ __forceinline__ uint32_t bits_h2(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
+
+// ---- codecs: decode one warp's half of a chunk record into the A ring ---------------------------------------------------
+// Row(a, rb, lane): what depends on the row-block only.  half<F>(rec, lane, row, ctx, taddr): family F of the record at `rec`
+// (shared memory) to the 16 tensor-memory lanes at taddr, columns 16 t + 8 h + {0..7} for octet t and group pair h.
+// The two values of a column are slots i, i + 2 of a quad (the bytes a 16-bit lane mask picks), columns c / 4 + c slots 0, 2 /
+// 1, 3 of quad c: x_tiles_kernel writes the activations in this order.
+template <int BITS, int T_>
+struct TileNint {
+    static constexpr int T = T_, TERMS = 1;
+    using BU = ByteUnit<BITS>;
+    static constexpr int WC = BU::words_for(8 * T);
+    static constexpr int MID = 1 << (BITS - 1);
+    // Bit position inside a byte at which register a (= r % 4) is read: where the packing leaves it, so that it is not shifted.
+    __host__ __device__ static constexpr int pos(int a) { return BITS == 2 ? 2 * a : ((BITS == 3 || BITS == 4) ? BITS * (a & 1) : 0); }
+    __host__ __device__ static size_t ctx_bytes(const NintDevB&) { return 0; }
+    __device__ static void ctx_init(unsigned char*, const TileArgs&, int, int) {}
+
+    struct Row {
+        __half2 step[2];      // a * scale * 2^-pos for rows q, q + 8, per group pair h
+        __half2 mid[2];       // a * scale * mid
+        __half2 nb_hi, nb_lo; // -b * scale, high and low part
+        __device__ __forceinline__ Row(const TileArgs&, const NintDevB& w, int rb, int lane) {
+            float a0, b0, a1, b1;
+            tile_row_factor(__ldg(w.anchors + rb * 16 + (lane >> 2)), BITS, a0, b0);
+            tile_row_factor(__ldg(w.anchors + rb * 16 + 8 + (lane >> 2)), BITS, a1, b1);
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                step[h] = __floats2half2_rn(a0 * (kTileWeightScale / (float)(1 << pos(2 * h))), a1 * (kTileWeightScale / (float)(1 << pos(2 * h + 1))));
+            mid[0] = mid[1] = __floats2half2_rn(a0 * (kTileWeightScale * MID), a1 * (kTileWeightScale * MID));
+            b0 *= -kTileWeightScale;
+            b1 *= -kTileWeightScale;
+            nb_hi = __floats2half2_rn(b0, b1);
+            nb_lo = __floats2half2_rn(b0 - __low2float(nb_hi), b1 - __high2float(nb_hi));
+        }
+    };
+    // register r as two f16 pairs 1024 + q 2^pos: bytes 0, 2 and bytes 1, 3
+    template <int R>
+    __device__ static __forceinline__ void pairs(const uint32_t* rec, int lane, __half2& even, __half2& odd) {
+        constexpr int P = pos(R % 4), TT = R % BU::NP, UNIT = R / BU::NP;
+        constexpr uint32_t M = ((1u << BITS) - 1u) << P, MASK = M | (M << 16);
+        uint32_t v;
+        if constexpr (TT < BU::U * BU::F) {   // a whole field of one word, at its place
+            static_assert((TT % BU::F) * BITS == P, "field position");
+            v = rec[(UNIT * BU::U + TT / BU::F) * 32 + lane];
+        } else {
+            uint32_t u[BU::U];
+#pragma unroll
+            for (int i = 0; i < BU::U; ++i) u[i] = rec[(UNIT * BU::U + i) * 32 + lane];
+            v = BU::at(u, TT) << P;
+        }
+        even = h2_bits((v & MASK) | 0x64006400u);
+        odd = h2_bits(((v >> 8) & MASK) | 0x64006400u);
+    }
+    template <int R>
+    __device__ static __forceinline__ void weights(const uint32_t* rec, int lane, __half2 d, __half2 n, uint32_t& lo, uint32_t& hi) {
+        __half2 even, odd;
+        pairs<R>(rec, lane, even, odd);
+        const __half2 bias = __float2half2_rn(1024.f + (float)(MID << pos(R % 4)));
+        lo = bits_h2(__hfma2(__hsub2(even, bias), d, n));
+        hi = bits_h2(__hfma2(__hsub2(odd, bias), d, n));
+    }
+    template <int F, int TI>
+    __device__ static __forceinline__ void octets(const uint32_t* rec, int lane, const __half2 (&d)[4], const __half2 (&n)[4], uint32_t taddr) {
+        if constexpr (TI < T) {
+            constexpr int R = (F * T + TI) * 4;
+            uint32_t r[8];
+            weights<R>(rec, lane, d[0], n[0], r[0], r[2]);
+            weights<R + 1>(rec, lane, d[1], n[1], r[1], r[3]);
+            weights<R + 2>(rec, lane, d[2], n[2], r[4], r[6]);
+            weights<R + 3>(rec, lane, d[3], n[3], r[5], r[7]);
+            tmem_st_16x128b_x4(taddr + 16 * TI, r);
+            octets<F, TI + 1>(rec, lane, d, n, taddr);
+        }
+    }
+    template <int F>
+    __device__ static __forceinline__ void half(const uint32_t* rec, int lane, const Row& row, const unsigned char*, uint32_t taddr) {
+        const uint32_t sel = (lane & 2) ? 0x4341u : 0x4240u;   // this lane's group of a pair: bytes (row q, row q + 8)
+        const __half2 k1024 = __float2half2_rn(1024.f);
+        __half2 d[4], n[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t* sc = rec + WC * 32 + (lane & ~3) + 2 * F + h;
+            const __half2 ss = __hsub2(h2_bits(__byte_perm(sc[0], 0x64646464u, sel)), k1024);
+            const __half2 sm = __hsub2(h2_bits(__byte_perm(sc[32], 0x64646464u, sel)), k1024);
+            const __half2 d2 = __hmul2(ss, row.step[h]);
+            const __half2 n2 = __hfma2(sm, row.nb_lo, __hfma2(sm, row.nb_hi, __hmul2(ss, row.mid[h])));
+            d[2 * h] = __low2half2(d2);
+            d[2 * h + 1] = __high2half2(d2);
+            n[2 * h] = __low2half2(n2);
+            n[2 * h + 1] = __high2half2(n2);
+        }
+        octets<F, 0>(rec, lane, d, n, taddr);
+    }
+    // what the epilogue multiplies a row's sums by
+    __device__ static __forceinline__ float row_undo(const TileArgs&, uint32_t anchor) {
+        float a, b;
+        return tile_row_factor(anchor, BITS, a, b) * (1.f / kTileWeightScale);
+    }
+};
+
+// ---- the kernel ----------------------------------------------------------------------------------------------------------
+struct TileShared {
+    __align__(8) uint64_t rec_full[kTileRecStages], rec_empty[kTileRecStages], x_full[kTileXStages], x_empty[kTileXStages];
+    uint64_t a_full[kTileAStages], a_empty[kTileAStages], d_full[2], d_empty[2], drain;
+    uint32_t tmem;
+    int failed;
+    unsigned last;
+    int finish;   // 1 + column table of the shared tile that this CTA finishes at its end, 0: none
+    TileSeg fin;
+    __align__(16) float row_factor[kTileRows];
+    __align__(16) int2 col[2][256];   // the epilogue's tile (two in turn): factor (float bits) and output row of every column
+};
+
+struct TileRing {
+    int stage = 0;
+    uint32_t phase = 0;
+    __device__ __forceinline__ void step(int n) {
+        if (++stage == n) { stage = 0; phase ^= 1u; }
+    }
+};
+template <int N, int I = 0, class Fn>
+__device__ __forceinline__ void tile_static_for(Fn&& f) {
+    if constexpr (I < N) {
+        f(std::integral_constant<int, I>{});
+        tile_static_for<N, I + 1>(f);
+    }
+}
+__device__ __forceinline__ bool tile_wait(uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity)); }
+
+// Both barriers with one round trip where both phases are already complete.
+__device__ __forceinline__ bool tile_wait2(uint64_t* bar0, uint32_t parity0, uint64_t* bar1, uint32_t parity1) {
+    const bool r0 = mbar_test(bar0, parity0), r1 = mbar_test(bar1, parity1);
+    if (__all_sync(0xffffffffu, r0 && r1)) return true;
+    return tile_wait(bar0, parity0) && tile_wait(bar1, parity1);
+}
+
+// Global stores that the compiler does not order against shared-memory loads: with plain stores every look-up of a column's
+// table entry waited for the store before it, 70 cycles a column.
+__device__ __forceinline__ void st_global(float* p, float v) { asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v)); }
+__device__ __forceinline__ void st_global(__nv_bfloat16* p, __nv_bfloat16 v) { asm volatile("st.global.b16 [%0], %1;" ::"l"(p), "h"(__bfloat16_as_ushort(v))); }
+
+// True for the four epilogue warps when it is true for all of them: they leave together, none waits at a barrier for one that gave up.
+__device__ __forceinline__ bool tile_epilogue_all(bool ok) {
+    uint32_t all;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(all) : "r"((uint32_t)ok) : "memory");
+    return all != 0u;
+}
+
+// The decoder warps' share of one stretch.
+template <class C, int F>
+__device__ __forceinline__ bool tile_decode(const TileArgs& a, TileShared& sh, const TileSeg& s, unsigned char* rec_ring, const unsigned char* ctx, TileRing& rr,
+                                            TileRing& ar, int rbl, int lane, uint32_t taddr) {
+    const NintDevB& w = a.pools[s.pool];
+    const bool mine = rbl < s.nrb;   // a tile at the end of the matrix has fewer row-blocks: their rows of D are never read
+    const typename C::Row row(a, w, s.rb0 + (mine ? rbl : 0), lane);
+    for (int ch = s.ch0; ch < s.ch1; ch += a.step) {
+        if (!tile_wait2(&sh.rec_full[rr.stage], rr.phase, &sh.a_empty[ar.stage], ar.phase ^ 1u)) return false;
+        if (mine) {
+            tc_fence_after_sync();
+            const uint32_t* rec = reinterpret_cast<const uint32_t*>(rec_ring + (size_t)rr.stage * a.rec_stage_bytes) + rbl * a.step * w.rec_words;
+            const uint32_t at = taddr + ar.stage * a.a_cols;
+            C::template half<F>(rec, lane, row, ctx, at);
+            if (a.step > 1 && ch + 1 < s.ch1) C::template half<F>(rec + w.rec_words, lane, row, ctx, at + 16 * C::T * C::TERMS);
+            __syncwarp();
+        }
+        if (lane == 0) mbar_arrive(&sh.rec_empty[rr.stage]);
+        if (mine) {
+            tmem_wait_st();
+            tc_fence_before_sync();
+            __syncwarp();
+        }
+        if (lane == 0) mbar_arrive(&sh.a_full[ar.stage]);
+        rr.step(a.rec_stages);
+        ar.step(a.a_stages);   // the other half's stage, then this half's next one
+        ar.step(a.a_stages);
+    }
+    return true;
+}
+
+// The issuer's share of one chunk of T octets: 4T slabs of 16 columns of K, 2T per decoder half.  An elected lane issues runs of
+// instructions between the waits; the runs are unrolled and their operands made warp-uniform with a shuffle, so that descriptors
+// stay in uniform registers (an issue inside a rolled loop, operands in lane registers, took 200 cycles, more than its 128
+// tensor cycles for N = 256).  tile_issue: activation stages of 64 columns.  tile_issue_step: small N, an activation stage holds
+// the n <= 2 chunks of a step and each half is one run; with a wait costing 200 cycles, what counts there is their number.
+template <int TERMS, int T>
+__device__ __forceinline__ bool tile_issue_step(const TileArgs& a, TileShared& sh, TileRing& ar, TileRing& xr, unsigned char* x_ring, uint32_t x_pitch, uint32_t tmem_a,
+                                                uint32_t td, uint32_t idesc, bool acc, int n) {
+    if (!tile_wait(&sh.x_full[xr.stage], xr.phase)) return false;
+    const uint32_t xb = __shfl_sync(0xffffffffu, smem_u32(x_ring) + (uint32_t)(xr.stage * a.x_stage_bytes), 0);
+#pragma unroll
+    for (int f = 0; f < 2; ++f) {
+        if (!tile_wait(&sh.a_full[ar.stage], ar.phase)) return false;
+        tc_fence_after_sync();
+        const uint32_t at = __shfl_sync(0xffffffffu, tmem_a + (uint32_t)(ar.stage * a.a_cols), 0);
+        if (elect_one()) {
+#pragma unroll
+            for (int g = 0; g < 2; ++g)
+                if (g < n) {
+#pragma unroll
+                    for (int i = 0; i < 2 * T; ++i) {
+                        const int sl = (g * 2 + f) * 2 * T + i;
+                        const uint64_t bdesc = smem_desc_sw128(xb + (uint32_t)(sl >> 2) * x_pitch) + (uint64_t)(2 * (sl & 3));
+#pragma unroll
+                        for (int term = 0; term < TERMS; ++term)
+                            tc_mma_f16_ts(td, at + (uint32_t)(16 * T * (g * TERMS + term) + 8 * i), bdesc, idesc, sl > 0 || term > 0 || acc);
+                    }
+                }
+            if (f == 1) tc_commit(&sh.x_empty[xr.stage]);
+            tc_commit(&sh.a_empty[ar.stage]);
+        }
+        __syncwarp();
+        ar.step(a.a_stages);
+    }
+    xr.step(a.x_stages);
+    return true;
+}
+
+template <int TERMS, int T>
+__device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, TileRing& ar, TileRing& xr, unsigned char* x_ring, uint32_t tmem_a, uint32_t td, uint32_t idesc,
+                                           bool acc) {
+    auto run = [&](auto first_c, auto len_c, bool x_done) {   // slabs [first, first + len) of the chunk, all in half first / 2T
+        constexpr int FIRST = decltype(first_c)::value, LEN = decltype(len_c)::value, H0 = FIRST % (2 * T);
+        const uint32_t at = __shfl_sync(0xffffffffu, tmem_a + (uint32_t)(ar.stage * a.a_cols), 0);
+        const uint32_t xb = __shfl_sync(0xffffffffu, smem_u32(x_ring) + (uint32_t)(xr.stage * a.x_stage_bytes), 0);
+        if (elect_one()) {
+#pragma unroll
+            for (int i = 0; i < LEN; ++i) {
+                const int sl = FIRST + i;
+                const uint64_t bdesc = smem_desc_sw128(xb) + (uint64_t)(2 * (sl & 3));
+#pragma unroll
+                for (int term = 0; term < TERMS; ++term)
+                    tc_mma_f16_ts(td, at + (uint32_t)(16 * T * term + 8 * (H0 + i)), bdesc, idesc, sl > 0 || term > 0 || acc);
+            }
+            if (x_done) tc_commit(&sh.x_empty[xr.stage]);
+            if (H0 + LEN == 2 * T) tc_commit(&sh.a_empty[ar.stage]);
+        }
+        __syncwarp();
+        if (x_done) xr.step(a.x_stages);
+        if (H0 + LEN == 2 * T) ar.step(a.a_stages);
+    };
+    auto wait_a = [&]() {
+        const bool ok = tile_wait(&sh.a_full[ar.stage], ar.phase);
+        tc_fence_after_sync();
+        return ok;
+    };
+    auto wait_x = [&]() { return tile_wait(&sh.x_full[xr.stage], xr.phase); };
+    using std::integral_constant;
+    constexpr int ODD = T & 1;   // an odd number of octets: the middle 64-column slab belongs to both halves
+    bool ok = wait_a();
+    auto atoms = [&](auto first_c, auto count_c) {
+        constexpr int A0 = decltype(first_c)::value, N = decltype(count_c)::value;
+        tile_static_for<N>([&](auto i_c) {
+            if (ok && (ok = wait_x())) run(integral_constant<int, 4 * A0 + 4 * decltype(i_c)::value>{}, integral_constant<int, 4>{}, true);
+        });
+    };
+    atoms(integral_constant<int, 0>{}, integral_constant<int, T / 2>{});
+    if constexpr (ODD) {
+        if (ok && (ok = wait_x())) run(integral_constant<int, 2 * T - 2>{}, integral_constant<int, 2>{}, false);
+        if (ok && (ok = wait_a())) run(integral_constant<int, 2 * T>{}, integral_constant<int, 2>{}, true);
+    } else {
+        ok = ok && wait_a();
+    }
+    // remaining whole slabs of the second half
+    tile_static_for<T / 2>([&](auto i_c) {
+        if (ok && (ok = wait_x())) run(integral_constant<int, 4 * (T / 2 + ODD) + 4 * decltype(i_c)::value>{}, integral_constant<int, 4>{}, true);
+    });
+    return ok;
+}
+
+// Sets::dispatch(w, f) calls f(Codec{}) for the codec of a cohort; Sets::ctx describes the codec context (lattice tables).
+template <class Sets>
+__global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_constant__ TileArgs a) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ TileShared sh;
+    unsigned char* x_ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+    const uint32_t x_stage_bytes = (uint32_t)a.x_stage_bytes;
+    unsigned char* rec_ring = x_ring + (size_t)a.x_stages * x_stage_bytes;
+    unsigned char* ctx = rec_ring + (size_t)a.rec_stages * a.rec_stage_bytes;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+
+    if (tid == 0) {
+        for (int i = 0; i < kTileRecStages; ++i) { mbar_init(&sh.rec_full[i], 1); mbar_init(&sh.rec_empty[i], kTileDecoders); }
+        for (int i = 0; i < kTileXStages; ++i) { mbar_init(&sh.x_full[i], 1); mbar_init(&sh.x_empty[i], 1); }
+        for (int i = 0; i < kTileAStages; ++i) { mbar_init(&sh.a_full[i], kTileDecoders / 2); mbar_init(&sh.a_empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { mbar_init(&sh.d_full[i], 1); mbar_init(&sh.d_empty[i], kTileEpilogue); }
+        mbar_init(&sh.drain, 1);
+        sh.finish = 0;
+        sh.failed = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == kTileWarpMma) tmem_alloc(&sh.tmem, 512u);
+    Sets::ctx_init(ctx, a, tid, kTileThreads);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tmem_d = sh.tmem, tmem_a = tmem_d + (uint32_t)(a.d_bufs * a.d_cols);
+
+    // Only the record loader of a plain product runs ahead of the previous kernel (weights are constants); everything else
+    // reads what that kernel wrote, or is bounded by it.
+    if (warp != kTileWarpRec || a.tile_bounds != nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    int cursor = tile_first(a);
+    TileSeg s;
+    if (warp < kTileDecoders) {
+        // -------- decoders: row-block 2 (warp & 3) + ((warp >> 2) & 1) of the tile, half (warp >> 3) of the chunk --------
+        const int rbl = 2 * (warp & 3) + ((warp >> 2) & 1), f = warp >> 3;
+        const uint32_t taddr = tmem_a + ((uint32_t)(rbl * 16) << 16);
+        TileRing rr, ar;
+        if (f) ar.step(a.a_stages);
+        bool ok = true;
+        while (ok && tile_next(a, cursor, s))
+            Sets::dispatch(a.pools[s.pool], [&](auto codec) {
+                using C = decltype(codec);
+                ok = f ? tile_decode<C, 1>(a, sh, s, rec_ring, ctx, rr, ar, rbl, lane, taddr) : tile_decode<C, 0>(a, sh, s, rec_ring, ctx, rr, ar, rbl, lane, taddr);
+            });
+        if (!ok) sh.failed = 1;
+    } else if (warp < kTileWarpMma) {
+        // -------- epilogue: lane = row of the warp's quarter of the tile --------
+        const int quarter = warp & 3, row_l = quarter * 32 + lane;
+        TileRing dr;
+        bool ok = true;
+        for (int buf = 0; ok && tile_next(a, cursor, s); buf ^= 1) {
+            const NintDevB& w = a.pools[s.pool];
+            const int row = s.row0 + row_l;
+            const bool row_ok = row < s.row_limit;
+            float undo = 0.f;
+            if (row_ok) {
+                const uint32_t anchor = __ldg(w.anchors + (size_t)s.rb0 * 16 + row_l);
+                Sets::dispatch(w, [&](auto codec) { undo = decltype(codec)::row_undo(a, anchor); });
+            }
+            for (int i = tid - kTileDecoders * 32; i < s.ncols; i += kTileEpilogue * 32)
+                sh.col[buf][i] = make_int2(__float_as_int(__ldcg(a.x_down + s.tok0 + i)), a.scatter ? __ldcg(a.pair_order + s.tok0 + i) : s.tok0 + i);
+            ok = tile_epilogue_all(tile_wait(&sh.d_full[dr.stage], dr.phase));
+            if (!ok) break;
+            tc_fence_after_sync();
+            const uint32_t td = tmem_d + (uint32_t)(dr.stage * a.d_cols) + ((uint32_t)(quarter * 32) << 16);
+            // finished sums of columns cb .. cb + 7, this lane's row
+            auto put8 = [&](int cb, const float (&v)[8]) {
+                int2 col[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) col[i] = sh.col[buf][cb + i];
+                const int n = row_ok ? s.ncols - cb : 0;
+                if (a.y_dtype == 0 /* MFQB_F32 */) {
+                    float* y = reinterpret_cast<float*>(a.y) + row;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < n) st_global(y + (size_t)col[i].y * a.ldy, v[i] * (undo * __int_as_float(col[i].x)));
+                } else {
+                    __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y) + row;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < n) st_global(y + (size_t)col[i].y * a.ldy, __float2bfloat16_rn(v[i] * (undo * __int_as_float(col[i].x))));
+                }
+            };
+            if (s.parts == 1) {
+                for (int cb = 0; cb < s.ncols; cb += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(td + (uint32_t)cb, r);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        float v[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[8 * h + i]);
+                        put8(cb + 8 * h, v);
+                    }
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.d_empty[dr.stage]);
+            } else {
+                // this CTA's part of a tile that others share: added into the tile's float32 copy in L2; the last to arrive
+                // takes the sums and leaves zeros
+                float* sums = a.partial + (size_t)s.slot0 * a.n_mma * kTileRows + row_l;
+                for (int cb = 0; cb < s.ncols; cb += 16) {
+                    uint32_t r[16];
+                    tmem_ld16(td + (uint32_t)cb, r);
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(sums + (size_t)(cb + i) * kTileRows), "f"(__uint_as_float(r[i])) : "memory");
+                }
+                tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&sh.d_empty[dr.stage]);
+                __threadfence();
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (warp == kTileDecoders && lane == 0) sh.last = atomicAdd(a.counters + s.slot0, 1u);
+                asm volatile("bar.sync 1, 128;" ::: "memory");
+                if (sh.last == (unsigned)(s.parts - 1)) {
+                    __threadfence();
+                    if (cursor >= tile_unit_begin(blockIdx.x + 1, a.units, gridDim.x)) {   // nothing left for this CTA: every warp helps, below
+                        if (lane == 0 && quarter == 0) { sh.finish = buf + 1; sh.fin = s; }
+                        break;
+                    }
+                    for (int cb = 0; cb < s.ncols; cb += 16) {
+                        float v[2][8];
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) v[i >> 3][i & 7] = __ldcg(sums + (size_t)(cb + i) * kTileRows);
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) __stcg(sums + (size_t)(cb + i) * kTileRows, 0.f);
+                        put8(cb, v[0]);
+                        put8(cb + 8, v[1]);
+                    }
+                    if (warp == kTileDecoders && lane == 0) a.counters[s.slot0] = 0u;
+                }
+            }
+            dr.step(a.d_bufs);
+        }
+        if (!ok) sh.failed = 1;
+    } else if (warp == kTileWarpMma) {
+        // -------- mma issuer: the warp stays together, an elected lane issues --------
+        const uint32_t idesc = instr_desc_f16(kTileRows, a.n_mma);
+        TileRing ar, xr, dr;
+        bool ok = true;
+        while (ok && tile_next(a, cursor, s)) {
+            const int t8 = a.pools[s.pool].t8;
+            if (!tile_wait(&sh.d_empty[dr.stage], dr.phase ^ 1u)) { ok = false; break; }
+            tc_fence_after_sync();
+            const uint32_t td = __shfl_sync(0xffffffffu, tmem_d + (uint32_t)(dr.stage * a.d_cols), 0);
+            const uint32_t x_pitch = (uint32_t)((s.ncols + 7) & ~7) * 128u;
+            bool acc = false;
+            for (int ch = s.ch0; ch < s.ch1 && ok; ch += a.step, acc = true) {
+                const int n = min(a.step, s.ch1 - ch);
+                auto issue = [&](auto t_c) {
+                    constexpr int T = decltype(t_c)::value;
+                    ok = a.x_whole ? tile_issue_step<Sets::TERMS, T>(a, sh, ar, xr, x_ring, x_pitch, tmem_a, td, idesc, acc, n)
+                                   : tile_issue<Sets::TERMS, T>(a, sh, ar, xr, x_ring, tmem_a, td, idesc, acc);
+                };
+                switch (t8) {
+                    case 2: issue(std::integral_constant<int, 2>{}); break;
+                    case 3: issue(std::integral_constant<int, 3>{}); break;
+                    case 4: issue(std::integral_constant<int, 4>{}); break;
+                    case 5: issue(std::integral_constant<int, 5>{}); break;
+                    case 6: issue(std::integral_constant<int, 6>{}); break;
+                    default: issue(std::integral_constant<int, 8>{}); break;
+                }
+            }
+            if (ok && elect_one()) tc_commit(&sh.d_full[dr.stage]);
+            __syncwarp();
+            dr.step(a.d_bufs);
+        }
+        if (!ok) {
+            sh.failed = 1;
+            if (elect_one()) tc_commit(&sh.drain);   // what was issued still reads the rings and the tensor memory
+            tile_wait(&sh.drain, 0);
+        }
+    } else if (warp == kTileWarpRec) {
+        // -------- record loader --------
+        TileRing rr;
+        bool ok = true;
+        int issued = 0;
+        while (ok && tile_next(a, cursor, s)) {
+            const NintDevB& w = a.pools[s.pool];
+            const uint32_t pitch = (uint32_t)(a.step * w.rec_words) * 4u;
+            const size_t rb_words = (size_t)w.nchunks * w.rec_words;
+            const uint32_t* src = w.items + (size_t)s.rb0 * rb_words + (size_t)s.ch0 * w.rec_words;
+            for (int ch = s.ch0; ch < s.ch1; ch += a.step, src += (size_t)a.step * w.rec_words) {
+                const uint32_t bytes = (uint32_t)(min(a.step, s.ch1 - ch) * w.rec_words) * 4u;   // a row-block's records of a step are neighbours
+                if (!tile_wait(&sh.rec_empty[rr.stage], rr.phase ^ 1u)) { ok = false; break; }
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sh.rec_full[rr.stage], bytes * (uint32_t)s.nrb);
+                    unsigned char* dst = rec_ring + (size_t)rr.stage * a.rec_stage_bytes;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < s.nrb) bulk_load(dst + i * pitch, src + (size_t)i * rb_words, bytes, &sh.rec_full[rr.stage]);
+                }
+                __syncwarp();
+                rr.step(a.rec_stages);
+                ++issued;
+            }
+        }
+        if (!ok) {
+            sh.failed = 1;
+            for (int i = 0; i < min(issued, a.rec_stages); ++i) tile_wait(&sh.rec_full[(rr.stage + a.rec_stages - 1 - i) % a.rec_stages], rr.phase ^ (i >= rr.stage ? 1u : 0u));
+        }
+    } else {
+        // -------- activation loader --------
+        TileRing xr;
+        bool ok = true;
+        int issued = 0;
+        while (ok && tile_next(a, cursor, s)) {
+            const int t8 = a.pools[s.pool].t8, atoms = a.x_whole ? a.step * t8 : 1;
+            const uint32_t pitch = (uint32_t)((s.ncols + 7) & ~7) * 128u;
+            const unsigned char* src = a.x + s.x_off + (size_t)s.ch0 * t8 * pitch;
+            for (int at = s.ch0 * t8; at < s.ch1 * t8; at += atoms, src += (size_t)atoms * pitch) {
+                const uint32_t bytes = pitch * (uint32_t)min(atoms, s.ch1 * t8 - at);
+                if (!tile_wait(&sh.x_empty[xr.stage], xr.phase ^ 1u)) { ok = false; break; }
+                if (elect_one()) {
+                    mbar_arrive_expect_tx(&sh.x_full[xr.stage], bytes);
+                    bulk_load(x_ring + (size_t)xr.stage * x_stage_bytes, src, bytes, &sh.x_full[xr.stage]);
+                }
+                __syncwarp();
+                xr.step(a.x_stages);
+                ++issued;
+            }
+        }
+        if (!ok) {
+            sh.failed = 1;
+            for (int i = 0; i < min(issued, a.x_stages); ++i) tile_wait(&sh.x_full[(xr.stage + a.x_stages - 1 - i) % a.x_stages], xr.phase ^ (i >= xr.stage ? 1u : 0u));
+        }
+    }
+    __syncwarp();
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == kTileWarpMma) {
+        tc_fence_after_sync();
+        tmem_free(tmem_d, 512u);
+        if (lane == 0 && sh.failed) atomicExch(a.error, MFQB_ERR_TIMEOUT);
+    }
+    if (sh.finish && !sh.failed) {
+        // The sums of the tile this CTA was the last to add to (up to 128 KB in L2, stored column by column): fetched into the
+        // rings' memory with one bulk copy per 64 columns, then a warp writes a column, four rows a lane.  (The four epilogue
+        // warps alone, sixteen loads in flight each, took 40,000 cycles for N = 256, a third of the kernel.)
+        const TileSeg& t = sh.fin;
+        const float* sums = a.partial + (size_t)t.slot0 * a.n_mma * kTileRows;
+        float* stage = reinterpret_cast<float*>(x_ring);
+        const int ncols16 = (t.ncols + 15) & ~15;   // what was added, and what has to be zero again
+        if (tid == 0) {
+            asm volatile("fence.proxy.async;" ::: "memory");
+            mbar_arrive_expect_tx(&sh.drain, (uint32_t)ncols16 * kTileRows * 4u);
+            for (int c = 0; c < ncols16; c += 64) bulk_load(stage + c * kTileRows, sums + c * kTileRows, (uint32_t)min(64, ncols16 - c) * kTileRows * 4u, &sh.drain);
+            a.counters[t.slot0] = 0u;
+        }
+        for (int r = tid; r < kTileRows; r += kTileThreads)
+            if (t.row0 + r < t.row_limit) {
+                const NintDevB& w = a.pools[t.pool];
+                const uint32_t anchor = __ldg(w.anchors + (size_t)t.rb0 * 16 + r);
+                Sets::dispatch(w, [&](auto codec) { sh.row_factor[r] = decltype(codec)::row_undo(a, anchor); });
+            }
+        __syncthreads();
+        if (!tile_wait(&sh.drain, 0)) {
+            if (tid == 0) atomicExch(a.error, MFQB_ERR_TIMEOUT);
+            return;
+        }
+        const int row = t.row0 + 4 * lane, n = min(4, t.row_limit - row);
+        const float4 f = *reinterpret_cast<const float4*>(sh.row_factor + 4 * lane);
+        const bool vec = n == 4 && (a.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
+        for (int c = warp; c < ncols16; c += kTileThreads / 32) {
+            __stcg(reinterpret_cast<float4*>(const_cast<float*>(sums) + c * kTileRows + 4 * lane), make_float4(0.f, 0.f, 0.f, 0.f));
+            if (c >= t.ncols) continue;
+            const int2 col = sh.col[sh.finish - 1][c];
+            const float down = __int_as_float(col.x);
+            const float4 v = *reinterpret_cast<const float4*>(stage + c * kTileRows + 4 * lane);
+            const float o[4] = {v.x * (f.x * down), v.y * (f.y * down), v.z * (f.z * down), v.w * (f.w * down)};
+            const size_t at = (size_t)col.y * a.ldy + row;
+            if (a.y_dtype == 0 /* MFQB_F32 */) {
+                float* y = reinterpret_cast<float*>(a.y) + at;
+                if (vec) *reinterpret_cast<float4*>(y) = make_float4(o[0], o[1], o[2], o[3]);
+                else
+                    for (int i = 0; i < n; ++i) y[i] = o[i];
+            } else {
+                __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y) + at;
+                if (vec) {
+                    const __nv_bfloat162 p0 = __floats2bfloat162_rn(o[0], o[1]), p1 = __floats2bfloat162_rn(o[2], o[3]);
+                    *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
+                } else {
+                    for (int i = 0; i < n; ++i) y[i] = __float2bfloat16_rn(o[i]);
+                }
+            }
+        }
+    }
+}
+
+}  // namespace mfqb

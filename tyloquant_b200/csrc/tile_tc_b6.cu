@@ -1,0 +1,6 @@
+// NINT6 instantiations of the tensor-memory tile kernel.
+#include "tile_tc_launch.cuh"
+
+namespace mfqb {
+MFQB_TILE_INSTANTIATE(6)
+}  // namespace mfqb

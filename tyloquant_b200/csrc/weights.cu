@@ -14,6 +14,7 @@
 #include "nint_blayout.h"
 #include "nvq.h"
 #include "nvq_blayout.h"
+#include "tile_tc.h"
 
 namespace mfqb {
 
@@ -414,8 +415,7 @@ int mfqb_mul_mat(const mfqb_weight* w, const void* x, int m, void* y, int y_dtyp
         const int64_t n = w->info.n, k = w->info.k;
         const size_t ysz = y_dtype == MFQB_F32 ? 4 : 2;
         if (w->family == MFQB_FAMILY_NINT) {
-            // more than 16 rows: tensor-core tile kernel (x conversion buffer is library scratch)
-            if (m > 16 && launch_nint_gemm(w->nint, x, m, y, y_dtype, w->device, stream)) return;
+            if (m >= 5 && launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
             if (m == 1 && gemv1_use_streamed(w->nint) &&
                 launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->fix.p, w->status, stream))
                 return;
