@@ -1,0 +1,72 @@
+"""Edges of loading: pieces, slices, whole-byte storage, padded experts -- decoded bit for bit."""
+
+import struct
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from oracle import mfq_oracle as O  # noqa: E402
+from tyloquant_b200 import QuantWeight, encode, moe  # noqa: E402
+
+
+def _same(a, b):
+    return np.array_equal(np.asarray(a).view(np.uint32), np.asarray(b).view(np.uint32))
+
+
+@pytest.mark.parametrize("profile", [(2, 16, 5), (3, 24, 5), (4, 32, 6), (5, 28, 7), (6, 24, 7), (8, 48, 7), (8, 22, 7)])
+def test_scalar_tensors_of_one_and_many_pieces(profile):
+    bits, gs, sb = profile
+    for n, k in [(1, 1), (17, 333), (1500, 5000), (40, 1 << 19)]:   # the last: a row-block alone exceeds a staging piece
+        blob = encode.random_nint_blob(n, k, bits, gs, sb, seed=n + bits, device="cuda")
+        ref = O.dequant_nint(O.unpack_nint(blob))
+        w = QuantWeight.from_blob(f"NINT{bits}", blob)
+        assert _same(w.dequantize().cpu().numpy(), ref), (profile, n, k)
+        w.free()
+        if n > 16 and k < 1 << 19:
+            cut = min(n, 1201)
+            rows = QuantWeight.from_blob(f"NINT{bits}", blob, axis=0, begin=13, end=cut)
+            assert _same(rows.dequantize().cpu().numpy(), ref[13:cut])
+            lo, hi = 3 * gs, (k // gs - 2) * gs
+            cols = QuantWeight.from_blob(f"NINT{bits}", blob, axis=1, begin=lo, end=hi)
+            assert _same(cols.dequantize().cpu().numpy(), ref[:, lo:hi])
+
+
+def test_whole_byte_storage_of_older_writers():
+    t = encode.quantize_nint(np.random.default_rng(1).standard_normal((33, 250)).astype(np.float32), 4, 24, 6)
+    legacy = b"".join([struct.pack("<BBiii", 4, 6, 24, 0, 250), struct.pack("<I", 2), struct.pack("<2q", 33, 250), struct.pack("<II", 33, t["ng"]),
+                       t["neuron_scale"].astype("<f2").tobytes(), t["neuron_min"].astype("<f2").tobytes(), t["sub_scale"].numpy().tobytes(),
+                       t["sub_min"].numpy().tobytes(), t["q"].numpy().tobytes()])
+    a, b = QuantWeight.from_blob("NINT4", legacy), QuantWeight.from_blob("NINT4", encode.nint_blob(t))
+    assert _same(a.dequantize().cpu().numpy(), b.dequantize().cpu().numpy())
+
+
+@pytest.mark.parametrize("jsc", [False, True])
+def test_lattice_tensors(jsc):
+    banks = encode.synthetic_d4_banks(512, 2, seed=5) if jsc else O.d4_256_codebook()[None]
+    for n, k in [(1, 5), (50, 1003), (3000, 4800)]:
+        wt = np.random.default_rng(n).standard_normal((n, k), dtype=np.float32)
+        blob = encode.nvq_blob(encode.quantize_nvq3(wt, banks, jsc=jsc, device="cuda"))
+        ref = O.dequant_nvq(O.unpack_nvq(blob))
+        w = QuantWeight.from_blob("NVQ3J-512" if jsc else "NVQ3", blob)
+        assert _same(w.dequantize().cpu().numpy(), ref), (n, k)
+        if n > 2000:
+            part = QuantWeight.from_blob("NVQ3J-512" if jsc else "NVQ3", blob, axis=0, begin=1001, end=2900)
+            assert _same(part.dequantize().cpu().numpy(), ref[1001:2900])
+
+
+def test_experts_with_padded_rows_and_a_shard():
+    e, out, k = 12, 100, 300   # 100 rows: padded to 112 on the device
+    w = (np.random.default_rng(3).standard_normal((e, out, k)) * 0.02).astype(np.float32)
+    bits = [2, 3, 4, 6, 2, 3, 4, 6, 5, 5, 8, 8]
+    blob = encode.quantize_expertwise(w, bits, device="cuda")
+    whole, shard = moe.MoeWeight(blob), moe.MoeWeight(blob, 0, 3, 9)
+    for i in range(e):
+        b, gs, sb = encode.CANONICAL_NINT[bits[i]]
+        ref = O.dequant_nint(O.unpack_nint(encode.nint_blob(encode.quantize_nint(w[i], b, gs, sb, device="cuda"))))
+        assert _same(whole.dequantize_expert(i).cpu().numpy(), ref), i
+        if 3 <= i < 9:
+            assert _same(shard.dequantize_expert(i).cpu().numpy(), ref), i

@@ -131,9 +131,9 @@ def check(status: int) -> None:
 
 def buffer_address(data) -> tuple[int, int, object]:
     """(address, nbytes, keepalive) of a bytes-like object, without copying when possible."""
-    mv = memoryview(data)
-    if mv.readonly:
-        keep = (C.c_char * mv.nbytes).from_buffer_copy(mv)
-    else:
-        keep = (C.c_char * mv.nbytes).from_buffer(mv)
-    return C.addressof(keep), mv.nbytes, keep
+    import numpy as np
+    if memoryview(data).nbytes == 0:
+        keep = (C.c_char * 1)()
+        return C.addressof(keep), 0, keep
+    a = np.frombuffer(data, dtype=np.uint8)   # a view, also of read-only buffers
+    return a.ctypes.data, a.nbytes, a

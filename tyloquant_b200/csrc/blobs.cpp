@@ -51,9 +51,9 @@ bool dtype_is_nvq(const std::string& d) {
     return d == "NVQ3" || d == "NIQ3" || d == "NVQ3J" || d == "NVQ3J-512" || d == "NVQ3J-L";
 }
 
-HostNint parse_nint(const void* blob, uint64_t nbytes) {
+NintView parse_nint_view(const void* blob, uint64_t nbytes) {
     Cursor c(blob, nbytes);
-    HostNint t;
+    NintView t;
     t.bits = c.get<uint8_t>("NINT header");
     t.sub_bits = c.get<uint8_t>("NINT header");
     t.gs = c.get<int32_t>("NINT header");
@@ -76,82 +76,67 @@ HostNint parse_nint(const void* blob, uint64_t nbytes) {
     t.k = neuron_len;
     t.ng = ng;
     const uint64_t nsub = (uint64_t)out * ng, nq = nsub * (uint64_t)t.gs;
-    const uint8_t* ns = c.take(2ull * out, "NINT neuron_scale");
-    const uint8_t* nm = c.take(2ull * out, "NINT neuron_min");
-    t.ns.resize(out);
-    t.nm.resize(out);
-    memcpy(t.ns.data(), ns, 2ull * out);
-    memcpy(t.nm.data(), nm, 2ull * out);
+    t.ns = c.take(2ull * out, "NINT neuron_scale");
+    t.nm = c.take(2ull * out, "NINT neuron_min");
     const uint64_t packed_tail = 2 * packed_nbytes(nsub, t.sub_bits) + packed_nbytes(nq, t.bits);
     const uint64_t legacy_tail = 2 * nsub + nq;  // whole-uint8 storage of older writers
     const uint64_t remaining = nbytes - c.off;
-    // sizes come from the header: nothing is allocated for them before the tail length has confirmed them
     if (remaining != legacy_tail && remaining != packed_tail)
         fail(MFQB_ERR_FORMAT, "invalid NINT blob tail: remaining=%llu packed=%llu legacy=%llu",
              (unsigned long long)remaining, (unsigned long long)packed_tail, (unsigned long long)legacy_tail);
-    t.ss.resize(nsub);
-    t.sm.resize(nsub);
-    t.q.resize(nq);
-    if (remaining == legacy_tail) {
-        memcpy(t.ss.data(), c.take(nsub, "NINT sub_scale"), nsub);
-        memcpy(t.sm.data(), c.take(nsub, "NINT sub_min"), nsub);
-        memcpy(t.q.data(), c.take(nq, "NINT q"), nq);
-    } else if (remaining == packed_tail) {
-        unpack_bits(c.take(packed_nbytes(nsub, t.sub_bits), "NINT sub_scale"), nsub, t.sub_bits, t.ss.data());
-        unpack_bits(c.take(packed_nbytes(nsub, t.sub_bits), "NINT sub_min"), nsub, t.sub_bits, t.sm.data());
-        unpack_bits(c.take(packed_nbytes(nq, t.bits), "NINT q"), nq, t.bits, t.q.data());
-    } else {
-        fail(MFQB_ERR_FORMAT, "invalid NINT blob tail: remaining=%llu packed=%llu legacy=%llu",
-             (unsigned long long)remaining, (unsigned long long)packed_tail, (unsigned long long)legacy_tail);
-    }
+    const bool legacy = remaining == legacy_tail;
+    t.sub_width = legacy ? 8 : t.sub_bits;
+    t.q_width = legacy ? 8 : t.bits;
+    t.ss = c.take(packed_nbytes(nsub, t.sub_width), "NINT sub_scale");
+    t.sm = c.take(packed_nbytes(nsub, t.sub_width), "NINT sub_min");
+    t.q = c.take(packed_nbytes(nq, t.q_width), "NINT q");
     return t;
 }
 
-uint64_t nint_payload_bytes(const HostNint& t) {
-    const uint64_t nsub = (uint64_t)t.n * t.ng;
-    return 4ull * t.n + 2 * packed_nbytes(nsub, t.sub_bits) + packed_nbytes(nsub * t.gs, t.bits);
+HostNint parse_nint(const void* blob, uint64_t nbytes) {
+    const NintView v = parse_nint_view(blob, nbytes);
+    HostNint t;
+    t.bits = v.bits;
+    t.sub_bits = v.sub_bits;
+    t.gs = v.gs;
+    t.n = v.n;
+    t.k = v.k;
+    t.ng = v.ng;
+    const uint64_t nsub = (uint64_t)v.n * v.ng;
+    t.ns.resize(v.n);
+    t.nm.resize(v.n);
+    t.ss.resize(nsub);
+    t.sm.resize(nsub);
+    t.q.resize(nsub * v.gs);
+    memcpy(t.ns.data(), v.ns, 2ull * v.n);
+    memcpy(t.nm.data(), v.nm, 2ull * v.n);
+    unpack_bits(v.ss, nsub, v.sub_width, t.ss.data());
+    unpack_bits(v.sm, nsub, v.sub_width, t.sm.data());
+    unpack_bits(v.q, nsub * v.gs, v.q_width, t.q.data());
+    return t;
 }
 
-HostNint slice_nint(const HostNint& t, int axis, int64_t begin, int64_t end) {
+uint64_t nint_payload_bytes(const NintView& t, int64_t n, int64_t ng) {
+    const uint64_t nsub = (uint64_t)n * ng;
+    return 4ull * n + 2 * packed_nbytes(nsub, t.sub_bits) + packed_nbytes(nsub * t.gs, t.bits);
+}
+
+SliceRange slice_nint(const NintView& t, int axis, int64_t begin, int64_t end) {
     if (axis == 0) {
         if (end < 0) end = t.n;
         if (begin < 0 || begin >= end || end > t.n) fail(MFQB_ERR_ARG, "NINT row slice [%lld,%lld) out of range", (long long)begin, (long long)end);
-        HostNint r = t;
-        r.n = end - begin;
-        r.ns.assign(t.ns.begin() + begin, t.ns.begin() + end);
-        r.nm.assign(t.nm.begin() + begin, t.nm.begin() + end);
-        r.ss.assign(t.ss.begin() + begin * t.ng, t.ss.begin() + end * t.ng);
-        r.sm.assign(t.sm.begin() + begin * t.ng, t.sm.begin() + end * t.ng);
-        r.q.assign(t.q.begin() + begin * t.ng * t.gs, t.q.begin() + end * t.ng * t.gs);
-        return r;
+        return SliceRange{begin, end - begin, 0, t.k, t.ng};
     }
     if (axis != 1) fail(MFQB_ERR_ARG, "slice axis must be 0 (rows) or 1 (columns)");
     if (end < 0) end = t.k;
     if (begin < 0 || begin >= end || end > t.k) fail(MFQB_ERR_ARG, "NINT column slice [%lld,%lld) out of range", (long long)begin, (long long)end);
     if (begin % t.gs != 0 || (end != t.k && end % t.gs != 0))
         fail(MFQB_ERR_ARG, "NINT column slices must start and end on group boundaries (gs=%d)", t.gs);
-    const int64_t g0 = begin / t.gs, g1 = (end + t.gs - 1) / t.gs, ngs = g1 - g0;
-    HostNint r;
-    r.bits = t.bits;
-    r.sub_bits = t.sub_bits;
-    r.gs = t.gs;
-    r.n = t.n;
-    r.k = end - begin;
-    r.ng = ngs;
-    r.ns = t.ns;
-    r.nm = t.nm;
-    r.ss.resize((size_t)t.n * ngs);
-    r.sm.resize((size_t)t.n * ngs);
-    r.q.resize((size_t)t.n * ngs * t.gs);
-    for (int64_t row = 0; row < t.n; ++row) {
-        memcpy(&r.ss[row * ngs], &t.ss[row * t.ng + g0], ngs);
-        memcpy(&r.sm[row * ngs], &t.sm[row * t.ng + g0], ngs);
-        memcpy(&r.q[row * ngs * t.gs], &t.q[(row * t.ng + g0) * t.gs], (size_t)ngs * t.gs);
-    }
-    return r;
+    const int64_t g0 = begin / t.gs, g1 = (end + t.gs - 1) / t.gs;
+    return SliceRange{0, t.n, g0, end - begin, g1 - g0};
 }
 
-HostNvq parse_nvq(const void* blob, uint64_t nbytes) {
+HostNvq parse_nvq_header(const void* blob, uint64_t nbytes, NvqStreams* streams) {
     Cursor c(blob, nbytes);
     const uint8_t* magic = c.take(4, "NVQ magic");
     if (memcmp(magic, "NVQ1", 4) != 0 && memcmp(magic, "NIQ1", 4) != 0) fail(MFQB_ERR_FORMAT, "invalid NVQ magic");
@@ -227,39 +212,40 @@ HostNvq parse_nvq(const void* blob, uint64_t nbytes) {
     t.ng = (t.k + t.gs - 1) / t.gs;
     t.nvec = (t.k + 3) / 4;
     t.nsign = (t.k + 7) / 8;
-    const uint8_t* an = c.take(2ull * out, "NVQ anchors");
-    t.anchors.resize(out);
-    memcpy(t.anchors.data(), an, 2ull * out);
     const uint64_t nsub = (uint64_t)out * t.ng, nidx = (uint64_t)out * t.nvec, nsg = (uint64_t)out * t.nsign;
-    t.sub.resize(nsub);
-    t.idx.resize(nidx);
-    t.signs.resize(nsg);
-    unpack_bits(c.take(packed_nbytes(nsub, t.sub_bits), "NVQ sub-scales"), nsub, t.sub_bits, t.sub.data());
-    unpack_bits16(c.take(packed_nbytes(nidx, t.index_bits), "NVQ indices"), nidx, t.index_bits, t.idx.data());
-    unpack_bits(c.take(packed_nbytes(nsg, 7), "NVQ signs"), nsg, 7, t.signs.data());
+    streams->anchors = c.take(2ull * out, "NVQ anchors");
+    streams->sub = c.take(packed_nbytes(nsub, t.sub_bits), "NVQ sub-scales");   // (a joint state has four bits: always in range)
+    streams->idx = c.take(packed_nbytes(nidx, t.index_bits), "NVQ indices");
+    streams->signs = c.take(packed_nbytes(nsg, 7), "NVQ signs");
     if (c.off != nbytes) fail(MFQB_ERR_FORMAT, "invalid NVQ blob tail: consumed=%llu size=%llu", (unsigned long long)c.off, (unsigned long long)nbytes);
-    if (t.jsc)
-        for (uint8_t s : t.sub)
-            if (s > 15) fail(MFQB_ERR_FORMAT, "NVQ-JSC state out of range");
     return t;
 }
 
-uint64_t nvq_payload_bytes(const HostNvq& t) {
-    return 2ull * t.n + packed_nbytes((uint64_t)t.n * t.ng, t.sub_bits) + packed_nbytes((uint64_t)t.n * t.nvec, t.index_bits) +
-           packed_nbytes((uint64_t)t.n * t.nsign, 7) + t.table_bytes;
+HostNvq parse_nvq(const void* blob, uint64_t nbytes) {
+    NvqStreams s;
+    HostNvq t = parse_nvq_header(blob, nbytes, &s);
+    const uint64_t nsub = (uint64_t)t.n * t.ng, nidx = (uint64_t)t.n * t.nvec, nsg = (uint64_t)t.n * t.nsign;
+    t.anchors.resize(t.n);
+    memcpy(t.anchors.data(), s.anchors, 2ull * t.n);
+    t.sub.resize(nsub);
+    t.idx.resize(nidx);
+    t.signs.resize(nsg);
+    unpack_bits(s.sub, nsub, t.sub_bits, t.sub.data());
+    unpack_bits16(s.idx, nidx, t.index_bits, t.idx.data());
+    unpack_bits(s.signs, nsg, 7, t.signs.data());
+    return t;
 }
 
-HostNvq slice_nvq(const HostNvq& t, int axis, int64_t begin, int64_t end) {
-    HostNvq r = t;
+uint64_t nvq_payload_bytes(const HostNvq& t, int64_t n, int64_t k) {
+    return 2ull * n + packed_nbytes((uint64_t)n * ((k + t.gs - 1) / t.gs), t.sub_bits) + packed_nbytes((uint64_t)n * ((k + 3) / 4), t.index_bits) +
+           packed_nbytes((uint64_t)n * ((k + 7) / 8), 7) + t.table_bytes;
+}
+
+SliceRange slice_nvq(const HostNvq& t, int axis, int64_t begin, int64_t end) {
     if (axis == 0) {
         if (end < 0) end = t.n;
         if (begin < 0 || begin >= end || end > t.n) fail(MFQB_ERR_ARG, "NVQ row slice out of range");
-        r.n = end - begin;
-        r.anchors.assign(t.anchors.begin() + begin, t.anchors.begin() + end);
-        r.sub.assign(t.sub.begin() + begin * t.ng, t.sub.begin() + end * t.ng);
-        r.idx.assign(t.idx.begin() + begin * t.nvec, t.idx.begin() + end * t.nvec);
-        r.signs.assign(t.signs.begin() + begin * t.nsign, t.signs.begin() + end * t.nsign);
-        return r;
+        return SliceRange{begin, end - begin, 0, t.k, t.ng};
     }
     if (axis != 1) fail(MFQB_ERR_ARG, "slice axis must be 0 (rows) or 1 (columns)");
     if (end < 0) end = t.k;
@@ -267,19 +253,7 @@ HostNvq slice_nvq(const HostNvq& t, int axis, int64_t begin, int64_t end) {
     // Groups (24), index vectors (4) and sign blocks (8) all restart at multiples of 24.
     if (begin % 24 != 0 || (end != t.k && end % 24 != 0))
         fail(MFQB_ERR_ARG, "NVQ column slices must start and end on multiples of 24");
-    r.k = end - begin;
-    r.ng = (r.k + 23) / 24;
-    r.nvec = (r.k + 3) / 4;
-    r.nsign = (r.k + 7) / 8;
-    r.sub.resize((size_t)t.n * r.ng);
-    r.idx.resize((size_t)t.n * r.nvec);
-    r.signs.resize((size_t)t.n * r.nsign);
-    for (int64_t row = 0; row < t.n; ++row) {
-        memcpy(&r.sub[row * r.ng], &t.sub[row * t.ng + begin / 24], r.ng);
-        memcpy(&r.idx[row * r.nvec], &t.idx[row * t.nvec + begin / 4], 2 * (size_t)r.nvec);
-        memcpy(&r.signs[row * r.nsign], &t.signs[row * t.nsign + begin / 8], r.nsign);
-    }
-    return r;
+    return SliceRange{0, t.n, begin / 24, end - begin, (end - begin + 23) / 24};
 }
 
 HostNintm parse_nintm(const void* blob, uint64_t nbytes) {
@@ -321,7 +295,7 @@ HostNintm parse_nintm(const void* blob, uint64_t nbytes) {
         if (!dtype_is_nint(pool.dtype))
             fail(MFQB_ERR_UNSUPPORTED, "NINTM cohort dtype '%s' is outside the NINT execution path", pool.dtype.c_str());
         if (runtime) fail(MFQB_ERR_FORMAT, "unexpected NINTM cohort runtime metadata for a NINT cohort");
-        pool.tensor = parse_nint(pl, payload);
+        pool.tensor = parse_nint_view(pl, payload);
         if (pool.tensor.n != (int64_t)count * t.out_per_expert || pool.tensor.k != t.k)
             fail(MFQB_ERR_FORMAT, "NINTM pool %u tensor shape does not match its expert count", p);
         for (int32_t e : pool.expert_ids) {

@@ -101,23 +101,41 @@ struct HostNvq {
     uint64_t table_bytes = 0;              // bytes of in-blob tables (JSC header+banks / custom codebook)
 };
 
+// A NINT blob's header and where its streams start; nothing is copied.
+struct NintView {
+    int bits = 0, sub_bits = 0, gs = 0;
+    int64_t n = 0, k = 0, ng = 0;
+    const uint8_t *ns = nullptr, *nm = nullptr, *ss = nullptr, *sm = nullptr, *q = nullptr;
+    int sub_width = 0, q_width = 0;        // bits per stored value (8 in the whole-byte storage of older writers)
+};
+// An NVQ blob's bulk streams (anchors: 16 bits, sub-scales: sub_bits, indices: index_bits, sign masks: 7 bits each).
+struct NvqStreams {
+    const uint8_t *anchors = nullptr, *sub = nullptr, *idx = nullptr, *signs = nullptr;
+};
+
 struct HostNintmPool {
     std::vector<int32_t> expert_ids;
     std::string dtype;
-    HostNint tensor;                       // rows = expert_ids.size() * out_per_expert
+    NintView tensor;                       // rows = expert_ids.size() * out_per_expert
 };
 struct HostNintm {
     int64_t n_experts = 0, out_per_expert = 0, k = 0;
     std::vector<HostNintmPool> pools;
 };
 
+NintView parse_nint_view(const void* blob, uint64_t nbytes);
 HostNint parse_nint(const void* blob, uint64_t nbytes);
+HostNvq parse_nvq_header(const void* blob, uint64_t nbytes, NvqStreams* streams);   // everything but sub, idx, signs, anchors
 HostNvq parse_nvq(const void* blob, uint64_t nbytes);
 HostNintm parse_nintm(const void* blob, uint64_t nbytes);
-HostNint slice_nint(const HostNint& t, int axis, int64_t begin, int64_t end);
-HostNvq slice_nvq(const HostNvq& t, int axis, int64_t begin, int64_t end);
-uint64_t nint_payload_bytes(const HostNint& t);
-uint64_t nvq_payload_bytes(const HostNvq& t);
+// A rectangle of a tensor: rows [row0, row0 + n), columns from group group0 on.
+struct SliceRange {
+    int64_t row0 = 0, n = 0, group0 = 0, k = 0, ng = 0;
+};
+SliceRange slice_nint(const NintView& t, int axis, int64_t begin, int64_t end);
+SliceRange slice_nvq(const HostNvq& t, int axis, int64_t begin, int64_t end);
+uint64_t nint_payload_bytes(const NintView& t, int64_t n, int64_t ng);
+uint64_t nvq_payload_bytes(const HostNvq& t, int64_t n, int64_t k);
 
 bool dtype_is_nint(const std::string& dtype);
 bool dtype_is_nvq(const std::string& dtype);

@@ -1,5 +1,6 @@
 // CUDA-side helpers shared by the .cu files of the library.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <mutex>
@@ -56,6 +57,26 @@ struct DevBuf {
     }
     ~DevBuf() { release(); }
 };
+
+#if defined(__CUDACC__)
+// Four neighbouring decoded weights, `live` of them inside the row: one vector store where the four are aligned.
+__device__ __forceinline__ void store_quad(void* out, int out_dtype, size_t off, const float (&v)[4], int live) {
+    if (out_dtype == MFQB_F32) {
+        float* p = static_cast<float*>(out) + off;
+        if (live == 4 && (reinterpret_cast<uintptr_t>(p) & 15) == 0) *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+        else
+            for (int e = 0; e < live; ++e) p[e] = v[e];
+    } else {
+        __nv_bfloat16* p = static_cast<__nv_bfloat16*>(out) + off;
+        if (live == 4 && (reinterpret_cast<uintptr_t>(p) & 7) == 0) {
+            const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+            *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b));
+        } else {
+            for (int e = 0; e < live; ++e) p[e] = __float2bfloat16_rn(v[e]);
+        }
+    }
+}
+#endif
 
 // Library scratch that only ever grows: one block per device, handed to kernels that may still be
 // in flight (or baked into a captured graph) when a later call needs more.  A larger request

@@ -66,8 +66,8 @@ struct LaneUnit {
         return r;
     }
 
-    // Host: store field t (codes at bit 0 of each lane of v) into zero-initialised units.
-    static inline void put(uint32_t* w, int t, uint32_t v) {
+    // Store field t (codes at bit 0 of each lane of v) into zero-initialised units; in kernels for compile-time t.
+    static MFQB_HD void put(uint32_t* w, int t, uint32_t v) {
         uint32_t* u = w + (t / NP) * U;
         const int tt = t % NP;
         if (tt < U * F) {
@@ -76,6 +76,9 @@ struct LaneUnit {
         }
         if constexpr (L > 0) {
             const int e = tt - U * F;
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
             for (int bit = 0; bit < B; ++bit) {
                 const int s = e * B + bit, i = s / L, off = F * B + (s % L);
                 u[i] |= ((v >> bit) & REP) << off;

@@ -2,8 +2,8 @@
 //
 // Every precision cohort of the record becomes one NINT device tensor whose rows are the held
 // experts of the cohort, each padded to whole 16-row blocks.  A routed matmul launches the
-// single-row kernel once per cohort over (row splits, pairs) CTAs (larger batches: the batched
-// kernel over route-plan tiles of 8 pairs of one expert); a CTA looks its pair's expert
+// single-row kernel once per cohort over (row splits, pairs) CTAs (larger batches: the batched kernel over route-plan
+// tiles of 2 or 4 pairs of one expert, then the tensor-memory tile kernel); a CTA looks its pair's expert
 // up in two small tables (cohort of the expert, position inside the cohort) and returns when
 // the expert belongs to another cohort or is not held by this handle (expert-parallel shard).
 #include <cuda_bf16.h>
@@ -14,7 +14,9 @@
 #include <mutex>
 
 #include "cuda_util.h"
+#include "load.h"
 #include "nint_gemv1_bl.cuh"
+#include "tile_tc.h"
 
 namespace mfqb {
 void launch_swiglu(const void* gate_up, int in_dtype, int rows, int f, void* hidden, cudaStream_t s);
@@ -40,21 +42,10 @@ struct PlanBufs {
 void launch_nint_bl_dequant(const NintDevB& w, void* out, int out_dtype, cudaStream_t s);
 void launch_nint_bl_gemv_routed(GemvArgsB a, int pairs, int device, cudaStream_t s);
 void launch_nint_bl_gemv_tiles(GemvArgsB a, int tile_m, int max_tiles, int device, cudaStream_t s);
-void check_nint_supported(const HostNint& t);
+void check_nint_supported(const NintView& t);
 int nint_bl_max_passes(const NintDevB& w);
-bool nint_gemm_grouped_supported(const NintDevB& w, int bn, int rows_per_expert);
-size_t nint_gemm_grouped_x_bytes(int pairs, int k);
-void launch_x_gather_f16(const void* x, bool x_f32, const int* pair_order, int div, int pairs, int k, void* x16, cudaStream_t s);
-void launch_nint_gemm_grouped(const NintDevB& w, const void* x16, int pairs, int bn, const int* expert_bounds, const int* tile_bounds,
-                              const int* pair_order, const int* expert_pool, const int* expert_local, int n_experts, int pool,
-                              int rb_per_expert, int rows_per_expert, int max_tiles, void* y, int y_dtype, int device, cudaStream_t s);
-bool moe_hetero_tilesh_supported(const NintDevB* pools, const int* held, int npools);
-bool launch_moe_hetero_tilesh(GemvArgsB base, const NintDevB* pools, const int* held, int npools, int tile_m, int max_tiles, int device, cudaStream_t s);
 // Twice the pairs per expert from which the f16 tile kernel is used (mfqb_tune "moe_f16_tiles_from_x2"); defined with mfqb_tune.
 extern int g_moe_f16_from_x2;
-size_t nint_bl_frag_tile_units(const NintDevB& w, int nt);
-size_t x_frags_bytes(int in_rows, int tiles, size_t tile_units);
-void launch_x_frags(XFragArgs fa, int in_rows, int tiles, int max_nchunks, void* buf, const uint2** xf, const float** down, cudaStream_t s);
 bool launch_moe_hetero_tiles(GemvArgsB base, const NintDevB* pools, const int* held, const uint2* const* xq, const float2* const* gtab,
                              int npools, int tile_m, int max_tiles, int device, cudaStream_t s);
 bool launch_moe_hetero_gemv1(GemvArgsB base, const NintDevB* pools, const int* held, int npools, int pairs, int device, cudaStream_t s);
@@ -63,36 +54,10 @@ void launch_x_planes(const NintDevB& w, const void* x, int rows, void* planes, c
                      bool x_f32);
 
 struct MoePool {
+    PackedDev dev;
     NintDevB d{};
-    DevBuf items, anchors;
     int held = 0;   // experts of this cohort held here
 };
-
-// Rows of the listed experts (positions inside the cohort tensor), each padded with all-zero
-// rows to `padded` rows.
-static HostNint gather_experts(const HostNint& t, const std::vector<int>& local, int64_t ope, int64_t padded) {
-    HostNint r;
-    r.bits = t.bits;
-    r.sub_bits = t.sub_bits;
-    r.gs = t.gs;
-    r.k = t.k;
-    r.ng = t.ng;
-    r.n = (int64_t)local.size() * padded;
-    r.ns.assign(r.n, 0);
-    r.nm.assign(r.n, 0);
-    r.ss.assign((size_t)r.n * t.ng, 0);
-    r.sm.assign((size_t)r.n * t.ng, 0);
-    r.q.assign((size_t)r.n * t.ng * t.gs, 0);
-    for (size_t i = 0; i < local.size(); ++i) {
-        const int64_t src = (int64_t)local[i] * ope, dst = (int64_t)i * padded;
-        std::copy(t.ns.begin() + src, t.ns.begin() + src + ope, r.ns.begin() + dst);
-        std::copy(t.nm.begin() + src, t.nm.begin() + src + ope, r.nm.begin() + dst);
-        std::copy(t.ss.begin() + src * t.ng, t.ss.begin() + (src + ope) * t.ng, r.ss.begin() + dst * t.ng);
-        std::copy(t.sm.begin() + src * t.ng, t.sm.begin() + (src + ope) * t.ng, r.sm.begin() + dst * t.ng);
-        std::copy(t.q.begin() + src * t.ng * t.gs, t.q.begin() + (src + ope) * t.ng * t.gs, r.q.begin() + dst * t.ng * t.gs);
-    }
-    return r;
-}
 
 // Per-device scratch for the FFN intermediates (slot 0) and for a stand-alone routed matmul's plan
 // and planes (slot 1): grow-only, see GrowOnlyScratch.
@@ -114,7 +79,7 @@ struct mfqb_moe_weight {
     int padded = 0;                                       // rows per expert on the device (multiple of 16)
 };
 
-static uint64_t expert_payload_bytes(const HostNint& t, int64_t ope) {
+static uint64_t expert_payload_bytes(const NintView& t, int64_t ope) {
     // share of the cohort's file streams: anchors + sub-scales + sub-mins + codes of `ope` rows
     const uint64_t per_row_bits = 32ull + 2ull * t.ng * t.sub_bits + (uint64_t)t.ng * t.gs * t.bits;
     return (per_row_bits * (uint64_t)ope + 7) / 8;
@@ -155,13 +120,11 @@ int mfqb_nintm_from_blob(const void* blob, uint64_t nbytes, int expert_begin, in
             auto pool = std::make_unique<MoePool>();
             pool->held = (int)local.size();
             if (!local.empty()) {
-                NintPackedB p = pack_nint_bytes(gather_experts(hp.tensor, local, ope, w->padded));
-                pool->items.upload(p.items.data(), p.items.size() * 4);
-                pool->anchors.upload(p.anchors.data(), p.anchors.size() * 4);
-                pool->d = p.d;
-                pool->d.items = static_cast<const uint32_t*>(pool->items.p);
-                pool->d.anchors = static_cast<const uint32_t*>(pool->anchors.p);
-                dev_bytes += pool->items.bytes + pool->anchors.bytes;
+                pool->dev.d = nint_geometry(hp.tensor, (int64_t)local.size() * w->padded, hp.tensor.k);
+                pool->dev.alloc();
+                load_nint(hp.tensor, 0, LoadRows{0, ope, w->padded, local}, device, pool->dev);   // each expert padded to whole row-blocks
+                pool->d = pool->dev.d;
+                dev_bytes += pool->dev.bytes;
             }
             w->pools.push_back(std::move(pool));
         }
@@ -221,70 +184,51 @@ int mfqb_moe_dequant_expert(const mfqb_moe_weight* w, int expert, void* out, int
     });
 }
 
-// Pairs per route-plan tile (2, 4 or 8, by the average number of pairs an expert sees), or
-// 0: fewer pairs than experts, every pair runs as a single-row problem of its own.
-// True when the f16 tile kernel can serve every held cohort of this record.
-static bool moe_f16_tiles_ok(const mfqb_moe_weight* w) {
+// The record's cohorts as the kernels take them.
+struct MoeCohorts {
     NintDevB devs[16];
-    int held[16];
-    if (w->pools.size() > 16) return false;
-    for (size_t pi = 0; pi < w->pools.size(); ++pi) {
-        devs[pi] = w->pools[pi]->d;
-        held[pi] = w->pools[pi]->held;
+    int held[16], n;
+    explicit MoeCohorts(const mfqb_moe_weight* w) : n((int)w->pools.size()) {   // at most 16 (mfqb_nintm_from_blob)
+        for (int i = 0; i < n; ++i) {
+            devs[i] = w->pools[i]->d;
+            held[i] = w->pools[i]->held;
+        }
     }
-    return moe_hetero_tilesh_supported(devs, held, (int)w->pools.size());
+};
+// True when the matmul over `pairs` pairs runs on the tensor-memory tile kernel (f16 weights): from two pairs per expert on.
+static bool moe_use_tiles_tc(const mfqb_moe_weight* w, int pairs) {
+    if (2 * (long long)pairs < (long long)mfqb::g_moe_f16_from_x2 * w->info.n_experts) return false;
+    const MoeCohorts c(w);
+    return tile_experts_supported(c.devs, c.held, c.n);
 }
-// 8-byte units per tile of the fragment-ordered input rows (the largest among the held cohorts) and the most chunks a row has.
-static size_t moe_frag_tile_units(const mfqb_moe_weight* w, int nt) {
-    size_t units = 0;
-    for (const auto& pool : w->pools)
-        if (pool->held) units = std::max(units, nint_bl_frag_tile_units(pool->d, nt));
-    return units;
+static size_t moe_tiles_tc_bytes(const mfqb_moe_weight* w, int pairs) {
+    const MoeCohorts c(w);
+    return tile_experts_x_bytes(c.devs, c.held, c.n, pairs, w->info.n_experts);
 }
-static int moe_max_nchunks(const mfqb_moe_weight* w) {
-    int n = 0;
-    for (const auto& pool : w->pools)
-        if (pool->held) n = std::max(n, pool->d.nchunks);
-    return n;
+// One matmul over the plan's tiles (tile_m pairs each) on that kernel; see launch_tile_experts_product.
+static void moe_tiles_tc(const mfqb_moe_weight* w, const PlanBufs& plan, int tile_m, int pairs, const void* x, TileX kind, int src_div, void* xbuf, void* y, int y_dtype,
+                         bool scatter, cudaStream_t s) {
+    const MoeCohorts c(w);
+    const TileRoutes r{plan.expert_bounds, plan.tile_bounds, plan.pair_order, static_cast<const int*>(w->d_expert_pool.p), static_cast<const int*>(w->d_expert_local.p),
+                       w->info.n_experts, pairs, tile_m};
+    launch_tile_experts_product(c.devs, c.held, c.n, r, x, kind, src_div, xbuf, y, y_dtype, scatter, w->info.out_per_expert, w->padded / 16, w->info.device, s);
 }
-// Upper bound on the route plan's tiles for `pairs` pairs in tiles of tile_m.
-static int moe_max_tiles(const mfqb_moe_weight* w, int pairs, int tile_m) { return pairs / tile_m + std::min(pairs, w->info.n_experts); }
 
-
+// Pairs per route-plan tile of the integer batched kernel (2, 4 or 8), or 0: fewer pairs than experts, every pair runs as a
+// single-row problem of its own.
 static int moe_tile_m(const mfqb_moe_weight* w, int pairs) {
     const int e = w->info.n_experts;
     if (pairs < e) return 0;
     int cap = 8;   // cohorts with wide records fit fewer batch rows per CTA
     for (const auto& pool : w->pools)
         if (pool->held) cap = std::min(cap, 2 * nint_bl_max_passes(pool->d));
-    // from about three pairs per expert the f16 tile kernel (tiles of 8, then 16 pairs: an expert's weights are
-    // decoded once per tile) is cheaper than the integer passes over tiles of 2 or 4
-    if (2 * (long long)pairs >= (long long)mfqb::g_moe_f16_from_x2 * e && moe_f16_tiles_ok(w)) return pairs >= 10 * e ? 16 : 8;
     // measured on the 128-expert top-8 layer: tiles of four win from two to about twenty pairs per expert
     return std::min(cap, 2 * pairs <= 3 * e ? 2 : (pairs <= 24 * e ? 4 : 8));
 }
 
-// Token tile of the tensor-core tile kernel for large batches (the route plan is then built with
-// this tile size), or 0 to stay on the integer kernels.  Measured on the 128-expert top-8 layer:
-// from about two dozen pairs per expert one f16 decode of an expert's weights per tile beats the
-// batched integer passes over them (the tile kernel's time hardly depends on the batch).
-static int moe_gemm_bn(const mfqb_moe_weight* w, int pairs) {
-    const int e = w->info.n_experts;
-    if (pairs < 24 * e) return 0;
-    int bn = 32;
-    while (bn < 256 && 4 * bn < 5 * (pairs / e)) bn *= 2;   // room for experts that draw more than the average
-    for (const auto& pool : w->pools)
-        if (pool->held && !nint_gemm_grouped_supported(pool->d, bn, w->info.out_per_expert)) return 0;
-    return bn;
-}
-
 // Bytes of quantised activation planes the tile path needs for `rows` input rows: one set per
 // distinct group size among the held cohorts (cohorts of equal group size share theirs).
-static size_t moe_planes_bytes(const mfqb_moe_weight* w, int rows, int pairs, int tile_m) {
-    // the f16 tile kernel's fragment-ordered input rows share the space
-    const size_t f16_rows = (tile_m == 8 || tile_m == 16)
-                                ? (x_frags_bytes(rows, moe_max_tiles(w, pairs, tile_m), moe_frag_tile_units(w, tile_m / 8)) + 255) / 256 * 256
-                                : 0;
+static size_t moe_planes_bytes(const mfqb_moe_weight* w, int rows) {
     size_t total = 0;
     for (size_t pi = 0; pi < w->pools.size(); ++pi) {
         if (!w->pools[pi]->held) continue;
@@ -292,7 +236,7 @@ static size_t moe_planes_bytes(const mfqb_moe_weight* w, int rows, int pairs, in
         for (size_t pj = 0; pj < pi; ++pj) seen = seen || (w->pools[pj]->held && w->pools[pj]->d.gs == w->pools[pi]->d.gs);
         if (!seen) total += (nint_bl_planes_bytes(w->pools[pi]->d, rows) + 255) / 256 * 256;
     }
-    return std::max(total, f16_rows);
+    return total;
 }
 
 // plan == nullptr: one single-row problem per pair.  Otherwise the batched kernel runs over the
@@ -300,7 +244,7 @@ static size_t moe_planes_bytes(const mfqb_moe_weight* w, int rows, int pairs, in
 // moe_planes_bytes() of device memory for the quantised input rows.
 constexpr size_t kFfnCounterBytes = 64 * 1024;   // route-sum counters at the start of the FFN scratch: zero between calls
 struct FfnLayout {
-    bool gemm, tiles, fused_tail;
+    bool tiles_tc, tiles, fused_tail;   // a route plan and the tensor-memory tile kernel / the integer batched kernel; the single-row kernel
     int tile_m;
     size_t o_gu, o_hid, o_dn, o_plan, o_planes, b_pgu, total;
 };
@@ -315,18 +259,21 @@ struct FfnTail {
     void* y;
     int y_dtype;
 };
+// Routes to experts this handle does not hold produce zeros (expert-parallel shards are summed afterwards), so the output is
+// cleared first when the handle is partial.
+static void clear_unheld(const mfqb_moe_weight* w, int pairs, void* out, int out_dtype, cudaStream_t stream) {
+    if (w->info.expert_end - w->info.expert_begin != w->info.n_experts)
+        MFQB_CUDA(cudaMemsetAsync(out, 0, (size_t)pairs * w->info.out_per_expert * (out_dtype == MFQB_F32 ? 4 : 2), stream));
+}
 static void mul_mat_id_impl(const mfqb_moe_weight* w, const void* x, int x_per_pair, const int32_t* ids, int tokens, int routes,
-                            void* out, int out_dtype, const PlanBufs* plan, int tile_m, void* planes, cudaStream_t stream, bool gemm = false,
+                            void* out, int out_dtype, const PlanBufs* plan, int tile_m, void* planes, cudaStream_t stream,
                             int x_mode = 0, const FfnTail* tail = nullptr) {
     const int pairs = tokens * routes, ope = w->info.out_per_expert;
     const int in_rows = x_per_pair ? pairs : tokens;
     struct PlaneSet { int gs; const uint2* xq; const float2* gtab; };
     std::vector<PlaneSet> sets;
     char* planes_next = static_cast<char*>(planes);
-    // Routes to experts this handle does not hold produce zeros (expert-parallel shards are
-    // summed afterwards), so clear the output when the handle is partial.
-    if (!tail && w->info.expert_end - w->info.expert_begin != w->info.n_experts)
-        MFQB_CUDA(cudaMemsetAsync(out, 0, (size_t)pairs * ope * (out_dtype == MFQB_F32 ? 4 : 2), stream));
+    if (!tail) clear_unheld(w, pairs, out, out_dtype, stream);
     if ((x_mode == 2 || tail) && plan) fail(MFQB_ERR_ARG, "mul_mat_id: the fused activation and the fused route sum belong to the single-row path");
     if (!plan && pairs <= 32768) {   // decode sizes: all cohorts in one launch when their codecs allow
         GemvArgsB a{};
@@ -358,61 +305,6 @@ static void mul_mat_id_impl(const mfqb_moe_weight* w, const void* x, int x_per_p
         if (launch_moe_hetero_gemv1(a, devs, held, (int)w->pools.size(), pairs, w->info.device, stream)) return;
     }
     if (x_mode == 2 || tail) fail(MFQB_ERR_UNSUPPORTED, "mul_mat_id: this record's cohorts have no all-cohort single-row kernel");
-    if (plan && gemm) {   // large batches: tensor-core tile kernel, `planes` holds the gathered f16 rows
-        launch_x_gather_f16(x, x_mode == 1, plan->pair_order, x_per_pair ? 1 : routes, pairs, w->info.k, planes, stream);
-        const int tiles = pairs / tile_m + std::min(pairs, w->info.n_experts);
-        if (tiles > 65535) fail(MFQB_ERR_ARG, "mfqb_mul_mat_id: too many route tiles (%d)", tiles);
-        for (size_t pi = 0; pi < w->pools.size(); ++pi) {
-            const MoePool& pool = *w->pools[pi];
-            if (!pool.held) continue;
-            launch_nint_gemm_grouped(pool.d, planes, pairs, tile_m, plan->expert_bounds, plan->tile_bounds, plan->pair_order,
-                                     static_cast<const int*>(w->d_expert_pool.p), static_cast<const int*>(w->d_expert_local.p),
-                                     w->info.n_experts, (int)pi, w->padded / 16, ope, tiles, out, out_dtype, w->info.device, stream);
-        }
-        return;
-    }
-    if (plan && (tile_m == 8 || tile_m == 16) && moe_f16_tiles_ok(w)) {   // f16 tile kernel, all cohorts in one launch
-        const int max_tiles_h = pairs / tile_m + std::min(pairs, w->info.n_experts);
-        if (max_tiles_h > 65535) fail(MFQB_ERR_ARG, "mfqb_mul_mat_id: too many route tiles (%d)", max_tiles_h);
-        GemvArgsB a{};
-        a.y = out;
-        a.ldy = ope;
-        a.y_dtype = out_dtype;
-        a.expert_pool = static_cast<const int*>(w->d_expert_pool.p);
-        a.expert_local = static_cast<const int*>(w->d_expert_local.p);
-        a.rb_per_expert = w->padded / 16;
-        a.routes = routes;
-        a.x_per_pair = x_per_pair ? 1 : 0;
-        a.expert_bounds = plan->expert_bounds;
-        a.tile_bounds = plan->tile_bounds;
-        a.pair_order = plan->pair_order;
-        a.n_experts = w->info.n_experts;
-        NintDevB devs[16];
-        int held[16];
-        XFragArgs fa{};
-        for (size_t pi = 0; pi < w->pools.size(); ++pi) {
-            devs[pi] = w->pools[pi]->d;
-            held[pi] = w->pools[pi]->held;
-            fa.pool_t8[pi] = w->pools[pi]->d.t8;
-            fa.pool_nchunks[pi] = w->pools[pi]->held ? w->pools[pi]->d.nchunks : 0;
-        }
-        fa.x = x;
-        fa.x_f32 = x_mode == 1;
-        fa.k = w->info.k;
-        fa.nt = tile_m / 8;
-        fa.tile_stride = moe_frag_tile_units(w, fa.nt);
-        fa.expert_bounds = plan->expert_bounds;
-        fa.tile_bounds = plan->tile_bounds;
-        fa.pair_order = plan->pair_order;
-        fa.expert_pool = static_cast<const int*>(w->d_expert_pool.p);
-        fa.n_experts = w->info.n_experts;
-        fa.routes = routes;
-        fa.x_per_pair = x_per_pair ? 1 : 0;
-        launch_x_frags(fa, in_rows, max_tiles_h, moe_max_nchunks(w), planes, &a.x16f, &a.x16_scale, stream);
-        a.x16f_tile_stride = fa.tile_stride;
-        if (launch_moe_hetero_tilesh(a, devs, held, (int)w->pools.size(), tile_m, max_tiles_h, w->info.device, stream)) return;
-        fail(MFQB_ERR_UNSUPPORTED, "mul_mat_id: tiles of %d pairs do not fit the f16 tile kernel for this record", tile_m);
-    }
     // quantised planes of the input rows, one set per distinct group size among the held cohorts
     const uint2* pool_xq[16] = {nullptr};
     const float2* pool_gtab[16] = {nullptr};
@@ -507,15 +399,20 @@ int mfqb_mul_mat_id(const mfqb_moe_weight* w, const void* x, int x_per_pair, con
         if (tokens == 0) return;
         DeviceGuard guard(w->info.device);
         const int pairs = tokens * routes;
-        const int gemm_bn = moe_gemm_bn(w, pairs);
-        const int tile_m = gemm_bn ? gemm_bn : moe_tile_m(w, pairs);
+        const bool tiles_tc = moe_use_tiles_tc(w, pairs);
+        const int tile_m = tiles_tc ? tile_experts_rows(pairs, w->info.n_experts) : moe_tile_m(w, pairs);
         if (tile_m) {   // larger batches: route plan in library scratch, batched or tile kernel over its tiles
             const size_t b_plan = PlanBufs::bytes(w->info.n_experts, pairs);
-            const size_t b_in = gemm_bn ? nint_gemm_grouped_x_bytes(pairs, w->info.k) : moe_planes_bytes(w, x_per_pair ? pairs : tokens, pairs, tile_m);
+            const size_t b_in = tiles_tc ? moe_tiles_tc_bytes(w, pairs) : moe_planes_bytes(w, x_per_pair ? pairs : tokens);
             char* s = static_cast<char*>(scratch_get(w->info.device, b_plan + b_in, stream, 1));
             PlanBufs plan = PlanBufs::carve(s, w->info.n_experts);
             launch_route_plan(ids, pairs, w->info.n_experts, tile_m, plan.expert_bounds, plan.tile_bounds, plan.pair_order, stream);
-            mul_mat_id_impl(w, x, x_per_pair, ids, tokens, routes, out, out_dtype, &plan, tile_m, s + b_plan, stream, gemm_bn != 0);
+            if (!tiles_tc) {
+                mul_mat_id_impl(w, x, x_per_pair, ids, tokens, routes, out, out_dtype, &plan, tile_m, s + b_plan, stream);
+                return;
+            }
+            clear_unheld(w, pairs, out, out_dtype, stream);
+            moe_tiles_tc(w, plan, tile_m, pairs, x, kTileXBf16, x_per_pair ? 1 : routes, s + b_plan, out, out_dtype, true, stream);
         } else {
             mul_mat_id_impl(w, x, x_per_pair, ids, tokens, routes, out, out_dtype, nullptr, 0, nullptr, stream);
         }
@@ -546,15 +443,22 @@ static void moe_ffn_run(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* d
     float* hid = reinterpret_cast<float*>(s + L.o_hid);
     float* dn = reinterpret_cast<float*>(s + L.o_dn);
     PlanBufs plan{};
-    if (L.tiles) {   // one route plan serves both matmuls
+    if (L.tiles || L.tiles_tc) {   // one route plan serves both matmuls
         plan = PlanBufs::carve(s + L.o_plan, gate_up->info.n_experts);
         launch_route_plan(ids, (int)pairs, gate_up->info.n_experts, L.tile_m, plan.expert_bounds, plan.tile_bounds, plan.pair_order, stream);
     }
     char* planes = s + L.o_planes;
-    mul_mat_id_impl(gate_up, x, 0, ids, tokens, routes, gu, MFQB_F32, L.tiles ? &plan : nullptr, L.tile_m, planes, stream, L.gemm);
+    if (L.tiles_tc) {   // the gate|up products stay in plan order; the down product's activation tiles form SwiGLU from them in float32
+        moe_tiles_tc(gate_up, plan, L.tile_m, (int)pairs, x, kTileXBf16, routes, planes, gu, MFQB_F32, false, stream);
+        clear_unheld(down, (int)pairs, dn, MFQB_F32, stream);
+        moe_tiles_tc(down, plan, L.tile_m, (int)pairs, gu, kTileXSwiglu, 0, planes, dn, MFQB_F32, true, stream);
+        launch_weighted_reduce(dn, MFQB_F32, weights, tokens, routes, h, y, y_dtype, stream);
+        return;
+    }
+    mul_mat_id_impl(gate_up, x, 0, ids, tokens, routes, gu, MFQB_F32, L.tiles ? &plan : nullptr, L.tile_m, planes, stream);
     if (L.fused_tail) {   // decode sizes: the down matmul reads the gate|up products and ends in the route sum
         const FfnTail tail{weights, dn, reinterpret_cast<unsigned*>(s), y, y_dtype};
-        mul_mat_id_impl(down, gu, 1, ids, tokens, routes, dn, MFQB_F32, nullptr, 0, nullptr, stream, false, 2, &tail);
+        mul_mat_id_impl(down, gu, 1, ids, tokens, routes, dn, MFQB_F32, nullptr, 0, nullptr, stream, 2, &tail);
         return;
     }
     if (!L.tiles) {   // cohorts without an all-cohort kernel: bf16 activation through the per-cohort launches
@@ -562,7 +466,7 @@ static void moe_ffn_run(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* d
         mul_mat_id_impl(down, hid, 1, ids, tokens, routes, dn, MFQB_F32, nullptr, 0, nullptr, stream);
     } else {          // the activation stays float32: no rounding between the two matmuls
         launch_swiglu_f32(gu, (int)pairs, f, hid, stream);
-        mul_mat_id_impl(down, hid, 1, ids, tokens, routes, dn, MFQB_F32, &plan, L.tile_m, planes + L.b_pgu, stream, L.gemm, 1);
+        mul_mat_id_impl(down, hid, 1, ids, tokens, routes, dn, MFQB_F32, &plan, L.tile_m, planes + L.b_pgu, stream, 1);
     }
     launch_weighted_reduce(dn, MFQB_F32, weights, tokens, routes, h, y, y_dtype, stream);
 }
@@ -576,23 +480,25 @@ static void check_ffn_args(const char* who, const mfqb_moe_weight* gate_up, cons
     if ((long long)tokens * routes > INT_MAX) fail(MFQB_ERR_ARG, "%s: %d tokens x %d routes is more than the kernels index", who, tokens, routes);
 }
 
-static FfnLayout ffn_layout(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* down, int tokens, int routes, bool allow_gemm) {
+static FfnLayout ffn_layout(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* down, int tokens, int routes) {
     FfnLayout L{};
-    const int h = gate_up->info.k, f2 = gate_up->info.out_per_expert, f = f2 / 2;
+    const int h = gate_up->info.k, f2 = gate_up->info.out_per_expert, f = f2 / 2, e = gate_up->info.n_experts;
     const size_t pairs = (size_t)tokens * routes;
     auto up256 = [](size_t v) { return (v + 255) / 256 * 256; };
-    // large batches: both matmuls on the tensor-core tile kernel, when every cohort of both has one
-    const int gemm_bn = allow_gemm ? std::min(moe_gemm_bn(gate_up, (int)pairs), moe_gemm_bn(down, (int)pairs)) : 0;
-    L.gemm = gemm_bn != 0;
-    L.tile_m = L.gemm ? gemm_bn : std::min(moe_tile_m(gate_up, (int)pairs), moe_tile_m(down, (int)pairs));
-    L.tiles = L.tile_m != 0;
-    L.fused_tail = !L.tiles && ffn_fused_tail_ok(down, tokens, (int)pairs) && ffn_fused_tail_ok(gate_up, tokens, (int)pairs);
-    const size_t b_plan = L.tiles ? PlanBufs::bytes(gate_up->info.n_experts, pairs) : 0;
-    L.b_pgu = L.gemm ? up256(nint_gemm_grouped_x_bytes((int)pairs, h)) : (L.tiles ? moe_planes_bytes(gate_up, tokens, (int)pairs, L.tile_m) : 0);
-    const size_t b_pdn = L.gemm ? nint_gemm_grouped_x_bytes((int)pairs, f) : (L.tiles ? moe_planes_bytes(down, (int)pairs, (int)pairs, L.tile_m) : 0);
+    L.tiles_tc = moe_use_tiles_tc(gate_up, (int)pairs) && moe_use_tiles_tc(down, (int)pairs);
+    L.tile_m = L.tiles_tc ? tile_experts_rows((int)pairs, e) : std::min(moe_tile_m(gate_up, (int)pairs), moe_tile_m(down, (int)pairs));
+    L.tiles = !L.tiles_tc && L.tile_m != 0;
+    L.fused_tail = !L.tile_m && ffn_fused_tail_ok(down, tokens, (int)pairs) && ffn_fused_tail_ok(gate_up, tokens, (int)pairs);
+    const size_t b_plan = L.tile_m ? PlanBufs::bytes(e, pairs) : 0;
+    size_t b_pdn = 0;
+    if (L.tiles_tc) L.b_pgu = std::max(moe_tiles_tc_bytes(gate_up, (int)pairs), moe_tiles_tc_bytes(down, (int)pairs));   // one after the other
+    else if (L.tiles) {
+        L.b_pgu = moe_planes_bytes(gate_up, tokens);
+        b_pdn = moe_planes_bytes(down, (int)pairs);
+    }
     L.o_gu = kFfnCounterBytes;
     L.o_hid = L.o_gu + up256(pairs * f2 * 4);
-    L.o_dn = L.o_hid + up256(pairs * f * 4);
+    L.o_dn = L.o_hid + (L.tiles_tc ? 0 : up256(pairs * f * 4));
     L.o_plan = L.o_dn + up256(pairs * h * 4);
     L.o_planes = L.o_plan + b_plan;
     L.total = L.o_planes + L.b_pgu + b_pdn;
@@ -606,7 +512,7 @@ int mfqb_moe_ffn(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* down, co
         check_ffn_args("mfqb_moe_ffn", gate_up, down, tokens, routes);
         if (tokens <= 0) return;
         DeviceGuard guard(gate_up->info.device);
-        const FfnLayout L = ffn_layout(gate_up, down, tokens, routes, true);
+        const FfnLayout L = ffn_layout(gate_up, down, tokens, routes);
         char* s = static_cast<char*>(scratch_get(gate_up->info.device, L.total, stream));
         moe_ffn_run(gate_up, down, x, ids, weights, tokens, routes, y, y_dtype, s, L, stream);
     });
@@ -647,8 +553,7 @@ int mfqb_moe_ffn_static(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* d
         if (!gate_up || !down || !x || !ids || !weights || !y) fail(MFQB_ERR_ARG, "mfqb_moe_ffn_static: null argument");
         check_ffn_args("mfqb_moe_ffn_static", gate_up, down, tokens, routes);
         if (tokens <= 0) return;
-        // the tensor-core tile path keeps its own growing buffers: this entry point stays on the integer kernels
-        const FfnLayout L = ffn_layout(gate_up, down, tokens, routes, false);
+        const FfnLayout L = ffn_layout(gate_up, down, tokens, routes);
         if (L.total > (size_t)MFQB_STATIC_SCRATCH_BYTES)
             fail(MFQB_ERR_ARG,
                  "mfqb_moe_ffn_static: %d tokens x %d routes need %llu bytes of scratch, the built-in array holds %llu; "

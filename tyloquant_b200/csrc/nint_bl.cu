@@ -39,15 +39,11 @@ __global__ void nint_bl_dequant_kernel(const NintDevB w, void* out, int out_dtyp
         const float2 nsm = __half22float2(*reinterpret_cast<const __half2*>(&an));
         const float d = __fmul_rn(nsm.x, ss), m = __fmul_rn(nsm.y, sm);
         const int k0 = grp * w.gs + 4 * j;
+        float v[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            if (4 * j + e < w.gs && k0 + e < w.k) {
-                const float v = __fsub_rn(__fmul_rn(d, (float)((codes >> (8 * e)) & 0xFF)), m);
-                const size_t off = (size_t)row * w.k + k0 + e;
-                if (out_dtype == MFQB_F32) reinterpret_cast<float*>(out)[off] = v;
-                else reinterpret_cast<__nv_bfloat16*>(out)[off] = __float2bfloat16_rn(v);
-            }
-        }
+        for (int e = 0; e < 4; ++e) v[e] = __fsub_rn(__fmul_rn(d, (float)((codes >> (8 * e)) & 0xFF)), m);
+        const int live = min(4, min(w.gs - 4 * j, w.k - k0));
+        if (live > 0) store_quad(out, out_dtype, (size_t)row * w.k + k0, v, live);
     }
 }
 

@@ -36,11 +36,14 @@
 #include <cstdint>
 #include <vector>
 
+struct uint4;   // CUDA's
+
 namespace mfqb {
 
 struct NintDevB {
     const uint32_t* items;    // [nrb * nchunks][rec_words]
     const uint32_t* anchors;  // [nrb * 16]
+    const uint4* rowc;        // [nrb * 16] row constants of the tile kernel, see TileRowConst in tile_tc.h
     int n, k, ng;        // rows, columns, groups per row
     int nrb, nchunks;    // row-blocks of 16, chunks of 8 groups
     int bits, gs, sub_bits;

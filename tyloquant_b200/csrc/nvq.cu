@@ -8,6 +8,7 @@
 #include <algorithm>
 
 #include "cuda_util.h"
+#include "load.h"
 #include "nvq.h"
 #include "nvq_blayout.h"
 #include "tile_tc.h"
@@ -18,7 +19,8 @@ void launch_bl_gemv(const NintDevB& w, const void* x, int m, void* y, int y_dtyp
 
 struct NvqDevice {
     NintDevB d{};
-    DevBuf items, anchors, table;
+    PackedDev dev;
+    DevBuf table;
     int device = 0;
 };
 void NvqDeviceDeleter::operator()(NvqDevice* p) const { delete p; }
@@ -34,32 +36,31 @@ void check_nvq_dtype(const std::string& dtype, const HostNvq& t) {
         fail(MFQB_ERR_FORMAT, "MFQ dtype/blob mismatch: %s contains a %d-entry codebook", dtype.c_str(), t.entries);
 }
 
-NvqDevicePtr make_nvq_device(const HostNvq& t, int device, mfqb_weight_info* info) {
+NvqDevicePtr make_nvq_device(const HostNvq& t, const NvqStreams& streams, const SliceRange& r, int device, mfqb_weight_info* info) {
     if ((size_t)t.banks * t.entries * 64 > 128 * 1024)
         fail(MFQB_ERR_UNSUPPORTED, "NVQ codebook of %d banks x %d entries is too large for the shared-memory table", t.banks, t.entries);
-    NvqPackedB p = pack_nvq_bytes(t);
     NvqDevicePtr w(new NvqDevice);
     DeviceGuard guard(device);
     w->device = device;
-    w->items.upload(p.items.data(), p.items.size() * 4);
-    w->anchors.upload(p.anchors.data(), p.anchors.size() * 4);
-    w->table.upload(p.table.data(), p.table.size() * 4);
-    w->d = p.d;
-    w->d.tile_terms = t.jsc ? lattice_terms(p.d.lut, t.codebooks.data(), t.codebooks.size()) : 1;
-    w->d.items = static_cast<const uint32_t*>(w->items.p);
-    w->d.anchors = static_cast<const uint32_t*>(w->anchors.p);
+    std::vector<uint32_t> table;
+    w->dev.d = nvq_geometry(t, r.n, r.k, table);
+    w->dev.alloc();
+    load_nvq(t, streams, r.row0, r.group0, device, w->dev);
+    w->table.upload(table.data(), table.size() * 4);
+    w->d = w->dev.d;
     w->d.table = static_cast<const uint32_t*>(w->table.p);
+    w->d.tile_terms = t.jsc ? lattice_terms(w->d.lut, t.codebooks.data(), t.codebooks.size()) : 1;
     if (info) {
         info->family = MFQB_FAMILY_NVQ;
         info->bits = t.index_bits;
         info->groupsize = t.gs;
         info->sub_bits = t.sub_bits;
-        info->n = t.n;
-        info->k = t.k;
+        info->n = r.n;
+        info->k = r.k;
         info->device = device;
         info->jsc_banks = t.jsc ? t.banks : 0;
-        info->payload_bytes = nvq_payload_bytes(t);
-        info->device_bytes = w->items.bytes + w->anchors.bytes + w->table.bytes;
+        info->payload_bytes = nvq_payload_bytes(t, r.n, r.k);
+        info->device_bytes = w->dev.bytes + w->table.bytes;
     }
     return w;
 }
@@ -89,14 +90,11 @@ __global__ void nvq_bl_dequant_kernel(const NintDevB w, void* out, int out_dtype
         const float scale = __fmul_rn(anchor, w.jsc ? w.lut[state] : (float)state);
         const uint32_t bank = (w.bankmap >> (2 * state)) & 3u;
         const uint32_t codes = w.table[((size_t)bank * w.entries + (field >> 4)) * 16 + (field & 15u)];
-        for (int j = 0; j < 4; ++j) {
-            const int k = grp * 24 + v * 4 + j;
-            if (k >= w.k) break;
-            const float val = __fmul_rn((float)(int)(signed char)(codes >> (8 * j)), scale);
-            const size_t off = (size_t)row * w.k + k;
-            if (out_dtype == MFQB_F32) reinterpret_cast<float*>(out)[off] = val;
-            else reinterpret_cast<__nv_bfloat16*>(out)[off] = __float2bfloat16_rn(val);
-        }
+        float val[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) val[j] = __fmul_rn((float)(int)(signed char)(codes >> (8 * j)), scale);
+        const int k = grp * 24 + v * 4, live = min(4, w.k - k);
+        if (live > 0) store_quad(out, out_dtype, (size_t)row * w.k + k, val, live);
     }
 }
 

@@ -14,7 +14,7 @@ struct NvqDeviceDeleter { void operator()(NvqDevice* p) const; };
 using NvqDevicePtr = std::unique_ptr<NvqDevice, NvqDeviceDeleter>;
 
 void check_nvq_dtype(const std::string& dtype, const HostNvq& t);
-NvqDevicePtr make_nvq_device(const HostNvq& t, int device, mfqb_weight_info* info);
+NvqDevicePtr make_nvq_device(const HostNvq& t, const NvqStreams& streams, const SliceRange& r, int device, mfqb_weight_info* info);
 struct NintDevB;
 const NintDevB& nvq_device_layout(const NvqDevice& w);
 void nvq_dequant(const NvqDevice& w, void* out, int out_dtype, cudaStream_t stream);

@@ -27,13 +27,12 @@ static uint32_t get_bits(const uint32_t* w, int pos, int nbits) {
     return (uint32_t)(v >> sh) & ((1u << nbits) - 1u);
 }
 
-NvqPackedB pack_nvq_bytes(const HostNvq& t) {
+NintDevB nvq_geometry(const HostNvq& t, int64_t n, int64_t k, std::vector<uint32_t>& table) {
     if (t.gs != 24 || t.vec != 4) fail(MFQB_ERR_UNSUPPORTED, "NVQ runtime layout needs 24-weight groups of 4-wide vectors");
-    NvqPackedB p;
-    NintDevB& d = p.d;
-    d.n = (int)t.n;
-    d.k = (int)t.k;
-    d.ng = (int)t.ng;
+    NintDevB d{};
+    d.n = (int)n;
+    d.k = (int)k;
+    d.ng = (int)((k + t.gs - 1) / t.gs);
     d.bits = 0;
     d.gs = 24;
     d.sub_bits = t.sub_bits;
@@ -53,7 +52,7 @@ NvqPackedB pack_nvq_bytes(const HostNvq& t) {
         d.bankmap |= (uint32_t)(t.jsc ? t.bank_for_state[s] : 0) << (2 * s);
     }
     // signed table: entry (bank, index, nibble) = the four int8 codes, negated where the nibble says so
-    p.table.resize((size_t)t.banks * t.entries * 16);
+    table.resize((size_t)t.banks * t.entries * 16);
     for (size_t e = 0; e < (size_t)t.banks * t.entries; ++e)
         for (uint32_t sg = 0; sg < 16; ++sg) {
             uint32_t v = 0;
@@ -61,9 +60,17 @@ NvqPackedB pack_nvq_bytes(const HostNvq& t) {
                 const int code = t.codebooks[e * 4 + j];
                 v |= (uint32_t)(uint8_t)(int8_t)(((sg >> j) & 1u) ? -code : code) << (8 * j);
             }
-            p.table[e * 16 + sg] = v;
+            table[e * 16 + sg] = v;
         }
-    d.table_words = (int)p.table.size();
+    d.table_words = (int)table.size();
+    return d;
+}
+
+NvqPackedB pack_nvq_bytes(const HostNvq& t) {
+    NvqPackedB p;
+    p.d = nvq_geometry(t, t.n, t.k, p.table);
+    const NintDevB& d = p.d;
+    const int fb = d.index_bits + 4;
     p.items.assign((size_t)d.nrb * d.nchunks * d.rec_words, 0u);
     p.anchors.assign((size_t)d.nrb * 16, 0u);
     for (int64_t r = 0; r < t.n; ++r) p.anchors[r] = t.anchors[r];

@@ -34,7 +34,9 @@ struct NvqPackedB {
     std::vector<uint32_t> items, anchors, table;
     NintDevB d{};   // pointers unset; geometry filled
 };
-NvqPackedB pack_nvq_bytes(const HostNvq& t);
+// Geometry, state scales and signed table of n rows x k columns of this tensor.
+NintDevB nvq_geometry(const HostNvq& t, int64_t n, int64_t k, std::vector<uint32_t>& table);
+NvqPackedB pack_nvq_bytes(const HostNvq& t);   // on the host, for the layout's self-check
 uint64_t selfcheck_nvq_bytes(const HostNvq& t);
 
 // Four sign bits of vector `vec` of a row (bit e set: weight 4*vec + e is negative).

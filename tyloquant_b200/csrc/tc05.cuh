@@ -23,6 +23,9 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+// A waiting warp sleeps in hardware for up to this long per poll: the polls of the warps that wait (loaders, issuer, epilogue)
+// otherwise take issue slots from the ones that work.
+constexpr uint32_t kMbarSuspendNs = 2000u;
 // Waits for the phase with the given parity to complete; gives up after `limit` polls and
 // returns false (the caller records the failure and leaves).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = 1u << 22) {
@@ -32,10 +35,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
         uint32_t done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
             "selp.u32 %0, 1, 0, p;\n\t}"
             : "=r"(done)
-            : "r"(addr), "r"(parity)
+            : "r"(addr), "r"(parity), "r"(kMbarSuspendNs)
             : "memory");
         if (done) return true;
     }

@@ -266,6 +266,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     const long long tiles = (long long)row_tiles * ((m + n - 1) / n), units = tiles * w.nchunks;
     if (units * (sms + 1) >= (1ll << 31) * 1ll * sms || units >= (1ll << 31)) return false;
     a.pools[0] = w;
+    a.lut_undo = 1.f;
     if (w.table) lattice_scales(w, a);
     a.m = m;
     a.ntok = (m + n - 1) / n;
@@ -305,6 +306,117 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
         fail(MFQB_ERR_CUDA, "%s%d gs=%d tile product launch (m = %d, %zu bytes of shared memory): %s", w.table ? "NVQ index bits " : "NINT", w.table ? w.index_bits : w.bits,
              w.gs, m, p.smem, cudaGetErrorString(e));
     return true;
+}
+
+// ---- expert products -----------------------------------------------------------------------------------------------------
+static bool experts_one_launch(const NintDevB* pools, const int* held, int npools) {   // the codecs of TileExperts
+    for (int i = 0; i < npools; ++i) {
+        const int c = pools[i].bits * 16 + pools[i].t8;
+        if (held[i] && c != 2 * 16 + 2 && c != 3 * 16 + 3 && c != 4 * 16 + 3 && c != 5 * 16 + 4 && c != 6 * 16 + 3 && c != 8 * 16 + 3 && c != 8 * 16 + 6) return false;
+    }
+    return true;
+}
+// Pairs per tile: one tile for nearly every expert, since each tile decodes the expert's weights once (three standard
+// deviations above the mean of evenly routed pairs); a tile's unused columns cost tensor time only, which the decoding hides.
+int tile_experts_rows(int pairs, int experts) {
+    const double mean = (double)pairs / std::max(experts, 1);
+    const int rows = (int)(mean + 3.0 * std::sqrt(mean) + 3.0);
+    return std::max(16, std::min(256, (rows + 15) / 16 * 16));
+}
+size_t tile_experts_x_bytes(const NintDevB* pools, const int* held, int npools, int pairs, int experts) {
+    size_t row = 0;
+    for (int i = 0; i < npools; ++i)
+        if (held[i]) row = std::max(row, x_row_bytes(pools[i]));
+    const size_t rows = (size_t)(pairs + 7) / 8 * 8 + 8 * ((size_t)experts + 1);   // tile_x_row
+    return (rows * row + 255) / 256 * 256 + ((size_t)pairs * 4 + 255) / 256 * 256;
+}
+bool tile_experts_supported(const NintDevB* pools, const int* held, int npools) {
+    if (npools > kTileMaxPools) return false;
+    TileArgs a{};
+    TilePlan p;
+    size_t rec = 0;
+    int t8 = 0;
+    for (int i = 0; i < npools; ++i) {
+        if (!held[i]) continue;
+        rec = std::max(rec, (size_t)pools[i].rec_words * 4);
+        t8 = std::max(t8, pools[i].t8);
+    }
+    return t8 == 0 || tile_plan(a, p, 256, rec, t8, 1, 0);   // the widest tile needs the most memory
+}
+
+void launch_tile_experts_product(const NintDevB* pools, const int* held, int npools, const TileRoutes& r, const void* x, TileX kind, int src_div, void* xbuf, void* y,
+                                 int y_dtype, bool scatter, int rows_per_expert, int rb_per_expert, int device, cudaStream_t s) {
+    TileArgs a{};
+    TilePlan p;
+    XTilesArgs xa{};
+    size_t rec = 0;
+    int t8 = 0, nslabs = 0, k = 0;
+    for (int i = 0; i < npools; ++i) {
+        if (!held[i]) continue;
+        const NintDevB& w = pools[i];
+        a.pools[i] = w;
+        rec = std::max(rec, (size_t)w.rec_words * 4);
+        t8 = std::max(t8, w.t8);
+        a.x_row_bytes = std::max(a.x_row_bytes, x_row_bytes(w));
+        nslabs = std::max(nslabs, w.nchunks * 4 * w.t8);
+        k = w.k;
+        xa.t8[i] = w.t8;
+        xa.gs[i] = w.gs;
+        xa.nchunks[i] = w.nchunks;
+    }
+    if (t8 == 0) return;   // nothing held here
+    const int n = std::max(16, r.tile_rows), sms = device_sm_count(device);
+    if (!tile_plan(a, p, n, rec, t8, 1, 0)) fail(MFQB_ERR_UNSUPPORTED, "expert tile product: tiles of %d pairs do not fit shared memory", n);
+    unsigned char* buf = static_cast<unsigned char*>(xbuf);
+    const size_t rows = (size_t)(r.pairs + 7) / 8 * 8 + 8 * ((size_t)r.n_experts + 1);
+    float* down = reinterpret_cast<float*>(buf + (rows * a.x_row_bytes + 255) / 256 * 256);
+    xa.x = x;
+    xa.kind = kind;
+    xa.k = k;
+    xa.x_rows = r.tile_rows;
+    xa.row_bytes = a.x_row_bytes;
+    xa.out = buf;
+    xa.down = down;
+    xa.expert_bounds = r.expert_bounds;
+    xa.tile_bounds = r.tile_bounds;
+    xa.pair_order = r.pair_order;
+    xa.expert_pool = r.expert_pool;
+    xa.n_experts = r.n_experts;
+    xa.src_div = src_div;
+    launch_x_tiles(xa, kind, r.pairs, nslabs, sms, s);
+    a.x = buf;
+    a.x_rows = r.tile_rows;
+    a.x_down = down;
+    a.y = y;
+    a.y_dtype = y_dtype;
+    a.ldy = rows_per_expert;
+    a.expert_bounds = r.expert_bounds;
+    a.tile_bounds = r.tile_bounds;
+    a.pair_order = r.pair_order;
+    a.expert_pool = r.expert_pool;
+    a.expert_local = r.expert_local;
+    a.n_experts = r.n_experts;
+    a.rb_per_expert = rb_per_expert;
+    a.rows_per_expert = rows_per_expert;
+    a.scatter = scatter;
+    a.error = device_status_word(device);
+    const long long items = (long long)((rows_per_expert + kTileRows - 1) / kTileRows) * (r.pairs / r.tile_rows + std::min(r.pairs, r.n_experts));
+    p.grid = (int)std::max<long long>(1, std::min<long long>(sms, items));
+    a.only_pool = -1;
+    a.lut_undo = 1.f;
+    if (experts_one_launch(pools, held, npools)) {
+        const cudaError_t e = launch_tile_experts(a, p, s);
+        if (e != cudaSuccess) fail(MFQB_ERR_CUDA, "expert tile product launch (tiles of %d, %zu bytes of shared memory): %s", n, p.smem, cudaGetErrorString(e));
+        return;
+    }
+    for (int i = 0; i < npools; ++i) {   // other profiles: cohort by cohort
+        if (!held[i]) continue;
+        TileArgs b = a;
+        b.pools[0] = pools[i];
+        b.only_pool = i;
+        const cudaError_t e = launch_one(b, p, 1, s);
+        if (e != cudaSuccess) fail(MFQB_ERR_CUDA, "NINT%d gs=%d expert tile product launch: %s", pools[i].bits, pools[i].gs, cudaGetErrorString(e));
+    }
 }
 
 }  // namespace mfqb

@@ -39,21 +39,21 @@
 #include "lane_unit.h"
 #include "nint_blayout.h"
 #include "tc05.cuh"
+#include "tile_tc.h"
 
 namespace mfqb {
 
 constexpr int kTileRows = 128, kTileDecoders = 16, kTileEpilogue = 4;
 constexpr int kTileWarpMma = kTileDecoders + kTileEpilogue, kTileWarpRec = kTileWarpMma + 1, kTileWarpX = kTileWarpMma + 2;
 constexpr int kTileThreads = (kTileDecoders + kTileEpilogue + 3) * 32;
-constexpr size_t kTileDynSmem = 221 * 1024;   // beside 5 KB of barriers and tables
-constexpr int kTileMaxPools = 8, kTileRecStages = 8, kTileXStages = 8, kTileAStages = 8;
-constexpr float kTileWeightScale = 0.25f;   // of the f16 weights: 8-bit codes x 8-bit sub-scales x offset head-room stay below 65504
+constexpr size_t kTileDynSmem = 212 * 1024;   // beside 14 KB of barriers and tables
+constexpr int kTileMaxPools = 8, kTileRecStages = 8, kTileXStages = 8, kTileAStages = 8, kTileSegs = 4;
 
 struct TileArgs {
     NintDevB pools[kTileMaxPools];   // the weight (entry 0), or the cohorts of an expert record
     // lattice records: f16 state scales normalised by a power of two, and its inverse
     uint16_t lut16[16];
-    float lut_undo;
+    float lut_undo;                  // (1 for scalar records)
     const unsigned char* x;          // activation tiles (x_tiles_kernel)
     size_t x_row_bytes;              // bytes of one row in the tiles' buffer (2 x the padded K, the largest among the cohorts)
     int x_rows;                      // most rows of a tile; a tile of c rows is stored with (c + 7) / 8 * 8 rows per 64-column slab
@@ -78,7 +78,7 @@ struct TileSeg {
     int pool, rb0, nrb, row0, row_limit, ch0, ch1, nchunks;
     int tok0, ncols;
     size_t x_off;
-    int tile, part, parts, slot0;   // slot0: CTA index of the tile's first part
+    int parts, slot0, last;   // CTAs that share the tile, the first of them; whether it is this CTA's last stretch
 };
 
 // Unit range of CTA b, and the CTA that owns a unit.
@@ -96,7 +96,6 @@ __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSe
         const NintDevB& w = a.pools[0];
         const int tile = cursor / w.nchunks, rt = tile / a.ntok, tt = tile - rt * a.ntok;
         s.pool = 0;
-        s.tile = tile;
         s.ch0 = cursor - tile * w.nchunks;
         s.ch1 = min(w.nchunks, s.ch0 + end - cursor);
         s.nchunks = w.nchunks;
@@ -109,8 +108,8 @@ __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSe
         s.x_off = (size_t)s.tok0 * a.x_row_bytes;
         s.slot0 = tile_unit_owner(tile * w.nchunks, a.units, gridDim.x);
         s.parts = tile_unit_owner((tile + 1) * w.nchunks - 1, a.units, gridDim.x) - s.slot0 + 1;
-        s.part = blockIdx.x - s.slot0;
         cursor += s.ch1 - s.ch0;
+        s.last = cursor >= end;
         return true;
     }
     const int row_tiles = (a.rows_per_expert + kTileRows - 1) / kTileRows, items = a.tile_bounds[a.n_experts] * row_tiles;
@@ -135,8 +134,7 @@ __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSe
         s.tok0 = a.expert_bounds[lo] + (t - a.tile_bounds[lo]) * a.x_rows;
         s.ncols = min(a.x_rows, a.expert_bounds[lo + 1] - s.tok0);
         s.x_off = (size_t)tile_x_row(a.expert_bounds[lo], lo, (t - a.tile_bounds[lo]) * a.x_rows) * a.x_row_bytes;
-        s.tile = t;
-        s.part = s.slot0 = 0;
+        s.slot0 = s.last = 0;
         s.parts = 1;
         cursor += gridDim.x;
         return true;
@@ -145,21 +143,11 @@ __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSe
 }
 __device__ __forceinline__ int tile_first(const TileArgs& a) { return a.tile_bounds == nullptr ? tile_unit_begin(blockIdx.x, a.units, gridDim.x) : (int)blockIdx.x; }
 
-// F of a row and its (a, b): see the head of the file.
-__device__ __forceinline__ float tile_row_factor(uint32_t anchor, int bits, float& a, float& b) {
-    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&anchor));   // (ns, nm)
-    float f = fmaxf(fabsf(v.x), fabsf(v.y) * __uint_as_float((uint32_t)(126 - bits) << 23));
-    if (f == 0.f) f = 1.f;
-    a = v.x / f;
-    b = v.y / f;
-    return f;
-}
-
 __device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t bits_h2(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
 
 // ---- codecs: decode one warp's half of a chunk record into the A ring ---------------------------------------------------
-// Row(a, rb, lane): what depends on the row-block only.  half<F>(rec, lane, row, ctx, taddr): family F of the record at `rec`
+// Row(consts, lane): what depends on the row-block only, from the 16 rows' constants.  half<F>(rec, lane, row, ctx, taddr): family F of the record at `rec`
 // (shared memory) to the 16 tensor-memory lanes at taddr, columns 16 t + 8 h + {0..7} for octet t and group pair h.
 // The two values of a column are slots i, i + 2 of a quad (the bytes a 16-bit lane mask picks), columns c / 4 + c slots 0, 2 /
 // 1, 3 of quad c: x_tiles_kernel writes the activations in this order.
@@ -176,20 +164,16 @@ struct TileNint {
 
     struct Row {
         __half2 step[2];      // a * scale * 2^-pos for rows q, q + 8, per group pair h
-        __half2 mid[2];       // a * scale * mid
+        __half2 mid;          // a * scale * mid
         __half2 nb_hi, nb_lo; // -b * scale, high and low part
-        __device__ __forceinline__ Row(const TileArgs&, const NintDevB& w, int rb, int lane) {
-            float a0, b0, a1, b1;
-            tile_row_factor(__ldg(w.anchors + rb * 16 + (lane >> 2)), BITS, a0, b0);
-            tile_row_factor(__ldg(w.anchors + rb * 16 + 8 + (lane >> 2)), BITS, a1, b1);
+        __device__ __forceinline__ Row(const NintDevB&, const uint4* consts, int lane) {
+            const uint4 c0 = consts[lane >> 2], c1 = consts[8 + (lane >> 2)];
+            const __half2 a2 = h2_bits(__byte_perm(c0.x, c1.x, 0x5410));
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                step[h] = __floats2half2_rn(a0 * (kTileWeightScale / (float)(1 << pos(2 * h))), a1 * (kTileWeightScale / (float)(1 << pos(2 * h + 1))));
-            mid[0] = mid[1] = __floats2half2_rn(a0 * (kTileWeightScale * MID), a1 * (kTileWeightScale * MID));
-            b0 *= -kTileWeightScale;
-            b1 *= -kTileWeightScale;
-            nb_hi = __floats2half2_rn(b0, b1);
-            nb_lo = __floats2half2_rn(b0 - __low2float(nb_hi), b1 - __high2float(nb_hi));
+            for (int h = 0; h < 2; ++h) step[h] = __hmul2(a2, __floats2half2_rn(1.f / (float)(1 << pos(2 * h)), 1.f / (float)(1 << pos(2 * h + 1))));
+            mid = __hmul2(a2, __float2half2_rn((float)MID));
+            nb_hi = h2_bits(__byte_perm(c0.x, c1.x, 0x7632));
+            nb_lo = h2_bits(__byte_perm(c0.y, c1.y, 0x5410));
         }
     };
     // register r as two f16 pairs 1024 + q 2^pos: bytes 0, 2 and bytes 1, 3
@@ -231,29 +215,27 @@ struct TileNint {
             octets<F, TI + 1>(rec, lane, d, n, taddr);
         }
     }
+    // Both halves of a chunk run the same code where the second one's registers start on a word.
+    static constexpr bool SPLIT = (4 * T) % BU::NP == 0;
+    static constexpr int FW = SPLIT ? 4 * T / BU::NP * BU::U : 0;
     template <int F>
-    __device__ static __forceinline__ void half(const uint32_t* rec, int lane, const Row& row, const unsigned char*, uint32_t taddr) {
+    __device__ static __forceinline__ void half(const uint32_t* rec, int lane, int f, const Row& row, const unsigned char*, uint32_t taddr) {
         const uint32_t sel = (lane & 2) ? 0x4341u : 0x4240u;   // this lane's group of a pair: bytes (row q, row q + 8)
         const __half2 k1024 = __float2half2_rn(1024.f);
         __half2 d[4], n[4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const uint32_t* sc = rec + WC * 32 + (lane & ~3) + 2 * F + h;
+            const uint32_t* sc = rec + WC * 32 + (lane & ~3) + 2 * f + h;
             const __half2 ss = __hsub2(h2_bits(__byte_perm(sc[0], 0x64646464u, sel)), k1024);
             const __half2 sm = __hsub2(h2_bits(__byte_perm(sc[32], 0x64646464u, sel)), k1024);
             const __half2 d2 = __hmul2(ss, row.step[h]);
-            const __half2 n2 = __hfma2(sm, row.nb_lo, __hfma2(sm, row.nb_hi, __hmul2(ss, row.mid[h])));
+            const __half2 n2 = __hfma2(sm, row.nb_lo, __hfma2(sm, row.nb_hi, __hmul2(ss, row.mid)));
             d[2 * h] = __low2half2(d2);
             d[2 * h + 1] = __high2half2(d2);
             n[2 * h] = __low2half2(n2);
             n[2 * h + 1] = __high2half2(n2);
         }
-        octets<F, 0>(rec, lane, d, n, taddr);
-    }
-    // what the epilogue multiplies a row's sums by
-    __device__ static __forceinline__ float row_undo(const TileArgs&, uint32_t anchor) {
-        float a, b;
-        return tile_row_factor(anchor, BITS, a, b) * (1.f / kTileWeightScale);
+        octets<F, 0>(rec + (SPLIT ? f * FW * 32 : 0), lane, d, n, taddr);
     }
 };
 
@@ -267,6 +249,9 @@ struct TileShared {
     int finish;   // 1 + column table of the shared tile that this CTA finishes at its end, 0: none
     TileSeg fin;
     __align__(16) float row_factor[kTileRows];
+    __align__(16) uint4 rowc[kTileSegs][kTileRows];   // the stretches' row constants
+    uint64_t seg_full[kTileSegs], seg_empty[kTileSegs];
+    TileSeg seg[kTileSegs];                            // stretches in order, from the record loader; parts == 0: no more
     __align__(16) int2 col[2][256];   // the epilogue's tile (two in turn): factor (float bits) and output row of every column
 };
 
@@ -309,18 +294,22 @@ __device__ __forceinline__ bool tile_epilogue_all(bool ok) {
 // The decoder warps' share of one stretch.
 template <class C, int F>
 __device__ __forceinline__ bool tile_decode(const TileArgs& a, TileShared& sh, const TileSeg& s, unsigned char* rec_ring, const unsigned char* ctx, TileRing& rr,
-                                            TileRing& ar, int rbl, int lane, uint32_t taddr) {
+                                            TileRing& ar, int rbl, int f, int lane, uint32_t taddr, const uint4* consts, uint64_t* seg_done, int& runway) {
     const NintDevB& w = a.pools[s.pool];
     const bool mine = rbl < s.nrb;   // a tile at the end of the matrix has fewer row-blocks: their rows of D are never read
-    const typename C::Row row(a, w, s.rb0 + (mine ? rbl : 0), lane);
+    const typename C::Row row(w, consts + (mine ? rbl : 0) * 16, lane);
+    __syncwarp();
+    if (lane == 0) mbar_arrive(seg_done);
     for (int ch = s.ch0; ch < s.ch1; ch += a.step) {
+        if (runway == 0) asm volatile("griddepcontrol.wait;" ::: "memory");   // from here on the A ring empties only once the activations are there
+        --runway;
         if (!tile_wait2(&sh.rec_full[rr.stage], rr.phase, &sh.a_empty[ar.stage], ar.phase ^ 1u)) return false;
         if (mine) {
             tc_fence_after_sync();
             const uint32_t* rec = reinterpret_cast<const uint32_t*>(rec_ring + (size_t)rr.stage * a.rec_stage_bytes) + rbl * a.step * w.rec_words;
             const uint32_t at = taddr + ar.stage * a.a_cols;
-            C::template half<F>(rec, lane, row, ctx, at);
-            if (a.step > 1 && ch + 1 < s.ch1) C::template half<F>(rec + w.rec_words, lane, row, ctx, at + 16 * C::T * C::TERMS);
+            C::template half<F>(rec, lane, f, row, ctx, at);
+            if (a.step > 1 && ch + 1 < s.ch1) C::template half<F>(rec + w.rec_words, lane, f, row, ctx, at + 16 * C::T * C::TERMS);
             __syncwarp();
         }
         if (lane == 0) mbar_arrive(&sh.rec_empty[rr.stage]);
@@ -442,6 +431,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
         for (int i = 0; i < kTileRecStages; ++i) { mbar_init(&sh.rec_full[i], 1); mbar_init(&sh.rec_empty[i], kTileDecoders); }
         for (int i = 0; i < kTileXStages; ++i) { mbar_init(&sh.x_full[i], 1); mbar_init(&sh.x_empty[i], 1); }
         for (int i = 0; i < kTileAStages; ++i) { mbar_init(&sh.a_full[i], kTileDecoders / 2); mbar_init(&sh.a_empty[i], 1); }
+        for (int i = 0; i < kTileSegs; ++i) { mbar_init(&sh.seg_full[i], 1); mbar_init(&sh.seg_empty[i], kTileDecoders + kTileEpilogue + 2); }
         for (int i = 0; i < 2; ++i) { mbar_init(&sh.d_full[i], 1); mbar_init(&sh.d_empty[i], kTileEpilogue); }
         mbar_init(&sh.drain, 1);
         sh.finish = 0;
@@ -456,12 +446,24 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t tmem_d = sh.tmem, tmem_a = tmem_d + (uint32_t)(a.d_bufs * a.d_cols);
 
-    // Only the record loader of a plain product runs ahead of the previous kernel (weights are constants); everything else
-    // reads what that kernel wrote, or is bounded by it.
-    if (warp != kTileWarpRec || a.tile_bounds != nullptr) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // Weights are constants: the record loader of a plain product fills its ring and the decoders theirs before the previous
+    // kernel has finished (each waits for it before it could block on what depends on it); all else waits here.
+    if (warp >= kTileDecoders && (warp != kTileWarpRec || a.tile_bounds != nullptr)) asm volatile("griddepcontrol.wait;" ::: "memory");
 
-    int cursor = tile_first(a);
     TileSeg s;
+    TileRing sr;
+    // The next stretch; false at the end or after a failure (ok).
+    auto next = [&](bool& ok) {
+        ok = tile_wait(&sh.seg_full[sr.stage], sr.phase);
+        if (!ok) return false;
+        s = sh.seg[sr.stage];
+        return s.parts != 0;
+    };
+    auto seg_done = [&]() {
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sh.seg_empty[sr.stage]);
+        sr.step(kTileSegs);
+    };
     if (warp < kTileDecoders) {
         // -------- decoders: row-block 2 (warp & 3) + ((warp >> 2) & 1) of the tile, half (warp >> 3) of the chunk --------
         const int rbl = 2 * (warp & 3) + ((warp >> 2) & 1), f = warp >> 3;
@@ -469,26 +471,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
         TileRing rr, ar;
         if (f) ar.step(a.a_stages);
         bool ok = true;
-        while (ok && tile_next(a, cursor, s))
+        int runway = (a.a_stages - f + 1) / 2;   // this half's stages of the ring
+        while (ok && next(ok)) {
+            const uint4* consts = sh.rowc[sr.stage];
+            uint64_t* done = &sh.seg_empty[sr.stage];
             Sets::dispatch(a.pools[s.pool], [&](auto codec) {
                 using C = decltype(codec);
-                ok = f ? tile_decode<C, 1>(a, sh, s, rec_ring, ctx, rr, ar, rbl, lane, taddr) : tile_decode<C, 0>(a, sh, s, rec_ring, ctx, rr, ar, rbl, lane, taddr);
+                if (C::SPLIT || !f) ok = tile_decode<C, 0>(a, sh, s, rec_ring, ctx, rr, ar, rbl, f, lane, taddr, consts, done, runway);
+                else ok = tile_decode<C, 1>(a, sh, s, rec_ring, ctx, rr, ar, rbl, f, lane, taddr, consts, done, runway);
             });
+            sr.step(kTileSegs);
+        }
         if (!ok) sh.failed = 1;
     } else if (warp < kTileWarpMma) {
         // -------- epilogue: lane = row of the warp's quarter of the tile --------
         const int quarter = warp & 3, row_l = quarter * 32 + lane;
         TileRing dr;
         bool ok = true;
-        for (int buf = 0; ok && tile_next(a, cursor, s); buf ^= 1) {
-            const NintDevB& w = a.pools[s.pool];
+        for (int buf = 0; ok && next(ok); buf ^= 1) {
             const int row = s.row0 + row_l;
             const bool row_ok = row < s.row_limit;
-            float undo = 0.f;
-            if (row_ok) {
-                const uint32_t anchor = __ldg(w.anchors + (size_t)s.rb0 * 16 + row_l);
-                Sets::dispatch(w, [&](auto codec) { undo = decltype(codec)::row_undo(a, anchor); });
-            }
+            const float undo = row_ok ? __uint_as_float(sh.rowc[sr.stage][row_l].z) * a.lut_undo : 0.f;
+            seg_done();
             for (int i = tid - kTileDecoders * 32; i < s.ncols; i += kTileEpilogue * 32)
                 sh.col[buf][i] = make_int2(__float_as_int(__ldcg(a.x_down + s.tok0 + i)), a.scatter ? __ldcg(a.pair_order + s.tok0 + i) : s.tok0 + i);
             ok = tile_epilogue_all(tile_wait(&sh.d_full[dr.stage], dr.phase));
@@ -548,7 +552,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
                 asm volatile("bar.sync 1, 128;" ::: "memory");
                 if (sh.last == (unsigned)(s.parts - 1)) {
                     __threadfence();
-                    if (cursor >= tile_unit_begin(blockIdx.x + 1, a.units, gridDim.x)) {   // nothing left for this CTA: every warp helps, below
+                    if (s.last) {   // nothing left for this CTA: every warp helps, below
                         if (lane == 0 && quarter == 0) { sh.finish = buf + 1; sh.fin = s; }
                         break;
                     }
@@ -572,7 +576,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
         const uint32_t idesc = instr_desc_f16(kTileRows, a.n_mma);
         TileRing ar, xr, dr;
         bool ok = true;
-        while (ok && tile_next(a, cursor, s)) {
+        while (ok && next(ok)) {
+            seg_done();
             const int t8 = a.pools[s.pool].t8;
             if (!tile_wait(&sh.d_empty[dr.stage], dr.phase ^ 1u)) { ok = false; break; }
             tc_fence_after_sync();
@@ -605,17 +610,30 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
             tile_wait(&sh.drain, 0);
         }
     } else if (warp == kTileWarpRec) {
-        // -------- record loader --------
+        // -------- record loader: also finds the stretches and hands them to the other warps with their row constants --------
         TileRing rr;
-        bool ok = true;
-        int issued = 0;
-        while (ok && tile_next(a, cursor, s)) {
-            const NintDevB& w = a.pools[s.pool];
+        bool ok = true, more = true;
+        int issued = 0, cursor = tile_first(a);
+        while (ok && more) {
+            more = tile_next(a, cursor, s);
+            if (!tile_wait(&sh.seg_empty[sr.stage], sr.phase ^ 1u)) { ok = false; break; }
+            const NintDevB& w = a.pools[more ? s.pool : 0];
+            if (elect_one()) {
+                if (!more) s.parts = 0;
+                sh.seg[sr.stage] = s;
+                const uint32_t bytes = more ? (uint32_t)s.nrb * 16u * 16u : 0u;
+                mbar_arrive_expect_tx(&sh.seg_full[sr.stage], bytes);
+                if (more) bulk_load(sh.rowc[sr.stage], w.rowc + (size_t)s.rb0 * 16, bytes, &sh.seg_full[sr.stage]);
+            }
+            __syncwarp();
+            sr.step(kTileSegs);
+            if (!more) break;
             const uint32_t pitch = (uint32_t)(a.step * w.rec_words) * 4u;
             const size_t rb_words = (size_t)w.nchunks * w.rec_words;
             const uint32_t* src = w.items + (size_t)s.rb0 * rb_words + (size_t)s.ch0 * w.rec_words;
             for (int ch = s.ch0; ch < s.ch1; ch += a.step, src += (size_t)a.step * w.rec_words) {
                 const uint32_t bytes = (uint32_t)(min(a.step, s.ch1 - ch) * w.rec_words) * 4u;   // a row-block's records of a step are neighbours
+                if (issued == a.rec_stages) asm volatile("griddepcontrol.wait;" ::: "memory");
                 if (!tile_wait(&sh.rec_empty[rr.stage], rr.phase ^ 1u)) { ok = false; break; }
                 if (elect_one()) {
                     mbar_arrive_expect_tx(&sh.rec_full[rr.stage], bytes * (uint32_t)s.nrb);
@@ -631,6 +649,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
         }
         if (!ok) {
             sh.failed = 1;
+            if (issued > 0) tile_wait(&sh.seg_full[(sr.stage + kTileSegs - 1) % kTileSegs], sr.phase ^ (sr.stage == 0 ? 1u : 0u));
             for (int i = 0; i < min(issued, a.rec_stages); ++i) tile_wait(&sh.rec_full[(rr.stage + a.rec_stages - 1 - i) % a.rec_stages], rr.phase ^ (i >= rr.stage ? 1u : 0u));
         }
     } else {
@@ -638,7 +657,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
         TileRing xr;
         bool ok = true;
         int issued = 0;
-        while (ok && tile_next(a, cursor, s)) {
+        while (ok && next(ok)) {
+            seg_done();
             const int t8 = a.pools[s.pool].t8, atoms = a.x_whole ? a.step * t8 : 1;
             const uint32_t pitch = (uint32_t)((s.ncols + 7) & ~7) * 128u;
             const unsigned char* src = a.x + s.x_off + (size_t)s.ch0 * t8 * pitch;
@@ -682,11 +702,8 @@ __global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_c
             a.counters[t.slot0] = 0u;
         }
         for (int r = tid; r < kTileRows; r += kTileThreads)
-            if (t.row0 + r < t.row_limit) {
-                const NintDevB& w = a.pools[t.pool];
-                const uint32_t anchor = __ldg(w.anchors + (size_t)t.rb0 * 16 + r);
-                Sets::dispatch(w, [&](auto codec) { sh.row_factor[r] = decltype(codec)::row_undo(a, anchor); });
-            }
+            if (t.row0 + r < t.row_limit)
+                sh.row_factor[r] = __uint_as_float(__ldg(&a.pools[t.pool].rowc[(size_t)t.rb0 * 16 + r]).z) * a.lut_undo;
         __syncthreads();
         if (!tile_wait(&sh.drain, 0)) {
             if (tid == 0) atomicExch(a.error, MFQB_ERR_TIMEOUT);

@@ -23,7 +23,7 @@ struct TileNvq {
     }
     struct Row {
         uint32_t bank_bytes, lut_off;
-        __device__ __forceinline__ Row(const TileArgs&, const NintDevB& w, int, int) : bank_bytes((uint32_t)w.entries * 64u), lut_off((uint32_t)w.table_words * 4u) {}
+        __device__ __forceinline__ Row(const NintDevB& w, const uint4*, int) : bank_bytes((uint32_t)w.entries * 64u), lut_off((uint32_t)w.table_words * 4u) {}
     };
     template <int R>
     __device__ static __forceinline__ uint32_t codes(const uint32_t* rec, int lane, uint32_t own, const Row& row, const unsigned char* ctx) {
@@ -76,8 +76,9 @@ struct TileNvq {
             octets<F, TI + 1>(rec, lane, own, row, ctx, d, bd, taddr);
         }
     }
+    static constexpr bool SPLIT = false;
     template <int F>
-    __device__ static __forceinline__ void half(const uint32_t* rec, int lane, const Row& row, const unsigned char* ctx, uint32_t taddr) {
+    __device__ static __forceinline__ void half(const uint32_t* rec, int lane, int, const Row& row, const unsigned char* ctx, uint32_t taddr) {
         const uint16_t* lut = reinterpret_cast<const uint16_t*>(ctx + row.lut_off);
         const int odd = (lane >> 1) & 1;
         const uint32_t own = rec[WC * 32 + lane];
@@ -93,9 +94,6 @@ struct TileNvq {
             }
         }
         octets<F, 0>(rec, lane, own, row, ctx, d, bd, taddr);
-    }
-    __device__ static __forceinline__ float row_undo(const TileArgs& a, uint32_t anchor) {
-        return __half2float(__ushort_as_half((unsigned short)(anchor & 0xFFFFu))) * a.lut_undo;
     }
 };
 

@@ -12,6 +12,7 @@
 #include "cuda_util.h"
 #include "nint_gemm_tc.cuh"
 #include "nint_blayout.h"
+#include "load.h"
 #include "nvq.h"
 #include "nvq_blayout.h"
 #include "tile_tc.h"
@@ -261,15 +262,14 @@ struct mfqb_weight {
     int family = 0, device = 0;
     mfqb_weight_info info{};
     NintDevB nint{};
-    DevBuf items, anchors;
-    DevBuf fix;          // streamed single-row kernel: partial rows of row-blocks shared by two CTAs, and their counters
+    PackedDev dev;       // its extra memory: the streamed single-row kernel's partial rows of row-blocks shared by two CTAs, and their counters
     int* status = nullptr;   // the device's host-visible status word
     NvqDevicePtr nvq;
 };
 
 namespace mfqb {
 
-void check_nint_supported(const HostNint& t) {
+void check_nint_supported(const NintView& t) {
     const int b = t.bits;
     if (!(b == 2 || b == 3 || b == 4 || b == 5 || b == 6 || b == 8))
         fail(MFQB_ERR_UNSUPPORTED, "NINT%d is not an executable code width (2,3,4,5,6,8)", b);
@@ -279,32 +279,29 @@ void check_nint_supported(const HostNint& t) {
 const NintDevB& weight_device_layout(const mfqb_weight* w);
 int weight_device_index(const mfqb_weight* w);
 
-static mfqb_weight* make_nint_weight(const HostNint& t, int device) {
+static mfqb_weight* make_nint_weight(const NintView& t, const SliceRange& r, int device) {
     check_nint_supported(t);
-    NintPackedB p = pack_nint_bytes(t);
     auto w = std::make_unique<mfqb_weight>();
     DeviceGuard guard(device);
     w->family = MFQB_FAMILY_NINT;
     w->device = device;
-    w->items.upload(p.items.data(), p.items.size() * 4);
-    w->anchors.upload(p.anchors.data(), p.anchors.size() * 4);
-    w->fix.alloc(gemvs_fix_bytes(device));
-    MFQB_CUDA(cudaMemset(w->fix.p, 0, w->fix.bytes));
+    w->dev.d = nint_geometry(t, r.n, r.k);
+    w->dev.alloc(gemvs_fix_bytes(device));
+    MFQB_CUDA(cudaMemset(w->dev.extra_at(), 0, gemvs_fix_bytes(device)));
+    load_nint(t, r.group0, LoadRows{r.row0, r.n, r.n, {0}}, device, w->dev);
     w->status = device_status_word(device);
-    w->nint = p.d;
-    w->nint.items = static_cast<const uint32_t*>(w->items.p);
-    w->nint.anchors = static_cast<const uint32_t*>(w->anchors.p);
+    w->nint = w->dev.d;
     mfqb_weight_info& i = w->info;
     i.family = MFQB_FAMILY_NINT;
     i.bits = t.bits;
     i.groupsize = t.gs;
     i.sub_bits = t.sub_bits;
-    i.n = t.n;
-    i.k = t.k;
+    i.n = r.n;
+    i.k = r.k;
     i.device = device;
     i.jsc_banks = 0;
-    i.payload_bytes = nint_payload_bytes(t);
-    i.device_bytes = w->items.bytes + w->anchors.bytes;
+    i.payload_bytes = nint_payload_bytes(t, r.n, r.ng);
+    i.device_bytes = w->dev.bytes;
     return w.release();
 }
 
@@ -337,16 +334,17 @@ int mfqb_weight_from_blob_slice(const char* dtype, const void* blob, uint64_t nb
         const std::string d(dtype);
         const bool whole = begin == 0 && end < 0;
         if (dtype_is_nint(d)) {
-            HostNint t = parse_nint(blob, nbytes);
+            const NintView t = parse_nint_view(blob, nbytes);
             if (d[4] - '0' != t.bits) fail(MFQB_ERR_FORMAT, "MFQ dtype/blob mismatch: %s contains NINT%d", dtype, t.bits);
-            *out = whole ? make_nint_weight(t, device) : make_nint_weight(slice_nint(t, axis, begin, end), device);
+            *out = make_nint_weight(t, whole ? SliceRange{0, t.n, 0, t.k, t.ng} : slice_nint(t, axis, begin, end), device);
         } else if (dtype_is_nvq(d)) {
-            HostNvq t = parse_nvq(blob, nbytes);
+            NvqStreams streams;
+            const HostNvq t = parse_nvq_header(blob, nbytes, &streams);
             check_nvq_dtype(d, t);
             auto w = std::make_unique<mfqb_weight>();
             w->family = MFQB_FAMILY_NVQ;
             w->device = device;
-            w->nvq = make_nvq_device(whole ? t : slice_nvq(t, axis, begin, end), device, &w->info);
+            w->nvq = make_nvq_device(t, streams, whole ? SliceRange{0, t.n, 0, t.k, t.ng} : slice_nvq(t, axis, begin, end), device, &w->info);
             *out = w.release();
         } else {
             fail(MFQB_ERR_UNSUPPORTED, "dtype '%s' is outside the packed-weight execution path", dtype);
@@ -374,16 +372,13 @@ int mfqb_weight_clone(const mfqb_weight* src, mfqb_weight** out) {
         w->family = src->family;
         w->device = src->device;
         w->info = src->info;
-        w->items.alloc(src->items.bytes);
-        w->anchors.alloc(src->anchors.bytes);
-        MFQB_CUDA(cudaMemcpy(w->items.p, src->items.p, src->items.bytes, cudaMemcpyDeviceToDevice));
-        MFQB_CUDA(cudaMemcpy(w->anchors.p, src->anchors.p, src->anchors.bytes, cudaMemcpyDeviceToDevice));
-        w->fix.alloc(src->fix.bytes);
-        MFQB_CUDA(cudaMemset(w->fix.p, 0, w->fix.bytes));
+        w->dev.d = src->dev.d;
+        const size_t fix = src->dev.mem.bytes - src->dev.extra_off;
+        w->dev.alloc(fix);
+        MFQB_CUDA(cudaMemcpy(w->dev.mem.p, src->dev.mem.p, src->dev.extra_off, cudaMemcpyDeviceToDevice));
+        MFQB_CUDA(cudaMemset(w->dev.extra_at(), 0, fix));
         w->status = src->status;
-        w->nint = src->nint;
-        w->nint.items = static_cast<const uint32_t*>(w->items.p);
-        w->nint.anchors = static_cast<const uint32_t*>(w->anchors.p);
+        w->nint = w->dev.d;
         *out = w.release();
     });
 }
@@ -417,7 +412,7 @@ int mfqb_mul_mat(const mfqb_weight* w, const void* x, int m, void* y, int y_dtyp
         if (w->family == MFQB_FAMILY_NINT) {
             if (m >= 5 && launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
             if (m == 1 && gemv1_use_streamed(w->nint) &&
-                launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->fix.p, w->status, stream))
+                launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->dev.extra_at(), w->status, stream))
                 return;
             const int per_launch = nint_bl_gemvh_supported(w->nint, 16) ? 16 : 8;   // batch rows one GEMV launch covers
             for (int m0 = 0; m0 < m; m0 += per_launch) {
@@ -675,8 +670,8 @@ int mfqb_selfcheck_layout(const char* dtype, const void* blob, uint64_t nbytes, 
         if (!dtype || !blob || !mismatches) fail(MFQB_ERR_ARG, "mfqb_selfcheck_layout: null argument");
         const std::string d(dtype);
         if (dtype_is_nint(d)) {
+            check_nint_supported(parse_nint_view(blob, nbytes));
             HostNint t = parse_nint(blob, nbytes);
-            check_nint_supported(t);
             *mismatches = selfcheck_nint_bytes(t);
         } else if (dtype_is_nvq(d)) {
             *mismatches = selfcheck_nvq_bytes(parse_nvq(blob, nbytes));
