@@ -124,6 +124,11 @@ for _name, (_res, _args) in _SIGNATURES.items():
     _fn.argtypes = _args
 
 
+from . import _fast  # noqa: E402  (built together with the library)
+
+_fast.bind(*(C.cast(getattr(lib, _name), C.c_void_p).value for _name in ("mfqb_mul_mat", "mfqb_moe_topk", "mfqb_moe_ffn")))
+
+
 def check(status: int) -> None:
     if status != OK:
         raise MfqbError(status, lib.mfqb_last_error().decode("utf-8", "replace"))

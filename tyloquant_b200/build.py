@@ -13,6 +13,7 @@ import hashlib
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -61,10 +62,23 @@ def _compile(src: str, hdr_digest: str, verbose: bool) -> str:
     return obj
 
 
+def _build_pyext() -> None:
+    """The Python extension with the direct calls (pyext/fast.c), next to the package's modules."""
+    src = os.path.join(HERE, "pyext", "fast.c")
+    out = os.path.join(HERE, "_fast" + sysconfig.get_config_var("EXT_SUFFIX"))
+    if os.path.exists(out) and os.path.getmtime(out) >= os.path.getmtime(src):
+        return
+    cmd = ["gcc", "-O2", "-fPIC", "-shared", "-Wall", "-I", sysconfig.get_paths()["include"], src, "-o", out]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"compiling fast.c failed:\n{r.stdout}\n{r.stderr}")
+
+
 def build(verbose: bool = False, jobs: int | None = None) -> str:
     os.makedirs(OBJDIR, exist_ok=True)
     sources = sorted(s for s in os.listdir(CSRC) if s.endswith((".cu", ".cpp")))
     digest = _headers_digest()
+    _build_pyext()
     with cf.ThreadPoolExecutor(max_workers=jobs or os.cpu_count() or 4) as pool:
         objs = list(pool.map(lambda s: _compile(s, digest, verbose), sources))
     stamp = hashlib.sha256(" ".join(sorted(objs)).encode()).hexdigest()

@@ -5,6 +5,8 @@
 #include "nint_gemvh_bl.cuh"
 #include "nint_gemvs.cuh"
 
+#include <algorithm>
+
 namespace mfqb {
 
 struct GemvPlanB {
@@ -52,11 +54,18 @@ static cudaError_t launch_gemvs_codec(const GemvSArgs& a, const GemvSPlan& p, cu
     return cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
-template <typename Kernel, typename... Extra>
-static cudaError_t launch_kernel_pdl(Kernel kernel, const GemvArgsB& a, const GemvPlanB& p, cudaStream_t stream, const Extra&... extra) {
-    if (p.smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem);
+template <auto kernel, typename... Extra>
+static cudaError_t launch_kernel_pdl(const GemvArgsB& a, const GemvPlanB& p, cudaStream_t stream, const Extra&... extra) {
+    if (p.smem > 48 * 1024) {   // once per kernel and device: the largest dynamic shared memory any plan asks for
+        static bool attr_set[64] = {};
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
+        if (dev < 0 || dev >= 64 || !attr_set[dev] || p.smem > 200 * 1024) {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(p.smem, (size_t)200 * 1024));
+            if (e != cudaSuccess) return e;
+            if (dev >= 0 && dev < 64) attr_set[dev] = true;
+        }
     }
     if (p.occupancy_out) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(p.occupancy_out, kernel, p.threads, p.smem);
     cudaLaunchConfig_t cfg = {};
@@ -75,19 +84,19 @@ static cudaError_t launch_kernel_pdl(Kernel kernel, const GemvArgsB& a, const Ge
 template <class C>
 static cudaError_t launch_gemv_codec(const GemvArgsB& a, const GemvPlanB& p, cudaStream_t stream) {
     switch (p.passes) {
-        case -4: return launch_kernel_pdl(gemv1_bl_norm_kernel<C>, a, p, stream);
-        case -3: return launch_kernel_pdl(gemv1_bl_routed_kernel<C>, a, p, stream);
-        case -2: return launch_kernel_pdl(gemv1_bl_swiglu_kernel<C>, a, p, stream);
-        case -1: return p.multi ? launch_kernel_pdl(gemv1_bl_multi_kernel<C>, a, p, stream, *p.multi) : cudaErrorInvalidValue;
+        case -4: return launch_kernel_pdl<gemv1_bl_norm_kernel<C>>(a, p, stream);
+        case -3: return launch_kernel_pdl<gemv1_bl_routed_kernel<C>>(a, p, stream);
+        case -2: return launch_kernel_pdl<gemv1_bl_swiglu_kernel<C>>(a, p, stream);
+        case -1: return p.multi ? launch_kernel_pdl<gemv1_bl_multi_kernel<C>>(a, p, stream, *p.multi) : cudaErrorInvalidValue;
         case 0:
-            if (a.glu || a.reduce.world > 0 || !C::PLAIN_FORM) return launch_kernel_pdl(gemv1_bl_epi_kernel<C>, a, p, stream);
-            if (a.route_ids == nullptr && p.grid_y == 1 && p.grid == a.w.nrb && a.private_sums) return launch_kernel_pdl(gemv1_bl_one_kernel<C>, a, p, stream);
-            return launch_kernel_pdl(gemv1_bl_kernel<C>, a, p, stream);
-        case 1: return launch_kernel_pdl(gemvn_bl_kernel<C, 1>, a, p, stream);
-        case 2: return launch_kernel_pdl(gemvn_bl_kernel<C, 2>, a, p, stream);
-        case 4: return launch_kernel_pdl(gemvn_bl_kernel<C, 4>, a, p, stream);
-        case 108: return launch_kernel_pdl(gemvh_bl_kernel<C, 1>, a, p, stream);
-        case 116: return launch_kernel_pdl(gemvh_bl_kernel<C, 2>, a, p, stream);
+            if (a.glu || a.reduce.world > 0 || !C::PLAIN_FORM) return launch_kernel_pdl<gemv1_bl_epi_kernel<C>>(a, p, stream);
+            if (a.route_ids == nullptr && p.grid_y == 1 && p.grid == a.w.nrb && a.private_sums) return launch_kernel_pdl<gemv1_bl_one_kernel<C>>(a, p, stream);
+            return launch_kernel_pdl<gemv1_bl_kernel<C>>(a, p, stream);
+        case 1: return launch_kernel_pdl<gemvn_bl_kernel<C, 1>>(a, p, stream);
+        case 2: return launch_kernel_pdl<gemvn_bl_kernel<C, 2>>(a, p, stream);
+        case 4: return launch_kernel_pdl<gemvn_bl_kernel<C, 4>>(a, p, stream);
+        case 108: return launch_kernel_pdl<gemvh_bl_kernel<C, 1>>(a, p, stream);
+        case 116: return launch_kernel_pdl<gemvh_bl_kernel<C, 2>>(a, p, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -8,17 +8,22 @@ from __future__ import annotations
 
 import ctypes as C
 
-from . import _capi
+from . import _capi, _fast
 from ._capi import BF16, F32, WeightInfo, check, lib
+
+_mod = None   # torch, once something needed it
 
 
 def _torch():
-    import torch
-    return torch
+    global _mod
+    if _mod is None:
+        import torch
+        _mod = torch
+    return _mod
 
 
 def _stream_ptr(device_index: int) -> int:
-    return _torch().cuda.current_stream(device_index).cuda_stream
+    return _torch()._C._cuda_getCurrentRawStream(device_index)   # current_stream() builds a Stream object around it
 
 
 class QuantWeight:
@@ -30,6 +35,7 @@ class QuantWeight:
         check(lib.mfqb_weight_info_get(self._h, C.byref(info)))
         self.info = info
         self.n, self.k, self.device = info.n, info.k, info.device
+        self._ptr = handle.value
 
     @classmethod
     def from_blob(cls, dtype: str, blob, device: int = 0, *, axis: int = 0, begin: int = 0, end: int = -1):
@@ -66,6 +72,19 @@ class QuantWeight:
         existing [m, n] float32 or bfloat16 tensor to write (graph capture wants fixed buffers)."""
         torch = _torch()
         squeeze = x.dim() == 1
+        # the plain call (a new output for contiguous rows on the weight's device), without the general path's views
+        if out is None and not squeeze and x.dtype is torch.bfloat16 and x.get_device() == self.device and x.is_contiguous():
+            shape = x.shape
+            if len(shape) == 2 and shape[1] == self.k and self._ptr:
+                m = shape[0]
+                if out_dtype is None or out_dtype is torch.bfloat16:
+                    y, code = x.new_empty(m, self.n), BF16
+                else:
+                    y, code = x.new_empty((m, self.n), dtype=out_dtype), F32 if out_dtype is torch.float32 else BF16
+                status = _fast.mul_mat(self._ptr, x.data_ptr(), m, y.data_ptr(), code, torch._C._cuda_getCurrentRawStream(self.device))
+                if status:
+                    check(status)
+                return y
         x2 = x.reshape(1, -1) if squeeze else x
         if x2.dtype != torch.bfloat16 or not x2.is_cuda or x2.device.index != self.device:
             raise ValueError(f"x must be a bfloat16 tensor on cuda:{self.device}")
@@ -149,6 +168,7 @@ class QuantWeight:
         if self._h:
             lib.mfqb_weight_free(self._h)
             self._h = C.c_void_p()
+            self._ptr = None
 
     def __del__(self):
         try:

@@ -7,19 +7,15 @@ from __future__ import annotations
 
 import ctypes as C
 
-from . import _capi
+from . import _capi, _fast
 from ._capi import BF16, F32, MoeInfo, check, lib
+from .linear import _torch
 
 SOFTMAX, SIGMOID, SQRT_SOFTPLUS, DELAYED_SOFTMAX = 0, 1, 2, 3
 
 
-def _torch():
-    import torch
-    return torch
-
-
 def _stream(t) -> int:
-    return _torch().cuda.current_stream(t.device.index).cuda_stream
+    return _torch()._C._cuda_getCurrentRawStream(t.get_device())
 
 
 def moe_topk(logits, k: int, mode: int = DELAYED_SOFTMAX, bias=None, normalize: bool = False, norm_floor: float = 0.0,
@@ -30,12 +26,16 @@ def moe_topk(logits, k: int, mode: int = DELAYED_SOFTMAX, bias=None, normalize: 
     if z.dtype != torch.float32 or not z.is_cuda or z.dim() != 2:
         raise ValueError("logits must be a float32 CUDA tensor [tokens, experts]")
     t, e = z.shape
-    ids = torch.empty((t, k), dtype=torch.int32, device=z.device)
-    w = torch.empty((t, k), dtype=torch.float32, device=z.device)
+    ids = z.new_empty((t, k), dtype=torch.int32)
+    w = z.new_empty(t, k)
     b = None if bias is None else bias.contiguous().float()
-    with torch.cuda.device(z.device):
-        check(lib.mfqb_moe_topk(z.data_ptr(), t, e, k, mode, None if b is None else b.data_ptr(), int(normalize),
-                                norm_floor, scale, ids.data_ptr(), w.data_ptr(), _stream(z)))
+    dev = z.get_device()
+    args = (z.data_ptr(), t, e, k, mode, None if b is None else b.data_ptr(), int(normalize), norm_floor, scale, ids.data_ptr(), w.data_ptr(), _stream(z))
+    if torch._C._cuda_getDevice() == dev:
+        check(_fast.moe_topk(*args))
+    else:
+        with torch.cuda.device(dev):
+            check(_fast.moe_topk(*args))
     return ids, w
 
 
@@ -132,7 +132,7 @@ def moe_ffn(gate_up: MoeWeight, down: MoeWeight, x, ids, weights, out_dtype=None
     weights = weights.contiguous()
     t, r = ids.shape
     tdt = out_dtype or torch.float32
-    y = torch.empty((t, down.info.out_per_expert), dtype=tdt, device=x.device)
-    check(lib.mfqb_moe_ffn(gate_up._h, down._h, x.data_ptr(), ids.data_ptr(), weights.data_ptr(), t, r, y.data_ptr(),
-                           F32 if tdt == torch.float32 else BF16, _stream(x)))
+    y = x.new_empty((t, down.info.out_per_expert), dtype=tdt)
+    check(_fast.moe_ffn(gate_up._h.value, down._h.value, x.data_ptr(), ids.data_ptr(), weights.data_ptr(), t, r, y.data_ptr(),
+                        F32 if tdt == torch.float32 else BF16, _stream(x)))
     return y
