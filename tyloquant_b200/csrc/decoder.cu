@@ -135,23 +135,38 @@ __device__ __forceinline__ uint4 pack_bf16x8(const float* f) {
     return make_uint4(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&b), *reinterpret_cast<const uint32_t*>(&c),
                       *reinterpret_cast<const uint32_t*>(&d));
 }
-__device__ __forceinline__ void bf16x8_to_f32(const uint4& r, float* f) {
-    f[0] = __uint_as_float(r.x << 16); f[1] = __uint_as_float(r.x & 0xFFFF0000u);
-    f[2] = __uint_as_float(r.y << 16); f[3] = __uint_as_float(r.y & 0xFFFF0000u);
-    f[4] = __uint_as_float(r.z << 16); f[5] = __uint_as_float(r.z & 0xFFFF0000u);
-    f[6] = __uint_as_float(r.w << 16); f[7] = __uint_as_float(r.w & 0xFFFF0000u);
-}
-
 constexpr int kMaxSplits = 64;
-constexpr int kAttnStages = 3;   // rounds of 32 tokens in flight per CTA
-// Dynamic shared memory of the attention kernel: the K/V ring (stages x 4 tokens x (K, V) x 128 threads x 16 bytes),
-// reused afterwards for the eight half-warps' results ([8][G][128] + 2 x [8][G] floats).
-constexpr size_t attn_smem_bytes(int g) {
-    const size_t ring = (size_t)kAttnStages * 4 * 2 * 128 * 16, meet = (size_t)8 * g * (kHeadDim + 2) * 4;
-    return ring > meet ? ring : meet;
+constexpr int kAttnWarps = 4, kAttnStages = 3;   // rounds of 16 tokens in flight per warp
+constexpr int kAttnStageBytes = 2 * 16 * kHeadDim * 2;   // K and V of 16 tokens
+// Dynamic shared memory of the attention kernel: the warps' K/V rings (reused afterwards for their results), the rotated queries.
+constexpr size_t attn_smem_bytes(int g) { return (size_t)kAttnWarps * kAttnStages * kAttnStageBytes + (size_t)g * kHeadDim * 4; }
+__device__ __forceinline__ void cp_async16_zfill(uint32_t smem_dst, const void* gsrc, bool valid) {   // zeros where not valid
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_dst), "l"(gsrc), "r"(valid ? 16 : 0) : "memory");
 }
-__device__ __forceinline__ void cp_async16_attn(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem_dst)), "l"(gsrc) : "memory");
+__device__ __forceinline__ void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ex2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// A pair of float32 values as three bf16 pairs whose sum carries 24 bits: t[0] + t[1] + t[2].
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&t)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
+        t[i] = *reinterpret_cast<const uint32_t*>(&h);
+        x -= __low2float(h);
+        y -= __high2float(h);
+    }
 }
 constexpr int kPartStride = kHeadDim + 4;   // a split's record per head: 128 output values | max | sum | pad (528 bytes)
 
@@ -160,165 +175,197 @@ constexpr int kPartStride = kHeadDim + 4;   // a split's record per head: 128 ou
 // the caches are [rows][nkv][max_ctx][128] bf16 for K and for V.
 //
 // CTA (split, kv head, row) scans its slice of the context for the G = nq / nkv query heads that share
-// the KV head.  Every CTA rotates those heads' queries itself (pre-scaled by 1/sqrt(128)); the CTA
-// whose slice holds the new position rotates the new key, rounds key and value to bf16 and writes
-// them into the caches before it scans (no other CTA reads that position in this step).  A
-// half-warp holds one token (16 lanes x 8 dimensions = one 16-byte load per lane for K and for V);
-// the CTA's eight half-warps take four tokens each per round of 32, eight 16-byte loads per lane in
-// flight, the first round requested before the queries are rotated.  Scores are reduced inside the
-// half-warp, the soft-max runs online per half-warp and head.  Each CTA leaves (unnormalised
-// output[128], max, sum) per head in `part`; the last CTA of a (row, kv head) to arrive -- a counter
-// per pair, left at zero -- merges the splits, a warp per head, and writes the bf16 attention output.
+// the KV head; the CTA whose slice holds the new position rotates the new key, rounds key and value to bf16 and writes
+// them into the caches before it scans (no other CTA reads that position in this step).
+//
+// The scan is bound by the cache bytes as long as the arithmetic stays off the float pipes: with a half-warp per token and
+// scalar products it took 30 instructions per 16 bytes (84 us for 16 sequences at a 4096-token context, 3.2 TB/s).  Here a
+// warp takes 16 tokens at a time through a private ring of asynchronous copies and multiplies on mma.m16n8k16: scores
+// S^T = Q K^T with the query heads in the rows, then O += P V with the scores' accumulators as they are for the A operand.
+// The caches are bf16; the float32 queries and probabilities enter as three bf16 terms each (exact to 24 bits), which are the
+// spare rows of the 16-row operand: rows 0-3 first terms of up to four heads, 4-7 second, 8-11 third.  Eight heads take a
+// second A operand for the third terms.
 template <int G>
-__global__ void __launch_bounds__(128, G <= 4 ? 4 : 2) attn_decode_kernel(const float* __restrict__ qkv, __nv_bfloat16* kcache, __nv_bfloat16* vcache,
+__global__ void __launch_bounds__(32 * kAttnWarps, 2) attn_decode_kernel(const float* __restrict__ qkv, __nv_bfloat16* kcache, __nv_bfloat16* vcache,
                                                              const int* __restrict__ pos, float* part, unsigned* counters,
                                                              __nv_bfloat16* __restrict__ out, int nq, int nkv, int max_ctx, int nsplit,
                                                              const float2* __restrict__ rope_table) {
+    constexpr int SETS = G > 4 ? 2 : 1;
     dep_wait();
+    extern __shared__ __align__(128) unsigned char attn_smem[];
     const int split = blockIdx.x, kvh = blockIdx.y, row = blockIdx.z;
-    const int lane = threadIdx.x & 31, l16 = lane & 15, slot = threadIdx.x >> 4;   // slot: half-warp 0..7 of the CTA
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane >> 2, c = lane & 3, l16 = lane & 15;
     const int p = pos[row], len = p + 1;   // the token written by this step takes part
     const int per = (len + nsplit - 1) / nsplit;
     const int t0 = split * per, t1 = min(len, t0 + per);
     const float* qkv_row = qkv + (size_t)row * (nq + 2 * nkv) * kHeadDim;
     const float2* tab = rope_table + (size_t)row * 64;
-    __nv_bfloat16* kb = kcache + ((size_t)row * nkv + kvh) * max_ctx * kHeadDim + 8 * l16;
-    __nv_bfloat16* vb = vcache + ((size_t)row * nkv + kvh) * max_ctx * kHeadDim + 8 * l16;
+    __nv_bfloat16* kb = kcache + ((size_t)row * nkv + kvh) * max_ctx * kHeadDim;
+    __nv_bfloat16* vb = vcache + ((size_t)row * nkv + kvh) * max_ctx * kHeadDim;
     if (t0 <= p && p < t1) {   // this CTA's slice holds the new position (uniform over the CTA)
-        if (threadIdx.x < 32) {   // warp 0 writes the new key and value
+        if (warp == 0) {       // warp 0 writes the new key and value
             float f[8];
             if (lane < 16) {
                 rope8(qkv_row + (size_t)(nq + kvh) * kHeadDim, tab, l16, 1.0f, f);
-                *reinterpret_cast<uint4*>(kb + (size_t)p * kHeadDim) = pack_bf16x8(f);
+                *reinterpret_cast<uint4*>(kb + (size_t)p * kHeadDim + 8 * l16) = pack_bf16x8(f);
             } else {
                 const float* src = qkv_row + (size_t)(nq + nkv + kvh) * kHeadDim + 8 * l16;
                 const float4 a = *reinterpret_cast<const float4*>(src), b = *reinterpret_cast<const float4*>(src + 4);
                 f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-                *reinterpret_cast<uint4*>(vb + (size_t)p * kHeadDim) = pack_bf16x8(f);
+                *reinterpret_cast<uint4*>(vb + (size_t)p * kHeadDim + 8 * l16) = pack_bf16x8(f);
             }
         }
         __syncthreads();   // visible to the whole CTA before anyone reads that position
     }
-    // A half-warp takes four tokens per round (slot, slot + 8, + 16, + 24 of a 32-token round).  Every lane copies
-    // the 16 bytes of K and of V it will use itself into its own slots of a ring in shared memory, kAttnStages
-    // rounds deep (asynchronous copies, no registers held, no synchronisation: a lane only reads what it copied),
-    // so the loads of the next rounds are in flight while a round is used.
-    constexpr int TPR = 4;
-    extern __shared__ __align__(16) unsigned char attn_smem[];
-    uint4* ring = reinterpret_cast<uint4*>(attn_smem);   // [stage][token of the round][K, V][thread]
-    auto slot_of = [&](int stage, int i, int kv) { return ring + ((stage * TPR + i) * 2 + kv) * 128 + threadIdx.x; };
-    auto request = [&](int base, int stage) {   // one copy group per round, empty past the end of the slice
+    // Ring of this warp: per stage 16 rows of K, then 16 rows of V, 256 bytes each, 16-byte pieces XORed with the row number.
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(attn_smem) + (uint32_t)(warp * kAttnStages * kAttnStageBytes);
+    auto request = [&](int base, int stage) {   // one copy group per round; zeros past the end of the slice
+        const uint32_t dst = ring + (uint32_t)(stage * kAttnStageBytes);
+        const int t = base + 16 * warp + (lane >> 4);
 #pragma unroll
-        for (int i = 0; i < TPR; ++i) {
-            const int t = base + slot + 8 * i;
-            if (t < t1) {
-                cp_async16_attn(slot_of(stage, i, 0), kb + (size_t)t * kHeadDim);
-                cp_async16_attn(slot_of(stage, i, 1), vb + (size_t)t * kHeadDim);
-            }
+        for (int i = 0; i < 8; ++i) {
+            const int r = 2 * i + (lane >> 4);
+            const bool in = t + 2 * i < t1;
+            const size_t off = in ? (size_t)(t + 2 * i) * kHeadDim + 8 * l16 : 0;
+            const uint32_t at = dst + (uint32_t)(r * 256 + ((l16 ^ (r & 7)) << 4));
+            cp_async16_zfill(at, kb + off, in);
+            cp_async16_zfill(at + 4096u, vb + off, in);
         }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 #pragma unroll
-    for (int sidx = 0; sidx < kAttnStages - 1; ++sidx) request(t0 + sidx * 8 * TPR, sidx);
-    float qv[G][8];
-    if (t0 < t1) {
-#pragma unroll
-        for (int g = 0; g < G; ++g) rope8(qkv_row + (size_t)(kvh * G + g) * kHeadDim, tab, l16, 0.08838834764831845f /* 1/sqrt(128) */, qv[g]);
+    for (int i = 0; i < kAttnStages - 1; ++i) request(t0 + i * 16 * kAttnWarps, i);
+    // the group's queries, rotated and scaled to log2 units by 1 / sqrt(128) * log2(e)
+    float* qs = reinterpret_cast<float*>(attn_smem + (size_t)kAttnWarps * kAttnStages * kAttnStageBytes);
+    for (int i = tid; i < G * 16; i += 32 * kAttnWarps) {
+        float f[8];
+        rope8(qkv_row + (size_t)(kvh * G + (i >> 4)) * kHeadDim, tab, i & 15, 0.08838834764831845f * 1.4426950408889634f, f);
+        float4* dst = reinterpret_cast<float4*>(qs + (i >> 4) * kHeadDim + 8 * (i & 15));
+        dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+        dst[1] = make_float4(f[4], f[5], f[6], f[7]);
     }
-    float m[G], l[G], acc[G][8];
+    __syncthreads();
+    // this lane's rows q and q + 8 of the A operands hold terms of head `h`
+    const int h = G > 4 ? q : (q & 3);
+    const bool live = h < G;
+    auto rows_of = [&](const uint32_t (&t)[3], int set, uint32_t& lo, uint32_t& hi) {   // A registers of rows q and q + 8
+        if (G > 4) {
+            lo = set ? t[2] : t[0];
+            hi = set ? 0u : t[1];
+        } else {
+            lo = q < 4 ? t[0] : t[1];
+            hi = q < 4 ? t[2] : 0u;
+        }
+    };
+    uint32_t qa[SETS][8][4];
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        m[g] = -INFINITY;
-        l[g] = 0.f;
+    for (int kk = 0; kk < 8; ++kk)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) acc[g][i] = 0.f;
-    }
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+        for (int half = 0; half < 2; ++half) {
+            const float2 v = live ? *reinterpret_cast<const float2*>(qs + h * kHeadDim + 16 * kk + 8 * half + 2 * c) : make_float2(0.f, 0.f);
+            uint32_t t[3];
+            split3(v.x, v.y, t);
+#pragma unroll
+            for (int st = 0; st < SETS; ++st) rows_of(t, st, qa[st][kk][2 * half], qa[st][kk][2 * half + 1]);
+        }
+    float acc[16][4];   // O: rows q, q + 8 x dimensions 8j + 2c, + 1
+#pragma unroll
+    for (int j = 0; j < 16; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    float m = -INFINITY, l = 0.f;   // of head h; l over this lane's tokens
+    const int kt = (lane >> 4) * 8 + (lane & 7), kc = (lane >> 3) & 1;   // row and piece this lane addresses for K, for V
+    const int vt = ((lane >> 3) & 1) * 8 + (lane & 7), vc = lane >> 4;
     int stage = 0, req_stage = kAttnStages - 1;
-    for (int base = t0; base < t1; base += 8 * TPR) {   // uniform trip count over the CTA: the shuffles below need whole warps
-        request(base + (kAttnStages - 1) * 8 * TPR, req_stage);   // the slot read in the previous iteration
+    for (int base = t0; base < t1; base += 16 * kAttnWarps) {
+        request(base + (kAttnStages - 1) * 16 * kAttnWarps, req_stage);   // the stage read in the previous iteration
         asm volatile("cp.async.wait_group %0;\n" ::"n"(kAttnStages - 1) : "memory");
-        float sc[TPR][G];
+        __syncwarp();
+        const int tw = base + 16 * warp;
+        if (tw < t1) {
+            const uint32_t ks = ring + (uint32_t)(stage * kAttnStageBytes), vs = ks + 4096u;
+            float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};   // tokens 0-7, 8-15
 #pragma unroll
-        for (int i = 0; i < TPR; ++i) {
-            float kf[8];
-            const uint4 ck = base + slot + 8 * i < t1 ? *slot_of(stage, i, 0) : zero;
-            bf16x8_to_f32(ck, kf);
+            for (int kk = 0; kk < 8; ++kk) {
+                uint32_t kf[4];
+                ldsm_x4(ks + (uint32_t)(kt * 256 + (((2 * kk + kc) ^ (kt & 7)) << 4)), kf);
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                float x = 0.f;
+                for (int st = 0; st < SETS; ++st) {
+                    mma_bf16(sc[0], qa[st][kk], kf[0], kf[1]);
+                    mma_bf16(sc[1], qa[st][kk], kf[2], kf[3]);
+                }
+            }
+            float sv[4];   // scores of head h for tokens 2c, 2c + 1, 2c + 8, 2c + 9: the terms' rows added up
 #pragma unroll
-                for (int d = 0; d < 8; ++d) x += qv[g][d] * kf[d];
-                sc[i][g] = x;
+            for (int i = 0; i < 4; ++i) {
+                float v = sc[i >> 1][i & 1] + sc[i >> 1][(i & 1) + 2];
+                if (G <= 4) v += __shfl_xor_sync(0xffffffffu, v, 16);
+                sv[i] = tw + 8 * (i >> 1) + 2 * c + (i & 1) < t1 ? v : -INFINITY;
+            }
+            float mn = fmaxf(m, fmaxf(fmaxf(sv[0], sv[1]), fmaxf(sv[2], sv[3])));
+            mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 1));
+            mn = fmaxf(mn, __shfl_xor_sync(0xffffffffu, mn, 2));
+            if (__any_sync(0xffffffffu, mn > m)) {
+                const float corr = ex2(m - mn);
+                l *= corr;
+#pragma unroll
+                for (int j = 0; j < 16; ++j) { acc[j][0] *= corr; acc[j][1] *= corr; acc[j][2] *= corr; acc[j][3] *= corr; }
+                m = mn;
+            }
+            float pr[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { pr[i] = ex2(sv[i] - m); l += pr[i]; }
+            uint32_t pa[SETS][4];
+#pragma unroll
+            for (int half = 0; half < 2; ++half) {
+                uint32_t t[3];
+                split3(pr[2 * half], pr[2 * half + 1], t);
+#pragma unroll
+                for (int st = 0; st < SETS; ++st) rows_of(t, st, pa[st][2 * half], pa[st][2 * half + 1]);
+            }
+#pragma unroll
+            for (int jj = 0; jj < 8; ++jj) {
+                uint32_t vf[4];
+                ldsm_x4_trans(vs + (uint32_t)(vt * 256 + (((2 * jj + vc) ^ (vt & 7)) << 4)), vf);
+#pragma unroll
+                for (int st = 0; st < SETS; ++st) {
+                    mma_bf16(acc[2 * jj], pa[st], vf[0], vf[1]);
+                    mma_bf16(acc[2 * jj + 1], pa[st], vf[2], vf[3]);
+                }
             }
         }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1)
-#pragma unroll
-            for (int i = 0; i < TPR; ++i)
-#pragma unroll
-                for (int g = 0; g < G; ++g) sc[i][g] += __shfl_xor_sync(0xffffffffu, sc[i][g], o);
-        if (base + slot < t1) {   // uniform over the half-warp; a later token of the round is valid only if the earlier ones are
-            float pr[TPR][G];
-#pragma unroll
-            for (int g = 0; g < G; ++g) {
-                float mn = m[g];
-#pragma unroll
-                for (int i = 0; i < TPR; ++i) {
-                    if (base + slot + 8 * i >= t1) sc[i][g] = -INFINITY;
-                    mn = fmaxf(mn, sc[i][g]);
-                }
-                const float corr = __expf(m[g] - mn);
-                float ps = 0.f;
-#pragma unroll
-                for (int i = 0; i < TPR; ++i) {
-                    pr[i][g] = __expf(sc[i][g] - mn);
-                    ps += pr[i][g];
-                }
-                l[g] = l[g] * corr + ps;
-#pragma unroll
-                for (int d = 0; d < 8; ++d) acc[g][d] *= corr;
-                m[g] = mn;
-            }
-#pragma unroll
-            for (int i = 0; i < TPR; ++i) {
-                float vf[8];
-                const uint4 cv = base + slot + 8 * i < t1 ? *slot_of(stage, i, 1) : zero;
-                bf16x8_to_f32(cv, vf);
-#pragma unroll
-                for (int g = 0; g < G; ++g)
-#pragma unroll
-                    for (int d = 0; d < 8; ++d) acc[g][d] += pr[i][g] * vf[d];
-            }
-        }
+        __syncwarp();   // every lane has read the stage before it is refilled
         if (++stage == kAttnStages) stage = 0;
         if (++req_stage == kAttnStages) req_stage = 0;
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    __syncthreads();   // the ring is done with: its memory now holds the half-warps' results
-    // the eight half-warps of the CTA meet in shared memory
-    float(*sm_acc)[G][kHeadDim] = reinterpret_cast<float(*)[G][kHeadDim]>(attn_smem);                       // [8][G][128]
-    float(*sm_m)[G] = reinterpret_cast<float(*)[G]>(attn_smem + (size_t)8 * G * kHeadDim * 4);              // [8][G]
-    float(*sm_l)[G] = reinterpret_cast<float(*)[G]>(attn_smem + (size_t)8 * G * kHeadDim * 4 + 8 * G * 4);  // [8][G]
+    __syncthreads();   // the rings are done with: their memory now holds the warps' results
+    float(*sm_acc)[G][kHeadDim] = reinterpret_cast<float(*)[G][kHeadDim]>(attn_smem);                                // [warps][G][128]
+    float(*sm_m)[G] = reinterpret_cast<float(*)[G]>(attn_smem + (size_t)kAttnWarps * G * kHeadDim * 4);              // [warps][G]
+    float(*sm_l)[G] = reinterpret_cast<float(*)[G]>(attn_smem + (size_t)kAttnWarps * G * (kHeadDim + 1) * 4);        // [warps][G]
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    const bool owner = q < G && (G > 4 || q < 4);
+    if (owner && c == 0) { sm_m[warp][h] = m; sm_l[warp][h] = l; }
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        if (l16 == 0) { sm_m[slot][g] = m[g]; sm_l[slot][g] = l[g]; }
-        float4* dst = reinterpret_cast<float4*>(&sm_acc[slot][g][8 * l16]);
-        dst[0] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
-        dst[1] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
+    for (int j = 0; j < 16; ++j) {
+        float x = acc[j][0] + acc[j][2], y = acc[j][1] + acc[j][3];   // the terms' rows
+        if (G <= 4) {
+            x += __shfl_xor_sync(0xffffffffu, x, 16);
+            y += __shfl_xor_sync(0xffffffffu, y, 16);
+        }
+        if (owner) *reinterpret_cast<float2*>(&sm_acc[warp][h][8 * j + 2 * c]) = make_float2(x, y);
     }
     __syncthreads();
-    for (int idx = threadIdx.x; idx < G * kHeadDim; idx += blockDim.x) {
+    for (int idx = tid; idx < G * kHeadDim; idx += 32 * kAttnWarps) {
         const int g = idx / kHeadDim, d = idx % kHeadDim;
         float mm = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) mm = fmaxf(mm, sm_m[w][g]);
+        for (int w = 0; w < kAttnWarps; ++w) mm = fmaxf(mm, sm_m[w][g]);
         float ll = 0.f, aa = 0.f;
 #pragma unroll
-        for (int w = 0; w < 8; ++w) {
-            const float c = sm_m[w][g] == -INFINITY ? 0.f : __expf(sm_m[w][g] - mm);
-            ll += sm_l[w][g] * c;
-            aa += sm_acc[w][g][d] * c;
+        for (int w = 0; w < kAttnWarps; ++w) {
+            const float cw = sm_m[w][g] == -INFINITY ? 0.f : ex2(sm_m[w][g] - mm);
+            ll += sm_l[w][g] * cw;
+            aa += sm_acc[w][g][d] * cw;
         }
         float* dst = part + (((size_t)row * nq + kvh * G + g) * nsplit + split) * kPartStride;
         dst[d] = aa;
@@ -340,7 +387,7 @@ __global__ void __launch_bounds__(128, G <= 4 ? 4 : 2) attn_decode_kernel(const 
         const float2 ml1 = h1 ? __ldcg(reinterpret_cast<const float2*>(src + (size_t)(lane + 32) * kPartStride + kHeadDim)) : make_float2(-INFINITY, 0.f);
         float mm = fmaxf(ml0.x, ml1.x);
         for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
-        const float c0 = ml0.x == -INFINITY ? 0.f : __expf(ml0.x - mm), c1 = ml1.x == -INFINITY ? 0.f : __expf(ml1.x - mm);
+        const float c0 = ml0.x == -INFINITY ? 0.f : ex2(ml0.x - mm), c1 = ml1.x == -INFINITY ? 0.f : ex2(ml1.x - mm);
         float ll = ml0.y * c0 + ml1.y * c1;
         for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
         float4 aa = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -473,13 +520,17 @@ struct mfqb_decoder {
     DevBuf h, h2, xn, qkv, attn, attn_count, inv_freq, rope_table, proj, proj_sum, act, logits, part, best_val, best_idx, part_val, part_idx, gathered, gathered_sum, pos;
 };
 
-// Context splits of the decode attention: as many CTAs as are resident at once (one wave: the merge
-// by the last CTA of a head group then follows the scan directly), but at least so many that a CTA
-// scans no more than 256 positions of a long context.
+// Context splits of the decode attention.  A CTA costs about as much as 96 tokens of its scan before and after it (queries,
+// first copies, merge); the split count with the shortest schedule, in tokens of the longest sequence of CTAs on a slot.
 static int attn_splits(const mfqb_decoder* d, int rows, int ctx_bound) {
-    const int one_wave = d->attn_per_sm * d->sms / (d->nkv * rows);
-    const int by_length = (ctx_bound + 255) / 256;
-    return std::max(1, std::min(kMaxSplits, std::max(one_wave, by_length)));
+    const long long slots = (long long)d->attn_per_sm * d->sms, groups = (long long)d->nkv * rows;
+    int best = 1;
+    long long best_cost = -1;
+    for (int n = 1; n <= kMaxSplits; ++n) {
+        const long long waves = (groups * n + slots - 1) / slots, cost = waves * ((ctx_bound + n - 1) / n + 96);
+        if (best_cost < 0 || cost < best_cost) { best = n; best_cost = cost; }
+    }
+    return best;
 }
 
 // The step's rotation table (cos, sin per sequence and pair), before the first block that uses it.
@@ -535,7 +586,7 @@ static const float* layer_forward(mfqb_decoder* d, int li, int rows, const float
     const int nsplit = attn_splits(d, rows, d->cfg.max_ctx);
     const dim3 agrid(nsplit, d->nkv, rows);
     auto attn = [&](auto kernel) {
-        launch_dep_smem(kernel, agrid, dim3(128), attn_smem_bytes(G), s, static_cast<const float*>(d->qkv.p), static_cast<__nv_bfloat16*>(L.kcache.p),
+        launch_dep_smem(kernel, agrid, dim3(32 * kAttnWarps), attn_smem_bytes(G), s, static_cast<const float*>(d->qkv.p), static_cast<__nv_bfloat16*>(L.kcache.p),
                    static_cast<__nv_bfloat16*>(L.vcache.p), static_cast<const int*>(d->pos.p), static_cast<float*>(d->part.p),
                    static_cast<unsigned*>(d->attn_count.p), static_cast<__nv_bfloat16*>(d->attn.p), d->nq, d->nkv, d->cfg.max_ctx, nsplit,
                    static_cast<const float2*>(d->rope_table.p));
@@ -633,19 +684,19 @@ int mfqb_decoder_create(const mfqb_decoder_config* cfg, int rank, int world, mfq
             switch (cfg->n_q_heads / cfg->n_kv_heads) {
                 case 1:
                     MFQB_CUDA(cudaFuncSetAttribute(attn_decode_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem_bytes(1)));
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<1>, 128, attn_smem_bytes(1));
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<1>, 32 * kAttnWarps, attn_smem_bytes(1));
                     break;
                 case 2:
                     MFQB_CUDA(cudaFuncSetAttribute(attn_decode_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem_bytes(2)));
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<2>, 128, attn_smem_bytes(2));
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<2>, 32 * kAttnWarps, attn_smem_bytes(2));
                     break;
                 case 4:
                     MFQB_CUDA(cudaFuncSetAttribute(attn_decode_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem_bytes(4)));
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<4>, 128, attn_smem_bytes(4));
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<4>, 32 * kAttnWarps, attn_smem_bytes(4));
                     break;
                 case 8:
                     MFQB_CUDA(cudaFuncSetAttribute(attn_decode_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_smem_bytes(8)));
-                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<8>, 128, attn_smem_bytes(8));
+                    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attn_decode_kernel<8>, 32 * kAttnWarps, attn_smem_bytes(8));
                     break;
                 default: fail(MFQB_ERR_UNSUPPORTED, "query heads per KV head must be 1, 2, 4 or 8, got %d", cfg->n_q_heads / cfg->n_kv_heads);
             }

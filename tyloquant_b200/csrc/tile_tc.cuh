@@ -418,7 +418,7 @@ __device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, Ti
 
 // Sets::dispatch(w, f) calls f(Codec{}) for the codec of a cohort; Sets::ctx describes the codec context (lattice tables).
 template <class Sets>
-__global__ void __launch_bounds__(kTileThreads, 1) tile_tc_kernel(const __grid_constant__ TileArgs a) {
+__global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ TileShared sh;
     unsigned char* x_ring = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
