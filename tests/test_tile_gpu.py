@@ -75,3 +75,20 @@ def test_shared_tiles_are_left_clean():
         y_ref = x.double() @ ref.double().T
         assert ((w.matmul(x, out_dtype=torch.float32).double() - y_ref).norm() / y_ref.norm()).item() <= REL_L2, i
     assert _status() == 0
+
+
+@pytest.mark.parametrize("n,k", [(32, 24), (160, 1000), (4128, 2600)])
+def test_gated_epilogue(n, k):
+    """Whole and shared tiles, the last row tile short of 128 rows."""
+    blob = encode.random_nint_blob(n, k, 6, 24, 7, seed=n, device="cuda")
+    w = QuantWeight.from_blob("NINT6", blob)
+    ref = torch.from_numpy(O.dequant_nint(O.unpack_nint(blob))).cuda().double().reshape(n // 32, 2, 16, k)
+    gen = torch.Generator("cuda").manual_seed(2)
+    for m in (5, 16, 17, 130, 300):
+        x = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+        g, u = (torch.einsum("mk,brk->mbr", x.double(), ref[:, i]).reshape(m, -1) for i in range(2))
+        want = u * g / (1 + torch.exp(-g))
+        for dtype, bound in ((torch.float32, 2 * REL_L2), (torch.bfloat16, 4e-3)):
+            got = w.matmul_glu(x, out_dtype=dtype).double()
+            assert ((got - want).norm() / want.norm()).item() <= bound, (n, m, dtype)
+    assert _status() == 0

@@ -21,8 +21,11 @@
 #include <cmath>
 
 #include "cuda_util.h"
+#include "tile_tc.h"
 
 namespace mfqb {
+
+const NintDevB& weight_device_layout(const mfqb_weight* w);
 
 constexpr int kHeadDim = 128;
 
@@ -477,12 +480,22 @@ __global__ void embed_rows_kernel(const int* __restrict__ ids, const __nv_bfloat
 }
 
 // Seeded synthetic cache contents (a stand-in for the prefill pass): values of unit scale.
-__global__ void fill_cache_kernel(__nv_bfloat16* __restrict__ p, size_t n, unsigned seed) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        unsigned x = (unsigned)i * 2654435761u ^ seed ^ (unsigned)(i >> 32) * 40503u;
-        x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-        p[i] = __float2bfloat16_rn(((float)(x & 0xFFFF) - 32768.f) * (1.f / 18918.f));   // uniform, unit variance
+__global__ void fill_cache_kernel(uint4* __restrict__ p, size_t n8, unsigned seed) {   // eight values a thread and turn
+    for (size_t i8 = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i8 < n8; i8 += (size_t)gridDim.x * blockDim.x) {
+        float f[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const size_t i = 8 * i8 + j;
+            unsigned x = (unsigned)i * 2654435761u ^ seed ^ (unsigned)(i >> 32) * 40503u;
+            x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
+            f[j] = ((float)(x & 0xFFFF) - 32768.f) * (1.f / 18918.f);   // uniform, unit variance
+        }
+        p[i8] = pack_bf16x8(f);
     }
+}
+__global__ void fill_pos_kernel(int* p, int n, int v) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) p[i] = v;
 }
 __global__ void fill_f32_kernel(float* p, size_t n, float v) {
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
@@ -557,6 +570,14 @@ static const float* rank_sum(mfqb_decoder* d, const float* in, float* out, size_
     return out;
 }
 
+// Batched steps: residual add, RMSNorm and product with the normalised row going straight into the tile kernel's activation
+// layout.  False when this weight or batch has no tile kernel: the caller normalises, then multiplies.
+static bool norm_mul_mat(mfqb_decoder* d, const mfqb_weight* w, const float* delta, const void* gamma, int rows, void* y, int y_dtype, bool glu, cudaStream_t s) {
+    if (rows < 5) return false;
+    const TileNorm norm{static_cast<float*>(d->h.p), delta, static_cast<const float*>(gamma), d->cfg.rms_eps};
+    return launch_tile_product(weight_device_layout(w), nullptr, rows, y, y_dtype, d->device, s, glu, &norm);
+}
+
 static void mul_mat(const mfqb_weight* w, const void* x, int m, void* y, cudaStream_t s) {
     const int rc = mfqb_mul_mat(w, x, m, y, MFQB_F32, s);
     if (rc != MFQB_OK) throw Error(rc, mfqb_last_error());
@@ -578,7 +599,7 @@ static const float* layer_forward(mfqb_decoder* d, int li, int rows, const float
         if (rc == MFQB_ERR_UNSUPPORTED) d->fused_norm = fused = false;   // weights this form does not take: the two-kernel form from here on
         else if (rc != MFQB_OK) throw Error(rc, mfqb_last_error());
     }
-    if (!fused) {
+    if (!fused && !norm_mul_mat(d, L.qkv, delta, L.gamma_attn.p, rows, d->qkv.p, MFQB_F32, false, s)) {
         launch_dep(add_rmsnorm_kernel, dim3(rows), dim3(1024), s, static_cast<float*>(d->h.p), delta, static_cast<const float*>(L.gamma_attn.p),
                    static_cast<__nv_bfloat16*>(d->xn.p), H, d->cfg.rms_eps);
         mul_mat(L.qkv, d->xn.p, rows, d->qkv.p, s);
@@ -613,7 +634,7 @@ static const float* layer_forward(mfqb_decoder* d, int li, int rows, const float
         const int rc = mfqb_mul_mat_rmsnorm(L.gate_up, static_cast<const float*>(d->h2.p), o_out, static_cast<const float*>(L.gamma_ffn.p), d->cfg.rms_eps,
                                             static_cast<float*>(d->h.p), d->act.p, MFQB_BF16, 1, s);
         if (rc != MFQB_OK) throw Error(rc, mfqb_last_error());
-    } else {
+    } else if (!norm_mul_mat(d, L.gate_up, o_out, L.gamma_ffn.p, rows, d->act.p, MFQB_BF16, true, s)) {
         launch_dep(add_rmsnorm_kernel, dim3(rows), dim3(1024), s, static_cast<float*>(d->h.p), o_out, static_cast<const float*>(L.gamma_ffn.p),
                    static_cast<__nv_bfloat16*>(d->xn.p), H, d->cfg.rms_eps);
         const int rc = mfqb_mul_mat_glu(L.gate_up, d->xn.p, rows, d->act.p, MFQB_BF16, s);
@@ -765,13 +786,13 @@ int mfqb_decoder_fill_cache(mfqb_decoder* d, int ctx_len, unsigned seed, mfqb_st
         DeviceGuard guard(d->device);
         unsigned s = seed;
         for (auto& L : d->layers) {
-            const size_t n = L.kcache.bytes / 2;
-            fill_cache_kernel<<<1024, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(L.kcache.p), n, s++);
-            fill_cache_kernel<<<1024, 256, 0, stream>>>(static_cast<__nv_bfloat16*>(L.vcache.p), n, s++);
+            const size_t n8 = L.kcache.bytes / 16;   // rows are 128 values
+            const unsigned grid = (unsigned)std::min<size_t>((n8 + 255) / 256, 8 * (size_t)d->sms);
+            fill_cache_kernel<<<grid, 256, 0, stream>>>(static_cast<uint4*>(L.kcache.p), n8, s++);
+            fill_cache_kernel<<<grid, 256, 0, stream>>>(static_cast<uint4*>(L.vcache.p), n8, s++);
         }
-        std::vector<int> pos((size_t)d->cfg.max_batch, ctx_len);
-        MFQB_CUDA(cudaMemcpyAsync(d->pos.p, pos.data(), pos.size() * 4, cudaMemcpyHostToDevice, stream));
-        MFQB_CUDA(cudaStreamSynchronize(stream));
+        fill_pos_kernel<<<(d->cfg.max_batch + 127) / 128, 128, 0, stream>>>(static_cast<int*>(d->pos.p), d->cfg.max_batch, ctx_len);
+        MFQB_CUDA(cudaGetLastError());
     });
 }
 
@@ -797,7 +818,7 @@ int mfqb_decoder_step(mfqb_decoder* d, const int32_t* ids_in, int batch, int32_t
             if (rc == MFQB_ERR_UNSUPPORTED) fused_head = false;
             else if (rc != MFQB_OK) throw Error(rc, mfqb_last_error());
         }
-        if (!fused_head) {
+        if (!fused_head && !norm_mul_mat(d, d->lm_head, delta, d->gamma_final.p, batch, d->logits.p, MFQB_F32, false, s)) {
             launch_dep(add_rmsnorm_kernel, dim3(batch), dim3(1024), s, static_cast<float*>(d->h.p), delta, static_cast<const float*>(d->gamma_final.p),
                        static_cast<__nv_bfloat16*>(d->xn.p), H, d->cfg.rms_eps);
             mul_mat(d->lm_head, d->xn.p, batch, d->logits.p, s);

@@ -35,6 +35,7 @@ __device__ __forceinline__ float2 x_row_scale(uint32_t absmax_bits) {
 
 template <int KIND>
 __device__ __forceinline__ float x_value(const void* row, int k, int j) {
+    if constexpr (KIND == kTileXShared) return __bfloat162float(static_cast<const __nv_bfloat16*>(row)[j]);
     if constexpr (KIND == kTileXBf16) return __bfloat162float(__ldcg(static_cast<const __nv_bfloat16*>(row) + j));
     const float v = __ldcg(static_cast<const float*>(row) + j);
     if constexpr (KIND == kTileXSwiglu) return __ldcg(static_cast<const float*>(row) + k + j) * v / (1.0f + expf(-v));
@@ -45,8 +46,9 @@ template <int KIND>
 __device__ __forceinline__ float4 x_quad(const void* row, int k, int j, bool aligned) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (aligned && j + 3 < k) {
-        if constexpr (KIND == kTileXBf16) {
-            const uint2 r = __ldcg(reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(row) + j));
+        if constexpr (KIND == kTileXBf16 || KIND == kTileXShared) {
+            const uint2* at = reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(row) + j);
+            const uint2 r = KIND == kTileXShared ? *at : __ldcg(at);
             v = make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
         } else {
             v = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + j));
@@ -67,6 +69,36 @@ __device__ __forceinline__ uint32_t x_pack(float a, float b) {   // non-finite -
     const __half ha = isfinite(a) ? __float2half_rn(a) : __ushort_as_half((unsigned short)0x7E00);
     const __half hb = isfinite(b) ? __float2half_rn(b) : __ushort_as_half((unsigned short)0x7E00);
     return (uint32_t)__half_as_ushort(ha) | ((uint32_t)__half_as_ushort(hb) << 16);
+}
+
+// Slabs first, first + step, ... of a row's tile: see x_tiles_kernel.  r: row of the tile, pitch: bytes of a 64-column slab of it.
+template <int KIND>
+__device__ __forceinline__ void x_write_slabs(const void* row, bool row_al, int k, int gs, int T, int nslabs, float scale, unsigned char* dst, int r, int pitch, int first,
+                                              int step) {
+    const bool quad_al = row_al && (gs & 3) == 0;
+    for (int js = first; js < nslabs; js += step) {
+        const int ch = js / (4 * T), jj = js - ch * 4 * T, h = jj & 1, ft = jj >> 1, f = ft / T, t = ft - f * T;
+        const int g = ch * kChunkGroupsB + 4 * f + 2 * h;
+        uint32_t w[8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int slot = 8 * t + 4 * (c & 1), k0 = (g + (c >> 1)) * gs + slot;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (slot + 3 < gs) {
+                v = x_quad<KIND>(row, k, k0, quad_al);
+            } else {
+                if (slot < gs && k0 < k) v.x = x_value<KIND>(row, k, k0);
+                if (slot + 1 < gs && k0 + 1 < k) v.y = x_value<KIND>(row, k, k0 + 1);
+                if (slot + 2 < gs && k0 + 2 < k) v.z = x_value<KIND>(row, k, k0 + 2);
+            }
+            w[c] = x_pack(v.x * scale, v.z * scale);
+            w[4 + c] = x_pack(v.y * scale, v.w * scale);
+        }
+        const int slab = js & 3;
+        unsigned char* at = dst + (size_t)(js >> 2) * pitch;
+        *reinterpret_cast<uint4*>(at + (((2 * slab) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+        *reinterpret_cast<uint4*>(at + (((2 * slab + 1) ^ (r & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+    }
 }
 
 // Scales a row to the top of the f16 range and writes it as B operand: per 64-column slab the tile's rows of 128 bytes with
@@ -135,30 +167,69 @@ __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XT
     if (blockIdx.x == 0 && tid == 0) a.down[p] = sc.y;
     const int r = p - tile_begin, pitch = ((ncols + 7) & ~7) * 128;
     unsigned char* dst = a.out + (size_t)base * a.row_bytes + (size_t)r * 128;
-    const bool quad_al = row_al && (gs & 3) == 0;
-    for (int js = blockIdx.x * 256 + tid; js < nslabs; js += gridDim.x * 256) {
-        const int ch = js / (4 * T), jj = js - ch * 4 * T, h = jj & 1, ft = jj >> 1, f = ft / T, t = ft - f * T;
-        const int g = ch * kChunkGroupsB + 4 * f + 2 * h;
-        uint32_t w[8];
+    x_write_slabs<KIND>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.x * 256 + tid, gridDim.x * 256);
+}
+
+// The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the
+// scaling, and in shared memory as bf16 between the scaling and the slabs.  In a decoder block this is one kernel (and one
+// trip through memory) less before q|k|v and before gate|up.
+__global__ void __launch_bounds__(1024) norm_tiles_kernel(const __grid_constant__ XTilesArgs a, const __grid_constant__ TileNorm nm) {
+    constexpr int KEEP = 2;
+    extern __shared__ __align__(16) unsigned char norm_row[];
+    __shared__ float red[32];
+    __shared__ uint32_t red_max[32];
+    const int tid = threadIdx.x, nv = a.k >> 2, p = blockIdx.x;
+    float4* row = reinterpret_cast<float4*>(nm.h + (size_t)p * a.k);
+    const float4* drow = nm.delta ? reinterpret_cast<const float4*>(nm.delta + (size_t)p * a.k) : nullptr;
+    const float4* g4 = reinterpret_cast<const float4*>(nm.gamma);
+    uint2* xs = reinterpret_cast<uint2*>(norm_row);
+    float4 v[KEEP], g[KEEP];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int slot = 8 * t + 4 * (c & 1), k0 = (g + (c >> 1)) * gs + slot;
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (slot + 3 < gs) {
-                v = x_quad<KIND>(row, k, k0, quad_al);
-            } else {
-                if (slot < gs && k0 < k) v.x = x_value<KIND>(row, k, k0);
-                if (slot + 1 < gs && k0 + 1 < k) v.y = x_value<KIND>(row, k, k0 + 1);
-                if (slot + 2 < gs && k0 + 2 < k) v.z = x_value<KIND>(row, k, k0 + 2);
-            }
-            w[c] = x_pack(v.x * sc.x, v.z * sc.x);
-            w[4 + c] = x_pack(v.y * sc.x, v.w * sc.x);
+    for (int j = 0; j < KEEP; ++j)   // gamma is a constant of the model: fetched while the predecessor still runs
+        if (tid + j * 1024 < nv) g[j] = __ldg(g4 + tid + j * 1024);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float ss = 0.f;
+    auto take = [&](int i) {
+        float4 t = row[i];
+        if (drow) {
+            const float4 d = drow[i];
+            t.x += d.x; t.y += d.y; t.z += d.z; t.w += d.w;
+            row[i] = t;
         }
-        const int slab = js & 3;
-        unsigned char* at = dst + (size_t)(js >> 2) * pitch;
-        *reinterpret_cast<uint4*>(at + (((2 * slab) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
-        *reinterpret_cast<uint4*>(at + (((2 * slab + 1) ^ (r & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
-    }
+        ss += t.x * t.x + t.y * t.y + t.z * t.z + t.w * t.w;
+        return t;
+    };
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j)
+        if (tid + j * 1024 < nv) v[j] = take(tid + j * 1024);
+    for (int i = tid + KEEP * 1024; i < nv; i += 1024) take(i);
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) red[tid >> 5] = ss;
+    __syncthreads();
+    float tot = red[tid & 31];
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    const float inv = rsqrtf(tot / (float)a.k + nm.eps);
+    uint32_t ab = 0u;
+    auto put = [&](int i, const float4& t, const float4& gm) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(t.x * inv * gm.x, t.y * inv * gm.y), hi = __floats2bfloat162_rn(t.z * inv * gm.z, t.w * inv * gm.w);
+        const uint32_t w0 = *reinterpret_cast<const uint32_t*>(&lo), w1 = *reinterpret_cast<const uint32_t*>(&hi);
+        ab = max(max(ab, max(w0 & 0x7FFF0000u, (w0 << 16) & 0x7FFF0000u)), max(w1 & 0x7FFF0000u, (w1 << 16) & 0x7FFF0000u));
+        xs[i] = make_uint2(w0, w1);
+    };
+#pragma unroll
+    for (int j = 0; j < KEEP; ++j)
+        if (tid + j * 1024 < nv) put(tid + j * 1024, v[j], g[j]);
+    for (int i = tid + KEEP * 1024; i < nv; i += 1024) put(i, row[i], __ldg(g4 + i));
+    for (int o = 16; o > 0; o >>= 1) ab = max(ab, __shfl_xor_sync(0xffffffffu, ab, o));
+    if ((tid & 31) == 0) red_max[tid >> 5] = ab;
+    __syncthreads();
+    ab = red_max[tid & 31];
+    for (int o = 16; o > 0; o >>= 1) ab = max(ab, __shfl_xor_sync(0xffffffffu, ab, o));
+    const float2 sc = x_row_scale(ab);
+    if (tid == 0) a.down[p] = sc.y;
+    const int T = a.t8[0], tile_begin = p / a.x_rows * a.x_rows, r = p - tile_begin, pitch = ((min(a.x_rows, a.m - tile_begin) + 7) & ~7) * 128;
+    x_write_slabs<kTileXShared>(norm_row, true, a.k, a.gs[0], T, a.nchunks[0] * 4 * T, sc.x, a.out + (size_t)tile_begin * a.row_bytes + (size_t)r * 128, r, pitch, tid, 1024);
 }
 
 static void launch_x_tiles(const XTilesArgs& a, int kind, int rows, int nslabs, int sms, cudaStream_t s) {
@@ -255,7 +326,8 @@ int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes) {
 }
 
 // y [m, n] = x [m, k] W^T.  False when this weight has no tile kernel.
-bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s) {
+bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s, bool glu, const TileNorm* norm) {
+    if (norm && (w.k % 4 || w.k > 20480)) return false;   // the row as bf16 in a CTA's 48 KB
     TileArgs a{};
     TilePlan p;
     const int terms = w.table ? w.tile_terms : 1;
@@ -274,7 +346,8 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     a.x_row_bytes = x_row_bytes(w);
     a.y = y;
     a.y_dtype = y_dtype;
-    a.ldy = w.n;
+    a.ldy = glu ? w.n / 2 : w.n;
+    a.glu = glu;
     a.units = (int)units;
     a.only_pool = -1;
     a.error = device_status_word(device);
@@ -299,7 +372,21 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     xa.t8[0] = w.t8;
     xa.gs[0] = w.gs;
     xa.nchunks[0] = w.nchunks;
-    launch_x_tiles(xa, kTileXBf16, m, w.nchunks * 4 * w.t8, sms, s);
+    if (norm) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)m);
+        cfg.blockDim = dim3(1024);
+        cfg.dynamicSmemBytes = (size_t)w.k * 2;
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        MFQB_CUDA(cudaLaunchKernelEx(&cfg, norm_tiles_kernel, xa, *norm));
+    } else {
+        launch_x_tiles(xa, kTileXBf16, m, w.nchunks * 4 * w.t8, sms, s);
+    }
     const cudaError_t e = launch_one(a, p, terms, s);
     if (e == cudaErrorNotSupported) return false;
     if (e != cudaSuccess)

@@ -60,6 +60,7 @@ struct TileArgs {
     const float* x_down;             // inverse scale per token, or per position of the route plan
     void* y;
     int y_dtype, ldy;
+    int glu;                         // plain product: rows come in 16-row blocks, gate and up in turn; y gets up * silu(gate)
     int m, ntok;                     // plain product: tokens, token tiles
     int units;                       // plain product: (tile, chunk) units
     float* partial;                  // [grid][N][128] float32 sums of tiles that several CTAs share, by the tile's first CTA; zero between calls
@@ -283,6 +284,8 @@ __device__ __forceinline__ bool tile_wait2(uint64_t* bar0, uint32_t parity0, uin
 __device__ __forceinline__ void st_global(float* p, float v) { asm volatile("st.global.f32 [%0], %1;" ::"l"(p), "f"(v)); }
 __device__ __forceinline__ void st_global(__nv_bfloat16* p, __nv_bfloat16 v) { asm volatile("st.global.b16 [%0], %1;" ::"l"(p), "h"(__bfloat16_as_ushort(v))); }
 
+__device__ __forceinline__ float tile_gated(float gate, float up) { return up * gate / (1.0f + expf(-gate)); }
+
 // True for the four epilogue warps when it is true for all of them: they leave together, none waits at a barrier for one that gave up.
 __device__ __forceinline__ bool tile_epilogue_all(bool ok) {
     uint32_t all;
@@ -504,8 +507,19 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
                 int2 col[8];
 #pragma unroll
                 for (int i = 0; i < 8; ++i) col[i] = sh.col[buf][cb + i];
-                const int n = row_ok ? s.ncols - cb : 0;
-                if (a.y_dtype == 0 /* MFQB_F32 */) {
+                int n = row_ok ? s.ncols - cb : 0;
+                if (a.glu) {   // gate rows are lanes 0-15 of the warp, their up rows lanes 16-31
+                    if (lane >= 16) n = 0;
+                    const int half = (row >> 5) * 16 + (row & 15);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float f = v[i] * (undo * __int_as_float(col[i].x)), up = __shfl_xor_sync(0xffffffffu, f, 16), o = tile_gated(f, up);
+                        if (i < n) {
+                            if (a.y_dtype == 0 /* MFQB_F32 */) st_global(reinterpret_cast<float*>(a.y) + (size_t)col[i].y * a.ldy + half, o);
+                            else st_global(reinterpret_cast<__nv_bfloat16*>(a.y) + (size_t)col[i].y * a.ldy + half, __float2bfloat16_rn(o));
+                        }
+                    }
+                } else if (a.y_dtype == 0 /* MFQB_F32 */) {
                     float* y = reinterpret_cast<float*>(a.y) + row;
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
@@ -709,7 +723,11 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
             if (tid == 0) atomicExch(a.error, MFQB_ERR_TIMEOUT);
             return;
         }
-        const int row = t.row0 + 4 * lane, n = min(4, t.row_limit - row);
+        int row = t.row0 + 4 * lane, n = min(4, t.row_limit - row);
+        if (a.glu) {   // gate rows are lanes 0-3 of every eight, their up rows lanes 4-7
+            if (lane & 4) n = 0;
+            row = (row >> 5) * 16 + (row & 15);
+        }
         const float4 f = *reinterpret_cast<const float4*>(sh.row_factor + 4 * lane);
         const bool vec = n == 4 && (a.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
         for (int c = warp; c < ncols16; c += kTileThreads / 32) {
@@ -718,7 +736,11 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
             const int2 col = sh.col[sh.finish - 1][c];
             const float down = __int_as_float(col.x);
             const float4 v = *reinterpret_cast<const float4*>(stage + c * kTileRows + 4 * lane);
-            const float o[4] = {v.x * (f.x * down), v.y * (f.y * down), v.z * (f.z * down), v.w * (f.w * down)};
+            float o[4] = {v.x * (f.x * down), v.y * (f.y * down), v.z * (f.z * down), v.w * (f.w * down)};
+            if (a.glu) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) o[i] = tile_gated(o[i], __shfl_xor_sync(0xffffffffu, o[i], 4));
+            }
             const size_t at = (size_t)col.y * a.ldy + row;
             if (a.y_dtype == 0 /* MFQB_F32 */) {
                 float* y = reinterpret_cast<float*>(a.y) + at;

@@ -9,7 +9,13 @@
 namespace mfqb {
 
 // What the activation rows are: bf16, float32, or float32 gate | up products whose SwiGLU activation is formed on the way.
-enum TileX { kTileXBf16 = 0, kTileXF32 = 1, kTileXSwiglu = 2 };
+enum TileX { kTileXBf16 = 0, kTileXF32 = 1, kTileXSwiglu = 2, kTileXShared = 3 /* bf16 in shared memory */ };
+// Residual add + RMSNorm on the way to the product: h [m, k] float32 += delta (may be null), x = bf16(h / rms(h) * gamma).
+struct TileNorm {
+    float* h;
+    const float *delta, *gamma;
+    float eps;
+};
 
 constexpr float kTileWeightScale = 0.25f;   // of the f16 weights: 8-bit codes x 8-bit sub-scales x offset head-room stay below 65504
 
@@ -33,8 +39,9 @@ __device__ __forceinline__ uint4 tile_row_const(uint32_t anchor, int bits) {
 }
 #endif
 
-// y [m, n] = x [m, k] W^T for bf16 x.  False when this weight has no tile kernel (its tables do not fit).
-bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s);
+// y [m, n] = x [m, k] W^T for bf16 x, or for the rows that `norm` gives (x unused).  glu: 16-row blocks of W alternate gate and
+// up rows and y [m, n / 2] = up * silu(gate).  False when this weight has no tile kernel (its tables do not fit).
+bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s, bool glu = false, const TileNorm* norm = nullptr);
 
 // f16 terms a lattice weight needs: 1 when every scale x code product is an f16 number, else 2.
 int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes);

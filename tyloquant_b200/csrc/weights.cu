@@ -468,6 +468,8 @@ int mfqb_mul_mat_glu(const mfqb_weight* w, const void* x, int m, void* y, int y_
             launch_bl_gemv(w->nint, x, 1, y, y_dtype, (int)w->info.n, w->device, stream, false, true);
             return;
         }
+        const NintDevB& dev = weight_device_layout(w);
+        if (m >= (w->family == MFQB_FAMILY_NINT ? 5 : 2) && launch_tile_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
         static GrowOnlyScratch pool;
         float* prod = static_cast<float*>(pool.get(w->device, (size_t)m * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)"));
         const int rc = mfqb_mul_mat(w, x, m, prod, MFQB_F32, stream);
