@@ -198,11 +198,25 @@ __global__ void __launch_bounds__(32 * kAttnWarps, 2) attn_decode_kernel(const f
     extern __shared__ __align__(128) unsigned char attn_smem[];
     const int split = blockIdx.x, kvh = blockIdx.y, row = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane >> 2, c = lane & 3, l16 = lane & 15;
+    const float* qkv_row = qkv + (size_t)row * (nq + 2 * nkv) * kHeadDim;
+    const float2* tab = rope_table + (size_t)row * 64;
+    // Rotation pair i of the group's queries: thread i, i + 128, ...; requested together with the position, used after the first
+    // copies are on their way.
+    constexpr int QPT = (G * 64 + 32 * kAttnWarps - 1) / (32 * kAttnWarps);
+    float q_lo[QPT], q_hi[QPT];
+    float2 q_cs[QPT];
+#pragma unroll
+    for (int j = 0; j < QPT; ++j) {
+        const int i = tid + 32 * kAttnWarps * j, g = i >> 6, d = i & 63;
+        if (g < G) {
+            q_lo[j] = __ldcg(qkv_row + (size_t)(kvh * G + g) * kHeadDim + d);
+            q_hi[j] = __ldcg(qkv_row + (size_t)(kvh * G + g) * kHeadDim + 64 + d);
+            q_cs[j] = __ldcg(tab + d);
+        }
+    }
     const int p = pos[row], len = p + 1;   // the token written by this step takes part
     const int per = (len + nsplit - 1) / nsplit;
     const int t0 = split * per, t1 = min(len, t0 + per);
-    const float* qkv_row = qkv + (size_t)row * (nq + 2 * nkv) * kHeadDim;
-    const float2* tab = rope_table + (size_t)row * 64;
     __nv_bfloat16* kb = kcache + ((size_t)row * nkv + kvh) * max_ctx * kHeadDim;
     __nv_bfloat16* vb = vcache + ((size_t)row * nkv + kvh) * max_ctx * kHeadDim;
     if (t0 <= p && p < t1) {   // this CTA's slice holds the new position (uniform over the CTA)
@@ -238,14 +252,16 @@ __global__ void __launch_bounds__(32 * kAttnWarps, 2) attn_decode_kernel(const f
     };
 #pragma unroll
     for (int i = 0; i < kAttnStages - 1; ++i) request(t0 + i * 16 * kAttnWarps, i);
-    // the group's queries, rotated and scaled to log2 units by 1 / sqrt(128) * log2(e)
+    // the group's queries, rotated and scaled to log2 units by 1 / sqrt(128) * log2(e): their loads were issued before the copies
     float* qs = reinterpret_cast<float*>(attn_smem + (size_t)kAttnWarps * kAttnStages * kAttnStageBytes);
-    for (int i = tid; i < G * 16; i += 32 * kAttnWarps) {
-        float f[8];
-        rope8(qkv_row + (size_t)(kvh * G + (i >> 4)) * kHeadDim, tab, i & 15, 0.08838834764831845f * 1.4426950408889634f, f);
-        float4* dst = reinterpret_cast<float4*>(qs + (i >> 4) * kHeadDim + 8 * (i & 15));
-        dst[0] = make_float4(f[0], f[1], f[2], f[3]);
-        dst[1] = make_float4(f[4], f[5], f[6], f[7]);
+#pragma unroll
+    for (int j = 0; j < QPT; ++j) {
+        const int i = tid + 32 * kAttnWarps * j, g = i >> 6, d = i & 63;
+        if (g < G) {
+            constexpr float kScale = 0.08838834764831845f * 1.4426950408889634f;
+            qs[g * kHeadDim + d] = (q_lo[j] * q_cs[j].x - q_hi[j] * q_cs[j].y) * kScale;
+            qs[g * kHeadDim + 64 + d] = (q_hi[j] * q_cs[j].x + q_lo[j] * q_cs[j].y) * kScale;
+        }
     }
     __syncthreads();
     // this lane's rows q and q + 8 of the A operands hold terms of head `h`
@@ -384,8 +400,13 @@ __global__ void __launch_bounds__(32 * kAttnWarps, 2) attn_decode_kernel(const f
     __threadfence();
     for (int g = threadIdx.x >> 5; g < G; g += 4) {
         const float* src = part + ((size_t)row * nq + kvh * G + g) * nsplit * kPartStride;
-        // weights of the splits (nsplit <= 64: two per lane)
+        // all loads of up to 32 splits at once, the weights' (nsplit <= 64: two per lane) among them: one trip to L2 each, and
+        // a rolled loop's remainder would make one per split
         const bool h0 = lane < nsplit, h1 = lane + 32 < nsplit;
+        float4 v[32];
+#pragma unroll
+        for (int u = 0; u < 32; ++u)
+            v[u] = u < nsplit ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)u * kPartStride) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
         const float2 ml0 = h0 ? __ldcg(reinterpret_cast<const float2*>(src + (size_t)lane * kPartStride + kHeadDim)) : make_float2(-INFINITY, 0.f);
         const float2 ml1 = h1 ? __ldcg(reinterpret_cast<const float2*>(src + (size_t)(lane + 32) * kPartStride + kHeadDim)) : make_float2(-INFINITY, 0.f);
         float mm = fmaxf(ml0.x, ml1.x);
@@ -394,11 +415,19 @@ __global__ void __launch_bounds__(32 * kAttnWarps, 2) attn_decode_kernel(const f
         float ll = ml0.y * c0 + ml1.y * c1;
         for (int o = 16; o > 0; o >>= 1) ll += __shfl_xor_sync(0xffffffffu, ll, o);
         float4 aa = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 16
-        for (int sp = 0; sp < nsplit; ++sp) {
-            const float c = __shfl_sync(0xffffffffu, sp < 32 ? c0 : c1, sp & 31);
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(src + (size_t)sp * kPartStride) + lane);
-            aa.x += c * v.x; aa.y += c * v.y; aa.z += c * v.z; aa.w += c * v.w;
+        auto add = [&](float cw) {
+#pragma unroll
+            for (int u = 0; u < 32; ++u) {
+                const float c = __shfl_sync(0xffffffffu, cw, u);
+                aa.x += c * v[u].x; aa.y += c * v[u].y; aa.z += c * v[u].z; aa.w += c * v[u].w;
+            }
+        };
+        add(c0);
+        if (nsplit > 32) {
+#pragma unroll
+            for (int u = 0; u < 32; ++u)
+                v[u] = u + 32 < nsplit ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(u + 32) * kPartStride) + lane) : make_float4(0.f, 0.f, 0.f, 0.f);
+            add(c1);
         }
         const float inv = 1.0f / ll;
         const __nv_bfloat162 o01 = __floats2bfloat162_rn(aa.x * inv, aa.y * inv), o23 = __floats2bfloat162_rn(aa.z * inv, aa.w * inv);

@@ -23,6 +23,7 @@ struct XTilesArgs {
     const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool;
     int n_experts, src_div, m;
     int t8[kTileMaxPools], gs[kTileMaxPools], nchunks[kTileMaxPools];
+    int staged;            // bf16 rows go through shared memory
 };
 
 // (2^e, 2^-e) with 2^e * max in [2^14, 2^15); (1, 1) for a zero, subnormal or non-finite maximum.
@@ -108,6 +109,7 @@ __device__ __forceinline__ void x_write_slabs(const void* row, bool row_al, int 
 // itself (from L2; a second launch for the maxima costs more for the rows of a decoding batch) and writes its share.
 template <int KIND>
 __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XTilesArgs a) {
+    extern __shared__ __align__(16) unsigned char x_row[];   // bf16 rows: kept between the two passes (a.staged)
     __shared__ uint32_t red[8];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -143,6 +145,7 @@ __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XT
             for (int u = 0; u < 8; ++u) v[u] = j0 + 256 * u < (k >> 3) ? __ldcg(reinterpret_cast<const uint4*>(row) + j0 + 256 * u) : make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
+                if (a.staged && j0 + 256 * u < (k >> 3)) reinterpret_cast<uint4*>(x_row)[j0 + 256 * u] = v[u];
                 const uint32_t w4[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) ab = max(ab, max(w4[i] & 0x7FFF0000u, (w4[i] << 16) & 0x7FFF0000u));
@@ -167,7 +170,10 @@ __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XT
     if (blockIdx.x == 0 && tid == 0) a.down[p] = sc.y;
     const int r = p - tile_begin, pitch = ((ncols + 7) & ~7) * 128;
     unsigned char* dst = a.out + (size_t)base * a.row_bytes + (size_t)r * 128;
-    x_write_slabs<KIND>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.x * 256 + tid, gridDim.x * 256);
+    if (KIND == kTileXBf16 && a.staged && (reinterpret_cast<uintptr_t>(row) & 15) == 0 && (k & 7) == 0)
+        x_write_slabs<kTileXShared>(x_row, true, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.x * 256 + tid, gridDim.x * 256);
+    else
+        x_write_slabs<KIND>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.x * 256 + tid, gridDim.x * 256);
 }
 
 // The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the
@@ -232,10 +238,13 @@ __global__ void __launch_bounds__(1024) norm_tiles_kernel(const __grid_constant_
     x_write_slabs<kTileXShared>(norm_row, true, a.k, a.gs[0], T, a.nchunks[0] * 4 * T, sc.x, a.out + (size_t)tile_begin * a.row_bytes + (size_t)r * 128, r, pitch, tid, 1024);
 }
 
-static void launch_x_tiles(const XTilesArgs& a, int kind, int rows, int nslabs, int sms, cudaStream_t s) {
+static void launch_x_tiles(XTilesArgs a, int kind, int rows, int nslabs, int sms, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     // one CTA per row fills the chip from a few hundred rows on; fewer rows are shared out
     const int splits = std::max(1, std::min((nslabs + 255) / 256, 2 * sms / std::max(rows, 1)));
+    // a second trip to L2 for the values costs a decoding batch 0.7 us of its chain; rows of up to 32 KB fit beside a tile CTA
+    a.staged = kind == kTileXBf16 && a.k <= 16384 && rows <= 64;
+    if (a.staged) cfg.dynamicSmemBytes = (size_t)(a.k + 7) / 8 * 16;
     cfg.gridDim = dim3((unsigned)splits, (unsigned)rows);
     cfg.blockDim = dim3(256);
     cfg.stream = s;
@@ -351,8 +360,16 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     a.units = (int)units;
     a.only_pool = -1;
     a.error = device_status_word(device);
-    // no more CTAs than two chunks each, nor than a dozen per tile: the last one adds the others' partial tiles
-    p.grid = (int)std::max<long long>(1, std::min<long long>(sms, std::min((units + 1) / 2, tiles * 12)));
+    // Fewer tiles than SMs: either as many CTAs per tile as fit, each with one part of one tile, or equal ranges over all SMs.
+    // The latter give a CTA less to do, but parts of two tiles, and two sums over CTAs that follow one another: each costs
+    // about as much as three chunks (1.5 to 2.5 us against 0.6 for a chunk of 16 tokens; both grow with the tokens), and half of
+    // the second one is hidden behind the CTA's other part: with six chunks instead of three for two sums, 16 rows through NINT6
+    // 4096 x 14336 took 22.4 us instead of 21.1, with none 8 rows through NVQ3 17408 x 5120 31.4 instead of 23.8.
+    // Without sharing there is no sum.  At most a dozen CTAs per tile: the last one adds the others' parts.
+    const long long split = std::min({(long long)sms / tiles, (long long)std::max(1, w.nchunks / 2), 12ll});
+    const long long chunks_split = split ? (w.nchunks + split - 1) / split + (split > 1 ? 3 : 0) : 0, chunks_equal = (units + sms - 1) / sms + 3;
+    a.split = split && chunks_split <= chunks_equal ? (int)split : 0;
+    p.grid = a.split ? (int)(tiles * split) : (int)std::max<long long>(1, std::min<long long>(sms, (units + 1) / 2));
     static GrowOnlyScratch xs[2], parts, counts;   // activations: decoding batches keep a small block of their own beside the prefill's
     const size_t xb = ((size_t)(m + 7) / 8 * 8 * a.x_row_bytes + 255) / 256 * 256;
     unsigned char* buf = static_cast<unsigned char*>(xs[m > 16].get(device, xb + (size_t)m * 4, s, "mfqb_mul_mat (f16 activation tiles)"));

@@ -60,9 +60,9 @@ struct TileArgs {
     const float* x_down;             // inverse scale per token, or per position of the route plan
     void* y;
     int y_dtype, ldy;
-    int glu;                         // plain product: rows come in 16-row blocks, gate and up in turn; y gets up * silu(gate)
+    int glu;                         // plain product: rows come in 16-row blocks, gate and up in turn; y gets up * silu(gate) (the launch picks the kernel)
     int m, ntok;                     // plain product: tokens, token tiles
-    int units;                       // plain product: (tile, chunk) units
+    int units, split;                // plain product: (tile, chunk) units; CTAs per tile, or 0: equal ranges of units
     float* partial;                  // [grid][N][128] float32 sums of tiles that several CTAs share, by the tile's first CTA; zero between calls
     unsigned* counters;              // [grid], zero between calls
     // expert product over a route plan with tiles of x_rows pairs; tile_bounds == nullptr: plain product
@@ -82,9 +82,25 @@ struct TileSeg {
     int parts, slot0, last;   // CTAs that share the tile, the first of them; whether it is this CTA's last stretch
 };
 
-// Unit range of CTA b, and the CTA that owns a unit.
-__device__ __forceinline__ int tile_unit_begin(int b, int units, int grid) { return (int)((long long)b * units / grid); }
-__device__ __forceinline__ int tile_unit_owner(int u, int units, int grid) { return (int)((((long long)u + 1) * grid - 1) / units); }
+// First unit of CTA b of a plain product.  split = 0: equal ranges; else `split` CTAs share every tile and none has a part of
+// two (see launch_tile_product).
+__device__ __forceinline__ int tile_unit_begin(const TileArgs& a, int b) {
+    if (a.split == 0) return (int)((long long)b * a.units / gridDim.x);
+    const int tile = b / a.split, part = b - tile * a.split, nch = a.pools[0].nchunks;
+    return tile * nch + part * nch / a.split;
+}
+// The CTAs that share a tile: the first one, and how many.
+__device__ __forceinline__ void tile_sharers(const TileArgs& a, int tile, int& slot0, int& parts) {
+    if (a.split) {
+        slot0 = tile * a.split;
+        parts = a.split;
+        return;
+    }
+    const int nch = a.pools[0].nchunks, grid = gridDim.x;
+    auto owner = [&](int u) { return (int)((((long long)u + 1) * grid - 1) / a.units); };
+    slot0 = owner(tile * nch);
+    parts = owner((tile + 1) * nch - 1) - slot0 + 1;
+}
 
 // First row of an expert's tile in the tiles' buffer: every tile starts on a multiple of eight rows, and experts do not overlap.
 __host__ __device__ __forceinline__ int tile_x_row(int expert_begin, int expert, int row_in_expert) { return (expert_begin + 7) / 8 * 8 + 8 * expert + row_in_expert; }
@@ -92,7 +108,7 @@ __host__ __device__ __forceinline__ int tile_x_row(int expert_begin, int expert,
 // Next stretch of this CTA; `cursor` starts at the CTA's first unit (plain) or item (experts).
 __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSeg& s) {
     if (a.tile_bounds == nullptr) {
-        const int end = tile_unit_begin(blockIdx.x + 1, a.units, gridDim.x);
+        const int end = tile_unit_begin(a, blockIdx.x + 1);
         if (cursor >= end) return false;
         const NintDevB& w = a.pools[0];
         const int tile = cursor / w.nchunks, rt = tile / a.ntok, tt = tile - rt * a.ntok;
@@ -107,8 +123,7 @@ __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSe
         s.tok0 = tt * a.x_rows;
         s.ncols = min(a.x_rows, a.m - s.tok0);
         s.x_off = (size_t)s.tok0 * a.x_row_bytes;
-        s.slot0 = tile_unit_owner(tile * w.nchunks, a.units, gridDim.x);
-        s.parts = tile_unit_owner((tile + 1) * w.nchunks - 1, a.units, gridDim.x) - s.slot0 + 1;
+        tile_sharers(a, tile, s.slot0, s.parts);
         cursor += s.ch1 - s.ch0;
         s.last = cursor >= end;
         return true;
@@ -142,7 +157,7 @@ __device__ __forceinline__ bool tile_next(const TileArgs& a, int& cursor, TileSe
     }
     return false;
 }
-__device__ __forceinline__ int tile_first(const TileArgs& a) { return a.tile_bounds == nullptr ? tile_unit_begin(blockIdx.x, a.units, gridDim.x) : (int)blockIdx.x; }
+__device__ __forceinline__ int tile_first(const TileArgs& a) { return a.tile_bounds == nullptr ? tile_unit_begin(a, blockIdx.x) : (int)blockIdx.x; }
 
 __device__ __forceinline__ __half2 h2_bits(uint32_t v) { return *reinterpret_cast<const __half2*>(&v); }
 __device__ __forceinline__ uint32_t bits_h2(__half2 v) { return *reinterpret_cast<const uint32_t*>(&v); }
@@ -420,7 +435,9 @@ __device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, Ti
 }
 
 // Sets::dispatch(w, f) calls f(Codec{}) for the codec of a cohort; Sets::ctx describes the codec context (lattice tables).
-template <class Sets>
+// GLU: the gated epilogue (TileArgs::glu).  1024 in the launch bound holds the kernel to 64 registers, which leaves room on the
+// SM for the CTAs of the kernel before it.
+template <class Sets, bool GLU>
 __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant__ TileArgs a) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ TileShared sh;
@@ -508,7 +525,7 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
 #pragma unroll
                 for (int i = 0; i < 8; ++i) col[i] = sh.col[buf][cb + i];
                 int n = row_ok ? s.ncols - cb : 0;
-                if (a.glu) {   // gate rows are lanes 0-15 of the warp, their up rows lanes 16-31
+                if constexpr (GLU) {   // gate rows are lanes 0-15 of the warp, their up rows lanes 16-31
                     if (lane >= 16) n = 0;
                     const int half = (row >> 5) * 16 + (row & 15);
 #pragma unroll
@@ -519,7 +536,9 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
                             else st_global(reinterpret_cast<__nv_bfloat16*>(a.y) + (size_t)col[i].y * a.ldy + half, __float2bfloat16_rn(o));
                         }
                     }
-                } else if (a.y_dtype == 0 /* MFQB_F32 */) {
+                    return;
+                }
+                if (a.y_dtype == 0 /* MFQB_F32 */) {
                     float* y = reinterpret_cast<float*>(a.y) + row;
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
@@ -724,7 +743,7 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
             return;
         }
         int row = t.row0 + 4 * lane, n = min(4, t.row_limit - row);
-        if (a.glu) {   // gate rows are lanes 0-3 of every eight, their up rows lanes 4-7
+        if constexpr (GLU) {   // gate rows are lanes 0-3 of every eight, their up rows lanes 4-7
             if (lane & 4) n = 0;
             row = (row >> 5) * 16 + (row & 15);
         }
@@ -737,7 +756,7 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
             const float down = __int_as_float(col.x);
             const float4 v = *reinterpret_cast<const float4*>(stage + c * kTileRows + 4 * lane);
             float o[4] = {v.x * (f.x * down), v.y * (f.y * down), v.z * (f.z * down), v.w * (f.w * down)};
-            if (a.glu) {
+            if constexpr (GLU) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) o[i] = tile_gated(o[i], __shfl_xor_sync(0xffffffffu, o[i], 4));
             }

@@ -20,9 +20,9 @@ struct TileOne {
     __device__ static void ctx_init(unsigned char* ctx, const TileArgs& a, int tid, int nthreads) { C::ctx_init(ctx, a, tid, nthreads); }
 };
 
-template <class Sets>
-static cudaError_t launch_tile(const TileArgs& a, const TilePlan& p, cudaStream_t stream) {
-    auto kernel = tile_tc_kernel<Sets>;
+template <class Sets, bool GLU>
+static cudaError_t launch_tile_form(const TileArgs& a, const TilePlan& p, cudaStream_t stream) {
+    auto kernel = tile_tc_kernel<Sets, GLU>;
     static bool attr_set[64] = {};   // per kernel and device: the largest dynamic shared memory any plan asks for
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -43,6 +43,11 @@ static cudaError_t launch_tile(const TileArgs& a, const TilePlan& p, cudaStream_
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
+template <class Sets>
+static cudaError_t launch_tile(const TileArgs& a, const TilePlan& p, cudaStream_t stream) {
+    return a.glu ? launch_tile_form<Sets, true>(a, p, stream) : launch_tile_form<Sets, false>(a, p, stream);
 }
 
 template <int BITS>

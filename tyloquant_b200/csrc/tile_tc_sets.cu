@@ -36,6 +36,6 @@ struct TileExperts {
     }
     __device__ static void ctx_init(unsigned char*, const TileArgs&, int, int) {}
 };
-cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, cudaStream_t stream) { return launch_tile<TileExperts>(a, p, stream); }
+cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, cudaStream_t stream) { return launch_tile_form<TileExperts, false>(a, p, stream); }
 
 }  // namespace mfqb
