@@ -238,6 +238,19 @@ __global__ void __launch_bounds__(1024) norm_tiles_kernel(const __grid_constant_
     x_write_slabs<kTileXShared>(norm_row, true, a.k, a.gs[0], T, a.nchunks[0] * 4 * T, sc.x, a.out + (size_t)tile_begin * a.row_bytes + (size_t)r * 128, r, pitch, tid, 1024);
 }
 
+// All of the SM's unified memory as shared memory.  Kernels of a chain that ask for different splits do not become resident
+// beside one another: the activation kernels (up to 33 KB) would wait for the tile kernel's CTAs to leave, and these for them
+// (16 rows through NINT6 4096 x 14336: 25.0 us instead of 20.9).
+template <auto kernel>
+static void whole_carveout() {
+    static bool done[64] = {};
+    int dev = 0;
+    MFQB_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && done[dev]) return;
+    MFQB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (dev >= 0 && dev < 64) done[dev] = true;
+}
+
 static void launch_x_tiles(XTilesArgs a, int kind, int rows, int nslabs, int sms, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     // one CTA per row fills the chip from a few hundred rows on; fewer rows are shared out
@@ -253,18 +266,24 @@ static void launch_x_tiles(XTilesArgs a, int kind, int rows, int nslabs, int sms
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
+    auto go = [&](auto kind_c) {
+        constexpr int KIND = decltype(kind_c)::value;
+        whole_carveout<x_tiles_kernel<KIND>>();
+        MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<KIND>, a));
+    };
     switch (kind) {
-        case kTileXBf16: MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<kTileXBf16>, a)); break;
-        case kTileXF32: MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<kTileXF32>, a)); break;
-        default: MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<kTileXSwiglu>, a)); break;
+        case kTileXBf16: go(std::integral_constant<int, kTileXBf16>{}); break;
+        case kTileXF32: go(std::integral_constant<int, kTileXF32>{}); break;
+        default: go(std::integral_constant<int, kTileXSwiglu>{}); break;
     }
 }
 
 // ---- plans ---------------------------------------------------------------------------------------------------------------
 static size_t x_row_bytes(const NintDevB& w) { return (size_t)w.nchunks * w.t8 * 128; }
 
-// Rings for tokens tiles of `n` columns: records first (two stages, then up to 64 KB of them, which is what keeps HBM busy),
-// activation slabs in the rest.  False when the codec's tables and two stages of each do not fit.
+// Rings for token tiles of `n` columns: two stages of each, then records up to 144 KB (what a decoder step frees comes back from
+// HBM 2 us later: with 64 KB the expert products waited for it, 128 experts and 32 tokens 183 us instead of 170) and activation
+// slabs.  False when the codec's tables and two stages of each do not fit.
 static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8, int terms, size_t ctx_bytes) {
     const size_t budget = kTileDynSmem - 1024, ctx = (ctx_bytes + 15) / 16 * 16;
     a.n_mma = n;
@@ -279,13 +298,13 @@ static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8,
         a.a_cols = 16 * t8 * terms * a.step;
         a.a_stages = std::min(kTileAStages, a_total / a.a_cols);
         const size_t rec_stage = 8 * rec_bytes * a.step, x_stage = (size_t)n * 128 * (a.x_whole ? a.step * t8 : 1);
-        if (a.a_stages < 2 || ctx + 2 * rec_stage + 2 * x_stage > budget || (a.x_whole && x_stage > 24 * 1024)) continue;
+        if (a.a_stages < 2 || ctx + (a.step > 1 ? 3 : 2) * rec_stage + 2 * x_stage > budget || (a.x_whole && x_stage > 24 * 1024)) continue;
         size_t left = budget - ctx - 2 * rec_stage - 2 * x_stage;
         int rs = 2, xs = 2;
         for (bool grown = true; grown;) {
             grown = false;
             if (xs < 4 && left >= x_stage) { ++xs; left -= x_stage; grown = true; }
-            if (rs < kTileRecStages && (size_t)rs * rec_stage < 64 * 1024 && left >= rec_stage) { ++rs; left -= rec_stage; grown = true; }
+            if (rs < kTileRecStages && (size_t)(rs + 1) * rec_stage <= 144 * 1024 && left >= rec_stage) { ++rs; left -= rec_stage; grown = true; }
         }
         while (xs < kTileXStages && !a.x_whole && left >= x_stage) { ++xs; left -= x_stage; }
         a.rec_stages = rs;
@@ -400,6 +419,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
+        whole_carveout<norm_tiles_kernel>();
         MFQB_CUDA(cudaLaunchKernelEx(&cfg, norm_tiles_kernel, xa, *norm));
     } else {
         launch_x_tiles(xa, kTileXBf16, m, w.nchunks * 4 * w.t8, sms, s);
