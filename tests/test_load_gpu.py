@@ -70,3 +70,26 @@ def test_experts_with_padded_rows_and_a_shard():
         assert _same(whole.dequantize_expert(i).cpu().numpy(), ref), i
         if 3 <= i < 9:
             assert _same(shard.dequantize_expert(i).cpu().numpy(), ref), i
+
+
+def test_memory_of_freed_tensors_is_taken_again_only_when_idle():
+    """Tensors loaded into the blocks of freed ones, with work on the freed ones still queued on another stream."""
+    side = torch.cuda.Stream()
+    x = torch.randn(1, 4096, device="cuda", dtype=torch.bfloat16)
+    last = None
+    for i, n in enumerate([2048, 2048, 1950, 2048, 300, 2048]):   # the same size, a little smaller, much smaller
+        blob = encode.random_nint_blob(n, 4096, 4, 24, 6, seed=i, device="cuda")
+        ref = O.dequant_nint(O.unpack_nint(blob))
+        w = QuantWeight.from_blob("NINT4", blob)
+        assert _same(w.dequantize().cpu().numpy(), ref), (i, n)
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            for _ in range(50):
+                y = w.matmul(x)
+        w.free()
+        if last is not None and last.shape == y.shape:
+            assert not torch.equal(last, y)
+        got = y.float().cpu().numpy()
+        want = x.float().cpu().numpy() @ ref.T
+        assert np.allclose(got, want, atol=2e-2 * np.abs(want).max()), (i, n)
+        last = y

@@ -30,6 +30,9 @@ struct DeviceGuard {
 
 int device_sm_count(int device);
 
+// cudaMalloc on the current device; where there is no room, after parked blocks of freed tensors have been given back.
+void device_malloc(void** p, size_t bytes);
+
 // Owning device buffer.
 struct DevBuf {
     void* p = nullptr;
@@ -43,7 +46,7 @@ struct DevBuf {
     }
     void alloc(size_t n) {
         release();
-        if (n) MFQB_CUDA(cudaMalloc(&p, n));
+        if (n) device_malloc(&p, n);
         bytes = n;
     }
     void upload(const void* src, size_t n) {

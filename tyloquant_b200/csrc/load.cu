@@ -323,6 +323,91 @@ NintDevB nint_geometry(const NintView& t, int64_t n, int64_t k) {
     return d;
 }
 
+namespace {
+struct Parked {
+    void* p;
+    size_t bytes;
+};
+struct ParkedList {   // oldest first
+    std::mutex mu;
+    std::vector<Parked> blocks;
+};
+ParkedList& parked(int device) {
+    static ParkedList* lists = new ParkedList[64];   // outlives tensors that are freed while the process ends
+    return lists[device];
+}
+}  // namespace
+
+void TensorBuf::alloc(size_t n) {
+    release();
+    bytes = n;
+    if (!n) return;
+    MFQB_CUDA(cudaGetDevice(&device_));
+    if (device_ >= 64) fail(MFQB_ERR_ARG, "device index %d out of range", device_);
+    {
+        ParkedList& l = parked(device_);
+        std::lock_guard<std::mutex> lock(l.mu);
+        auto best = l.blocks.end();   // the smallest that fits and wastes no more than an eighth
+        for (auto it = l.blocks.begin(); it != l.blocks.end(); ++it)
+            if (it->bytes >= n && it->bytes - n <= n / 8 && (best == l.blocks.end() || it->bytes < best->bytes)) best = it;
+        if (best != l.blocks.end()) {
+            p = best->p;
+            block_ = best->bytes;
+            l.blocks.erase(best);
+            return;
+        }
+    }
+    device_malloc(&p, n);
+    block_ = n;
+}
+
+void TensorBuf::release() {
+    if (!p) return;
+    void* const mem = p;
+    p = nullptr;
+    bytes = 0;
+    int prev = device_;
+    cudaGetDevice(&prev);
+    if (prev != device_) cudaSetDevice(device_);
+    std::vector<Parked> out;
+    if (block_ <= kParkedBytes && cudaDeviceSynchronize() == cudaSuccess) {
+        ParkedList& l = parked(device_);
+        std::lock_guard<std::mutex> lock(l.mu);
+        l.blocks.push_back(Parked{mem, block_});
+        size_t total = 0;
+        for (const Parked& b : l.blocks) total += b.bytes;
+        while (total > kParkedBytes || l.blocks.size() > kParkedBlocks) {
+            total -= l.blocks.front().bytes;
+            out.push_back(l.blocks.front());
+            l.blocks.erase(l.blocks.begin());
+        }
+    } else {
+        out.push_back(Parked{mem, block_});
+    }
+    for (const Parked& b : out) cudaFree(b.p);
+    if (prev != device_) cudaSetDevice(prev);
+}
+
+bool give_back_parked(int device) {
+    if (device < 0 || device >= 64) return false;
+    std::vector<Parked> out;
+    {
+        ParkedList& l = parked(device);
+        std::lock_guard<std::mutex> lock(l.mu);
+        out.swap(l.blocks);
+    }
+    for (const Parked& b : out) cudaFree(b.p);
+    return !out.empty();
+}
+
+void device_malloc(void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    int device = -1;
+    if (e == cudaErrorMemoryAllocation && cudaGetLastError() == e && cudaGetDevice(&device) == cudaSuccess && give_back_parked(device))
+        e = cudaMalloc(p, bytes);
+    MFQB_CUDA(e);
+}
+
 void PackedDev::alloc(size_t extra) {
     const size_t items = up256((size_t)d.nrb * d.nchunks * d.rec_words * 4), anchors = up256((size_t)d.nrb * 16 * 4), rowc = (size_t)d.nrb * 16 * sizeof(uint4);
     extra_off = items + anchors + up256(rowc);

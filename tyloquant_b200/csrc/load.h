@@ -9,9 +9,33 @@
 
 namespace mfqb {
 
+// Device memory of a tensor.  Mapping and unmapping 52 MB takes 360 and 320 us, a third of loading it (2390 -> 1570 us with decoding and freeing), so the blocks of freed
+// tensors are parked and taken again by tensors of about their size: at most kParkedBytes in kParkedBlocks of each device,
+// given back when newer ones push them out or when an allocation of the library finds no room.  A block is parked after
+// all work of its device has ended (what cudaFree waits for), so whatever stream takes it next may write at once.
+constexpr size_t kParkedBytes = 256u << 20;
+constexpr int kParkedBlocks = 16;
+
+struct TensorBuf {
+    void* p = nullptr;
+    size_t bytes = 0;   // asked for; the block may be larger
+    TensorBuf() = default;
+    TensorBuf(const TensorBuf&) = delete;
+    TensorBuf& operator=(const TensorBuf&) = delete;
+    TensorBuf(TensorBuf&& o) noexcept : p(o.p), bytes(o.bytes), block_(o.block_), device_(o.device_) { o.p = nullptr; }
+    void alloc(size_t n);   // on the current device
+    void release();
+    ~TensorBuf() { release(); }
+
+private:
+    size_t block_ = 0;
+    int device_ = 0;
+};
+bool give_back_parked(int device);   // true where the device got memory back
+
 // Device memory of one tensor in the byte-lane layout: records, anchors and row constants in one allocation.
 struct PackedDev {
-    DevBuf mem;
+    TensorBuf mem;
     NintDevB d{};
     uint64_t bytes = 0;   // records + anchors + row constants
     void alloc(size_t extra = 0);               // geometry in d is set; `extra` more bytes at extra_at()

@@ -47,7 +47,7 @@ void* GrowOnlyScratch::get(int device, size_t bytes, cudaStream_t stream, const 
              what, bytes, d.bytes);
     void* p = nullptr;
     const size_t want = bytes + bytes / 2;
-    MFQB_CUDA(cudaMalloc(&p, want));
+    device_malloc(&p, want);
     MFQB_CUDA(cudaMemset(p, 0, want));   // some users keep self-resetting counters in their block: they start at zero
     d.p = p;   // the previous block stays allocated: earlier launches and captured graphs may still use it
     d.bytes = want;
