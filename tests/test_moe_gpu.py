@@ -166,3 +166,27 @@ def test_route_plan_tiles_and_grouped_tile_kernel(tokens):
     assert rel_l2((parts[0] + parts[1]).cpu().numpy(), y) <= 1e-5
     gu.free()
     dn.free()
+
+
+def test_one_token_calls_back_to_back_past_the_expert_table():
+    """514 experts, two of them past the table a CTA keeps at hand; calls with other routes follow one another without a wait."""
+    e_count, h, f, k = 514, 72, 48, 4
+    gu_blob, dn_blob = _moe_case(e_count, h, f, np.random.default_rng(5).choice([3, 4, 6], e_count), seed=6)
+    gu_ref, dn_ref = O.dequant_nintm(O.unpack_nintm(gu_blob)), O.dequant_nintm(O.unpack_nintm(dn_blob))
+    gu, dn = moe.MoeWeight(gu_blob), moe.MoeWeight(dn_blob)
+    rng = np.random.default_rng(7)
+    x = encode.bf16_round(rng.standard_normal((1, h), dtype=np.float32))
+    zs = [rng.standard_normal((1, e_count)).astype(np.float32) for _ in range(12)]
+    for i, z in enumerate(zs):
+        z[0, [512, 513, i, 511]] += 9.0
+    xt, zt = bf16_tensor(x), [torch.from_numpy(z).cuda() for z in zs]
+    torch.cuda.synchronize()
+    ys = []
+    for z in zt:
+        ids, wts = moe.moe_topk(z, k)
+        ys.append(moe.moe_ffn(gu, dn, xt, ids, wts))
+    for y, z in zip(ys, zs):
+        rid, rw = O.moe_topk(z, k)
+        assert rel_l2(y.cpu().numpy(), O.moe_ffn(x, gu_ref, dn_ref, rid, rw)) <= REL_L2
+    gu.free()
+    dn.free()

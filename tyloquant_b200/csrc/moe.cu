@@ -290,6 +290,9 @@ static void mul_mat_id_impl(const mfqb_moe_weight* w, const void* x, int x_per_p
         a.n_experts = w->info.n_experts;
         a.x_mode = x_mode;
         if (tail) {
+            // the launch ahead in the stream is the gate|up product of the same routes, which lets this one start only after
+            // its own wait for them
+            a.ids_ready = 1;
             a.route_w = tail->route_w;
             a.pair_out = tail->pair_out;
             a.token_count = tail->token_count;

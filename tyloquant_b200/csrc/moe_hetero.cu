@@ -27,19 +27,35 @@ constexpr bool hetero_has_codec(int bits, int t8) {
            (bits == 8 && t8 == 3) || (bits == 8 && t8 == 6);
 }
 
+// A token's pairs are some ten microseconds of dependent trips: the route, its expert's cohort and position, the records, the
+// activations, the sum.  The expert tables are constants, so they are fetched while the kernel ahead still runs; the down
+// product, whose routes were complete before the gate|up product let it start, asks for its records before it waits.  One
+// token of 128 experts, 8 routes, 2048 x 768: router and both products 24.4 -> 22.0 us in a graph.  Three CTAs per SM (80
+// registers, spills) gave 24.5; even runs of records per warp with rings of 10 KB 23.0.
+constexpr int kHeteroTable = 512;   // experts whose (cohort, position) a CTA keeps at hand
 template <int XMODE>
 __global__ void __launch_bounds__(256, 2) moe_hetero_gemv1_kernel(const __grid_constant__ HeteroArgs h) {
     extern __shared__ __align__(16) unsigned char smem[];
-    pdl_wait_b();   // the routing table comes from the previous kernel
-    const int e = h.base.route_ids[blockIdx.y];
+    __shared__ int2 table[kHeteroTable];
+    const int n_experts = h.base.n_experts;
+    for (int i = threadIdx.x; i < min(n_experts, kHeteroTable); i += blockDim.x) table[i] = make_int2(h.base.expert_pool[i], h.base.expert_local[i]);
+    __syncthreads();
+    if (!h.base.ids_ready) pdl_wait_b();   // the routing table comes from the previous kernel
+    const int e = __ldcg(h.base.route_ids + blockIdx.y);
     // an id outside [0, n_experts) is ignored like a route to an expert that is not held here
-    const int pool = (e >= 0 && e < h.base.n_experts) ? h.base.expert_pool[e] : -1;
+    int2 at = make_int2(-1, 0);
+    if (e >= 0 && e < n_experts) at = e < kHeteroTable ? table[e] : make_int2(h.base.expert_pool[e], h.base.expert_local[e]);
+    const int pool = at.x;
     if (pool < 0) {
-        if (h.base.route_w != nullptr) routed_absent_pair(h.base, blockIdx.y);
+        if (h.base.route_w != nullptr) {
+            pdl_wait_b();
+            routed_absent_pair(h.base, blockIdx.y);
+        }
         return;
     }
     GemvArgsB a = h.base;
     a.pool = pool;
+    a.pair_local = at.y + 1;
     const NintDevB& w = h.pools[pool];
     switch (w.bits * 16 + w.t8) {
         case 2 * 16 + 2: gemv1_bl_body<NintCodec<2, 2>, XMODE, false, true>(a, w, smem); break;
@@ -262,7 +278,7 @@ bool launch_moe_hetero_gemv1(GemvArgsB base, const NintDevB* pools, const int* h
     const size_t smem = (size_t)((base.private_sums ? 8 : 1) + 1) * base.rb_per_cta * 16 * 4 + ring;
     auto kernel = base.x_mode == 2 ? moe_hetero_gemv1_kernel<2> : (base.x_mode == 1 ? moe_hetero_gemv1_kernel<1> : moe_hetero_gemv1_kernel<0>);
     static bool attr_set[3][64] = {};
-    if (smem > 48 * 1024 && !attr_set[base.x_mode][device]) {
+    if (smem + sizeof(int2) * kHeteroTable > 48 * 1024 && !attr_set[base.x_mode][device]) {
         MFQB_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         attr_set[base.x_mode][device] = true;
     }

@@ -66,6 +66,8 @@ struct GemvArgsB {
     const int* route_ids;    // [pairs] expert of each pair; nullptr = plain GEMV
     const int* expert_pool;  // [experts] cohort index of each expert (-1: not held here)
     const int* expert_local; // [experts] position of the expert inside its cohort
+    int ids_ready;           // route_ids were complete before the kernel ahead in the stream let this one start
+    int pair_local;          // all-cohort kernel: the pair's position inside its cohort + 1 once looked up, 0 = look it up here
     int pool;                // cohort this launch covers
     int rb_per_expert;       // rows_per_expert / 16
     int routes;              // routes per token (R)
@@ -523,11 +525,16 @@ __device__ __forceinline__ void gemv1_bl_body(const GemvArgsB& a, const NintDevB
     size_t y_off = 0;
     const bool routed = !DENSE && a.route_ids != nullptr;
     if (routed) {
-        pdl_wait_b();   // the routing table comes from the previous kernel
-        const int pair = blockIdx.y, e = a.route_ids[pair];
-        if (e < 0 || a.expert_pool[e] != a.pool) return;
+        const int pair = blockIdx.y;
+        int local = a.pair_local - 1;
+        if (local < 0) {
+            pdl_wait_b();   // the routing table comes from the previous kernel
+            const int e = a.route_ids[pair];
+            if (e < 0 || a.expert_pool[e] != a.pool) return;
+            local = a.expert_local[e];
+        }
         rb_total = a.rb_per_expert;
-        rb_base = a.expert_local[e] * a.rb_per_expert;
+        rb_base = local * a.rb_per_expert;
         if constexpr (XMODE == 0) xrow += (size_t)(a.x_per_pair ? pair : pair / a.routes) * w.k;
         y_off = (size_t)pair * a.ldy;
     }
