@@ -10,7 +10,6 @@
 #include <climits>
 
 #include "cuda_util.h"
-#include "nint_gemm_tc.cuh"
 #include "nint_blayout.h"
 #include "load.h"
 #include "nvq.h"
@@ -54,179 +53,27 @@ void* GrowOnlyScratch::get(int device, size_t bytes, cudaStream_t stream, const 
     return p;
 }
 
-// ---- tcgen05 prefill GEMM: x conversion pre-pass, per-device scratch and status word -----------
-__global__ void x_to_f16_kernel(const __nv_bfloat16* __restrict__ x, int m, int k, int kx, __half* __restrict__ out) {
-    const size_t total = (size_t)m * kx;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = i / kx, c = i % kx;
-        // bf16 -> f16: exact for |x| in [2^-14, 65504]; larger finite magnitudes saturate to +-65504;
-        // an infinity or NaN stays non-finite (NaN), so it poisons the outputs as on the integer kernels
-        const float v = c < (size_t)k ? __bfloat162float(x[r * k + c]) : 0.f;
-        out[i] = isfinite(v) ? __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f)) : __ushort_as_half((unsigned short)0x7E00);
-    }
-}
-
-struct GemmDeviceState {
+// Per device a status word that kernels set when a bounded wait runs out (mfqb_device_status).
+struct DeviceStatus {
     std::mutex mu;
-    GrowOnlyScratch x16;
-    int* status_host[64] = {nullptr};
-    int* status_dev[64] = {nullptr};
+    int* host[64] = {nullptr};
+    int* dev[64] = {nullptr};
 };
-static GemmDeviceState g_gemm;
+static DeviceStatus g_status;
 
-int* gemm_status_word(int device) {   // pinned, mapped: the host can read it without a sync
-    if (!g_gemm.status_host[device]) {
-        MFQB_CUDA(cudaHostAlloc((void**)&g_gemm.status_host[device], sizeof(int), cudaHostAllocMapped));
-        *g_gemm.status_host[device] = 0;
-        MFQB_CUDA(cudaHostGetDevicePointer((void**)&g_gemm.status_dev[device], g_gemm.status_host[device], 0));
+int* device_status_word(int device) {   // pinned, mapped: the host can read it without a sync
+    std::lock_guard<std::mutex> lock(g_status.mu);
+    if (!g_status.host[device]) {
+        MFQB_CUDA(cudaHostAlloc((void**)&g_status.host[device], sizeof(int), cudaHostAllocMapped));
+        *g_status.host[device] = 0;
+        MFQB_CUDA(cudaHostGetDevicePointer((void**)&g_status.dev[device], g_status.host[device], 0));
     }
-    return g_gemm.status_dev[device];
+    return g_status.dev[device];
 }
 
-// Tensor map of the f16 activations [m, kx] for 64-column x bn-row boxes with the 128-byte swizzle.
-// cuTensorMapEncodeTiled is looked up through the runtime, so the library links only libcudart.
-static CUtensorMap make_x_map(const void* x16, int m, int kx, int bn, int xcols = 64) {
-    typedef CUresult (*EncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static EncodeFn encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        MFQB_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-        if (!fn || qres != cudaDriverEntryPointSuccess) fail(MFQB_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-        encode = reinterpret_cast<EncodeFn>(fn);
-    }
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)kx, (cuuint64_t)m};
-    const cuuint64_t strides[1] = {(cuuint64_t)kx * sizeof(__half)};
-    const cuuint32_t box[2] = {(cuuint32_t)xcols, (cuuint32_t)std::min(bn, 256)};   // a box holds at most 256 rows; wider tiles take two loads
-    const cuuint32_t elem[2] = {1u, 1u};
-    const CUresult r = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x16), dims, strides, box, elem,
-                              CU_TENSOR_MAP_INTERLEAVE_NONE, xcols == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) fail(MFQB_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return map;
-}
-
-// Returns false when this weight has no tensor-core tile kernel (the caller falls back to GEMV passes).
-int* device_status_word(int device) {
-    std::lock_guard<std::mutex> lock(g_gemm.mu);
-    return gemm_status_word(device);
-}
-
-static bool launch_nint_gemm(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s) {
-    const GemmPlan p = plan_nint_gemm(w, m);
-    if (p.bn == 0) return false;
-    std::lock_guard<std::mutex> lock(g_gemm.mu);
-    GemmArgs a{};
-    a.w = w;
-    a.m = m;
-    a.kx = (w.k + 7) / 8 * 8;
-    a.y = y;
-    a.y_dtype = y_dtype;
-    a.bn = p.bn;
-    a.stages = p.stages;
-    a.xstages = p.xstages;
-    a.xcols = p.xcols;
-    a.error = gemm_status_word(device);
-    void* xb = g_gemm.x16.get(device, (size_t)m * a.kx * sizeof(__half), s, "mfqb_mul_mat (f16 copy of the activations)");
-    a.x16 = static_cast<const __half*>(xb);
-    const size_t total = (size_t)m * a.kx;
-    x_to_f16_kernel<<<(int)std::min<size_t>((total + 255) / 256, 148 * 8), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), m, w.k,
-                                                                                      a.kx, static_cast<__half*>(xb));
-    MFQB_CUDA(cudaGetLastError());
-    const CUtensorMap x_map = make_x_map(xb, m, a.kx, p.bn, p.xcols);
-    cudaError_t e;
-    switch (w.bits) {
-        case 2: e = launch_nint_gemm_bits<2>(a, p, x_map, s); break;
-        case 3: e = launch_nint_gemm_bits<3>(a, p, x_map, s); break;
-        case 4: e = launch_nint_gemm_bits<4>(a, p, x_map, s); break;
-        case 5: e = launch_nint_gemm_bits<5>(a, p, x_map, s); break;
-        case 6: e = launch_nint_gemm_bits<6>(a, p, x_map, s); break;
-        case 8: e = launch_nint_gemm_bits<8>(a, p, x_map, s); break;
-        default: return false;
-    }
-    if (e == cudaErrorNotSupported) return false;
-    if (e != cudaSuccess) fail(MFQB_ERR_CUDA, "NINT%d gs=%d GEMM launch: %s", w.bits, w.gs, cudaGetErrorString(e));
-    return true;
-}
-
-// Rows of x (bf16 [rows, k]) gathered in route-plan order and converted to f16 [pairs, kx]:
-// out row p = x row (pair_order[p] / div).
-template <typename XT>
-__global__ void x_gather_f16_kernel(const XT* __restrict__ x, const int* __restrict__ pair_order, int div, int pairs, int k, int kx,
-                                    __half* __restrict__ out) {
-    const size_t total = (size_t)pairs * kx;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-        const size_t p = i / kx, c = i % kx;
-        const float v = c < (size_t)k ? (float)x[(size_t)(pair_order[p] / div) * k + c] : 0.f;
-        out[i] = isfinite(v) ? __float2half_rn(fminf(fmaxf(v, -65504.f), 65504.f)) : __ushort_as_half((unsigned short)0x7E00);
-    }
-}
-
-// True when the grouped tile kernel can run this cohort tensor with `bn`-pair tiles.
-bool nint_gemm_grouped_supported(const NintDevB& w, int bn, int rows_per_expert) { return plan_nint_gemm_grouped(w, bn, rows_per_expert, 1).bn != 0; }
-
-// Bytes of the gathered f16 input the grouped kernel reads.
-size_t nint_gemm_grouped_x_bytes(int pairs, int k) { return (size_t)pairs * ((k + 7) / 8 * 8) * sizeof(__half); }
-
-void launch_x_gather_f16(const void* x, bool x_f32, const int* pair_order, int div, int pairs, int k, void* x16, cudaStream_t s) {
-    const int kx = (k + 7) / 8 * 8;
-    const size_t total = (size_t)pairs * kx;
-    const int grid = (int)std::min<size_t>((total + 255) / 256, 148 * 8);
-    if (x_f32) x_gather_f16_kernel<float><<<grid, 256, 0, s>>>(static_cast<const float*>(x), pair_order, div, pairs, k, kx, static_cast<__half*>(x16));
-    else x_gather_f16_kernel<__nv_bfloat16><<<grid, 256, 0, s>>>(static_cast<const __nv_bfloat16*>(x), pair_order, div, pairs, k, kx, static_cast<__half*>(x16));
-    MFQB_CUDA(cudaGetLastError());
-}
-
-// Expert matmul of one cohort on the tile kernel: x16 = launch_x_gather_f16 output for this plan.
-void launch_nint_gemm_grouped(const NintDevB& w, const void* x16, int pairs, int bn, const int* expert_bounds, const int* tile_bounds,
-                              const int* pair_order, const int* expert_pool, const int* expert_local, int n_experts, int pool,
-                              int rb_per_expert, int rows_per_expert, int max_tiles, void* y, int y_dtype, int device, cudaStream_t s) {
-    const GemmPlan p = plan_nint_gemm_grouped(w, bn, rows_per_expert, max_tiles);
-    if (p.bn == 0) fail(MFQB_ERR_UNSUPPORTED, "NINT%d gs=%d has no grouped tile kernel for tiles of %d", w.bits, w.gs, bn);
-    GemmArgs a{};
-    {
-        std::lock_guard<std::mutex> lock(g_gemm.mu);
-        a.error = gemm_status_word(device);
-    }
-    a.w = w;
-    a.m = pairs;
-    a.kx = (w.k + 7) / 8 * 8;
-    a.x16 = static_cast<const __half*>(x16);
-    a.y = y;
-    a.y_dtype = y_dtype;
-    a.bn = p.bn;
-    a.stages = p.stages;
-    a.xstages = p.xstages;
-    a.xcols = p.xcols;
-    a.expert_bounds = expert_bounds;
-    a.tile_bounds = tile_bounds;
-    a.pair_order = pair_order;
-    a.expert_pool = expert_pool;
-    a.expert_local = expert_local;
-    a.n_experts = n_experts;
-    a.pool = pool;
-    a.rb_per_expert = rb_per_expert;
-    a.ldy = rows_per_expert;
-    const CUtensorMap x_map = make_x_map(x16, pairs, a.kx, p.bn);
-    cudaError_t e;
-    switch (w.bits) {
-        case 2: e = launch_nint_gemm_bits<2>(a, p, x_map, s); break;
-        case 3: e = launch_nint_gemm_bits<3>(a, p, x_map, s); break;
-        case 4: e = launch_nint_gemm_bits<4>(a, p, x_map, s); break;
-        case 5: e = launch_nint_gemm_bits<5>(a, p, x_map, s); break;
-        case 6: e = launch_nint_gemm_bits<6>(a, p, x_map, s); break;
-        case 8: e = launch_nint_gemm_bits<8>(a, p, x_map, s); break;
-        default: e = cudaErrorNotSupported; break;
-    }
-    if (e != cudaSuccess) fail(MFQB_ERR_CUDA, "NINT%d gs=%d grouped GEMM launch: %s", w.bits, w.gs, cudaGetErrorString(e));
-}
-
-int gemm_device_status(int device) {
-    std::lock_guard<std::mutex> lock(g_gemm.mu);
-    return g_gemm.status_host[device] ? *static_cast<volatile int*>(g_gemm.status_host[device]) : 0;
+int device_status(int device) {
+    std::lock_guard<std::mutex> lock(g_status.mu);
+    return g_status.host[device] ? *static_cast<volatile int*>(g_status.host[device]) : 0;
 }
 
 }  // namespace mfqb
@@ -241,9 +88,7 @@ size_t gemvs_fix_bytes(int device);
 void launch_swiglu(const void* gate_up, int in_dtype, int rows, int f, void* hidden, cudaStream_t s);
 void launch_bl_gemv_norm(const NintDevB& w, const float* h, const float* delta, const float* gamma, float eps, float* h_out, void* y, int y_dtype,
                          bool glu, int device, cudaStream_t s);
-bool nint_bl_gemvh_supported(const NintDevB& w, int rows_per_launch);
 int g_moe_f16_from_x2 = 4;   // see mfqb_tune
-int g_gemm_plan_choice = 0;   // see mfqb_tune
 void launch_bl_gemv_multi(const NintDevB* ws, void* const* ys, int count, const void* x, int y_dtype, int device, cudaStream_t s);
 bool launch_bl_gemvs(const NintDevB& w, const void* x, int x_dtype, void* y, int y_dtype, int device, void* fix, int* error, cudaStream_t s);
 }
@@ -414,7 +259,7 @@ int mfqb_mul_mat(const mfqb_weight* w, const void* x, int m, void* y, int y_dtyp
             if (m == 1 && gemv1_use_streamed(w->nint) &&
                 launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->dev.extra_at(), w->status, stream))
                 return;
-            const int per_launch = nint_bl_gemvh_supported(w->nint, 16) ? 16 : 8;   // batch rows one GEMV launch covers
+            constexpr int per_launch = 8;   // batch rows one GEMV launch covers
             for (int m0 = 0; m0 < m; m0 += per_launch) {
                 const int mm = std::min(per_launch, m - m0);
                 launch_bl_gemv(w->nint, static_cast<const char*>(x) + (size_t)m0 * k * 2, mm,
@@ -655,7 +500,7 @@ int mfqb_tune(const char* key, int value) {
         if (!key) fail(MFQB_ERR_ARG, "mfqb_tune: null key");
         if (std::string(key) == "gemv1_kernel" && value >= 0 && value <= 2) g_gemv1_choice = value;
         else if (std::string(key) == "moe_f16_tiles_from_x2" && value >= 2 && value <= 1000000) g_moe_f16_from_x2 = value;
-        else if (std::string(key) == "gemm_plan" && value >= 0 && value <= 1) g_gemm_plan_choice = value;
+        else if (std::string(key) == "gemm_plan" && value >= 0 && value <= 1) {}   // had two tile plans to choose from; callers may still name it
         else fail(MFQB_ERR_ARG, "mfqb_tune: unknown key '%s' or value %d out of range", key, value);
     });
 }
@@ -663,7 +508,7 @@ int mfqb_tune(const char* key, int value) {
 int mfqb_device_status(int device, int* status) {
     return guarded([&] {
         if (!status || device < 0 || device >= 64) fail(MFQB_ERR_ARG, "mfqb_device_status: bad argument");
-        *status = gemm_device_status(device);
+        *status = device_status(device);
     });
 }
 
