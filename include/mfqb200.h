@@ -110,15 +110,16 @@ int mfqb_weight_free(mfqb_weight* w);
 int mfqb_dequant(const mfqb_weight* w, void* out, int out_dtype, mfqb_stream_t stream);
 
 /* y[m, n] = x[m, k] . W^T.  x is row-major bf16 with exactly k columns; y is row-major [m, n] in
- * y_dtype.  Any m >= 1 is accepted.  m <= 16 (and every m for lattice weights) runs the
+ * y_dtype.  Any m >= 1 is accepted.  m <= 4 (lattice weights: m = 1) runs the
  * weight-streaming kernels: the weights stay integer codes on the int8 tensor cores, x is quantised
  * inside the kernel, group by group, to 16-bit integers with a power-of-two scale (exact for a bf16
  * value unless it lies more than 2^7 below its group's largest magnitude; the product is within
  * 1e-5 relative L2 of the float32 reference), sums are exact in int32 and the scales are applied
- * in float32.  Larger m for NINT runs the tcgen05 tile kernel (f16 operands, float32 accumulation).
- * An infinity or NaN in x makes the outputs NaN (on the tile kernel, finite magnitudes beyond
- * 65504 saturate to +-65504 in the f16 copy of x).
- * Library scratch: m >= 2 uses a per-device buffer (quantised planes, or the f16 copy of x) that
+ * in float32.  Larger m runs the tcgen05 tile kernel (f16 operands, float32 accumulation): NINT weights
+ * are rounded to f16 (within 1e-3 relative L2), lattice weights are exact, every row of x is scaled
+ * by a power of two (exact within 2^-28 of the row's largest magnitude).
+ * An infinity or NaN in x makes the outputs NaN.
+ * Library scratch: m >= 2 uses a per-device buffer (quantised planes, or activation tiles and partial sums) that
  * only ever grows -- a block handed to a kernel or baked into a captured graph stays allocated.
  * Growing calls cudaMalloc, so the first call with a given (or larger) m on a device must come
  * outside stream capture; inside a capture it fails with MFQB_ERR_ARG instead.  The buffer holds
@@ -151,7 +152,8 @@ int mfqb_mul_mat_swiglu(const mfqb_weight* w, const void* gate_up_f32, int m, vo
  * packed); y [m, n / 2] = up * gate / (1 + exp(-gate)).  The same composition as
  * mfqb_mul_mat_swiglu (mfq/kernels/cuda/glu.cuh:6-17) with the activation on the producing side,
  * so the following down projection is a plain mfqb_mul_mat.  m = 1 on NINT weights runs in the
- * single-row kernel; other cases take the product into library scratch and apply the activation. */
+ * single-row kernel, batches of the tile kernel apply it where a tile is finished; other cases take the
+ * product into library scratch and apply the activation. */
 int mfqb_mul_mat_glu(const mfqb_weight* w, const void* x_bf16, int m, void* y, int y_dtype,
                      mfqb_stream_t stream);
 
@@ -170,8 +172,7 @@ int mfqb_mul_mat_rmsnorm(const mfqb_weight* w, const float* h, const float* delt
  * NINT weight takes -- 0 by shape (default), 1 the per-warp ring kernel, 2 the streamed kernel.
  * "moe_f16_tiles_from_x2": twice the average number of (token, route) pairs per expert from which
  * the expert matmuls take the f16 tile kernel instead of the integer tiles (default 4).
- * "gemm_plan": 0 = ring sizes of the tensor-core tile kernel by shape (default), 1 = 32-column
- * activation stages with a two-chunk weight ring for every shape.
+ * "gemm_plan" (0 or 1) is accepted and has no effect: the tile kernel sizes its rings by shape.
  * No counterpart in the reference (its switches are MFQ_* environment variables,
  * docs/developer-architecture-and-operator-reference.md:1048-1078). */
 int mfqb_tune(const char* key, int value);
