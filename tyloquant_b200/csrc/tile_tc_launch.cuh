@@ -14,6 +14,7 @@ struct TilePlan {
 // A plain product, or one cohort of an expert product: one codec.
 template <class C>
 struct TileOne {
+    static constexpr bool ONE = true;
     static constexpr int TERMS = C::TERMS;
     template <class Fn>
     __device__ static __forceinline__ void dispatch(const NintDevB&, Fn&& f) { f(C{}); }

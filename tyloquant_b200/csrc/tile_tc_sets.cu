@@ -20,6 +20,7 @@ cudaError_t launch_tile_nvq(const TileArgs& a, const TilePlan& p, int terms, cud
 
 // Every cohort of an expert record in one launch: the codecs of the per-expert precision profiles.
 struct TileExperts {
+    static constexpr bool ONE = false;
     static constexpr int TERMS = 1;
     template <class Fn>
     __device__ static __forceinline__ void dispatch(const NintDevB& w, Fn&& f) {
