@@ -190,3 +190,22 @@ def test_one_token_calls_back_to_back_past_the_expert_table():
         assert rel_l2(y.cpu().numpy(), O.moe_ffn(x, gu_ref, dn_ref, rid, rw)) <= REL_L2
     gu.free()
     dn.free()
+
+
+@pytest.mark.parametrize("tokens", [2, 6, 64])
+def test_gate_up_shard_beside_a_whole_down_weight(tokens):
+    """Routes to experts that only the down weight holds add nothing, whatever earlier calls left in the scratch: the single-row
+    kernels, the integer tiles and the tensor-memory tiles."""
+    e_count, h, f, k = 8, 256, 96, 2
+    gu_blob, dn_blob = _moe_case(e_count, h, f, [4, 6] * 4, seed=31)
+    gu, dn = moe.MoeWeight(gu_blob), moe.MoeWeight(dn_blob)
+    gu_shard, dn_shard = moe.MoeWeight(gu_blob, 0, 2, 5), moe.MoeWeight(dn_blob, 0, 2, 5)
+    rng = np.random.default_rng(32)
+    x = bf16_tensor(encode.bf16_round(rng.standard_normal((tokens, h), dtype=np.float32)))
+    ids, wts = moe.moe_topk(torch.from_numpy(rng.standard_normal((tokens, e_count)).astype(np.float32)).cuda(), k)
+    moe.moe_ffn(gu, dn, 64.0 * x, ids, wts)
+    got = moe.moe_ffn(gu_shard, dn, x, ids, wts)
+    want = moe.moe_ffn(gu_shard, dn_shard, x, ids, wts)
+    assert (got - want).abs().max().item() <= 1e-5 * want.abs().max().item()   # float32 sums in another order
+    for w in (gu, dn, gu_shard, dn_shard):
+        w.free()

@@ -452,6 +452,9 @@ static void moe_ffn_run(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* d
     }
     char* planes = s + L.o_planes;
     if (L.tiles_tc) {   // the gate|up products stay in plan order; the down product's activation tiles form SwiGLU from them in float32
+        // Experts that only `down` holds have no gate|up product: their rows are zeros, not what an earlier call left there.
+        if (gate_up->info.expert_begin > down->info.expert_begin || gate_up->info.expert_end < down->info.expert_end)
+            MFQB_CUDA(cudaMemsetAsync(gu, 0, pairs * gate_up->info.out_per_expert * sizeof(float), stream));
         moe_tiles_tc(gate_up, plan, L.tile_m, (int)pairs, x, kTileXBf16, routes, planes, gu, MFQB_F32, false, stream);
         clear_unheld(down, (int)pairs, dn, MFQB_F32, stream);
         moe_tiles_tc(down, plan, L.tile_m, (int)pairs, gu, kTileXSwiglu, 0, planes, dn, MFQB_F32, true, stream);
