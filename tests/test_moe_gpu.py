@@ -209,3 +209,25 @@ def test_gate_up_shard_beside_a_whole_down_weight(tokens):
     assert (got - want).abs().max().item() <= 1e-5 * want.abs().max().item()   # float32 sums in another order
     for w in (gu, dn, gu_shard, dn_shard):
         w.free()
+
+
+def test_more_pairs_than_a_grid_dimension():
+    """8200 tokens of 8 routes: 65,600 pairs through the routed product and the FFN."""
+    e_count, h, f, tokens, routes = 8, 48, 24, 8200, 8
+    gu_blob, dn_blob = _moe_case(e_count, h, f, [4, 6] * 4, seed=41)
+    gu, dn = moe.MoeWeight(gu_blob), moe.MoeWeight(dn_blob)
+    gen = torch.Generator("cuda").manual_seed(42)
+    x = torch.randn(tokens, h, device="cuda", generator=gen).to(torch.bfloat16)
+    ids, wts = moe.moe_topk(torch.randn(tokens, e_count, device="cuda", generator=gen), routes)
+    gw, dw = (torch.stack([w.dequantize_expert(e) for e in range(e_count)]).double() for w in (gu, dn))
+    every = torch.einsum("th,eoh->teo", x.double(), gw)
+    want = torch.gather(every, 1, ids.long()[:, :, None].expand(-1, -1, 2 * f))
+    got = gu.matmul_id(x, ids, out_dtype=torch.float32).double()
+    assert ((got - want).norm() / want.norm()).item() <= REL_L2
+    act = every[..., f:] * every[..., :f] / (1 + torch.exp(-every[..., :f]))
+    out = torch.gather(torch.einsum("tef,ehf->teh", act, dw), 1, ids.long()[:, :, None].expand(-1, -1, h))
+    want = (out * wts.double()[:, :, None]).sum(1)
+    got = moe.moe_ffn(gu, dn, x, ids, wts).double()
+    assert ((got - want).norm() / want.norm()).item() <= REL_L2
+    gu.free()
+    dn.free()

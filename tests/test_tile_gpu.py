@@ -92,3 +92,19 @@ def test_gated_epilogue(n, k):
             got = w.matmul_glu(x, out_dtype=dtype).double()
             assert ((got - want).norm() / want.norm()).item() <= bound, (n, m, dtype)
     assert _status() == 0
+
+
+@pytest.mark.parametrize("m", [65535, 65536, 70000])
+def test_more_rows_than_a_grid_dimension(m):
+    n, k = 40, 72
+    wt = np.random.default_rng(1).standard_normal((n, k)).astype(np.float32) * np.float32(0.02)
+    for dtype, blob, bound in (("NINT4", encode.random_nint_blob(n, k, 4, 24, 6, seed=3, device="cuda"), REL_L2),
+                               ("NVQ3", encode.nvq_blob(encode.quantize_nvq3(wt, O.d4_256_codebook()[None], jsc=False, device="cuda")), 1e-5)):
+        w = QuantWeight.from_blob(dtype, blob)
+        x = torch.randn(m, k, device="cuda", generator=torch.Generator("cuda").manual_seed(m)).to(torch.bfloat16)
+        want = x.double() @ w.dequantize().double().T
+        got = w.matmul(x, out_dtype=torch.float32).double()
+        assert ((got - want).norm() / want.norm()).item() <= bound, dtype
+        assert ((got[-64:] - want[-64:]).norm() / want[-64:].norm()).item() <= bound, dtype
+        w.free()
+    assert _status() == 0

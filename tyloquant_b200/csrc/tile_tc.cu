@@ -105,15 +105,16 @@ __device__ __forceinline__ void x_write_slabs(const void* row, bool row_al, int 
 // Scales a row to the top of the f16 range and writes it as B operand: per 64-column slab the tile's rows of 128 bytes with
 // the 128-byte swizzle, columns in the decoders' order (slab of 16 columns (f, t, h): octet t of groups 4f + 2h, + 1; quads
 // c = 0..3 of these 16 slots, their slots 0 and 2 in columns 2c, 2c + 1, slots 1 and 3 in columns 8 + 2c, + 1).  Slots past
-// the group size, groups and columns past the row are zero.  Grid (splits, rows): every CTA takes the row's maximum for
-// itself (from L2; a second launch for the maxima costs more for the rows of a decoding batch) and writes its share.
+// the group size, groups and columns past the row are zero.  Grid (rows, splits), for a grid's other dimensions end at 65535:
+// every CTA takes the row's maximum for itself (from L2; a second launch for the maxima costs more for the rows of a decoding
+// batch) and writes its share.
 template <int KIND>
 __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XTilesArgs a) {
     extern __shared__ __align__(16) unsigned char x_row[];   // bf16 rows: kept between the two passes (a.staged)
     __shared__ uint32_t red[8];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int p = blockIdx.y;
+    const int p = blockIdx.x;
     int pool = 0, src = p, tile_begin = p / a.x_rows * a.x_rows, ncols = min(a.x_rows, a.m - tile_begin), base = tile_begin;
     if (a.tile_bounds != nullptr) {
         if (p >= a.expert_bounds[a.n_experts]) return;
@@ -167,13 +168,13 @@ __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XT
 #pragma unroll
     for (int i = 0; i < 8; ++i) ab = max(ab, red[i]);
     const float2 sc = x_row_scale(ab);
-    if (blockIdx.x == 0 && tid == 0) a.down[p] = sc.y;
+    if (blockIdx.y == 0 && tid == 0) a.down[p] = sc.y;
     const int r = p - tile_begin, pitch = ((ncols + 7) & ~7) * 128;
     unsigned char* dst = a.out + (size_t)base * a.row_bytes + (size_t)r * 128;
     if (KIND == kTileXBf16 && a.staged && (reinterpret_cast<uintptr_t>(row) & 15) == 0 && (k & 7) == 0)
-        x_write_slabs<kTileXShared>(x_row, true, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.x * 256 + tid, gridDim.x * 256);
+        x_write_slabs<kTileXShared>(x_row, true, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.y * 256 + tid, gridDim.y * 256);
     else
-        x_write_slabs<KIND>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.x * 256 + tid, gridDim.x * 256);
+        x_write_slabs<KIND>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.y * 256 + tid, gridDim.y * 256);
 }
 
 // The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the
@@ -258,7 +259,7 @@ static void launch_x_tiles(XTilesArgs a, int kind, int rows, int nslabs, int sms
     // a second trip to L2 for the values costs a decoding batch 0.7 us of its chain; rows of up to 32 KB fit beside a tile CTA
     a.staged = kind == kTileXBf16 && a.k <= 16384 && rows <= 64;
     if (a.staged) cfg.dynamicSmemBytes = (size_t)(a.k + 7) / 8 * 16;
-    cfg.gridDim = dim3((unsigned)splits, (unsigned)rows);
+    cfg.gridDim = dim3((unsigned)rows, (unsigned)splits);
     cfg.blockDim = dim3(256);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
