@@ -82,3 +82,22 @@ def test_static_scratch_ffn_matches_allocating_ffn_twice_in_a_row():
     assert "scratch" in msg and str(8 << 20) in msg
     gu.free()
     dn.free()
+
+
+@pytest.mark.parametrize("tokens", [32, 40])
+def test_static_scratch_batches_whose_activation_tiles_do_not_fit(tokens):
+    """Two pairs per expert and more: where the tile kernel's scratch is too large for the array, the integer kernels run."""
+    e_count, h, f, k = 128, 2048, 768, 8
+    gen = torch.Generator("cuda").manual_seed(3)
+    bits = [3, 4, 5, 8] * 32
+    gu, dn = (moe.MoeWeight(encode.quantize_expertwise(torch.randn(shape, device="cuda", generator=gen) * 0.02, bits, device="cuda"))
+              for shape in ((e_count, 2 * f, h), (e_count, h, f)))
+    x = torch.randn(tokens, h, device="cuda", generator=gen).to(torch.bfloat16)
+    ids, wts = moe.moe_topk(torch.randn(tokens, e_count, device="cuda", generator=gen), k)
+    rc, want = _ffn(lib.mfqb_moe_ffn, gu, dn, x, ids, wts)
+    assert rc == 0, lib.mfqb_last_error()
+    rc, got = _ffn(lib.mfqb_moe_ffn_static, gu, dn, x, ids, wts)
+    assert rc == 0, lib.mfqb_last_error()
+    assert ((got - want).norm() / want.norm()).item() <= 1e-3
+    gu.free()
+    dn.free()

@@ -486,12 +486,13 @@ static void check_ffn_args(const char* who, const mfqb_moe_weight* gate_up, cons
     if ((long long)tokens * routes > INT_MAX) fail(MFQB_ERR_ARG, "%s: %d tokens x %d routes is more than the kernels index", who, tokens, routes);
 }
 
-static FfnLayout ffn_layout(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* down, int tokens, int routes) {
+// allow_tc: the tensor-memory tile kernel may be used (its activation tiles take more scratch than the integer kernels' planes).
+static FfnLayout ffn_layout(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* down, int tokens, int routes, bool allow_tc = true) {
     FfnLayout L{};
     const int h = gate_up->info.k, f2 = gate_up->info.out_per_expert, f = f2 / 2, e = gate_up->info.n_experts;
     const size_t pairs = (size_t)tokens * routes;
     auto up256 = [](size_t v) { return (v + 255) / 256 * 256; };
-    L.tiles_tc = moe_use_tiles_tc(gate_up, (int)pairs) && moe_use_tiles_tc(down, (int)pairs);
+    L.tiles_tc = allow_tc && moe_use_tiles_tc(gate_up, (int)pairs) && moe_use_tiles_tc(down, (int)pairs);
     L.tile_m = L.tiles_tc ? tile_experts_rows((int)pairs, e) : std::min(moe_tile_m(gate_up, (int)pairs), moe_tile_m(down, (int)pairs));
     L.tiles = !L.tiles_tc && L.tile_m != 0;
     L.fused_tail = !L.tile_m && ffn_fused_tail_ok(down, tokens, (int)pairs) && ffn_fused_tail_ok(gate_up, tokens, (int)pairs);
@@ -559,7 +560,8 @@ int mfqb_moe_ffn_static(const mfqb_moe_weight* gate_up, const mfqb_moe_weight* d
         if (!gate_up || !down || !x || !ids || !weights || !y) fail(MFQB_ERR_ARG, "mfqb_moe_ffn_static: null argument");
         check_ffn_args("mfqb_moe_ffn_static", gate_up, down, tokens, routes);
         if (tokens <= 0) return;
-        const FfnLayout L = ffn_layout(gate_up, down, tokens, routes);
+        FfnLayout L = ffn_layout(gate_up, down, tokens, routes);
+        if (L.total > (size_t)MFQB_STATIC_SCRATCH_BYTES) L = ffn_layout(gate_up, down, tokens, routes, false);   // the integer kernels need less
         if (L.total > (size_t)MFQB_STATIC_SCRATCH_BYTES)
             fail(MFQB_ERR_ARG,
                  "mfqb_moe_ffn_static: %d tokens x %d routes need %llu bytes of scratch, the built-in array holds %llu; "
