@@ -117,7 +117,8 @@ int mfqb_dequant(const mfqb_weight* w, void* out, int out_dtype, mfqb_stream_t s
  * 1e-5 relative L2 of the float32 reference), sums are exact in int32 and the scales are applied
  * in float32.  Larger m runs the tcgen05 tile kernel (f16 operands, float32 accumulation): NINT weights
  * are rounded to f16 (within 1e-3 relative L2), lattice weights are exact, every row of x is scaled
- * by a power of two (exact within 2^-28 of the row's largest magnitude).
+ * by a power of two (exact within 2^-28 of the row's largest magnitude), and sums are taken in a fixed
+ * order: the same call gives the same bits again.
  * An infinity or NaN in x makes the outputs NaN.
  * Library scratch: m >= 2 uses a per-device buffer (quantised planes, or activation tiles and partial sums) that
  * only ever grows -- a block handed to a kernel or baked into a captured graph stays allocated.

@@ -108,3 +108,28 @@ def test_more_rows_than_a_grid_dimension(m):
         assert ((got[-64:] - want[-64:]).norm() / want[-64:].norm()).item() <= bound, dtype
         w.free()
     assert _status() == 0
+
+
+# Shared tiles: two parts and whole tiles between them, one part of one tile per CTA, three parts, more parts than are added at once
+SHARED = [(14336, 4096, 4, 32, 6, 512), (4096, 14336, 6, 24, 7, 16), (5000, 2888, 4, 24, 6, 77), (520, 9000, 3, 24, 5, 33), (100, 24000, 2, 16, 5, 16),
+          (100, 24000, 2, 16, 5, 250), (300, 14336, 8, 48, 7, 8)]
+
+
+@pytest.mark.parametrize("n,k,bits,gs,sb,m", SHARED)
+def test_shared_tiles_have_the_same_bits_in_every_call(n, k, bits, gs, sb, m):
+    w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(n, k, bits, gs, sb, seed=n, device="cuda"))
+    other = QuantWeight.from_blob("NINT4", encode.random_nint_blob(700, 3000, 4, 24, 6, seed=1, device="cuda"))
+    gen = torch.Generator("cuda").manual_seed(m)
+    x = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+    xo = torch.randn(50, 3000, device="cuda", generator=gen).to(torch.bfloat16)
+    first = w.matmul(x, out_dtype=torch.float32)
+    want = x.double() @ w.dequantize().double().T
+    assert ((first.double() - want).norm() / want.norm()).item() <= REL_L2
+    for _ in range(20):
+        other.matmul(xo)
+        assert torch.equal(first, w.matmul(x, out_dtype=torch.float32))
+    if n % 32 == 0:
+        glu = w.matmul_glu(x, out_dtype=torch.float32)
+        for _ in range(5):
+            assert torch.equal(glu, w.matmul_glu(x, out_dtype=torch.float32))
+    assert _status() == 0

@@ -312,7 +312,8 @@ static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8,
         a.rec_stage_bytes = (int)rec_stage;
         a.x_stages = xs;
         a.x_stage_bytes = (int)x_stage;
-        p.smem = 1024 + std::max((size_t)xs * x_stage + (size_t)rs * rec_stage + ctx, (size_t)n * kTileRows * 4);   // a shared tile is finished there
+        p.smem = 1024 + std::max((size_t)xs * x_stage + (size_t)rs * rec_stage + ctx, std::max<size_t>(n, 32) * kTileRows * 4);   // a shared tile's parts are added there
+        a.sum_bytes = (int)p.smem - 1024;
         return true;
     }
     return false;
@@ -385,8 +386,8 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     // about as much as three chunks (1.5 to 2.5 us against 0.6 for a chunk of 16 tokens; both grow with the tokens), and half of
     // the second one is hidden behind the CTA's other part: with six chunks instead of three for two sums, 16 rows through NINT6
     // 4096 x 14336 took 22.4 us instead of 21.1, with none 8 rows through NVQ3 17408 x 5120 31.4 instead of 23.8.
-    // Without sharing there is no sum.  At most a dozen CTAs per tile: the last one adds the others' parts.
-    const long long split = std::min({(long long)sms / tiles, (long long)std::max(1, w.nchunks / 2), 12ll});
+    // Without sharing there is no sum.  At most a dozen CTAs per tile (kTileGroup): the last one adds the others' parts.
+    const long long split = std::min({(long long)sms / tiles, (long long)std::max(1, w.nchunks / 2), (long long)kTileGroup});
     const long long chunks_split = split ? (w.nchunks + split - 1) / split + (split > 1 ? 3 : 0) : 0, chunks_equal = (units + sms - 1) / sms + 3;
     a.split = split && chunks_split <= chunks_equal ? (int)split : 0;
     p.grid = a.split ? (int)(tiles * split) : (int)std::max<long long>(1, std::min<long long>(sms, (units + 1) / 2));
@@ -395,8 +396,8 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     unsigned char* buf = static_cast<unsigned char*>(xs[m > 16].get(device, xb + (size_t)m * 4, s, "mfqb_mul_mat (f16 activation tiles)"));
     a.x = buf;
     a.x_down = reinterpret_cast<const float*>(buf + xb);
-    a.partial = static_cast<float*>(parts.get(device, (size_t)p.grid * n * kTileRows * 4, s, "mfqb_mul_mat (partial tiles)"));
-    a.counters = static_cast<unsigned*>(counts.get(device, (size_t)p.grid * 4, s, "mfqb_mul_mat (tile counters)"));
+    a.partial = static_cast<float*>(parts.get(device, (size_t)p.grid * 2 * n * kTileRows * 4, s, "mfqb_mul_mat (parts of shared tiles)"));
+    a.counters = static_cast<unsigned*>(counts.get(device, (size_t)p.grid * 2 * 4, s, "mfqb_mul_mat (tile counters)"));
     XTilesArgs xa{};
     xa.x = x;
     xa.kind = kTileXBf16;

@@ -23,9 +23,12 @@
 // bits the weight is fed as two f16 terms whose sum is exact.  Activations: one power-of-two scale per token
 // (largest magnitude next to 2^15), exact for bf16 values within 2^-28 of the row's largest.
 //
-// Work split.  Plain products: the (tile, chunk) units are cut into equal contiguous ranges, one per CTA; a tile that
-// straddles CTAs is summed with float32 reductions in L2, and the last CTA to arrive finishes it (no CTA ever waits for
-// another; a first form in which it added up the others' partial tiles spent 25,000 cycles on the loads).  Expert products (route plan): item = (row tile, token tile of one expert), strided over the CTAs.
+// Work split.  Plain products: the (tile, chunk) units are cut into equal contiguous ranges, one per CTA, or every tile into
+// as many parts.  The CTAs that share a tile leave their parts in L2, and the last one to arrive adds them up in the order of
+// K, so a product has the same bits in every call (no CTA ever waits for another; float32 reductions into one copy, whose order
+// is that of arrival, took 84.1 us for four products of 16 rows, NINT6 4096 x 14336, this 84.4; 77 rows, three parts of 80
+// columns, NINT5 5000 x 2888: 70.6 and 76.0).  Expert products (route plan): item = (row
+// tile, token tile of one expert), strided over the CTAs.
 //
 // Every mbarrier wait is bounded: on expiry the CTA raises the device's status word, waits (bounded) for its own copies and
 // leaves through the common exit, which frees the tensor memory.
@@ -47,6 +50,7 @@ constexpr int kTileRows = 128, kTileDecoders = 16, kTileEpilogue = 4;
 constexpr int kTileWarpMma = kTileDecoders + kTileEpilogue, kTileWarpRec = kTileWarpMma + 1, kTileWarpX = kTileWarpMma + 2;
 constexpr int kTileThreads = (kTileDecoders + kTileEpilogue + 3) * 32;
 constexpr size_t kTileDynSmem = 212 * 1024;   // beside 14 KB of barriers and tables
+constexpr int kTileGroup = 12;   // parts of a shared tile that are added at once; more go in two steps
 constexpr int kTileMaxPools = 8, kTileRecStages = 8, kTileXStages = 8, kTileAStages = 8, kTileSegs = 4;
 
 struct TileArgs {
@@ -63,8 +67,9 @@ struct TileArgs {
     int glu;                         // plain product: rows come in 16-row blocks, gate and up in turn; y gets up * silu(gate) (the launch picks the kernel)
     int m, ntok;                     // plain product: tokens, token tiles
     int units, split;                // plain product: (tile, chunk) units; CTAs per tile, or 0: equal ranges of units
-    float* partial;                  // [grid][N][128] float32 sums of tiles that several CTAs share, by the tile's first CTA; zero between calls
-    unsigned* counters;              // [grid], zero between calls
+    float* partial;                  // [2 grid][N][128] float32 parts of tiles that several CTAs share, see tile_part
+    unsigned* counters;              // arrivals at a group of parts [grid], by the group's first CTA, and of groups at a tile [grid], by the tile's; zero between calls
+    int sum_bytes;                   // shared memory that the addition of parts may use
     // expert product over a route plan with tiles of x_rows pairs; tile_bounds == nullptr: plain product
     const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool, *expert_local;
     int n_experts, rb_per_expert, rows_per_expert, only_pool /* -1: every cohort */, scatter /* rows go to pair_order[p], else to p */;
@@ -100,6 +105,11 @@ __device__ __forceinline__ void tile_sharers(const TileArgs& a, int tile, int& s
     auto owner = [&](int u) { return (int)((((long long)u + 1) * grid - 1) / a.units); };
     slot0 = owner(tile * nch);
     parts = owner((tile + 1) * nch - 1) - slot0 + 1;
+}
+
+// Part p of a shared tile: a CTA has at most the end of one tile (or a middle part) and the beginning (part 0) of another.
+__device__ __forceinline__ float* tile_part(const TileArgs& a, int slot0, int p) {
+    return a.partial + (size_t)(2 * (slot0 + p) + (p == 0)) * a.n_mma * kTileRows;
 }
 
 // First row of an expert's tile in the tiles' buffer: every tile starts on a multiple of eight rows, and experts do not overlap.
@@ -262,8 +272,11 @@ struct TileShared {
     uint32_t tmem;
     int failed;
     unsigned last;
-    int finish;   // 1 + column table of the shared tile that this CTA finishes at its end, 0: none
-    TileSeg fin;
+    uint64_t sum_full[2];
+    // Groups of parts that this CTA was the last to arrive at, and adds up at its end: [0] with its last stretch, [1] with an
+    // earlier one (parts == 0: none).
+    TileSeg fin[2];
+    int fin_col;   // column table of fin[0]; its row factors are in row_factor
     __align__(16) float row_factor[kTileRows];
     __align__(16) uint4 rowc[kTileSegs][kTileRows];   // the stretches' row constants
     uint64_t seg_full[kTileSegs], seg_empty[kTileSegs];
@@ -307,6 +320,117 @@ __device__ __forceinline__ bool tile_epilogue_all(bool ok) {
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbarrier.cta.red.and.pred p, 1, 128, q;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(all) : "r"((uint32_t)ok) : "memory");
     return all != 0u;
+}
+
+// Adding up parts p0, p0 + step, ... of a shared tile, in this order (up to 128 KB each in L2, stored column by column): a block
+// of columns at a time comes into the rings' memory with bulk copies, two blocks in flight, then a warp takes a column, four
+// rows a lane.  (The four epilogue warps alone, sixteen loads in flight each, took 40,000 cycles for one part of N = 256.)
+struct TileSum {
+    int slot0, p0, step, count, ncols, cols, blocks;
+    __device__ __forceinline__ TileSum(const TileArgs& a, const TileSeg& t, int p0_, int step_, int count_) : slot0(t.slot0), p0(p0_), step(step_), count(count_), ncols(t.ncols) {
+        cols = max(1, min(ncols, a.sum_bytes / (2 * count * kTileRows * 4)));
+        blocks = (ncols + cols - 1) / cols;
+    }
+    __device__ __forceinline__ void request(const TileArgs& a, TileShared& sh, float* stage, int b) const {   // one thread
+        const int c0 = b * cols;
+        const uint32_t bytes = (uint32_t)min(cols, ncols - c0) * kTileRows * 4u;
+        asm volatile("fence.proxy.async;" ::: "memory");
+        mbar_arrive_expect_tx(&sh.sum_full[b & 1], bytes * (uint32_t)count);
+        for (int q = 0; q < count; ++q)
+            bulk_load(stage + (size_t)((b & 1) * count + q) * cols * kTileRows, tile_part(a, slot0, p0 + q * step) + (size_t)c0 * kTileRows, bytes, &sh.sum_full[b & 1]);
+    }
+    __device__ __forceinline__ void request_first(const TileArgs& a, TileShared& sh, float* stage) const {   // the stage is free
+        request(a, sh, stage, 0);
+        if (blocks > 1) request(a, sh, stage, 1);
+    }
+    // The whole CTA; the first blocks are requested.  phase: bit b, parity of the next wait on sum_full[b].
+    template <class Put>
+    __device__ __forceinline__ bool run(const TileArgs& a, TileShared& sh, float* stage, uint32_t& phase, Put&& put) const {
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        bool ok = true;
+        for (int b = 0; b < blocks && ok; ++b) {
+            ok = tile_wait(&sh.sum_full[b & 1], (phase >> (b & 1)) & 1u);
+            phase ^= 1u << (b & 1);
+            const float* src = stage + (size_t)(b & 1) * count * cols * kTileRows + 4 * lane;
+            const int c0 = b * cols, n = min(cols, ncols - c0);
+            if (ok)
+                for (int c = warp; c < n; c += kTileThreads / 32) {
+                    float4 v = *reinterpret_cast<const float4*>(src + c * kTileRows);
+                    for (int q = 1; q < count; ++q) {
+                        const float4 x = *reinterpret_cast<const float4*>(src + (q * cols + c) * kTileRows);
+                        v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+                    }
+                    put(c0 + c, v);
+                }
+            ok = __syncthreads_and(ok);
+            if (ok && threadIdx.x == 0 && b + 2 < blocks) request(a, sh, stage, b + 2);
+        }
+        return ok;
+    }
+};
+
+// First part of the group that this CTA's part belongs to, and how many the group has.
+__device__ __forceinline__ int2 tile_group(const TileSeg& t) {
+    const int p0 = ((int)blockIdx.x - t.slot0) / kTileGroup * kTileGroup;
+    return make_int2(p0, min(kTileGroup, t.parts - p0));
+}
+// Adds up a group of parts that this CTA was the last to arrive at, and where that is the last of the tile's groups, writes the
+// tile.  The whole CTA; sh.row_factor and `down` (x: the token's factor) are filled, the sum's first blocks requested.
+template <bool GLU>
+__device__ __forceinline__ bool tile_finish(const TileArgs& a, TileShared& sh, const TileSeg& t, const int2* down_of, float* stage, uint32_t& phase) {
+    const int tid = threadIdx.x, lane = tid & 31, groups = (t.parts + kTileGroup - 1) / kTileGroup;
+    const int2 g = tile_group(t);
+    TileSum sum(a, t, g.x, 1, g.y);
+    bool ok = true;
+    if (groups > 1) {
+        float* group_sum = tile_part(a, t.slot0, g.x) + 4 * lane;
+        ok = sum.run(a, sh, stage, phase, [&](int c, const float4& v) { __stcg(reinterpret_cast<float4*>(group_sum + (size_t)c * kTileRows), v); });
+        __threadfence();
+        __syncthreads();
+        sum = TileSum(a, t, 0, kTileGroup, groups);
+        if (ok && tid == 0) {
+            unsigned* counter = a.counters + gridDim.x + t.slot0;
+            sh.last = atomicAdd(counter, 1u);
+            if (sh.last == (unsigned)(groups - 1)) {
+                __threadfence();
+                *counter = 0u;
+                sum.request_first(a, sh, stage);
+            }
+        }
+        __syncthreads();
+        if (ok && sh.last != (unsigned)(groups - 1)) return true;
+    }
+    int row = t.row0 + 4 * lane, n = min(4, t.row_limit - row);
+    if constexpr (GLU) {   // gate rows are lanes 0-3 of every eight, their up rows lanes 4-7
+        if (lane & 4) n = 0;
+        row = (row >> 5) * 16 + (row & 15);
+    }
+    const float4 f = *reinterpret_cast<const float4*>(sh.row_factor + 4 * lane);
+    const bool vec = n == 4 && (a.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
+    ok = ok && sum.run(a, sh, stage, phase, [&](int c, const float4& v) {
+        const float down = __int_as_float(down_of[c].x);
+        float o[4] = {v.x * (f.x * down), v.y * (f.y * down), v.z * (f.z * down), v.w * (f.w * down)};
+        if constexpr (GLU) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = tile_gated(o[i], __shfl_xor_sync(0xffffffffu, o[i], 4));
+        }
+        const size_t at = (size_t)(t.tok0 + c) * a.ldy + row;   // (a plain product: its output rows are the tokens)
+        if (a.y_dtype == 0 /* MFQB_F32 */) {
+            float* y = reinterpret_cast<float*>(a.y) + at;
+            if (vec) *reinterpret_cast<float4*>(y) = make_float4(o[0], o[1], o[2], o[3]);
+            else
+                for (int i = 0; i < n; ++i) y[i] = o[i];
+        } else {
+            __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y) + at;
+            if (vec) {
+                const __nv_bfloat162 b0 = __floats2bfloat162_rn(o[0], o[1]), b1 = __floats2bfloat162_rn(o[2], o[3]);
+                *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&b0), *reinterpret_cast<const uint32_t*>(&b1));
+            } else {
+                for (int i = 0; i < n; ++i) y[i] = __float2bfloat16_rn(o[i]);
+            }
+        }
+    });
+    return ok;
 }
 
 // The decoder warps' share of one stretch.
@@ -454,7 +578,8 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
         for (int i = 0; i < kTileSegs; ++i) { mbar_init(&sh.seg_full[i], 1); mbar_init(&sh.seg_empty[i], kTileDecoders + kTileEpilogue + 2); }
         for (int i = 0; i < 2; ++i) { mbar_init(&sh.d_full[i], 1); mbar_init(&sh.d_empty[i], kTileEpilogue); }
         mbar_init(&sh.drain, 1);
-        sh.finish = 0;
+        for (int i = 0; i < 2; ++i) mbar_init(&sh.sum_full[i], 1);
+        sh.fin[0].parts = sh.fin[1].parts = 0;
         sh.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -572,7 +697,7 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
                         if (i < n) st_global(y + (size_t)col[i].y * a.ldy, __float2bfloat16_rn(v[i] * (undo * __int_as_float(col[i].x))));
                 }
             };
-            if (s.parts == 1) {
+            if (!Sets::ONE || s.parts == 1) {   // (the all-cohort expert kernel shares no tiles)
                 for (int cb = 0; cb < s.ncols; cb += 16) {
                     uint32_t r[16];
                     tmem_ld16(td + (uint32_t)cb, r);
@@ -587,40 +712,32 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.d_empty[dr.stage]);
-            } else {
-                // this CTA's part of a tile that others share: added into the tile's float32 copy in L2; the last to arrive
-                // takes the sums and leaves zeros
-                float* sums = a.partial + (size_t)s.slot0 * a.n_mma * kTileRows + row_l;
+            } else if constexpr (Sets::ONE) {
+                // this CTA's part of a tile that others share
+                float* mine = tile_part(a, s.slot0, (int)blockIdx.x - s.slot0) + row_l;
                 for (int cb = 0; cb < s.ncols; cb += 16) {
                     uint32_t r[16];
                     tmem_ld16(td + (uint32_t)cb, r);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i)
-                        asm volatile("red.relaxed.gpu.global.add.f32 [%0], %1;" ::"l"(sums + (size_t)(cb + i) * kTileRows), "f"(__uint_as_float(r[i])) : "memory");
+                    for (int i = 0; i < 16; ++i) st_global(mine + (size_t)(cb + i) * kTileRows, __uint_as_float(r[i]));
                 }
                 tc_fence_before_sync();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&sh.d_empty[dr.stage]);
+                if (s.last) sh.row_factor[row_l] = undo;
+                const int2 g = tile_group(s);
+                const TileSum sum(a, s, g.x, 1, g.y);
                 __threadfence();
                 asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp == kTileDecoders && lane == 0) sh.last = atomicAdd(a.counters + s.slot0, 1u);
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (sh.last == (unsigned)(s.parts - 1)) {
-                    __threadfence();
-                    if (s.last) {   // nothing left for this CTA: every warp helps, below
-                        if (lane == 0 && quarter == 0) { sh.finish = buf + 1; sh.fin = s; }
-                        break;
+                if (warp == kTileDecoders && lane == 0) {
+                    unsigned* counter = a.counters + s.slot0 + g.x;
+                    if (atomicAdd(counter, 1u) == (unsigned)(g.y - 1)) {   // nearly always with the last stretch: part 0 of a tile is one
+                        __threadfence();
+                        if (s.last) sum.request_first(a, sh, reinterpret_cast<float*>(x_ring));   // nothing uses the rings' memory any more
+                        *counter = 0u;
+                        sh.fin[s.last ? 0 : 1] = s;
+                        sh.fin_col = buf;
                     }
-                    for (int cb = 0; cb < s.ncols; cb += 16) {
-                        float v[2][8];
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) v[i >> 3][i & 7] = __ldcg(sums + (size_t)(cb + i) * kTileRows);
-#pragma unroll
-                        for (int i = 0; i < 16; ++i) __stcg(sums + (size_t)(cb + i) * kTileRows, 0.f);
-                        put8(cb, v[0]);
-                        put8(cb + 8, v[1]);
-                    }
-                    if (warp == kTileDecoders && lane == 0) a.counters[s.slot0] = 0u;
                 }
             }
             dr.step(a.d_bufs);
@@ -742,61 +859,23 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
         tmem_free(tmem_d, 512u);
         if (lane == 0 && sh.failed) atomicExch(a.error, MFQB_ERR_TIMEOUT);
     }
-    if (sh.finish && !sh.failed) {
-        // The sums of the tile this CTA was the last to add to (up to 128 KB in L2, stored column by column): fetched into the
-        // rings' memory with one bulk copy per 64 columns, then a warp writes a column, four rows a lane.  (The four epilogue
-        // warps alone, sixteen loads in flight each, took 40,000 cycles for N = 256, a third of the kernel.)
-        const TileSeg& t = sh.fin;
-        const float* sums = a.partial + (size_t)t.slot0 * a.n_mma * kTileRows;
-        float* stage = reinterpret_cast<float*>(x_ring);
-        const int ncols16 = (t.ncols + 15) & ~15;   // what was added, and what has to be zero again
-        if (tid == 0) {
-            asm volatile("fence.proxy.async;" ::: "memory");
-            mbar_arrive_expect_tx(&sh.drain, (uint32_t)ncols16 * kTileRows * 4u);
-            for (int c = 0; c < ncols16; c += 64) bulk_load(stage + c * kTileRows, sums + c * kTileRows, (uint32_t)min(64, ncols16 - c) * kTileRows * 4u, &sh.drain);
-            a.counters[t.slot0] = 0u;
-        }
-        for (int r = tid; r < kTileRows; r += kTileThreads)
-            if (t.row0 + r < t.row_limit)
-                sh.row_factor[r] = __uint_as_float(__ldg(&a.pools[t.pool].rowc[(size_t)t.rb0 * 16 + r]).z) * a.lut_undo;
-        __syncthreads();
-        if (!tile_wait(&sh.drain, 0)) {
-            if (tid == 0) atomicExch(a.error, MFQB_ERR_TIMEOUT);
-            return;
-        }
-        int row = t.row0 + 4 * lane, n = min(4, t.row_limit - row);
-        if constexpr (GLU) {   // gate rows are lanes 0-3 of every eight, their up rows lanes 4-7
-            if (lane & 4) n = 0;
-            row = (row >> 5) * 16 + (row & 15);
-        }
-        const float4 f = *reinterpret_cast<const float4*>(sh.row_factor + 4 * lane);
-        const bool vec = n == 4 && (a.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(a.y) & 15) == 0;
-        for (int c = warp; c < ncols16; c += kTileThreads / 32) {
-            __stcg(reinterpret_cast<float4*>(const_cast<float*>(sums) + c * kTileRows + 4 * lane), make_float4(0.f, 0.f, 0.f, 0.f));
-            if (c >= t.ncols) continue;
-            const int2 col = sh.col[sh.finish - 1][c];
-            const float down = __int_as_float(col.x);
-            const float4 v = *reinterpret_cast<const float4*>(stage + c * kTileRows + 4 * lane);
-            float o[4] = {v.x * (f.x * down), v.y * (f.y * down), v.z * (f.z * down), v.w * (f.w * down)};
-            if constexpr (GLU) {
-#pragma unroll
-                for (int i = 0; i < 4; ++i) o[i] = tile_gated(o[i], __shfl_xor_sync(0xffffffffu, o[i], 4));
+    if constexpr (Sets::ONE) {
+        if (!sh.failed && (sh.fin[0].parts | sh.fin[1].parts)) {
+            float* stage = reinterpret_cast<float*>(x_ring);
+            bool ok = true;
+            uint32_t phase = 0u;
+            if (sh.fin[0].parts) ok = tile_finish<GLU>(a, sh, sh.fin[0], sh.col[sh.fin_col], stage, phase);
+            if (ok && sh.fin[1].parts) {   // its tables have made room for later stretches'
+                const TileSeg& t = sh.fin[1];
+                __syncthreads();
+                for (int r = tid; r < kTileRows; r += kTileThreads)
+                    sh.row_factor[r] = t.row0 + r < t.row_limit ? __uint_as_float(__ldg(&a.pools[0].rowc[(size_t)t.rb0 * 16 + r]).z) * a.lut_undo : 0.f;
+                for (int c = tid; c < t.ncols; c += kTileThreads) sh.col[0][c].x = __float_as_int(__ldcg(a.x_down + t.tok0 + c));
+                if (tid == 0) TileSum(a, t, tile_group(t).x, 1, tile_group(t).y).request_first(a, sh, stage);
+                __syncthreads();
+                ok = tile_finish<GLU>(a, sh, t, sh.col[0], stage, phase);
             }
-            const size_t at = (size_t)col.y * a.ldy + row;
-            if (a.y_dtype == 0 /* MFQB_F32 */) {
-                float* y = reinterpret_cast<float*>(a.y) + at;
-                if (vec) *reinterpret_cast<float4*>(y) = make_float4(o[0], o[1], o[2], o[3]);
-                else
-                    for (int i = 0; i < n; ++i) y[i] = o[i];
-            } else {
-                __nv_bfloat16* y = reinterpret_cast<__nv_bfloat16*>(a.y) + at;
-                if (vec) {
-                    const __nv_bfloat162 p0 = __floats2bfloat162_rn(o[0], o[1]), p1 = __floats2bfloat162_rn(o[2], o[3]);
-                    *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&p0), *reinterpret_cast<const uint32_t*>(&p1));
-                } else {
-                    for (int i = 0; i < n; ++i) y[i] = __float2bfloat16_rn(o[i]);
-                }
-            }
+            if (!ok && tid == 0) atomicExch(a.error, MFQB_ERR_TIMEOUT);
         }
     }
 }
