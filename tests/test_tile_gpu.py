@@ -1,6 +1,10 @@
 """Edges of the tensor-memory tile kernel behind batched products: token tiles, row tiles, shared tiles, both f16 forms of
 lattice weights."""
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -133,3 +137,49 @@ def test_shared_tiles_have_the_same_bits_in_every_call(n, k, bits, gs, sb, m):
         for _ in range(5):
             assert torch.equal(glu, w.matmul_glu(x, out_dtype=torch.float32))
     assert _status() == 0
+
+
+GROWING_CALL = """
+import ctypes, sys, torch
+sys.path.insert(0, %r)
+from tyloquant_b200 import QuantWeight, encode, moe
+w, small = (QuantWeight.from_blob("NINT6", encode.random_nint_blob(n, k, 6, 24, 7, seed=1, device="cuda")) for n, k in ((4096, 14336), (100, 400)))
+gen = torch.Generator("cuda").manual_seed(1)
+x, xe = (torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16) for m, k in ((16, 14336), (3, 256)))
+want = x.double() @ w.dequantize().double().T
+gu, dn = (moe.MoeWeight(encode.quantize_expertwise(torch.randn(shape, device="cuda", generator=gen) * 0.02, [4] * 8, device="cuda"))
+          for shape in ((8, 192, 256), (8, 256, 96)))
+ids, wts = moe.moe_topk(torch.randn(3, 8, device="cuda", generator=gen), 2)
+gw, dw = (torch.stack([m.dequantize_expert(i) for i in range(8)]).double()[ids.long()] for m in (gu, dn))   # [token, route, out, in]
+h = torch.einsum("troi,ti->tro", gw, xe.double())
+act = h[..., 96:] * h[..., :96] / (1 + torch.exp(-h[..., :96]))
+ffn = (torch.einsum("trho,tro->trh", dw, act) * wts.double()[..., None]).sum(1)
+y, z = small.matmul(x[:, :400].contiguous()), moe.moe_ffn(gu, dn, xe[:1], ids[:1], wts[:1])   # the kernels' code is loaded, the scratch small
+rt, blocks = ctypes.CDLL("libcudart.so.12"), []
+for size in [1 << i for i in range(8, 20) for _ in range(48)]:
+    p = ctypes.c_void_p()
+    assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(size)) == 0 and rt.cudaMemset(p, 0x3f, ctypes.c_size_t(size)) == 0
+    blocks.append(p)
+torch.cuda.synchronize()
+for p in blocks:
+    assert rt.cudaFree(p) == 0
+y, z = torch.zeros(16, 4096, device="cuda"), None
+side = torch.cuda.Stream()
+torch.cuda.synchronize()
+torch.cuda._sleep(400_000_000)   # the default stream is busy for a fifth of a second
+with torch.cuda.stream(side):
+    w.matmul(x, out=y)
+    z = moe.moe_ffn(gu, dn, xe, ids, wts)
+side.synchronize()
+busy = not torch.cuda.default_stream().query()
+err = [((a.double() - b).norm() / b.norm()).item() for a, b in ((y, want), (z, ffn))]
+print(busy, err)
+assert max(err) <= 1e-3, err
+"""
+
+
+def test_call_that_grows_the_scratch_while_the_default_stream_is_busy():
+    """New scratch, in memory that held something else, is cleared in the order of the call's own stream (here a non-blocking one)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", GROWING_CALL % root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr[-2000:]

@@ -47,7 +47,7 @@ void* GrowOnlyScratch::get(int device, size_t bytes, cudaStream_t stream, const 
     void* p = nullptr;
     const size_t want = bytes + bytes / 2;
     device_malloc(&p, want);
-    MFQB_CUDA(cudaMemset(p, 0, want));   // some users keep self-resetting counters in their block: they start at zero
+    MFQB_CUDA(cudaMemsetAsync(p, 0, want, stream));   // some users keep self-resetting counters in their block: they start at zero, in the call's own order
     d.p = p;   // the previous block stays allocated: earlier launches and captured graphs may still use it
     d.bytes = want;
     return p;
