@@ -183,3 +183,22 @@ def test_call_that_grows_the_scratch_while_the_default_stream_is_busy():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", GROWING_CALL % root], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr[-2000:]
+
+
+def test_overlapping_calls_spoil_no_later_ones():
+    """Calls on one device share scratch and have to be ordered by their streams.  Two that overlap all the same may be wrong, but
+    leave nothing behind: arrival counts belong to one call."""
+    ws = [QuantWeight.from_blob("NINT6", encode.random_nint_blob(n, k, 6, 24, 7, seed=n, device="cuda")) for n, k in ((4096, 14336), (1000, 9000))]
+    gen = torch.Generator("cuda").manual_seed(1)
+    xs = [torch.randn(m, w.k, device="cuda", generator=gen).to(torch.bfloat16) for m, w in zip((16, 40), ws)]
+    want = [w.matmul(x, out_dtype=torch.float32) for w, x in zip(ws, xs)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for _ in range(40):
+        for s, w, x in zip(streams, ws, xs):
+            with torch.cuda.stream(s):
+                w.matmul(x)
+    torch.cuda.synchronize()
+    for _ in range(3):
+        for w, x, y in zip(ws, xs, want):
+            assert torch.equal(w.matmul(x, out_dtype=torch.float32), y)

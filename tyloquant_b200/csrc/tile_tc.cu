@@ -24,6 +24,8 @@ struct XTilesArgs {
     int n_experts, src_div, m;
     int t8[kTileMaxPools], gs[kTileMaxPools], nchunks[kTileMaxPools];
     int staged;            // bf16 rows go through shared memory
+    unsigned* counters;    // the product's arrival counts, cleared here: nothing is left over from a call that was cut short
+    int n_counters;
 };
 
 // (2^e, 2^-e) with 2^e * max in [2^14, 2^15); (1, 1) for a zero, subnormal or non-finite maximum.
@@ -169,6 +171,8 @@ __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XT
     for (int i = 0; i < 8; ++i) ab = max(ab, red[i]);
     const float2 sc = x_row_scale(ab);
     if (blockIdx.y == 0 && tid == 0) a.down[p] = sc.y;
+    if (p == 0 && blockIdx.y == 0)
+        for (int i = tid; i < a.n_counters; i += 256) a.counters[i] = 0u;
     const int r = p - tile_begin, pitch = ((ncols + 7) & ~7) * 128;
     unsigned char* dst = a.out + (size_t)base * a.row_bytes + (size_t)r * 128;
     if (KIND == kTileXBf16 && a.staged && (reinterpret_cast<uintptr_t>(row) & 15) == 0 && (k & 7) == 0)
@@ -235,6 +239,8 @@ __global__ void __launch_bounds__(1024) norm_tiles_kernel(const __grid_constant_
     for (int o = 16; o > 0; o >>= 1) ab = max(ab, __shfl_xor_sync(0xffffffffu, ab, o));
     const float2 sc = x_row_scale(ab);
     if (tid == 0) a.down[p] = sc.y;
+    if (p == 0)
+        for (int i = tid; i < a.n_counters; i += 1024) a.counters[i] = 0u;
     const int T = a.t8[0], tile_begin = p / a.x_rows * a.x_rows, r = p - tile_begin, pitch = ((min(a.x_rows, a.m - tile_begin) + 7) & ~7) * 128;
     x_write_slabs<kTileXShared>(norm_row, true, a.k, a.gs[0], T, a.nchunks[0] * 4 * T, sc.x, a.out + (size_t)tile_begin * a.row_bytes + (size_t)r * 128, r, pitch, tid, 1024);
 }
@@ -407,6 +413,8 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     xa.row_bytes = a.x_row_bytes;
     xa.out = buf;
     xa.down = reinterpret_cast<float*>(buf + xb);
+    xa.counters = a.counters;
+    xa.n_counters = 2 * p.grid;
     xa.t8[0] = w.t8;
     xa.gs[0] = w.gs;
     xa.nchunks[0] = w.nchunks;

@@ -68,7 +68,7 @@ struct TileArgs {
     int m, ntok;                     // plain product: tokens, token tiles
     int units, split;                // plain product: (tile, chunk) units; CTAs per tile, or 0: equal ranges of units
     float* partial;                  // [2 grid][N][128] float32 parts of tiles that several CTAs share, see tile_part
-    unsigned* counters;              // arrivals at a group of parts [grid], by the group's first CTA, and of groups at a tile [grid], by the tile's; zero between calls
+    unsigned* counters;              // arrivals at a group of parts [grid], by the group's first CTA, and of groups at a tile [grid], by the tile's; zero from x_tiles_kernel
     int sum_bytes;                   // shared memory that the addition of parts may use
     // expert product over a route plan with tiles of x_rows pairs; tile_bounds == nullptr: plain product
     const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool, *expert_local;
@@ -393,7 +393,6 @@ __device__ __forceinline__ bool tile_finish(const TileArgs& a, TileShared& sh, c
             sh.last = atomicAdd(counter, 1u);
             if (sh.last == (unsigned)(groups - 1)) {
                 __threadfence();
-                *counter = 0u;
                 sum.request_first(a, sh, stage);
             }
         }
@@ -734,7 +733,6 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
                     if (atomicAdd(counter, 1u) == (unsigned)(g.y - 1)) {   // nearly always with the last stretch: part 0 of a tile is one
                         __threadfence();
                         if (s.last) sum.request_first(a, sh, reinterpret_cast<float*>(x_ring));   // nothing uses the rings' memory any more
-                        *counter = 0u;
                         sh.fin[s.last ? 0 : 1] = s;
                         sh.fin_col = buf;
                     }
