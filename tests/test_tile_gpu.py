@@ -4,6 +4,7 @@ lattice weights."""
 import os
 import subprocess
 import sys
+import threading
 
 import numpy as np
 import pytest
@@ -202,3 +203,28 @@ def test_overlapping_calls_spoil_no_later_ones():
     for _ in range(3):
         for w, x, y in zip(ws, xs, want):
             assert torch.equal(w.matmul(x, out_dtype=torch.float32), y)
+
+
+def test_two_threads_on_one_stream():
+    """A product is two launches over scratch of the device: those of two threads on the same stream do not mix."""
+    w = QuantWeight.from_blob("NINT4", encode.random_nint_blob(256, 512, 4, 32, 6, seed=1, device="cuda"))
+    gen = torch.Generator("cuda").manual_seed(1)
+    xs = [torch.randn(40, 512, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(4)]
+    want = [w.matmul(x) for x in xs]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.cuda.stream(stream):
+            for _ in range(20):
+                ys = [w.matmul(xs[i]) for _ in range(100)]
+                stream.synchronize()
+                wrong.extend(i for y in ys if not torch.equal(y, want[i]))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, len(wrong)

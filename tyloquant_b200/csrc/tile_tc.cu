@@ -1,6 +1,7 @@
 // Host side of the tensor-memory tile kernel (tile_tc.cuh): activation tiles, shared-memory plan, launches.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 
 #include "cuda_util.h"
 #include "tile_tc.h"
@@ -397,6 +398,9 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     const long long chunks_split = split ? (w.nchunks + split - 1) / split + (split > 1 ? 3 : 0) : 0, chunks_equal = (units + sms - 1) / sms + 3;
     a.split = split && chunks_split <= chunks_equal ? (int)split : 0;
     p.grid = a.split ? (int)(tiles * split) : (int)std::max<long long>(1, std::min<long long>(sms, (units + 1) / 2));
+    // The two launches below belong together: another thread's on the same stream would take the scratch between them.
+    static std::mutex launches[64];
+    std::lock_guard<std::mutex> lock(launches[device]);
     static GrowOnlyScratch xs[2], parts, counts;   // activations: decoding batches keep a small block of their own beside the prefill's
     const size_t xb = ((size_t)(m + 7) / 8 * 8 * a.x_row_bytes + 255) / 256 * 256;
     unsigned char* buf = static_cast<unsigned char*>(xs[m > 16].get(device, xb + (size_t)m * 4, s, "mfqb_mul_mat (f16 activation tiles)"));
