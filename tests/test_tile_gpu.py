@@ -228,3 +228,32 @@ def test_two_threads_on_one_stream():
     for t in threads:
         t.join()
     assert not wrong, len(wrong)
+
+
+def _kernels(fn):
+    """Names of the kernels that a call launches."""
+    from torch.profiler import ProfilerActivity, profile
+    fn()
+    torch.cuda.synchronize()
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+
+
+@pytest.mark.parametrize("dtype,entries,banks", [("NVQ3J-512", 512, 4), ("NVQ3J-L", 1024, 2)])
+def test_codebooks_that_fill_shared_memory(dtype, entries, banks):
+    """Wide batches take narrower token tiles where the tables leave no room for 256 columns, not passes of a few rows."""
+    n, k = 300, 1000
+    wt = np.random.default_rng(1).standard_normal((n, k), dtype=np.float32) * np.float32(0.02)
+    w = QuantWeight.from_blob(dtype, encode.nvq_blob(encode.quantize_nvq3(wt, encode.synthetic_d4_banks(entries, banks, seed=5), jsc=True, device="cuda")))
+    ref = w.dequantize().double()
+    gen = torch.Generator("cuda").manual_seed(1)
+    for m in (208, 224, 240, 256, 257, 500, 512):
+        x = torch.randn(m, k, device="cuda", generator=gen).to(torch.bfloat16)
+        want = x.double() @ ref.T
+        got = w.matmul(x, out_dtype=torch.float32).double()
+        assert ((got - want).norm() / want.norm()).item() <= 1e-5, m
+        names = _kernels(lambda: w.matmul(x))
+        assert len(names) == 2 and any("tile_tc_kernel" in name for name in names), (m, names)
+    assert _status() == 0

@@ -368,9 +368,16 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     TileArgs a{};
     TilePlan p;
     const int terms = w.table ? w.tile_terms : 1;
-    // token tiles: as few as 256 columns allow, of equal size
-    const int ntok = (m + 255) / 256, n = std::max(16, ((m + ntok - 1) / ntok + 15) / 16 * 16);
-    if (!tile_plan(a, p, n, (size_t)w.rec_words * 4, w.t8, terms, w.table ? (size_t)w.table_words * 4 + 64 : 0)) return false;
+    // token tiles: as few as 256 columns allow, or fewer columns where a codebook of 128 KB leaves no room for the rings of that many
+    // (giving up there cost a product of 256 rows 32 passes of the single-row kernel), of equal size
+    const size_t rec_bytes = (size_t)w.rec_words * 4, ctx_bytes = w.table ? (size_t)w.table_words * 4 + 64 : 0;
+    auto equal_tiles = [m](int most) {
+        const int ntok = (m + most - 1) / most;
+        return std::max(16, ((m + ntok - 1) / ntok + 15) / 16 * 16);
+    };
+    int n = equal_tiles(256);
+    for (int most = n; !tile_plan(a, p, n, rec_bytes, w.t8, terms, ctx_bytes); n = equal_tiles(most))
+        if ((most -= 16) < 16) return false;
     const int row_tiles = (w.n + kTileRows - 1) / kTileRows, sms = device_sm_count(device);
     const long long tiles = (long long)row_tiles * ((m + n - 1) / n), units = tiles * w.nchunks;
     if (units * (sms + 1) >= (1ll << 31) * 1ll * sms || units >= (1ll << 31)) return false;
