@@ -116,7 +116,8 @@ int mfqb_dequant(const mfqb_weight* w, void* out, int out_dtype, mfqb_stream_t s
  * value unless it lies more than 2^7 below its group's largest magnitude; the product is within
  * 1e-5 relative L2 of the float32 reference), sums are exact in int32 and the scales are applied
  * in float32.  Larger m runs the tcgen05 tile kernel (f16 operands, float32 accumulation): NINT weights
- * are rounded to f16 (within 1e-3 relative L2), lattice weights are exact, every row of x is scaled
+ * are rounded to f16 (within 1e-3 relative L2; where the group size is no multiple of 8 they are two f16
+ * terms, within 1e-5), lattice weights are exact, every row of x is scaled
  * by a power of two (exact within 2^-28 of the row's largest magnitude), and sums are taken in a fixed
  * order: the same call gives the same bits again.
  * An infinity or NaN in x makes the outputs NaN.

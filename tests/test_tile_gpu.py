@@ -257,3 +257,28 @@ def test_codebooks_that_fill_shared_memory(dtype, entries, banks):
         names = _kernels(lambda: w.matmul(x))
         assert len(names) == 2 and any("tile_tc_kernel" in name for name in names), (m, names)
     assert _status() == 0
+
+
+@pytest.mark.parametrize("profile", [(5, 28, 7), (8, 22, 7), (4, 27, 6), (4, 12, 6), (6, 36, 7), (8, 44, 8), (8, 60, 7)])
+def test_padded_groups_keep_the_integer_kernels_accuracy(profile):
+    """Group sizes that are no multiple of eight: two f16 terms per weight (the last one: the integer kernels), within the 1e-5 of
+    the paths with fewer rows; rows whose minimum dwarfs their scale among them."""
+    bits, gs, sb = profile
+    for n, k in ((1, 24), (129, 1001), (272, 4104), (1000, 776)):
+        t = encode.quantize_nint(np.random.default_rng(n).standard_normal((n, k)).astype(np.float32), bits, gs, sb)
+        scale, minimum = (np.array(t[name], dtype=np.float16) for name in ("neuron_scale", "neuron_min"))
+        scale[3::7] *= np.float16(2.0 ** -9)
+        scale[5::11] = 0
+        minimum[6::13] = 0
+        t["neuron_scale"], t["neuron_min"] = scale, minimum
+        blob = encode.nint_blob(t)
+        w = QuantWeight.from_blob(f"NINT{bits}", blob)
+        ref = O.dequant_nint(O.unpack_nint(blob))
+        for m in (4, 5, 16, 17, 64, 65, 129, 257, 520):
+            x = encode.bf16_round(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32))
+            y = w.matmul(bf16_tensor(x), out_dtype=torch.float32).cpu().numpy()
+            err = y.astype(np.float64) - x.astype(np.float64) @ ref.astype(np.float64).T
+            size = np.sqrt(np.square(x, dtype=np.float64) @ np.square(ref, dtype=np.float64).T)
+            assert np.linalg.norm(err) <= 1e-5 * np.linalg.norm(size), (profile, n, k, m)
+        w.free()
+    assert _status() == 0

@@ -320,6 +320,7 @@ NintDevB nint_geometry(const NintView& t, int64_t n, int64_t k) {
     d.nchunks = (d.ng + kChunkGroupsB - 1) / kChunkGroupsB;
     d.wc = byte_unit_words(d.bits, 8 * d.t8);
     d.rec_words = (d.wc + 2) * 32;
+    d.tile_terms = t.gs % 8 ? 2 : 1;
     return d;
 }
 

@@ -56,7 +56,7 @@ struct NintDevB {
     int index_bits, entries, banks, jsc;
     float lut[16];           // scale of each state (JSC); plain NVQ uses the sub-scale itself
     uint32_t bankmap;        // 2 bits per state: codebook bank
-    int tile_terms;          // f16 terms per weight in the tile kernel (lattice_terms)
+    int tile_terms;          // f16 terms per weight in the tile kernel: 2 for padded groups, lattice weights see lattice_terms
 };
 
 constexpr int kChunkGroupsB = 8;

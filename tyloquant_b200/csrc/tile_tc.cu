@@ -295,8 +295,9 @@ static size_t x_row_bytes(const NintDevB& w) { return (size_t)w.nchunks * w.t8 *
 static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8, int terms, size_t ctx_bytes) {
     const size_t budget = kTileDynSmem - 1024, ctx = (ctx_bytes + 15) / 16 * 16;
     a.n_mma = n;
-    a.d_bufs = n <= 128 ? 2 : 1;
     a.d_cols = n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256));
+    // a second accumulator, unless two-term weights need its columns for two stages of either half
+    a.d_bufs = n <= 128 && (terms == 1 || (512 - 2 * a.d_cols) / (16 * t8 * terms) >= 4) ? 2 : 1;
     const int a_total = 512 - a.d_bufs * a.d_cols;
     // Small N: every barrier round trip costs more than the tensor work between two of them, so a step takes two chunks and an
     // activation stage all of a step.  Large N: one chunk a step, activations in 64-column slabs.
@@ -367,7 +368,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     if (norm && (w.k % 4 || w.k > 20480)) return false;   // the row as bf16 in a CTA's 48 KB
     TileArgs a{};
     TilePlan p;
-    const int terms = w.table ? w.tile_terms : 1;
+    const int terms = w.tile_terms;
     // token tiles: as few as 256 columns allow, or fewer columns where a codebook of 128 KB leaves no room for the rings of that many
     // (giving up there cost a product of 256 rows 32 passes of the single-row kernel), of equal size
     const size_t rec_bytes = (size_t)w.rec_words * 4, ctx_bytes = w.table ? (size_t)w.table_words * 4 + 64 : 0;
@@ -500,6 +501,7 @@ void launch_tile_experts_product(const NintDevB* pools, const int* held, int npo
         if (!held[i]) continue;
         const NintDevB& w = pools[i];
         a.pools[i] = w;
+        a.pools[i].tile_terms = 1;
         rec = std::max(rec, (size_t)w.rec_words * 4);
         t8 = std::max(t8, w.t8);
         a.x_row_bytes = std::max(a.x_row_bytes, x_row_bytes(w));

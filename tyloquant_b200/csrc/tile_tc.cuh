@@ -15,10 +15,11 @@
 //   * mma issuer: one thread, tcgen05.mma with A from tensor memory, B from shared memory, D in tensor memory;
 //   * 4 epilogue warps: tcgen05.ld, scaling by row and token factors, stores.
 //
-// Arithmetic.  A row of W is factored as F * (a ss (q - mid) + (mid a ss - b sm)) with F = max(|ns|, |nm| 2^-(BITS+1)),
-// a = ns / F, b = nm / F: F is applied to the finished sums in float32, and since F = ns for every ordinary row the step
-// a ss is an integer and exact in f16.  The offset is formed with two fused multiply-adds (b as high and low f16 part), so a
-// weight is rounded twice in f16, about 2e-4 relative L2 on the product.  Lattice weights are integers ss * code <= 225,
+// Arithmetic.  A row of W is factored as F * (a ss (q - mid) + (mid a ss - b sm)) with a = ns / F, b = nm / F (tile_row_const):
+// F is applied to the finished sums in float32, and since a is a power of two the step a ss is exact in f16.  The offset is
+// formed with two fused multiply-adds (b as high and low f16 part), so a weight is rounded twice in f16, about 2.4e-4 relative
+// L2 on the product.  Group sizes that are no multiple of eight have integer kernels (4e-6) as their other path, so their
+// weights are fed as two f16 terms that carry 22 bits.  Lattice weights are integers ss * code <= 225,
 // exact in f16; the scales of a joint-codebook record are f16 numbers, and where some product with a code has more than 11
 // bits the weight is fed as two f16 terms whose sum is exact.  Activations: one power-of-two scale per token
 // (largest magnitude next to 2^15), exact for bf16 values within 2^-28 of the row's largest.
@@ -177,9 +178,10 @@ __device__ __forceinline__ uint32_t bits_h2(__half2 v) { return *reinterpret_cas
 // (shared memory) to the 16 tensor-memory lanes at taddr, columns 16 t + 8 h + {0..7} for octet t and group pair h.
 // The two values of a column are slots i, i + 2 of a quad (the bytes a 16-bit lane mask picks), columns c / 4 + c slots 0, 2 /
 // 1, 3 of quad c: x_tiles_kernel writes the activations in this order.
-template <int BITS, int T_>
+// TERMS 2: two terms whose sum carries some 22 bits, by error-free sums and products.
+template <int BITS, int T_, int TERMS_ = 1>
 struct TileNint {
-    static constexpr int T = T_, TERMS = 1;
+    static constexpr int T = T_, TERMS = TERMS_;
     using BU = ByteUnit<BITS>;
     static constexpr int WC = BU::words_for(8 * T);
     static constexpr int MID = 1 << (BITS - 1);
@@ -228,9 +230,34 @@ struct TileNint {
         lo = bits_h2(__hfma2(__hsub2(even, bias), d, n));
         hi = bits_h2(__hfma2(__hsub2(odd, bias), d, n));
     }
+    // q d + n + nl in two terms: p + pe = q d and s + se = p + n exactly.
+    __device__ static __forceinline__ void terms(__half2 q, __half2 d, __half2 n, __half2 nl, uint32_t& first, uint32_t& second) {
+        const __half2 p = __hmul2_rn(q, d), pe = __hfma2(q, d, __hneg2(p));
+        const __half2 s = __hadd2_rn(p, n), b = __hsub2_rn(s, p), se = __hadd2_rn(__hsub2_rn(p, __hsub2_rn(s, b)), __hsub2_rn(n, b));
+        first = bits_h2(s);
+        second = bits_h2(__hadd2_rn(__hadd2_rn(se, pe), nl));
+    }
+    template <int R>
+    __device__ static __forceinline__ void weights2(const uint32_t* rec, int lane, __half2 d, __half2 n, __half2 nl, uint32_t& lo, uint32_t& hi, uint32_t& lo2, uint32_t& hi2) {
+        __half2 even, odd;
+        pairs<R>(rec, lane, even, odd);
+        const __half2 bias = __float2half2_rn(1024.f + (float)(MID << pos(R % 4)));
+        terms(__hsub2(even, bias), d, n, nl, lo, lo2);
+        terms(__hsub2(odd, bias), d, n, nl, hi, hi2);
+    }
     template <int F, int TI>
-    __device__ static __forceinline__ void octets(const uint32_t* rec, int lane, const __half2 (&d)[4], const __half2 (&n)[4], uint32_t taddr) {
-        if constexpr (TI < T) {
+    __device__ static __forceinline__ void octets(const uint32_t* rec, int lane, const __half2 (&d)[4], const __half2 (&n)[4], const __half2 (&nl)[4], uint32_t taddr) {
+        if constexpr (TI < T && TERMS == 2) {
+            constexpr int R = (F * T + TI) * 4;
+            uint32_t r[8], e[8];
+            weights2<R>(rec, lane, d[0], n[0], nl[0], r[0], r[2], e[0], e[2]);
+            weights2<R + 1>(rec, lane, d[1], n[1], nl[1], r[1], r[3], e[1], e[3]);
+            weights2<R + 2>(rec, lane, d[2], n[2], nl[2], r[4], r[6], e[4], e[6]);
+            weights2<R + 3>(rec, lane, d[3], n[3], nl[3], r[5], r[7], e[5], e[7]);
+            tmem_st_16x128b_x4(taddr + 16 * TI, r);
+            tmem_st_16x128b_x4(taddr + 16 * T + 16 * TI, e);
+            octets<F, TI + 1>(rec, lane, d, n, nl, taddr);
+        } else if constexpr (TI < T) {
             constexpr int R = (F * T + TI) * 4;
             uint32_t r[8];
             weights<R>(rec, lane, d[0], n[0], r[0], r[2]);
@@ -238,7 +265,7 @@ struct TileNint {
             weights<R + 2>(rec, lane, d[2], n[2], r[4], r[6]);
             weights<R + 3>(rec, lane, d[3], n[3], r[5], r[7]);
             tmem_st_16x128b_x4(taddr + 16 * TI, r);
-            octets<F, TI + 1>(rec, lane, d, n, taddr);
+            octets<F, TI + 1>(rec, lane, d, n, nl, taddr);
         }
     }
     // Both halves of a chunk run the same code where the second one's registers start on a word.
@@ -248,20 +275,30 @@ struct TileNint {
     __device__ static __forceinline__ void half(const uint32_t* rec, int lane, int f, const Row& row, const unsigned char*, uint32_t taddr) {
         const uint32_t sel = (lane & 2) ? 0x4341u : 0x4240u;   // this lane's group of a pair: bytes (row q, row q + 8)
         const __half2 k1024 = __float2half2_rn(1024.f);
-        __half2 d[4], n[4];
+        __half2 d[4], n[4], nl[4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const uint32_t* sc = rec + WC * 32 + (lane & ~3) + 2 * f + h;
             const __half2 ss = __hsub2(h2_bits(__byte_perm(sc[0], 0x64646464u, sel)), k1024);
             const __half2 sm = __hsub2(h2_bits(__byte_perm(sc[32], 0x64646464u, sel)), k1024);
             const __half2 d2 = __hmul2(ss, row.step[h]);
-            const __half2 n2 = __hfma2(sm, row.nb_lo, __hfma2(sm, row.nb_hi, __hmul2(ss, row.mid)));
+            __half2 n2, l2;
+            if constexpr (TERMS == 2) {   // m + (v + ve) in two terms, m and v + ve exact
+                const __half2 m = __hmul2_rn(ss, row.mid), v = __hmul2_rn(sm, row.nb_hi), ve = __hfma2(sm, row.nb_hi, __hneg2(v));
+                n2 = __hadd2_rn(m, v);
+                const __half2 b = __hsub2_rn(n2, m), ne = __hadd2_rn(__hsub2_rn(m, __hsub2_rn(n2, b)), __hsub2_rn(v, b));
+                l2 = __hfma2(sm, row.nb_lo, __hadd2_rn(ne, ve));
+            } else {
+                n2 = l2 = __hfma2(sm, row.nb_lo, __hfma2(sm, row.nb_hi, __hmul2(ss, row.mid)));
+            }
+            nl[2 * h] = __low2half2(l2);
+            nl[2 * h + 1] = __high2half2(l2);
             d[2 * h] = __low2half2(d2);
             d[2 * h + 1] = __high2half2(d2);
             n[2 * h] = __low2half2(n2);
             n[2 * h + 1] = __high2half2(n2);
         }
-        octets<F, 0>(rec + (SPLIT ? f * FW * 32 : 0), lane, d, n, taddr);
+        octets<F, 0>(rec + (SPLIT ? f * FW * 32 : 0), lane, d, n, nl, taddr);
     }
 };
 

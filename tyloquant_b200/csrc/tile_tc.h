@@ -21,14 +21,17 @@ constexpr float kTileWeightScale = 0.25f;   // of the f16 weights: 8-bit codes x
 
 #if defined(__CUDACC__)
 // Constants of a weight row for the tile kernel, 16 bytes: x = f16 a (times kTileWeightScale) | f16 high part of -b << 16,
-// y = f16 low part of -b, z = float32 factor of the row's sums.  Scalar rows: F = max(|ns|, |nm| 2^-(bits + 1)), a = ns / F,
-// b = nm / F, factor F; lattice rows (bits = 0): factor = anchor.
+// y = f16 low part of -b, z = float32 factor of the row's sums.  Scalar rows: F = |ns| 2^j >= |nm| 2^-(bits + 1) with the smallest
+// such j >= 0 (a = ns / F is a power of two), F = |nm| 2^-(bits + 1) where ns = 0, b = nm / F, factor F; lattice rows (bits = 0):
+// factor = anchor.
 __device__ __forceinline__ uint4 tile_row_const(uint32_t anchor, int bits) {
     const float ns = __half2float(__ushort_as_half((unsigned short)(anchor & 0xFFFFu))), nm = __half2float(__ushort_as_half((unsigned short)(anchor >> 16)));
     uint4 c = make_uint4(0u, 0u, __float_as_uint(ns), 0u);
     if (bits) {
-        float f = fmaxf(fabsf(ns), fabsf(nm) * __uint_as_float((uint32_t)(126 - bits) << 23));
-        if (f == 0.f) f = 1.f;
+        const float least = fabsf(nm) * __uint_as_float((uint32_t)(126 - bits) << 23);
+        float f = fabsf(ns);
+        if (f == 0.f) f = least > 0.f ? least : 1.f;
+        else if (least > f) f = ldexpf(f, ilogbf(least / f) + 1);
         const float nb = -nm / f * kTileWeightScale;
         const __half hi = __float2half_rn(nb);
         c.x = (uint32_t)__half_as_ushort(__float2half_rn(ns / f * kTileWeightScale)) | (uint32_t)__half_as_ushort(hi) << 16;

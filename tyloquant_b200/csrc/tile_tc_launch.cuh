@@ -59,8 +59,11 @@ cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, cudaStream
 
 template <int BITS, int T>
 static cudaError_t launch_tile_if_catalog(const TileArgs& a, const TilePlan& p, cudaStream_t stream) {
-    if constexpr (nint_bl_in_catalog(BITS, T)) return launch_tile<TileOne<TileNint<BITS, T>>>(a, p, stream);
-    else return cudaErrorNotSupported;
+    if constexpr (nint_bl_in_catalog(BITS, T)) {
+        if (a.pools[0].tile_terms != 2) return launch_tile<TileOne<TileNint<BITS, T>>>(a, p, stream);
+        if constexpr (T <= 6) return launch_tile<TileOne<TileNint<BITS, T, 2>>>(a, p, stream);   // beyond, two stages of two terms do not fit tensor memory
+    }
+    return cudaErrorNotSupported;
 }
 #define MFQB_TILE_INSTANTIATE(BITS)                                                                          \
     template <>                                                                                              \
