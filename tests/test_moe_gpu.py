@@ -231,3 +231,27 @@ def test_more_pairs_than_a_grid_dimension():
     assert ((got - want).norm() / want.norm()).item() <= REL_L2
     gu.free()
     dn.free()
+
+
+@pytest.mark.parametrize("tokens", [4, 8, 16, 100, 260, 400])
+def test_records_with_padded_groups_keep_the_integer_kernels_accuracy(tokens):
+    """NINT5's groups of 28 are padded to 32: such a record's products stay within 1e-5 at every batch size (two f16 terms for
+    weights and float32 activations on the tile kernel), and the FFN within what its activations' 16 bits cost at fewer pairs."""
+    e_count, h, f, k = 8, 520, 200, 2
+    gu_blob, dn_blob = _moe_case(e_count, h, f, [3, 4, 5, 8] * 2, seed=51)
+    gu, dn = moe.MoeWeight(gu_blob), moe.MoeWeight(dn_blob)
+    gen = torch.Generator("cuda").manual_seed(52)
+    x = torch.randn(tokens, h, device="cuda", generator=gen).to(torch.bfloat16)
+    ids, wts = moe.moe_topk(torch.randn(tokens, e_count, device="cuda", generator=gen), k)
+    gw, dw = (torch.stack([w.dequantize_expert(e) for e in range(e_count)]).double() for w in (gu, dn))
+    every = torch.einsum("th,eoh->teo", x.double(), gw)
+    pick = lambda t: torch.gather(t, 1, ids.long()[:, :, None].expand(-1, -1, t.shape[2]))
+    want = pick(every)
+    got = gu.matmul_id(x, ids, out_dtype=torch.float32).double()
+    assert ((got - want).norm() / want.norm()).item() <= 1e-5
+    act = every[..., f:] * every[..., :f] / (1 + torch.exp(-every[..., :f]))
+    want = (pick(torch.einsum("tef,ehf->teh", act, dw)) * wts.double()[:, :, None]).sum(1)
+    got = moe.moe_ffn(gu, dn, x, ids, wts).double()
+    assert ((got - want).norm() / want.norm()).item() <= (2e-5 if tokens * k >= 2 * e_count else 2e-4)
+    gu.free()
+    dn.free()

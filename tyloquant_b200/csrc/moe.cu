@@ -195,15 +195,16 @@ struct MoeCohorts {
         }
     }
 };
-// True when the matmul over `pairs` pairs runs on the tensor-memory tile kernel (f16 weights): from two pairs per expert on.
-static bool moe_use_tiles_tc(const mfqb_moe_weight* w, int pairs) {
-    if (2 * (long long)pairs < (long long)mfqb::g_moe_f16_from_x2 * w->info.n_experts) return false;
+// Most pairs per tile when the matmul over `pairs` pairs runs on the tensor-memory tile kernel (from two pairs per expert on), 0 when
+// it does not.  float_x: the activations are the FFN's float32 gate|up products.
+static int moe_tiles_tc_rows(const mfqb_moe_weight* w, int pairs, bool float_x) {
+    if (2 * (long long)pairs < (long long)mfqb::g_moe_f16_from_x2 * w->info.n_experts) return 0;
     const MoeCohorts c(w);
-    return tile_experts_supported(c.devs, c.held, c.n);
+    return tile_experts_max_rows(c.devs, c.held, c.n, tile_experts_terms(c.devs, c.held, c.n, pairs, w->info.n_experts), float_x);
 }
-static size_t moe_tiles_tc_bytes(const mfqb_moe_weight* w, int pairs) {
+static size_t moe_tiles_tc_bytes(const mfqb_moe_weight* w, int pairs, bool float_x) {
     const MoeCohorts c(w);
-    return tile_experts_x_bytes(c.devs, c.held, c.n, pairs, w->info.n_experts);
+    return tile_experts_x_bytes(c.devs, c.held, c.n, pairs, w->info.n_experts, tile_experts_terms(c.devs, c.held, c.n, pairs, w->info.n_experts), float_x);
 }
 // One matmul over the plan's tiles (tile_m pairs each) on that kernel; see launch_tile_experts_product.
 static void moe_tiles_tc(const mfqb_moe_weight* w, const PlanBufs& plan, int tile_m, int pairs, const void* x, TileX kind, int src_div, void* xbuf, void* y, int y_dtype,
@@ -211,7 +212,7 @@ static void moe_tiles_tc(const mfqb_moe_weight* w, const PlanBufs& plan, int til
     const MoeCohorts c(w);
     const TileRoutes r{plan.expert_bounds, plan.tile_bounds, plan.pair_order, static_cast<const int*>(w->d_expert_pool.p), static_cast<const int*>(w->d_expert_local.p),
                        w->info.n_experts, pairs, tile_m};
-    launch_tile_experts_product(c.devs, c.held, c.n, r, x, kind, src_div, xbuf, y, y_dtype, scatter, w->info.out_per_expert, w->padded / 16, w->info.device, s);
+    launch_tile_experts_product(c.devs, c.held, c.n, r, tile_experts_terms(c.devs, c.held, c.n, pairs, w->info.n_experts), x, kind, src_div, xbuf, y, y_dtype, scatter, w->info.out_per_expert, w->padded / 16, w->info.device, s);
 }
 
 // Pairs per route-plan tile of the integer batched kernel (2, 4 or 8), or 0: fewer pairs than experts, every pair runs as a
@@ -402,11 +403,11 @@ int mfqb_mul_mat_id(const mfqb_moe_weight* w, const void* x, int x_per_pair, con
         if (tokens == 0) return;
         DeviceGuard guard(w->info.device);
         const int pairs = tokens * routes;
-        const bool tiles_tc = moe_use_tiles_tc(w, pairs);
-        const int tile_m = tiles_tc ? tile_experts_rows(pairs, w->info.n_experts) : moe_tile_m(w, pairs);
+        const int tiles_tc = moe_tiles_tc_rows(w, pairs, false);
+        const int tile_m = tiles_tc ? tile_experts_rows(pairs, w->info.n_experts, tiles_tc) : moe_tile_m(w, pairs);
         if (tile_m) {   // larger batches: route plan in library scratch, batched or tile kernel over its tiles
             const size_t b_plan = PlanBufs::bytes(w->info.n_experts, pairs);
-            const size_t b_in = tiles_tc ? moe_tiles_tc_bytes(w, pairs) : moe_planes_bytes(w, x_per_pair ? pairs : tokens);
+            const size_t b_in = tiles_tc ? moe_tiles_tc_bytes(w, pairs, false) : moe_planes_bytes(w, x_per_pair ? pairs : tokens);
             char* s = static_cast<char*>(scratch_get(w->info.device, b_plan + b_in, stream, 1));
             PlanBufs plan = PlanBufs::carve(s, w->info.n_experts);
             launch_route_plan(ids, pairs, w->info.n_experts, tile_m, plan.expert_bounds, plan.tile_bounds, plan.pair_order, stream);
@@ -492,13 +493,14 @@ static FfnLayout ffn_layout(const mfqb_moe_weight* gate_up, const mfqb_moe_weigh
     const int h = gate_up->info.k, f2 = gate_up->info.out_per_expert, f = f2 / 2, e = gate_up->info.n_experts;
     const size_t pairs = (size_t)tokens * routes;
     auto up256 = [](size_t v) { return (v + 255) / 256 * 256; };
-    L.tiles_tc = allow_tc && moe_use_tiles_tc(gate_up, (int)pairs) && moe_use_tiles_tc(down, (int)pairs);
-    L.tile_m = L.tiles_tc ? tile_experts_rows((int)pairs, e) : std::min(moe_tile_m(gate_up, (int)pairs), moe_tile_m(down, (int)pairs));
+    const int max_rows = allow_tc ? std::min(moe_tiles_tc_rows(gate_up, (int)pairs, false), moe_tiles_tc_rows(down, (int)pairs, true)) : 0;
+    L.tiles_tc = max_rows > 0;
+    L.tile_m = L.tiles_tc ? tile_experts_rows((int)pairs, e, max_rows) : std::min(moe_tile_m(gate_up, (int)pairs), moe_tile_m(down, (int)pairs));
     L.tiles = !L.tiles_tc && L.tile_m != 0;
     L.fused_tail = !L.tile_m && ffn_fused_tail_ok(down, tokens, (int)pairs) && ffn_fused_tail_ok(gate_up, tokens, (int)pairs);
     const size_t b_plan = L.tile_m ? PlanBufs::bytes(e, pairs) : 0;
     size_t b_pdn = 0;
-    if (L.tiles_tc) L.b_pgu = std::max(moe_tiles_tc_bytes(gate_up, (int)pairs), moe_tiles_tc_bytes(down, (int)pairs));   // one after the other
+    if (L.tiles_tc) L.b_pgu = std::max(moe_tiles_tc_bytes(gate_up, (int)pairs, false), moe_tiles_tc_bytes(down, (int)pairs, true));   // one after the other
     else if (L.tiles) {
         L.b_pgu = moe_planes_bytes(gate_up, tokens);
         b_pdn = moe_planes_bytes(down, (int)pairs);

@@ -75,15 +75,21 @@ __device__ __forceinline__ uint32_t x_pack(float a, float b) {   // non-finite -
     return (uint32_t)__half_as_ushort(ha) | ((uint32_t)__half_as_ushort(hb) << 16);
 }
 
+__device__ __forceinline__ uint32_t x_pack_rest(float a, float b, uint32_t packed) {   // what rounding cut off; 0 beside a NaN
+    const float2 r = __half22float2(*reinterpret_cast<const __half2*>(&packed));
+    const __half2 h = __floats2half2_rn(isfinite(a) ? a - r.x : 0.f, isfinite(b) ? b - r.y : 0.f);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
 // Slabs first, first + step, ... of a row's tile: see x_tiles_kernel.  r: row of the tile, pitch: bytes of a 64-column slab of it.
-template <int KIND>
+template <int KIND, int XTERMS = 1>
 __device__ __forceinline__ void x_write_slabs(const void* row, bool row_al, int k, int gs, int T, int nslabs, float scale, unsigned char* dst, int r, int pitch, int first,
                                               int step) {
     const bool quad_al = row_al && (gs & 3) == 0;
     for (int js = first; js < nslabs; js += step) {
         const int ch = js / (4 * T), jj = js - ch * 4 * T, h = jj & 1, ft = jj >> 1, f = ft / T, t = ft - f * T;
         const int g = ch * kChunkGroupsB + 4 * f + 2 * h;
-        uint32_t w[8];
+        uint32_t w[8], e[8];
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int slot = 8 * t + 4 * (c & 1), k0 = (g + (c >> 1)) * gs + slot;
@@ -97,11 +103,20 @@ __device__ __forceinline__ void x_write_slabs(const void* row, bool row_al, int 
             }
             w[c] = x_pack(v.x * scale, v.z * scale);
             w[4 + c] = x_pack(v.y * scale, v.w * scale);
+            if constexpr (XTERMS == 2) {
+                e[c] = x_pack_rest(v.x * scale, v.z * scale, w[c]);
+                e[4 + c] = x_pack_rest(v.y * scale, v.w * scale, w[4 + c]);
+            }
         }
         const int slab = js & 3;
-        unsigned char* at = dst + (size_t)(js >> 2) * pitch;
+        unsigned char* at = dst + (size_t)(js >> 2) * XTERMS * pitch;
         *reinterpret_cast<uint4*>(at + (((2 * slab) ^ (r & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
         *reinterpret_cast<uint4*>(at + (((2 * slab + 1) ^ (r & 7)) << 4)) = make_uint4(w[4], w[5], w[6], w[7]);
+        if constexpr (XTERMS == 2) {
+            at += pitch;
+            *reinterpret_cast<uint4*>(at + (((2 * slab) ^ (r & 7)) << 4)) = make_uint4(e[0], e[1], e[2], e[3]);
+            *reinterpret_cast<uint4*>(at + (((2 * slab + 1) ^ (r & 7)) << 4)) = make_uint4(e[4], e[5], e[6], e[7]);
+        }
     }
 }
 
@@ -111,7 +126,7 @@ __device__ __forceinline__ void x_write_slabs(const void* row, bool row_al, int 
 // the group size, groups and columns past the row are zero.  Grid (rows, splits), for a grid's other dimensions end at 65535:
 // every CTA takes the row's maximum for itself (from L2; a second launch for the maxima costs more for the rows of a decoding
 // batch) and writes its share.
-template <int KIND>
+template <int KIND, int XTERMS>
 __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XTilesArgs a) {
     extern __shared__ __align__(16) unsigned char x_row[];   // bf16 rows: kept between the two passes (a.staged)
     __shared__ uint32_t red[8];
@@ -179,7 +194,7 @@ __global__ void __launch_bounds__(256) x_tiles_kernel(const __grid_constant__ XT
     if (KIND == kTileXBf16 && a.staged && (reinterpret_cast<uintptr_t>(row) & 15) == 0 && (k & 7) == 0)
         x_write_slabs<kTileXShared>(x_row, true, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.y * 256 + tid, gridDim.y * 256);
     else
-        x_write_slabs<KIND>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.y * 256 + tid, gridDim.y * 256);
+        x_write_slabs<KIND, XTERMS>(row, row_al, k, gs, T, nslabs, sc.x, dst, r, pitch, blockIdx.y * 256 + tid, gridDim.y * 256);
 }
 
 // The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the
@@ -259,7 +274,7 @@ static void whole_carveout() {
     if (dev >= 0 && dev < 64) done[dev] = true;
 }
 
-static void launch_x_tiles(XTilesArgs a, int kind, int rows, int nslabs, int sms, cudaStream_t s) {
+static void launch_x_tiles(XTilesArgs a, int kind, int x_terms, int rows, int nslabs, int sms, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     // one CTA per row fills the chip from a few hundred rows on; fewer rows are shared out
     const int splits = std::max(1, std::min((nslabs + 255) / 256, 2 * sms / std::max(rows, 1)));
@@ -274,16 +289,15 @@ static void launch_x_tiles(XTilesArgs a, int kind, int rows, int nslabs, int sms
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    auto go = [&](auto kind_c) {
-        constexpr int KIND = decltype(kind_c)::value;
-        whole_carveout<x_tiles_kernel<KIND>>();
-        MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<KIND>, a));
+    auto go = [&](auto kind_c, auto terms_c) {
+        constexpr int KIND = decltype(kind_c)::value, XTERMS = decltype(terms_c)::value;
+        whole_carveout<x_tiles_kernel<KIND, XTERMS>>();
+        MFQB_CUDA(cudaLaunchKernelEx(&cfg, x_tiles_kernel<KIND, XTERMS>, a));
     };
-    switch (kind) {
-        case kTileXBf16: go(std::integral_constant<int, kTileXBf16>{}); break;
-        case kTileXF32: go(std::integral_constant<int, kTileXF32>{}); break;
-        default: go(std::integral_constant<int, kTileXSwiglu>{}); break;
-    }
+    using std::integral_constant;
+    if (kind == kTileXBf16) go(integral_constant<int, kTileXBf16>{}, integral_constant<int, 1>{});
+    else if (x_terms == 1) go(integral_constant<int, kTileXSwiglu>{}, integral_constant<int, 1>{});
+    else go(integral_constant<int, kTileXSwiglu>{}, integral_constant<int, 2>{});
 }
 
 // ---- plans ---------------------------------------------------------------------------------------------------------------
@@ -292,7 +306,7 @@ static size_t x_row_bytes(const NintDevB& w) { return (size_t)w.nchunks * w.t8 *
 // Rings for token tiles of `n` columns: two stages of each, then records up to 144 KB (what a decoder step frees comes back from
 // HBM 2 us later: with 64 KB the expert products waited for it, 128 experts and 32 tokens 183 us instead of 170) and activation
 // slabs.  False when the codec's tables and two stages of each do not fit.
-static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8, int terms, size_t ctx_bytes) {
+static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8, int terms, int x_terms, size_t ctx_bytes) {
     const size_t budget = kTileDynSmem - 1024, ctx = (ctx_bytes + 15) / 16 * 16;
     a.n_mma = n;
     a.d_cols = n <= 32 ? 32 : (n <= 64 ? 64 : (n <= 128 ? 128 : 256));
@@ -306,7 +320,7 @@ static bool tile_plan(TileArgs& a, TilePlan& p, int n, size_t rec_bytes, int t8,
         a.step = std::max(step, 1);
         a.a_cols = 16 * t8 * terms * a.step;
         a.a_stages = std::min(kTileAStages, a_total / a.a_cols);
-        const size_t rec_stage = 8 * rec_bytes * a.step, x_stage = (size_t)n * 128 * (a.x_whole ? a.step * t8 : 1);
+        const size_t rec_stage = 8 * rec_bytes * a.step, x_stage = (size_t)n * 128 * x_terms * (a.x_whole ? a.step * t8 : 1);
         if (a.a_stages < 2 || ctx + (a.step > 1 ? 3 : 2) * rec_stage + 2 * x_stage > budget || (a.x_whole && x_stage > 24 * 1024)) continue;
         size_t left = budget - ctx - 2 * rec_stage - 2 * x_stage;
         int rs = 2, xs = 2;
@@ -377,7 +391,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
         return std::max(16, ((m + ntok - 1) / ntok + 15) / 16 * 16);
     };
     int n = equal_tiles(256);
-    for (int most = n; !tile_plan(a, p, n, rec_bytes, w.t8, terms, ctx_bytes); n = equal_tiles(most))
+    for (int most = n; !tile_plan(a, p, n, rec_bytes, w.t8, terms, 1, ctx_bytes); n = equal_tiles(most))
         if ((most -= 16) < 16) return false;
     const int row_tiles = (w.n + kTileRows - 1) / kTileRows, sms = device_sm_count(device);
     const long long tiles = (long long)row_tiles * ((m + n - 1) / n), units = tiles * w.nchunks;
@@ -444,7 +458,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
         whole_carveout<norm_tiles_kernel>();
         MFQB_CUDA(cudaLaunchKernelEx(&cfg, norm_tiles_kernel, xa, *norm));
     } else {
-        launch_x_tiles(xa, kTileXBf16, m, w.nchunks * 4 * w.t8, sms, s);
+        launch_x_tiles(xa, kTileXBf16, 1, m, w.nchunks * 4 * w.t8, sms, s);
     }
     const cudaError_t e = launch_one(a, p, terms, s);
     if (e == cudaErrorNotSupported) return false;
@@ -462,22 +476,30 @@ static bool experts_one_launch(const NintDevB* pools, const int* held, int npool
     }
     return true;
 }
+// Two terms where a group size is no multiple of eight, or a codec outside the one-launch kernel below two dozen pairs per expert:
+// these ran on the integer kernels before there was a tile kernel for them.
+int tile_experts_terms(const NintDevB* pools, const int* held, int npools, int pairs, int experts) {
+    for (int i = 0; i < npools; ++i)
+        if (held[i] && pools[i].tile_terms == 2) return 2;
+    return experts_one_launch(pools, held, npools) || pairs / 24 >= experts ? 1 : 2;
+}
+static int x_terms_of(int terms, bool float_x) { return terms == 2 && float_x ? 2 : 1; }   // bf16 values are f16 numbers
 // Pairs per tile: one tile for nearly every expert, since each tile decodes the expert's weights once (three standard
 // deviations above the mean of evenly routed pairs); a tile's unused columns cost tensor time only, which the decoding hides.
-int tile_experts_rows(int pairs, int experts) {
+int tile_experts_rows(int pairs, int experts, int max_rows) {
     const double mean = (double)pairs / std::max(experts, 1);
     const int rows = (int)(mean + 3.0 * std::sqrt(mean) + 3.0);
-    return std::max(16, std::min(256, (rows + 15) / 16 * 16));
+    return std::max(16, std::min(max_rows, (rows + 15) / 16 * 16));
 }
-size_t tile_experts_x_bytes(const NintDevB* pools, const int* held, int npools, int pairs, int experts) {
+size_t tile_experts_x_bytes(const NintDevB* pools, const int* held, int npools, int pairs, int experts, int terms, bool float_x) {
     size_t row = 0;
     for (int i = 0; i < npools; ++i)
-        if (held[i]) row = std::max(row, x_row_bytes(pools[i]));
+        if (held[i]) row = std::max(row, x_row_bytes(pools[i]) * x_terms_of(terms, float_x));
     const size_t rows = (size_t)(pairs + 7) / 8 * 8 + 8 * ((size_t)experts + 1);   // tile_x_row
     return (rows * row + 255) / 256 * 256 + ((size_t)pairs * 4 + 255) / 256 * 256;
 }
-bool tile_experts_supported(const NintDevB* pools, const int* held, int npools) {
-    if (npools > kTileMaxPools) return false;
+int tile_experts_max_rows(const NintDevB* pools, const int* held, int npools, int terms, bool float_x) {
+    if (npools > kTileMaxPools || (terms == 2 && !experts_one_launch(pools, held, npools))) return 0;
     TileArgs a{};
     TilePlan p;
     size_t rec = 0;
@@ -487,11 +509,14 @@ bool tile_experts_supported(const NintDevB* pools, const int* held, int npools) 
         rec = std::max(rec, (size_t)pools[i].rec_words * 4);
         t8 = std::max(t8, pools[i].t8);
     }
-    return t8 == 0 || tile_plan(a, p, 256, rec, t8, 1, 0);   // the widest tile needs the most memory
+    int n = 256;
+    while (n > 0 && t8 && !tile_plan(a, p, n, rec, t8, terms, x_terms_of(terms, float_x), 0)) n -= 16;
+    return n;
 }
 
-void launch_tile_experts_product(const NintDevB* pools, const int* held, int npools, const TileRoutes& r, const void* x, TileX kind, int src_div, void* xbuf, void* y,
+void launch_tile_experts_product(const NintDevB* pools, const int* held, int npools, const TileRoutes& r, int terms, const void* x, TileX kind, int src_div, void* xbuf, void* y,
                                  int y_dtype, bool scatter, int rows_per_expert, int rb_per_expert, int device, cudaStream_t s) {
+    const int x_terms = x_terms_of(terms, kind != kTileXBf16);
     TileArgs a{};
     TilePlan p;
     XTilesArgs xa{};
@@ -501,10 +526,10 @@ void launch_tile_experts_product(const NintDevB* pools, const int* held, int npo
         if (!held[i]) continue;
         const NintDevB& w = pools[i];
         a.pools[i] = w;
-        a.pools[i].tile_terms = 1;
+        a.pools[i].tile_terms = terms;
         rec = std::max(rec, (size_t)w.rec_words * 4);
         t8 = std::max(t8, w.t8);
-        a.x_row_bytes = std::max(a.x_row_bytes, x_row_bytes(w));
+        a.x_row_bytes = std::max(a.x_row_bytes, x_row_bytes(w) * x_terms);
         nslabs = std::max(nslabs, w.nchunks * 4 * w.t8);
         k = w.k;
         xa.t8[i] = w.t8;
@@ -513,7 +538,7 @@ void launch_tile_experts_product(const NintDevB* pools, const int* held, int npo
     }
     if (t8 == 0) return;   // nothing held here
     const int n = std::max(16, r.tile_rows), sms = device_sm_count(device);
-    if (!tile_plan(a, p, n, rec, t8, 1, 0)) fail(MFQB_ERR_UNSUPPORTED, "expert tile product: tiles of %d pairs do not fit shared memory", n);
+    if (!tile_plan(a, p, n, rec, t8, terms, x_terms, 0)) fail(MFQB_ERR_UNSUPPORTED, "expert tile product: tiles of %d pairs do not fit shared memory", n);
     unsigned char* buf = static_cast<unsigned char*>(xbuf);
     const size_t rows = (size_t)(r.pairs + 7) / 8 * 8 + 8 * ((size_t)r.n_experts + 1);
     float* down = reinterpret_cast<float*>(buf + (rows * a.x_row_bytes + 255) / 256 * 256);
@@ -530,7 +555,7 @@ void launch_tile_experts_product(const NintDevB* pools, const int* held, int npo
     xa.expert_pool = r.expert_pool;
     xa.n_experts = r.n_experts;
     xa.src_div = src_div;
-    launch_x_tiles(xa, kind, r.pairs, nslabs, sms, s);
+    launch_x_tiles(xa, kind, x_terms, r.pairs, nslabs, sms, s);
     a.x = buf;
     a.x_rows = r.tile_rows;
     a.x_down = down;
@@ -552,7 +577,7 @@ void launch_tile_experts_product(const NintDevB* pools, const int* held, int npo
     a.only_pool = -1;
     a.lut_undo = 1.f;
     if (experts_one_launch(pools, held, npools)) {
-        const cudaError_t e = launch_tile_experts(a, p, s);
+        const cudaError_t e = launch_tile_experts(a, p, terms, x_terms, s);
         if (e != cudaSuccess) fail(MFQB_ERR_CUDA, "expert tile product launch (tiles of %d, %zu bytes of shared memory): %s", n, p.smem, cudaGetErrorString(e));
         return;
     }

@@ -509,7 +509,15 @@ __device__ __forceinline__ bool tile_decode(const TileArgs& a, TileShared& sh, c
 // stay in uniform registers (an issue inside a rolled loop, operands in lane registers, took 200 cycles, more than its 128
 // tensor cycles for N = 256).  tile_issue: activation stages of 64 columns.  tile_issue_step: small N, an activation stage holds
 // the n <= 2 chunks of a step and each half is one run; with a wait costing 200 cycles, what counts there is their number.
-template <int TERMS, int T>
+// XTERMS 2: activations in two terms; the product of two second terms is left out (2^-22).
+template <int TERMS, int XTERMS>
+__device__ __forceinline__ void tile_mma(uint32_t td, uint32_t at, uint32_t second_at, uint64_t bdesc, uint32_t second_b, uint32_t idesc, bool acc) {
+    tc_mma_f16_ts(td, at, bdesc, idesc, acc);
+    if constexpr (TERMS == 2) tc_mma_f16_ts(td, at + second_at, bdesc, idesc, true);
+    if constexpr (XTERMS == 2) tc_mma_f16_ts(td, at, bdesc + (uint64_t)(second_b >> 4), idesc, true);
+}
+
+template <int TERMS, int XTERMS, int T>
 __device__ __forceinline__ bool tile_issue_step(const TileArgs& a, TileShared& sh, TileRing& ar, TileRing& xr, unsigned char* x_ring, uint32_t x_pitch, uint32_t tmem_a,
                                                 uint32_t td, uint32_t idesc, bool acc, int n) {
     if (!tile_wait(&sh.x_full[xr.stage], xr.phase)) return false;
@@ -526,10 +534,8 @@ __device__ __forceinline__ bool tile_issue_step(const TileArgs& a, TileShared& s
 #pragma unroll
                     for (int i = 0; i < 2 * T; ++i) {
                         const int sl = (g * 2 + f) * 2 * T + i;
-                        const uint64_t bdesc = smem_desc_sw128(xb + (uint32_t)(sl >> 2) * x_pitch) + (uint64_t)(2 * (sl & 3));
-#pragma unroll
-                        for (int term = 0; term < TERMS; ++term)
-                            tc_mma_f16_ts(td, at + (uint32_t)(16 * T * (g * TERMS + term) + 8 * i), bdesc, idesc, sl > 0 || term > 0 || acc);
+                        const uint64_t bdesc = smem_desc_sw128(xb + (uint32_t)((sl >> 2) * XTERMS) * x_pitch) + (uint64_t)(2 * (sl & 3));
+                        tile_mma<TERMS, XTERMS>(td, at + (uint32_t)(16 * T * g * TERMS + 8 * i), 16u * T, bdesc, x_pitch, idesc, sl > 0 || acc);
                     }
                 }
             if (f == 1) tc_commit(&sh.x_empty[xr.stage]);
@@ -542,8 +548,8 @@ __device__ __forceinline__ bool tile_issue_step(const TileArgs& a, TileShared& s
     return true;
 }
 
-template <int TERMS, int T>
-__device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, TileRing& ar, TileRing& xr, unsigned char* x_ring, uint32_t tmem_a, uint32_t td, uint32_t idesc,
+template <int TERMS, int XTERMS, int T>
+__device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, TileRing& ar, TileRing& xr, unsigned char* x_ring, uint32_t x_pitch, uint32_t tmem_a, uint32_t td, uint32_t idesc,
                                            bool acc) {
     auto run = [&](auto first_c, auto len_c, bool x_done) {   // slabs [first, first + len) of the chunk, all in half first / 2T
         constexpr int FIRST = decltype(first_c)::value, LEN = decltype(len_c)::value, H0 = FIRST % (2 * T);
@@ -554,9 +560,7 @@ __device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, Ti
             for (int i = 0; i < LEN; ++i) {
                 const int sl = FIRST + i;
                 const uint64_t bdesc = smem_desc_sw128(xb) + (uint64_t)(2 * (sl & 3));
-#pragma unroll
-                for (int term = 0; term < TERMS; ++term)
-                    tc_mma_f16_ts(td, at + (uint32_t)(16 * T * term + 8 * (H0 + i)), bdesc, idesc, sl > 0 || term > 0 || acc);
+                tile_mma<TERMS, XTERMS>(td, at + (uint32_t)(8 * (H0 + i)), 16u * T, bdesc, x_pitch, idesc, sl > 0 || acc);
             }
             if (x_done) tc_commit(&sh.x_empty[xr.stage]);
             if (H0 + LEN == 2 * T) tc_commit(&sh.a_empty[ar.stage]);
@@ -594,7 +598,8 @@ __device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, Ti
     return ok;
 }
 
-// Sets::dispatch(w, f) calls f(Codec{}) for the codec of a cohort; Sets::ctx describes the codec context (lattice tables).
+// Sets::dispatch(w, f) calls f(Codec{}) for the codec of a cohort; Sets::ctx describes the codec context (lattice tables);
+// Sets::XTERMS: f16 terms per activation (2: a 64-column slab of second terms follows every slab of first terms).
 // GLU: the gated epilogue (TileArgs::glu).  1024 in the launch bound holds the kernel to 64 registers, which leaves room on the
 // SM for the CTAs of the kernel before it.
 template <class Sets, bool GLU>
@@ -795,8 +800,8 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
                 const int n = min(a.step, s.ch1 - ch);
                 auto issue = [&](auto t_c) {
                     constexpr int T = decltype(t_c)::value;
-                    ok = a.x_whole ? tile_issue_step<Sets::TERMS, T>(a, sh, ar, xr, x_ring, x_pitch, tmem_a, td, idesc, acc, n)
-                                   : tile_issue<Sets::TERMS, T>(a, sh, ar, xr, x_ring, tmem_a, td, idesc, acc);
+                    ok = a.x_whole ? tile_issue_step<Sets::TERMS, Sets::XTERMS, T>(a, sh, ar, xr, x_ring, x_pitch, tmem_a, td, idesc, acc, n)
+                                   : tile_issue<Sets::TERMS, Sets::XTERMS, T>(a, sh, ar, xr, x_ring, x_pitch, tmem_a, td, idesc, acc);
                 };
                 switch (t8) {
                     case 2: issue(std::integral_constant<int, 2>{}); break;
@@ -867,7 +872,7 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
         while (ok && next(ok)) {
             seg_done();
             const int t8 = a.pools[s.pool].t8, atoms = a.x_whole ? a.step * t8 : 1;
-            const uint32_t pitch = (uint32_t)((s.ncols + 7) & ~7) * 128u;
+            const uint32_t pitch = (uint32_t)((s.ncols + 7) & ~7) * 128u * (uint32_t)Sets::XTERMS;
             const unsigned char* src = a.x + s.x_off + (size_t)s.ch0 * t8 * pitch;
             for (int at = s.ch0 * t8; at < s.ch1 * t8; at += atoms, src += (size_t)atoms * pitch) {
                 const uint32_t bytes = pitch * (uint32_t)min(atoms, s.ch1 * t8 - at);

@@ -54,12 +54,16 @@ struct TileRoutes {
     const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool, *expert_local;
     int n_experts, pairs, tile_rows;
 };
-// Routed expert product over the cohorts of a record: row p of the plan takes x row pair_order[p] / src_div (src_div = 0: row p)
-// and writes y row pair_order[p] (scatter) or p.  xbuf: tile_experts_x_bytes of device memory.
-bool tile_experts_supported(const NintDevB* pools, const int* held, int npools);
-int tile_experts_rows(int pairs, int experts);
-size_t tile_experts_x_bytes(const NintDevB* pools, const int* held, int npools, int pairs, int experts);
-void launch_tile_experts_product(const NintDevB* pools, const int* held, int npools, const TileRoutes& r, const void* x, TileX kind, int src_div, void* xbuf, void* y,
+// Routed expert products over the cohorts of a record.  Weights and the float32 activations of a gated FFN go in as `terms` f16
+// terms: two where the record's other kernels are the integer ones, whose accuracy they keep (tile_experts_terms).
+int tile_experts_terms(const NintDevB* pools, const int* held, int npools, int pairs, int experts);
+// Most pairs per tile that fit, 0: no tile kernel for this record; the pairs per tile to take.
+int tile_experts_max_rows(const NintDevB* pools, const int* held, int npools, int terms, bool float_x);
+int tile_experts_rows(int pairs, int experts, int max_rows);
+size_t tile_experts_x_bytes(const NintDevB* pools, const int* held, int npools, int pairs, int experts, int terms, bool float_x);
+// Row p of the plan takes x row pair_order[p] / src_div (src_div = 0: row p) and writes y row pair_order[p] (scatter) or p.  xbuf:
+// tile_experts_x_bytes of device memory.
+void launch_tile_experts_product(const NintDevB* pools, const int* held, int npools, const TileRoutes& r, int terms, const void* x, TileX kind, int src_div, void* xbuf, void* y,
                                  int y_dtype, bool scatter, int rows_per_expert, int rb_per_expert, int device, cudaStream_t s);
 
 }  // namespace mfqb

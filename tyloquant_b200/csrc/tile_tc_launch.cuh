@@ -15,7 +15,7 @@ struct TilePlan {
 template <class C>
 struct TileOne {
     static constexpr bool ONE = true;
-    static constexpr int TERMS = C::TERMS;
+    static constexpr int TERMS = C::TERMS, XTERMS = 1;
     template <class Fn>
     __device__ static __forceinline__ void dispatch(const NintDevB&, Fn&& f) { f(C{}); }
     __device__ static void ctx_init(unsigned char* ctx, const TileArgs& a, int tid, int nthreads) { C::ctx_init(ctx, a, tid, nthreads); }
@@ -55,7 +55,7 @@ static cudaError_t launch_tile(const TileArgs& a, const TilePlan& p, cudaStream_
 template <int BITS>
 cudaError_t launch_tile_bits(const TileArgs& a, const TilePlan& p, cudaStream_t stream);
 cudaError_t launch_tile_nvq(const TileArgs& a, const TilePlan& p, int terms, cudaStream_t stream);
-cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, cudaStream_t stream);
+cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, int terms, int x_terms, cudaStream_t stream);
 
 template <int BITS, int T>
 static cudaError_t launch_tile_if_catalog(const TileArgs& a, const TilePlan& p, cudaStream_t stream) {

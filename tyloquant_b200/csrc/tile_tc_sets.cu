@@ -19,24 +19,28 @@ cudaError_t launch_tile_nvq(const TileArgs& a, const TilePlan& p, int terms, cud
 }
 
 // Every cohort of an expert record in one launch: the codecs of the per-expert precision profiles.
+template <int TERMS_, int XTERMS_>
 struct TileExperts {
     static constexpr bool ONE = false;
-    static constexpr int TERMS = 1;
+    static constexpr int TERMS = TERMS_, XTERMS = XTERMS_;
     template <class Fn>
     __device__ static __forceinline__ void dispatch(const NintDevB& w, Fn&& f) {
         switch (w.bits * 16 + w.t8) {
-            case 2 * 16 + 2: f(TileNint<2, 2>{}); break;
-            case 3 * 16 + 3: f(TileNint<3, 3>{}); break;
-            case 4 * 16 + 3: f(TileNint<4, 3>{}); break;
-            case 5 * 16 + 4: f(TileNint<5, 4>{}); break;
-            case 6 * 16 + 3: f(TileNint<6, 3>{}); break;
-            case 8 * 16 + 3: f(TileNint<8, 3>{}); break;
-            case 8 * 16 + 6: f(TileNint<8, 6>{}); break;
+            case 2 * 16 + 2: f(TileNint<2, 2, TERMS>{}); break;
+            case 3 * 16 + 3: f(TileNint<3, 3, TERMS>{}); break;
+            case 4 * 16 + 3: f(TileNint<4, 3, TERMS>{}); break;
+            case 5 * 16 + 4: f(TileNint<5, 4, TERMS>{}); break;
+            case 6 * 16 + 3: f(TileNint<6, 3, TERMS>{}); break;
+            case 8 * 16 + 3: f(TileNint<8, 3, TERMS>{}); break;
+            case 8 * 16 + 6: f(TileNint<8, 6, TERMS>{}); break;
             default: break;
         }
     }
     __device__ static void ctx_init(unsigned char*, const TileArgs&, int, int) {}
 };
-cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, cudaStream_t stream) { return launch_tile_form<TileExperts, false>(a, p, stream); }
+cudaError_t launch_tile_experts(const TileArgs& a, const TilePlan& p, int terms, int x_terms, cudaStream_t stream) {
+    if (terms == 1) return launch_tile_form<TileExperts<1, 1>, false>(a, p, stream);
+    return x_terms == 1 ? launch_tile_form<TileExperts<2, 1>, false>(a, p, stream) : launch_tile_form<TileExperts<2, 2>, false>(a, p, stream);
+}
 
 }  // namespace mfqb
