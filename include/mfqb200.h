@@ -99,7 +99,10 @@ int mfqb_weight_info_get(const mfqb_weight* w, mfqb_weight_info* info);
 /* A second handle with its own device copy of the same weight, on the same device (device-to-device
  * copy: the host-side re-layout is not repeated).  No counterpart in the reference. */
 int mfqb_weight_clone(const mfqb_weight* w, mfqb_weight** out);
+/* Frees the handle and its device memory.  Up to 256 MB of such memory per device (16 blocks) stay with the library for the
+ * tensors loaded next; mfqb_memory_trim gives them back to the device. */
 int mfqb_weight_free(mfqb_weight* w);
+int mfqb_memory_trim(int device);
 
 /* Reference decoder on the GPU: writes the [n, k] row-major dequantized tensor.
  * out_dtype MFQB_F32 is bit-identical to nint_quant.dequantize / nvq_quant.dequantize /

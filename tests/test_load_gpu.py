@@ -1,6 +1,7 @@
 """Edges of loading: pieces, slices, whole-byte storage, padded experts -- decoded bit for bit."""
 
 import struct
+import threading
 
 import numpy as np
 import pytest
@@ -10,7 +11,7 @@ pytestmark = pytest.mark.gpu
 torch = pytest.importorskip("torch")
 
 from oracle import mfq_oracle as O  # noqa: E402
-from tyloquant_b200 import QuantWeight, encode, moe  # noqa: E402
+from tyloquant_b200 import QuantWeight, _capi, encode, moe  # noqa: E402
 
 
 def _same(a, b):
@@ -93,3 +94,58 @@ def test_memory_of_freed_tensors_is_taken_again_only_when_idle():
         want = x.float().cpu().numpy() @ ref.T
         assert np.allclose(got, want, atol=2e-2 * np.abs(want).max()), (i, n)
         last = y
+
+
+@pytest.mark.parametrize("mode", ["relaxed", "thread_local"])
+def test_a_weight_freed_beside_a_capture_does_not_end_it(mode):
+    """Freeing is allowed there: in the capturing thread in the relaxed mode, and in other threads in both."""
+    w, other, third = (QuantWeight.from_blob("NINT4", encode.random_nint_blob(512, 512, 4, 24, 6, seed=i, device="cuda")) for i in range(3))
+    x = torch.randn(1, 512, device="cuda").to(torch.bfloat16)
+    want, out = w.matmul(x), torch.empty(1, 512, device="cuda", dtype=torch.bfloat16)
+    w.matmul(x, out=out)
+    torch.cuda.synchronize()
+    graph, stream = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        graph.capture_begin(capture_error_mode=mode)
+        w.matmul(x, out=out)
+        t = threading.Thread(target=other.free)
+        t.start()
+        t.join()
+        if mode == "relaxed":
+            third.free()
+        w.matmul(x, out=out)
+        graph.capture_end()
+    out.zero_()
+    torch.cuda.synchronize()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("replay", [False, True])
+def test_freeing_waits_for_work_on_any_stream(replay):
+    """A freed tensor's block may be written by the next load, so freeing returns after kernels and graphs that could read it."""
+    ws = [QuantWeight.from_blob("NINT4", encode.random_nint_blob(512, 512, 4, 24, 6, seed=i, device="cuda")) for i in range(4)]
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    if replay:
+        with torch.cuda.graph(graph):
+            torch.cuda._sleep(100_000_000)
+    for w in ws:
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            graph.replay() if replay else torch.cuda._sleep(100_000_000)
+        done = stream.record_event()
+        w.free()
+        assert done.query()
+
+
+def test_parked_memory_is_given_back():
+    _capi.check(_capi.lib.mfqb_memory_trim(0))
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    w = QuantWeight.from_blob("NINT4", encode.random_nint_blob(8192, 8192, 4, 24, 6, seed=1, device="cuda"))
+    torch.cuda.empty_cache()
+    w.free()
+    kept = before - torch.cuda.mem_get_info()[0]
+    _capi.check(_capi.lib.mfqb_memory_trim(0))
+    assert kept > 30 << 20 and before - torch.cuda.mem_get_info()[0] < kept - (30 << 20)

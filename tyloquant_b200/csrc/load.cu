@@ -345,6 +345,7 @@ void TensorBuf::alloc(size_t n) {
     if (!n) return;
     MFQB_CUDA(cudaGetDevice(&device_));
     if (device_ >= 64) fail(MFQB_ERR_ARG, "device index %d out of range", device_);
+    device_malloc(&fence_, 256);
     {
         ParkedList& l = parked(device_);
         std::lock_guard<std::mutex> lock(l.mu);
@@ -363,15 +364,16 @@ void TensorBuf::alloc(size_t n) {
 }
 
 void TensorBuf::release() {
-    if (!p) return;
-    void* const mem = p;
-    p = nullptr;
     bytes = 0;
+    if (!p && !fence_) return;
+    void *const mem = p, *const fence = fence_;
+    p = fence_ = nullptr;
     int prev = device_;
     cudaGetDevice(&prev);
     if (prev != device_) cudaSetDevice(device_);
+    const bool idle = cudaFree(fence) == cudaSuccess;   // waits for the device, see above
     std::vector<Parked> out;
-    if (block_ <= kParkedBytes && cudaDeviceSynchronize() == cudaSuccess) {
+    if (idle && mem && block_ <= kParkedBytes) {
         ParkedList& l = parked(device_);
         std::lock_guard<std::mutex> lock(l.mu);
         l.blocks.push_back(Parked{mem, block_});
@@ -382,7 +384,7 @@ void TensorBuf::release() {
             out.push_back(l.blocks.front());
             l.blocks.erase(l.blocks.begin());
         }
-    } else {
+    } else if (mem) {
         out.push_back(Parked{mem, block_});
     }
     for (const Parked& b : out) cudaFree(b.p);

@@ -9,10 +9,14 @@
 
 namespace mfqb {
 
-// Device memory of a tensor.  Mapping and unmapping 52 MB takes 360 and 320 us, a third of loading it (2390 -> 1570 us with decoding and freeing), so the blocks of freed
-// tensors are parked and taken again by tensors of about their size: at most kParkedBytes in kParkedBlocks of each device,
-// given back when newer ones push them out or when an allocation of the library finds no room.  A block is parked after
-// all work of its device has ended (what cudaFree waits for), so whatever stream takes it next may write at once.
+// Device memory of a tensor.  Mapping and unmapping 52 MB takes 0.7 to 5 ms, up to twice what loading it takes (1.5 ms with
+// decoding and freeing), so the blocks of freed tensors are parked and taken again by tensors of about their size: at most
+// kParkedBytes in kParkedBlocks of each device, given back when newer ones push them out, when an allocation of the library
+// finds no room, or by mfqb_memory_trim.
+//
+// A block is parked after all work of its device has ended, so whatever stream takes it next may write at once.  What waits for
+// that work is cudaFree, of a few bytes that every tensor has beside its block: where a stream is being captured
+// (cudaStreamCaptureModeRelaxed, or by another thread) freeing is allowed, and synchronising the device would end the capture.
 constexpr size_t kParkedBytes = 256u << 20;
 constexpr int kParkedBlocks = 16;
 
@@ -22,12 +26,13 @@ struct TensorBuf {
     TensorBuf() = default;
     TensorBuf(const TensorBuf&) = delete;
     TensorBuf& operator=(const TensorBuf&) = delete;
-    TensorBuf(TensorBuf&& o) noexcept : p(o.p), bytes(o.bytes), block_(o.block_), device_(o.device_) { o.p = nullptr; }
+    TensorBuf(TensorBuf&& o) noexcept : p(o.p), bytes(o.bytes), fence_(o.fence_), block_(o.block_), device_(o.device_) { o.p = o.fence_ = nullptr; }
     void alloc(size_t n);   // on the current device
     void release();
     ~TensorBuf() { release(); }
 
 private:
+    void* fence_ = nullptr;   // freed before the block is parked
     size_t block_ = 0;
     int device_ = 0;
 };

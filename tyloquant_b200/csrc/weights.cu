@@ -505,6 +505,14 @@ int mfqb_tune(const char* key, int value) {
     });
 }
 
+int mfqb_memory_trim(int device) {
+    return guarded([&] {
+        if (device < 0 || device >= 64) fail(MFQB_ERR_ARG, "mfqb_memory_trim: bad device index %d", device);
+        DeviceGuard guard(device);
+        give_back_parked(device);
+    });
+}
+
 int mfqb_device_status(int device, int* status) {
     return guarded([&] {
         if (!status || device < 0 || device >= 64) fail(MFQB_ERR_ARG, "mfqb_device_status: bad argument");
