@@ -176,7 +176,8 @@ int mfqb_mul_mat_rmsnorm(const mfqb_weight* w, const float* h, const float* delt
 /* Tuning switches, for measurements.  "gemv1_kernel": which kernel a single-row product of a plain
  * NINT weight takes -- 0 by shape (default), 1 the per-warp ring kernel, 2 the streamed kernel.
  * "moe_f16_tiles_from_x2": twice the average number of (token, route) pairs per expert from which
- * the expert matmuls take the f16 tile kernel instead of the integer tiles (default 4).
+ * the expert matmuls take the f16 tile kernel instead of the integer tiles (default 4; records with
+ * padded groups, whose weights go in as two f16 terms, from one and a half times as many).
  * "gemm_plan" (0 or 1) is accepted and has no effect: the tile kernel sizes its rings by shape.
  * No counterpart in the reference (its switches are MFQ_* environment variables,
  * docs/developer-architecture-and-operator-reference.md:1048-1078). */

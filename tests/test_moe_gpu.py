@@ -233,7 +233,7 @@ def test_more_pairs_than_a_grid_dimension():
     dn.free()
 
 
-@pytest.mark.parametrize("tokens", [4, 8, 16, 100, 260, 400])
+@pytest.mark.parametrize("tokens", [4, 8, 11, 12, 16, 100, 260, 400])
 def test_records_with_padded_groups_keep_the_integer_kernels_accuracy(tokens):
     """NINT5's groups of 28 are padded to 32: such a record's products stay within 1e-5 at every batch size (two f16 terms for
     weights and float32 activations on the tile kernel), and the FFN within what its activations' 16 bits cost at fewer pairs."""
@@ -252,6 +252,6 @@ def test_records_with_padded_groups_keep_the_integer_kernels_accuracy(tokens):
     act = every[..., f:] * every[..., :f] / (1 + torch.exp(-every[..., :f]))
     want = (pick(torch.einsum("tef,ehf->teh", act, dw)) * wts.double()[:, :, None]).sum(1)
     got = moe.moe_ffn(gu, dn, x, ids, wts).double()
-    assert ((got - want).norm() / want.norm()).item() <= (2e-5 if tokens * k >= 2 * e_count else 2e-4)
+    assert ((got - want).norm() / want.norm()).item() <= (2e-5 if tokens * k >= 3 * e_count else 2e-4)
     gu.free()
     dn.free()

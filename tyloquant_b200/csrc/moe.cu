@@ -195,12 +195,15 @@ struct MoeCohorts {
         }
     }
 };
-// Most pairs per tile when the matmul over `pairs` pairs runs on the tensor-memory tile kernel (from two pairs per expert on), 0 when
-// it does not.  float_x: the activations are the FFN's float32 gate|up products.
+// Most pairs per tile when the matmul over `pairs` pairs runs on the tensor-memory tile kernel, 0 when it does not: from two pairs
+// per expert on, with two-term weights from three (128 experts of 2048 x 768, widths 3, 4, 5, 8, top 8: 339 us on the integer
+// kernels and 385 here at two pairs per expert, 518 and 427 at four).  float_x: the activations are the FFN's float32 gate|up
+// products.
 static int moe_tiles_tc_rows(const mfqb_moe_weight* w, int pairs, bool float_x) {
-    if (2 * (long long)pairs < (long long)mfqb::g_moe_f16_from_x2 * w->info.n_experts) return 0;
     const MoeCohorts c(w);
-    return tile_experts_max_rows(c.devs, c.held, c.n, tile_experts_terms(c.devs, c.held, c.n, pairs, w->info.n_experts), float_x);
+    const int terms = tile_experts_terms(c.devs, c.held, c.n, pairs, w->info.n_experts);
+    if (4 * (long long)pairs < (terms + 1ll) * mfqb::g_moe_f16_from_x2 * w->info.n_experts) return 0;
+    return tile_experts_max_rows(c.devs, c.held, c.n, terms, float_x);
 }
 static size_t moe_tiles_tc_bytes(const mfqb_moe_weight* w, int pairs, bool float_x) {
     const MoeCohorts c(w);
