@@ -1,6 +1,9 @@
 """Edges of loading: pieces, slices, whole-byte storage, padded experts -- decoded bit for bit."""
 
+import os
 import struct
+import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -149,3 +152,49 @@ def test_parked_memory_is_given_back():
     kept = before - torch.cuda.mem_get_info()[0]
     _capi.check(_capi.lib.mfqb_memory_trim(0))
     assert kept > 30 << 20 and before - torch.cuda.mem_get_info()[0] < kept - (30 << 20)
+
+
+NO_ROOM = """
+import ctypes, os, sys
+sys.path.insert(0, %r)
+import numpy as np, torch
+from oracle import mfq_oracle as O
+from tyloquant_b200 import QuantWeight, encode
+shim = ctypes.CDLL(os.environ["LD_PRELOAD"])
+blob = encode.random_nint_blob(8000, 4000, 4, 24, 6, seed=1, device="cuda")
+torch.cuda.synchronize()
+shim.fail_next(%d)
+try:
+    QuantWeight.from_blob("NINT4", blob)
+except Exception as e:
+    assert "memory" in str(e), e
+else:
+    raise SystemExit("the load should have failed")
+shim.fail_next(0)
+w = QuantWeight.from_blob("NINT4", blob)
+assert np.array_equal(w.dequantize().cpu().numpy(), O.dequant_nint(O.unpack_nint(blob)))
+"""
+
+SHIM = """
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static int at;
+void fail_next(int n) { at = n; }
+int cudaMalloc(void** p, size_t n) {
+    int (*real)(void**, size_t) = (int (*)(void**, size_t))dlsym(RTLD_NEXT, "cudaMalloc");
+    if (n == (2u << 20) && at && --at == 0) return 2;
+    return real(p, n);
+}
+"""
+
+
+@pytest.mark.parametrize("block", [1, 3])
+def test_load_after_one_that_found_no_room(tmp_path, block):
+    """The first staging block, or one of several.  Staging survives between loads; one whose device half could not be allocated is not taken for complete."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src, lib = tmp_path / "shim.c", tmp_path / "shim.so"
+    src.write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", str(src), "-o", str(lib), "-ldl"], check=True)
+    r = subprocess.run([sys.executable, "-c", NO_ROOM % (root, block)], env={**os.environ, "LD_PRELOAD": str(lib)}, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr[-2000:]

@@ -1,6 +1,7 @@
 """Edges of the tensor-memory tile kernel behind batched products: token tiles, row tiles, shared tiles, both f16 forms of
 lattice weights."""
 
+import ctypes
 import os
 import subprocess
 import sys
@@ -230,15 +231,32 @@ def test_two_threads_on_one_stream():
     assert not wrong, len(wrong)
 
 
+class _NodeParams(ctypes.Structure):   # cudaKernelNodeParams
+    _fields_ = [("func", ctypes.c_void_p), ("grid", ctypes.c_uint * 3), ("block", ctypes.c_uint * 3), ("smem", ctypes.c_uint), ("args", ctypes.c_void_p),
+                ("extra", ctypes.c_void_p)]
+
+
 def _kernels(fn):
-    """Names of the kernels that a call launches."""
-    from torch.profiler import ProfilerActivity, profile
+    """Names of the kernels that a call launches: those of its captured graph."""
+    rt = ctypes.CDLL("libcudart.so.12")
     fn()
     torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
         fn()
-        torch.cuda.synchronize()
-    return [e.name for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA]
+    raw, count = ctypes.c_void_p(graph.raw_cuda_graph()), ctypes.c_size_t(0)
+    assert rt.cudaGraphGetNodes(raw, None, ctypes.byref(count)) == 0
+    nodes = (ctypes.c_void_p * count.value)()
+    assert rt.cudaGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0
+    names = []
+    for node in nodes:
+        kind, params, name = ctypes.c_int(-1), _NodeParams(), ctypes.c_char_p()
+        assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
+        if kind.value == 0:   # a kernel
+            assert rt.cudaGraphKernelNodeGetParams(ctypes.c_void_p(node), ctypes.byref(params)) == 0
+            assert rt.cudaFuncGetName(ctypes.byref(name), ctypes.c_void_p(params.func)) == 0
+            names.append(name.value.decode())
+    return names
 
 
 @pytest.mark.parametrize("dtype,entries,banks", [("NVQ3J-512", 512, 4), ("NVQ3J-L", 1024, 2)])

@@ -12,6 +12,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -154,10 +155,16 @@ struct Slot {
     char *host = nullptr, *dev = nullptr;
     cudaEvent_t done = nullptr;
     bool used = false;
-    void alloc(size_t bytes) {
-        MFQB_CUDA(cudaHostAlloc((void**)&host, bytes, cudaHostAllocDefault));
-        MFQB_CUDA(cudaMalloc((void**)&dev, bytes));
-        MFQB_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+    void alloc(size_t bytes) {   // all three, or none: a slot outlives the load that could not have it
+        try {
+            MFQB_CUDA(cudaHostAlloc((void**)&host, bytes, cudaHostAllocDefault));
+            MFQB_CUDA(cudaMalloc((void**)&dev, bytes));
+            MFQB_CUDA(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
+        } catch (...) {
+            (void)cudaGetLastError();   // the launches of a later load look at it
+            release();
+            throw;
+        }
     }
     void release() {
         if (host) cudaFreeHost(host);
@@ -281,7 +288,10 @@ void run_pieces(const std::vector<Piece>& pieces, const std::vector<StreamSpec>&
         }
     };
     std::vector<std::thread> threads;
-    for (int i = 1; i < workers; ++i) threads.emplace_back(work, i);
+    try {
+        for (int i = 1; i < workers; ++i) threads.emplace_back(work, i);
+    } catch (const std::system_error&) {   // no more threads to be had: the ones there are do the work
+    }
     work(0);
     for (auto& t : threads) t.join();
     big_slot.release();
