@@ -198,3 +198,18 @@ def test_load_after_one_that_found_no_room(tmp_path, block):
     subprocess.run(["gcc", "-shared", "-fPIC", "-O1", str(src), "-o", str(lib), "-ldl"], check=True)
     r = subprocess.run([sys.executable, "-c", NO_ROOM % (root, block)], env={**os.environ, "LD_PRELOAD": str(lib)}, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr[-2000:]
+
+
+def test_experts_larger_than_a_staging_piece():
+    """Experts are cut by row-blocks; 100 and 500 rows are padded to whole ones, the last piece with them."""
+    for e, out, k in ((3, 100, 40000), (5, 500, 9000)):
+        w = torch.randn(e, out, k, device="cuda", generator=torch.Generator("cuda").manual_seed(out)) * 0.02
+        bits = [(6, 4, 8, 6, 6)[i] for i in range(e)]
+        blob = encode.quantize_expertwise(w, bits, device="cuda")
+        whole, shard = moe.MoeWeight(blob), moe.MoeWeight(blob, 0, 1, 3)
+        for i in range(e):
+            b, gs, sb = encode.CANONICAL_NINT[bits[i]]
+            ref = O.dequant_nint(O.unpack_nint(encode.nint_blob(encode.quantize_nint(w[i], b, gs, sb, device="cuda"))))
+            assert _same(whole.dequantize_expert(i).cpu().numpy(), ref), i
+            if 1 <= i < 3:
+                assert _same(shard.dequantize_expert(i).cpu().numpy(), ref), i

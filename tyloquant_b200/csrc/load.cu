@@ -41,6 +41,20 @@ __device__ __forceinline__ uint32_t stream_bits(const uint32_t* s, uint32_t bit,
     const uint32_t v = __funnelshift_r(__ldg(s + (bit >> 5)), __ldg(s + (bit >> 5) + 1), bit & 31);
     return n == 32 ? v : v & ((1u << n) - 1u);
 }
+// Where a file row of a stream begins (64 bits: a row-block can be as wide as an int says), for values counted inside the row.
+struct RowBits {
+    const uint32_t* p;
+    uint32_t bit;
+    __device__ __forceinline__ RowBits(const PackArgs& a, int k, int src, uint32_t per_row) {
+        const uint64_t b = a.bit0[k] + (uint64_t)max(src, 0) * per_row * (uint32_t)a.width[k];
+        p = a.stream[k] + (b >> 5);
+        bit = (uint32_t)b & 31u;
+    }
+    __device__ __forceinline__ uint32_t get(uint64_t first_bit, int n) const {
+        const uint64_t b = bit + first_bit;
+        return stream_bits(p + (b >> 5), (uint32_t)b & 31u, n);
+    }
+};
 __device__ __forceinline__ int pack_src_row(const PackArgs& a, int r) {   // file row of a device row, -1: padding
     if (r >= a.rows) return -1;
     const int u = r / a.padded, o = r - u * a.padded, src = u * a.ope + o;
@@ -56,6 +70,8 @@ __global__ void __launch_bounds__(256) pack_nint_kernel(const __grid_constant__ 
     for (long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); item < (long long)nrb * a.nchunks; item += (long long)gridDim.x * 8) {
         const int rb = (int)(item / a.nchunks), ch = (int)(item - (long long)rb * a.nchunks);
         const int src[2] = {pack_src_row(a, rb * 16 + q), pack_src_row(a, rb * 16 + q + 8)};
+        const uint32_t per_row = (uint32_t)a.ng_file;
+        const RowBits code[2] = {{a, 4, src[0], per_row * a.gs}, {a, 4, src[1], per_row * a.gs}};
         uint32_t w[WC];
 #pragma unroll
         for (int i = 0; i < WC; ++i) w[i] = 0u;
@@ -65,9 +81,8 @@ __global__ void __launch_bounds__(256) pack_nint_kernel(const __grid_constant__ 
             const int grp = ch * kChunkGroupsB + 4 * f + 2 * ((r >> 1) & 1) + (c >> 1);
             uint32_t v = 0u;
             if (src[hi] >= 0 && grp < a.ng && slot < a.gs) {
-                const uint32_t at = ((uint32_t)src[hi] * a.ng_file + a.group0 + grp) * a.gs + slot;
                 const int wq = a.width[4], cnt = min(4, a.gs - slot);
-                const uint32_t four = stream_bits(a.stream[4], a.bit0[4] + at * wq, 4 * wq);
+                const uint32_t four = code[hi].get(((uint64_t)(a.group0 + grp) * a.gs + slot) * wq, 4 * wq);
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     if (i < cnt) v |= ((four >> (i * wq)) & ((1u << BITS) - 1u)) << (8 * i);
@@ -82,9 +97,9 @@ __global__ void __launch_bounds__(256) pack_nint_kernel(const __grid_constant__ 
         for (int i = 0; i < 4; ++i) {
             const int grp = ch * kChunkGroupsB + 2 * c + (i & 1);
             if (src[i >> 1] < 0 || grp >= a.ng) continue;
-            const uint32_t at = (uint32_t)src[i >> 1] * a.ng_file + a.group0 + grp;
-            s0 |= stream_bits(a.stream[2], a.bit0[2] + at * a.width[2], a.width[2]) << (8 * i);
-            s1 |= stream_bits(a.stream[3], a.bit0[3] + at * a.width[3], a.width[3]) << (8 * i);
+            const uint64_t at = (uint64_t)(a.group0 + grp);
+            s0 |= RowBits(a, 2, src[i >> 1], per_row).get(at * a.width[2], a.width[2]) << (8 * i);
+            s1 |= RowBits(a, 3, src[i >> 1], per_row).get(at * a.width[3], a.width[3]) << (8 * i);
         }
         rec[WC * 32 + lane] = s0;
         rec[(WC + 1) * 32 + lane] = s1;
@@ -99,9 +114,12 @@ __global__ void __launch_bounds__(256) pack_nvq_kernel(const __grid_constant__ P
     for (long long item = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); item < (long long)nrb * a.nchunks; item += (long long)gridDim.x * 8) {
         const int rb = (int)(item / a.nchunks), ch = (int)(item - (long long)rb * a.nchunks);
         const int src[2] = {pack_src_row(a, rb * 16 + q), pack_src_row(a, rb * 16 + q + 8)};
+        const RowBits sub[2] = {{a, 1, src[0], (uint32_t)a.ng_file}, {a, 1, src[1], (uint32_t)a.ng_file}};
+        const RowBits index[2] = {{a, 2, src[0], (uint32_t)a.nvec_file}, {a, 2, src[1], (uint32_t)a.nvec_file}};
+        const RowBits sign[2] = {{a, 3, src[0], (uint32_t)a.nsign_file}, {a, 3, src[1], (uint32_t)a.nsign_file}};
         auto state = [&](int hi, int grp) {
             if (src[hi] < 0 || grp >= a.ng) return 0u;
-            return stream_bits(a.stream[1], a.bit0[1] + ((uint32_t)src[hi] * a.ng_file + a.group0 + grp) * a.width[1], a.width[1]);
+            return sub[hi].get((uint64_t)(a.group0 + grp) * a.width[1], a.width[1]);
         };
         uint32_t w[WC + 1], sword = 0u;
 #pragma unroll
@@ -111,8 +129,8 @@ __global__ void __launch_bounds__(256) pack_nvq_kernel(const __grid_constant__ P
             const int hi = r & 1, ft = r >> 2, f = ft / 3, t = ft % 3;
             const int grp = ch * kChunkGroupsB + 4 * f + 2 * ((r >> 1) & 1) + (c >> 1), vec = grp * 6 + 2 * t + (c & 1);
             if (src[hi] < 0 || grp >= a.ng || vec >= a.nvec) continue;
-            const uint32_t idx = stream_bits(a.stream[2], a.bit0[2] + ((uint32_t)src[hi] * a.nvec_file + a.group0 * 6 + vec) * IB, IB);
-            const uint32_t mask = stream_bits(a.stream[3], a.bit0[3] + ((uint32_t)src[hi] * a.nsign_file + a.group0 * 3 + (vec >> 1)) * 7u, 7);
+            const uint32_t idx = index[hi].get((uint64_t)(a.group0 * 6 + vec) * IB, IB);
+            const uint32_t mask = sign[hi].get((uint64_t)(a.group0 * 3 + (vec >> 1)) * 7u, 7);
             const uint32_t full = mask | ((uint32_t)(__popc(mask) & 1) << 7);   // the eighth sign is the parity of the seven stored ones
             const uint32_t field = ((full >> ((vec & 1) * 4)) & 15u) | (idx << 4);
             const int pos = r * FB, wi = pos >> 5, sh = pos & 31;
@@ -201,25 +219,25 @@ size_t stage_bytes(const std::vector<StreamSpec>& st, int64_t src_rows) {
     return n;
 }
 
-// Pieces of at most kSlotBytes of streams where the tensor allows (whole row-blocks, or whole units for padded ones).
+// Pieces of at most kSlotBytes of streams: several whole units, or row-blocks of one (at least one row-block).
 std::vector<Piece> cut_pieces(const LoadRows& rows, const std::vector<StreamSpec>& st) {
     std::vector<Piece> out;
-    const bool plain = rows.units.size() == 1 && rows.ope == rows.padded;
     auto fits = [&](int64_t r) { return stage_bytes(st, r) <= kSlotBytes; };
-    if (plain) {
-        int64_t per = rows.ope;
-        while (per > 16 && !fits(per)) per = std::max<int64_t>(16, (per / 2 + 15) / 16 * 16);
-        for (int64_t r = 0; r < rows.ope; r += per) {
-            const int n = (int)std::min(per, rows.ope - r);
-            out.push_back(Piece{r, rows.row0 + rows.units[0] * rows.ope + r, n, n, n, n});
-        }
-        return out;
-    }
+    int64_t per = rows.ope;   // rows of a piece inside a unit
+    while (per > 16 && !fits(per)) per = std::max<int64_t>(16, (per / 2 + 15) / 16 * 16);
     for (size_t i = 0; i < rows.units.size();) {
+        const int64_t dev0 = (int64_t)i * rows.padded, src0 = rows.row0 + rows.units[i] * rows.ope;
+        if (per < rows.ope) {
+            for (int64_t r = 0; r < rows.ope; r += per) {
+                const int64_t src = std::min(per, rows.ope - r), dev = r + per < rows.ope ? per : rows.padded - r;
+                out.push_back(Piece{dev0 + r, src0 + r, (int)dev, (int)dev, (int)src, (int)src});
+            }
+            ++i;
+            continue;
+        }
         size_t n = 1;
         while (i + n < rows.units.size() && rows.units[i + n] == rows.units[i] + (int)n && fits((int64_t)(n + 1) * rows.ope)) ++n;
-        out.push_back(Piece{(int64_t)i * rows.padded, rows.row0 + rows.units[i] * rows.ope, (int)(n * rows.padded), (int)rows.padded, (int)rows.ope,
-                            (int)(n * rows.ope)});
+        out.push_back(Piece{dev0, src0, (int)(n * rows.padded), (int)rows.padded, (int)rows.ope, (int)(n * rows.ope)});
         i += n;
     }
     return out;
@@ -233,7 +251,7 @@ void run_pieces(const std::vector<Piece>& pieces, const std::vector<StreamSpec>&
     std::lock_guard<std::mutex> lock(pool.mu);
     size_t need = 0;
     for (const Piece& pc : pieces) need = std::max(need, stage_bytes(st, pc.src_rows));
-    const bool big = need > kSlotBytes;   // a row-block (or an expert) of a very wide tensor: staging of this load only
+    const bool big = need > kSlotBytes;   // a row-block of a very wide tensor: staging of this load only
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency());
     const int workers = big ? 1 : (int)std::min<size_t>(std::min(kLoadWorkers, hw), pieces.size());
     Slot big_slot;
