@@ -11,6 +11,7 @@ torch = pytest.importorskip("torch")
 from oracle import mfq_oracle as O  # noqa: E402
 from tyloquant_b200 import encode, moe  # noqa: E402
 from test_nint_gpu import rel_l2, bf16_tensor, REL_L2  # noqa: E402
+from test_tile_gpu import _kernels  # noqa: E402
 
 
 @pytest.mark.parametrize("tokens,experts,k", [(1, 128, 8), (33, 128, 8), (7, 256, 6), (5, 16, 16), (9, 384, 12), (3, 100, 8), (64, 4096, 4)])
@@ -253,5 +254,34 @@ def test_records_with_padded_groups_keep_the_integer_kernels_accuracy(tokens):
     want = (pick(torch.einsum("tef,ehf->teh", act, dw)) * wts.double()[:, :, None]).sum(1)
     got = moe.moe_ffn(gu, dn, x, ids, wts).double()
     assert ((got - want).norm() / want.norm()).item() <= (2e-5 if tokens * k >= 3 * e_count else 2e-4)
+    gu.free()
+    dn.free()
+
+
+@pytest.mark.parametrize("cohorts,tokens", [(9, 400), (16, 400), (16, 2100)])
+def test_records_of_many_cohorts(cohorts, tokens):
+    """Up to sixteen cohorts take the tile kernel, however many experts share one."""
+    e_count, h, f, k = 16, 72, 48, 8
+    gen = torch.Generator("cuda").manual_seed(cohorts)
+    blobs = []
+    for shape in ((e_count, 2 * f, h), (e_count, h, f)):
+        w = torch.randn(shape, device="cuda", generator=gen) * 0.02
+        pools = []
+        for c in range(cohorts):
+            ids = list(range(c, e_count, cohorts))
+            bits, gs, sb = encode.CANONICAL_NINT[(3, 4, 6)[c % 3]]
+            pools.append((ids, f"NINT{bits}", encode.nint_blob(encode.quantize_nint(w[ids].reshape(-1, shape[2]), bits, gs, sb, device="cuda"))))
+        blobs.append(encode.nintm_blob(e_count, shape[1], shape[2], pools))
+    gu, dn = (moe.MoeWeight(b) for b in blobs)
+    x = torch.randn(tokens, h, device="cuda", generator=gen).to(torch.bfloat16)
+    ids, wts = moe.moe_topk(torch.randn(tokens, e_count, device="cuda", generator=gen), k)
+    gw, dw = (torch.stack([w.dequantize_expert(e) for e in range(e_count)]).double() for w in (gu, dn))
+    every = torch.einsum("th,eoh->teo", x.double(), gw)
+    act = every[..., f:] * every[..., :f] / (1 + torch.exp(-every[..., :f]))
+    out = torch.gather(torch.einsum("tef,ehf->teh", act, dw), 1, ids.long()[:, :, None].expand(-1, -1, h))
+    want = (out * wts.double()[:, :, None]).sum(1)
+    names = _kernels(lambda: moe.moe_ffn(gu, dn, x, ids, wts))
+    assert sum("tile_tc_kernel" in name for name in names) == 2, names
+    assert ((moe.moe_ffn(gu, dn, x, ids, wts).double() - want).norm() / want.norm()).item() <= REL_L2
     gu.free()
     dn.free()

@@ -52,7 +52,7 @@ constexpr int kTileWarpMma = kTileDecoders + kTileEpilogue, kTileWarpRec = kTile
 constexpr int kTileThreads = (kTileDecoders + kTileEpilogue + 3) * 32;
 constexpr size_t kTileDynSmem = 212 * 1024;   // beside 14 KB of barriers and tables
 constexpr int kTileGroup = 12;   // parts of a shared tile that are added at once; more go in two steps
-constexpr int kTileMaxPools = 8, kTileRecStages = 8, kTileXStages = 8, kTileAStages = 8, kTileSegs = 4;
+constexpr int kTileMaxPools = 16, kTileRecStages = 8, kTileXStages = 8, kTileAStages = 8, kTileSegs = 4;
 
 struct TileArgs {
     NintDevB pools[kTileMaxPools];   // the weight (entry 0), or the cohorts of an expert record
@@ -79,6 +79,8 @@ struct TileArgs {
     int rec_stages, rec_stage_bytes, x_stages, x_stage_bytes, x_whole /* 0: an activation stage is one 64-column slab; 1: the slabs of a step */, step /* chunks per step */, a_stages, a_cols, d_bufs, d_cols;
     int* error;
 };
+
+static_assert(sizeof(TileArgs) <= 4096, "kernel parameters");
 
 // One stretch of work: chunks [ch0, ch1) of a tile.
 struct TileSeg {
