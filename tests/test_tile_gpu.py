@@ -300,3 +300,25 @@ def test_padded_groups_keep_the_integer_kernels_accuracy(profile):
             assert np.linalg.norm(err) <= 1e-5 * np.linalg.norm(size), (profile, n, k, m)
         w.free()
     assert _status() == 0
+
+
+def test_state_scales_far_apart():
+    """State scales that are no f16 numbers side by side: rows that only have small ones keep their accuracy."""
+    n, k = 100, 400
+    wt = np.random.default_rng(1).standard_normal((n, k), dtype=np.float32) * np.float32(0.02)
+    t = encode.quantize_nvq3(wt, encode.synthetic_d4_banks(512, 2, seed=5), jsc=True, device="cuda")
+    t["sub"][:n // 2] = t["sub"][:n // 2] % 4            # states 0 .. 3 for the first rows
+    t["sub"][n // 2:] = 12 + t["sub"][n // 2:] % 4
+    blob = encode.nvq_blob(t)
+    at = blob.index(bytes([1, 2, 16, 1]), 36) + 4
+    lut = np.where(np.arange(16) < 4, 1.37 * 2.0 ** -18, 2.0 ** 14).astype("<f2")
+    blob = blob[:at] + lut.tobytes() + blob[at + 32:]
+    ref = O.dequant_nvq(O.unpack_nvq(blob)).astype(np.float64)
+    w = QuantWeight.from_blob("NVQ3J-512", blob)
+    for m in (2, 40, 300):
+        x = encode.bf16_round(np.random.default_rng(m).standard_normal((m, k), dtype=np.float32))
+        y = w.matmul(bf16_tensor(x), out_dtype=torch.float32).cpu().numpy()
+        err, size = y - x.astype(np.float64) @ ref.T, np.sqrt(np.square(x, dtype=np.float64) @ np.square(ref).T)
+        for rows in (slice(0, n // 2), slice(n // 2, n)):
+            assert np.linalg.norm(err[:, rows]) <= 1e-5 * np.linalg.norm(size[:, rows]), (m, rows)
+    assert _status() == 0

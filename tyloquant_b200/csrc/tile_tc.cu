@@ -354,27 +354,37 @@ static cudaError_t launch_one(const TileArgs& a, const TilePlan& p, int terms, c
     }
 }
 
+// Exponent that takes the state scales of a joint-codebook record to the top of what their products with the codes (up to 127)
+// may reach in f16.
+static int lattice_shift(const float* lut) {
+    float top = 0.f;
+    for (int i = 0; i < 16; ++i) top = std::max(top, std::fabs(lut[i]));
+    int e = 0;
+    if (top > 0.f && std::isfinite(top)) std::frexp(top, &e);   // top = m 2^e, m in [0.5, 1)
+    return 8 - e;
+}
 // f16 state scales of a lattice record, normalised so that code x scale stays below 2^15.
 static void lattice_scales(const NintDevB& w, TileArgs& a) {
-    float top = 0.f;
-    for (int i = 0; i < 16; ++i) top = std::max(top, std::fabs(w.jsc ? w.lut[i] : (float)i));
-    int e = 0;
-    if (w.jsc && top > 0.f && std::isfinite(top)) std::frexp(top, &e);   // top = m 2^e, m in [0.5, 1)
-    const int shift = w.jsc ? 8 - e : 0;                                 // codes reach 127
+    const int shift = w.jsc ? lattice_shift(w.lut) : 0;
     for (int i = 0; i < 16; ++i) a.lut16[i] = __half_as_ushort(__float2half(std::ldexp(w.jsc ? w.lut[i] : (float)i, shift)));
     a.lut_undo = std::ldexp(1.f, -shift);
 }
 int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes) {
     bool used[128] = {};
     for (size_t i = 0; i < n_codes; ++i) used[codes[i] & 127] = true;
-    for (int s = 0; s < 16; ++s)
+    const int shift = lattice_shift(lut);
+    int terms = 1;
+    for (int s = 0; s < 16; ++s) {
+        const float scaled = std::ldexp(lut[s], shift);
+        if (std::isfinite(lut[s]) && __half2float(__float2half(scaled)) != scaled) return 0;   // scales more than some 2^21 apart
         for (int c = 0; c < 128; ++c) {
             if (!used[c] || lut[s] == 0.f) continue;
             int e;
             const float m = std::frexp(lut[s] * (float)c, &e) * 2048.f;   // 11 significant bits are an f16
-            if (c && m != std::floor(m)) return 2;
+            if (c && m != std::floor(m)) terms = 2;
         }
-    return 1;
+    }
+    return terms;
 }
 
 // y [m, n] = x [m, k] W^T.  False when this weight has no tile kernel.
@@ -383,6 +393,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     TileArgs a{};
     TilePlan p;
     const int terms = w.tile_terms;
+    if (terms == 0) return false;
     // token tiles: as few as 256 columns allow, or fewer columns where a codebook of 128 KB leaves no room for the rings of that many
     // (giving up there cost a product of 256 rows 32 passes of the single-row kernel), of equal size
     const size_t rec_bytes = (size_t)w.rec_words * 4, ctx_bytes = w.table ? (size_t)w.table_words * 4 + 64 : 0;

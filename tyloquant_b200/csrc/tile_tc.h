@@ -46,7 +46,8 @@ __device__ __forceinline__ uint4 tile_row_const(uint32_t anchor, int bits) {
 // up rows and y [m, n / 2] = up * silu(gate).  False when this weight has no tile kernel (its tables do not fit).
 bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s, bool glu = false, const TileNorm* norm = nullptr);
 
-// f16 terms a lattice weight needs: 1 when every scale x code product is an f16 number, else 2.
+// f16 terms a lattice weight needs: 1 when every scale x code product is an f16 number, else 2; 0 when the state scales lie too far
+// apart to be f16 numbers side by side (no tile kernel then).
 int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes);
 
 // A route plan whose tiles hold up to tile_rows pairs, and where each expert lives.
