@@ -126,7 +126,7 @@ int mfqb_dequant(const mfqb_weight* w, void* out, int out_dtype, mfqb_stream_t s
  * An infinity or NaN in x makes the outputs NaN.
  * Library scratch: m >= 2 uses a per-device buffer (quantised planes, or activation tiles and partial sums) that
  * only ever grows -- a block handed to a kernel or baked into a captured graph stays allocated.
- * Growing calls cudaMalloc, so the first call with a given (or larger) m on a device must come
+ * Growing calls cudaMalloc, so one call with the same weight and the same or a larger m must come first,
  * outside stream capture; inside a capture it fails with MFQB_ERR_ARG instead.  The buffer holds
  * one call's data at a time: calls with m >= 2 on one device must be ordered by their streams.
  * A single-row (m = 1) product of a NINT weight uses a few KB of scratch owned by the weight

@@ -180,6 +180,34 @@ assert max(err) <= 1e-3, err
 """
 
 
+WARM_CALL = """
+import sys, torch
+sys.path.insert(0, %r)
+from tyloquant_b200 import QuantWeight, encode
+ws = [QuantWeight.from_blob("NINT4", encode.random_nint_blob(14336, 4096, 4, 32, 6, seed=1, device="cuda")),
+      QuantWeight.from_blob("NVQ3", encode.nvq_blob(encode.quantize_nvq3(torch.randn(640, 4096).numpy(), encode.d4_256_codebook()[None], jsc=False, device="cuda")))]
+x = torch.randn(600, 4096, device="cuda").to(torch.bfloat16)
+for w in ws:
+    for warm, later in ((8, (2, 3, 5)), (257, (256, 40, 16, 3)), (512, (300, 8, 1))):
+        for fn in (lambda m, w=w: w.matmul(x[:m]), lambda m, w=w: w.matmul_glu(x[:m])):
+            fn(warm)
+            torch.cuda.synchronize()
+            for m in later:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph):
+                    y = fn(m)
+                graph.replay()
+                torch.cuda.synchronize()
+                assert torch.isfinite(y.float()).all() and ((fn(m).float() - y.float()).norm() / y.float().norm()).item() < 1e-3, m
+"""
+
+
+def test_one_call_makes_room_for_captures_of_smaller_batches():
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", WARM_CALL % root], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr[-2000:]
+
+
 def test_call_that_grows_the_scratch_while_the_default_stream_is_busy():
     """New scratch, in memory that held something else, is cleared in the order of the call's own stream (here a non-blocking one)."""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))

@@ -88,7 +88,9 @@ __device__ __forceinline__ void store_quad(void* out, int out_dtype, size_t off,
 // fails with a message instead of breaking the capture.  Calls that share a block on one device
 // must be ordered by their streams (the block holds one call's intermediates at a time).
 struct GrowOnlyScratch {
-    void* get(int device, size_t bytes, cudaStream_t stream, const char* what);
+    void* get(int device, size_t bytes, cudaStream_t stream, const char* what, bool exact = false);   // exact: no room for growth
+    // Grows the block for a call that may follow, which could be captured; does nothing while the stream is.
+    void reserve(int device, size_t bytes, cudaStream_t stream, const char* what);
 
 private:
     struct PerDevice {

@@ -150,10 +150,10 @@ void launch_x_planes(const NintDevB& w, const void* x, int rows, void* planes, c
 }
 
 // Library scratch for the planes of a plain batched product (per device, grow-only).
-static void* planes_scratch(int device, size_t bytes, cudaStream_t s) {
-    static GrowOnlyScratch pool;
-    return pool.get(device, bytes, s, "mfqb_mul_mat (quantised activation planes)");
-}
+static GrowOnlyScratch g_planes;
+static void* planes_scratch(int device, size_t bytes, cudaStream_t s) { return g_planes.get(device, bytes, s, "mfqb_mul_mat (quantised activation planes)"); }
+// Room for the batches that the tile kernel leaves to the integer one (up to four rows).
+void reserve_planes(const NintDevB& w, int device, cudaStream_t s) { g_planes.reserve(device, nint_bl_planes_bytes(w, 4), s, "mfqb_mul_mat (quantised activation planes)"); }
 
 static int passes_for(int m) { return m <= 2 ? 1 : (m <= 4 ? 2 : 4); }
 

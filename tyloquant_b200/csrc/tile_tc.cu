@@ -434,13 +434,18 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     // The two launches below belong together: another thread's on the same stream would take the scratch between them.
     static std::mutex launches[64];
     std::lock_guard<std::mutex> lock(launches[device]);
-    static GrowOnlyScratch xs[2], parts, counts;   // activations: decoding batches keep a small block of their own beside the prefill's
-    const size_t xb = ((size_t)(m + 7) / 8 * 8 * a.x_row_bytes + 255) / 256 * 256;
-    unsigned char* buf = static_cast<unsigned char*>(xs[m > 16].get(device, xb + (size_t)m * 4, s, "mfqb_mul_mat (f16 activation tiles)"));
+    // One call with this weight makes room for every smaller batch of it: decoding batches keep a small block of their own beside
+    // the prefill's, and the parts of shared tiles are as many as any plan may have.
+    static GrowOnlyScratch xs[2], parts, counts;
+    const char* what = "mfqb_mul_mat (f16 activation tiles)";
+    auto x_bytes = [&](int rows) { return ((size_t)(rows + 7) / 8 * 8 * a.x_row_bytes + 255) / 256 * 256; };
+    const size_t xb = x_bytes(m);
+    if (m > 16) xs[0].reserve(device, x_bytes(16) + 64, s, what);
+    unsigned char* buf = static_cast<unsigned char*>(xs[m > 16].get(device, xb + (size_t)m * 4, s, what));
     a.x = buf;
     a.x_down = reinterpret_cast<const float*>(buf + xb);
-    a.partial = static_cast<float*>(parts.get(device, (size_t)p.grid * 2 * n * kTileRows * 4, s, "mfqb_mul_mat (parts of shared tiles)"));
-    a.counters = static_cast<unsigned*>(counts.get(device, (size_t)p.grid * 2 * 4, s, "mfqb_mul_mat (tile counters)"));
+    a.partial = static_cast<float*>(parts.get(device, (size_t)sms * 2 * 256 * kTileRows * 4, s, "mfqb_mul_mat (parts of shared tiles)", true));
+    a.counters = static_cast<unsigned*>(counts.get(device, (size_t)sms * 2 * 4, s, "mfqb_mul_mat (tile counters)", true));
     XTilesArgs xa{};
     xa.x = x;
     xa.kind = kTileXBf16;

@@ -31,21 +31,31 @@ int device_sm_count(int device) {
     return cache[device];
 }
 
-void* GrowOnlyScratch::get(int device, size_t bytes, cudaStream_t stream, const char* what) {
-    static std::mutex mu;   // one lock for every pool: growth is rare
-    std::lock_guard<std::mutex> lock(mu);
+static bool capturing(cudaStream_t stream) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) (void)cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+static std::mutex g_scratch_mu;   // one lock for every pool: growth is rare
+void GrowOnlyScratch::reserve(int device, size_t bytes, cudaStream_t stream, const char* what) {
+    {
+        std::lock_guard<std::mutex> lock(g_scratch_mu);
+        if (device >= 0 && device < 64 && dev_[device].bytes >= bytes) return;
+    }
+    if (!capturing(stream)) get(device, bytes, stream, what);
+}
+void* GrowOnlyScratch::get(int device, size_t bytes, cudaStream_t stream, const char* what, bool exact) {
+    std::lock_guard<std::mutex> lock(g_scratch_mu);
     if (device < 0 || device >= 64) fail(MFQB_ERR_ARG, "device index %d out of range", device);
     PerDevice& d = dev_[device];
     if (d.bytes >= bytes) return d.p;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &st) != cudaSuccess) (void)cudaGetLastError();
-    if (st != cudaStreamCaptureStatusNone)
+    if (capturing(stream))
         fail(MFQB_ERR_ARG,
              "%s needs %zu bytes of library scratch (it holds %zu) while the stream is being captured: "
              "run one call of this size outside the capture first",
              what, bytes, d.bytes);
     void* p = nullptr;
-    const size_t want = bytes + bytes / 2;
+    const size_t want = exact ? bytes : bytes + bytes / 2;
     device_malloc(&p, want);
     MFQB_CUDA(cudaMemsetAsync(p, 0, want, stream));   // some users keep self-resetting counters in their block: they start at zero, in the call's own order
     d.p = p;   // the previous block stays allocated: earlier launches and captured graphs may still use it
@@ -86,6 +96,7 @@ void launch_bl_gemv(const NintDevB& w, const void* x, int m, void* y, int y_dtyp
 bool nint_bl_supported(int bits, int gs);
 size_t gemvs_fix_bytes(int device);
 void launch_swiglu(const void* gate_up, int in_dtype, int rows, int f, void* hidden, cudaStream_t s);
+void reserve_planes(const NintDevB& w, int device, cudaStream_t s);
 void launch_bl_gemv_norm(const NintDevB& w, const float* h, const float* delta, const float* gamma, float eps, float* h_out, void* y, int y_dtype,
                          bool glu, int device, cudaStream_t s);
 int g_moe_f16_from_x2 = 4;   // see mfqb_tune
@@ -255,7 +266,10 @@ int mfqb_mul_mat(const mfqb_weight* w, const void* x, int m, void* y, int y_dtyp
         const int64_t n = w->info.n, k = w->info.k;
         const size_t ysz = y_dtype == MFQB_F32 ? 4 : 2;
         if (w->family == MFQB_FAMILY_NINT) {
-            if (m >= 5 && launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
+            if (m >= 5) {
+                reserve_planes(w->nint, w->device, stream);   // a call with fewer rows may follow inside a capture
+                if (launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
+            }
             if (m == 1 && gemv1_use_streamed(w->nint) &&
                 launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->dev.extra_at(), w->status, stream))
                 return;
@@ -314,8 +328,13 @@ int mfqb_mul_mat_glu(const mfqb_weight* w, const void* x, int m, void* y, int y_
             return;
         }
         const NintDevB& dev = weight_device_layout(w);
-        if (m >= (w->family == MFQB_FAMILY_NINT ? 5 : 2) && launch_tile_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
+        const int tile_from = w->family == MFQB_FAMILY_NINT ? 5 : 2;
         static GrowOnlyScratch pool;
+        if (m >= tile_from) {
+            pool.reserve(w->device, (size_t)(tile_from - 1) * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)");   // as in mfqb_mul_mat
+            if (w->family == MFQB_FAMILY_NINT) reserve_planes(dev, w->device, stream);
+            if (launch_tile_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
+        }
         float* prod = static_cast<float*>(pool.get(w->device, (size_t)m * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)"));
         const int rc = mfqb_mul_mat(w, x, m, prod, MFQB_F32, stream);
         if (rc != MFQB_OK) throw Error(rc, mfqb_last_error());
