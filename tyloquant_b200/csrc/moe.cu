@@ -226,7 +226,8 @@ static int moe_tile_m(const mfqb_moe_weight* w, int pairs) {
     int cap = 8;   // cohorts with wide records fit fewer batch rows per CTA
     for (const auto& pool : w->pools)
         if (pool->held) cap = std::min(cap, 2 * nint_bl_max_passes(pool->d));
-    // measured on the 128-expert top-8 layer: tiles of four win from two to about twenty pairs per expert
+    // measured on the 128-expert top-8 layer among the integer kernel's own tiles: pairs up to 1.5 per expert, fours to about
+    // twenty (the tile kernel takes over from two on, wherever the record has one)
     return std::min(cap, 2 * pairs <= 3 * e ? 2 : (pairs <= 24 * e ? 4 : 8));
 }
 

@@ -42,8 +42,7 @@ __device__ __forceinline__ float x_value(const void* row, int k, int j) {
     if constexpr (KIND == kTileXShared) return __bfloat162float(static_cast<const __nv_bfloat16*>(row)[j]);
     if constexpr (KIND == kTileXBf16) return __bfloat162float(__ldcg(static_cast<const __nv_bfloat16*>(row) + j));
     const float v = __ldcg(static_cast<const float*>(row) + j);
-    if constexpr (KIND == kTileXSwiglu) return __ldcg(static_cast<const float*>(row) + k + j) * v / (1.0f + expf(-v));
-    return v;
+    return __ldcg(static_cast<const float*>(row) + k + j) * v / (1.0f + expf(-v));
 }
 // Four consecutive values from column j on, zero past the row.
 template <int KIND>
@@ -56,10 +55,8 @@ __device__ __forceinline__ float4 x_quad(const void* row, int k, int j, bool ali
             v = make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
         } else {
             v = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + j));
-            if constexpr (KIND == kTileXSwiglu) {
-                const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k + j));
-                v = make_float4(u.x * v.x / (1.0f + expf(-v.x)), u.y * v.y / (1.0f + expf(-v.y)), u.z * v.z / (1.0f + expf(-v.z)), u.w * v.w / (1.0f + expf(-v.w)));
-            }
+            const float4 u = __ldcg(reinterpret_cast<const float4*>(static_cast<const float*>(row) + k + j));
+            v = make_float4(u.x * v.x / (1.0f + expf(-v.x)), u.y * v.y / (1.0f + expf(-v.y)), u.z * v.z / (1.0f + expf(-v.z)), u.w * v.w / (1.0f + expf(-v.w)));
         }
     } else {
         if (j < k) v.x = x_value<KIND>(row, k, j);

@@ -8,8 +8,8 @@
 
 namespace mfqb {
 
-// What the activation rows are: bf16, float32, or float32 gate | up products whose SwiGLU activation is formed on the way.
-enum TileX { kTileXBf16 = 0, kTileXF32 = 1, kTileXSwiglu = 2, kTileXShared = 3 /* bf16 in shared memory */ };
+// What the activation rows are: bf16, or float32 gate | up products whose SwiGLU activation is formed on the way.
+enum TileX { kTileXBf16 = 0, kTileXSwiglu = 1, kTileXShared = 2 /* bf16 in shared memory */ };
 // Residual add + RMSNorm on the way to the product: h [m, k] float32 += delta (may be null), x = bf16(h / rms(h) * gamma).
 struct TileNorm {
     float* h;
