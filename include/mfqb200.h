@@ -69,8 +69,8 @@ int mfqb_file_blob(const mfqb_file* f, int i, const void** data, uint64_t* nbyte
  * slice_nvq_cpu (cpp_runtime/mfq_decode.cpp:1663-1744, 3579-3677).
  *
  * dtype is the record's label ("NINT2".."NINT8", "NVQ3", "NVQ3J-512", "NVQ3J",
- * "NIQ3").  The blob is decoded on the host, re-laid into the device format and
- * uploaded to `device`; the call returns after the upload has completed.
+ * "NIQ3").  The blob's streams are copied to `device` as they are and re-laid into the
+ * device format there; the call returns when the device holds the tensor.
  *
  * axis: 0 = output rows [begin,end), 1 = input columns [begin,end).  Input slices must
  * start on a group boundary (NINT) / a multiple of 24 (NVQ); begin=0,end=-1 = whole.

@@ -191,7 +191,8 @@ int cudaMalloc(void** p, size_t n) {
 
 @pytest.mark.parametrize("block", [1, 3])
 def test_load_after_one_that_found_no_room(tmp_path, block):
-    """The first staging block, or one of several.  Staging survives between loads; one whose device half could not be allocated is not taken for complete."""
+    """Staging survives between loads; a block (the first, or one of several) whose device half could not be allocated is not taken
+    for complete."""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     src, lib = tmp_path / "shim.c", tmp_path / "shim.so"
     src.write_text(SHIM)

@@ -139,9 +139,8 @@ def test_mixed_precision_layer_and_expert_shards(tokens):
 
 @pytest.mark.parametrize("tokens", [16, 40, 400])
 def test_route_plan_tiles_and_grouped_tile_kernel(tokens):
-    """48 experts, top-4: 16 tokens give tiles of two pairs, 40 tokens tiles of four (with the four
-    canonical precisions every cohort then runs in the same launch), 400 tokens (33 pairs per expert)
-    go to the tensor-core tile kernel grouped by expert.  Also through an expert shard."""
+    """48 experts, top-4, the four canonical precisions in one launch: 16 tokens give integer tiles of two pairs, 40 tokens
+    (3.3 pairs per expert) and 400 (33) go to the tensor-memory tile kernel.  Also through an expert shard."""
     e_count, h, f, k = 48, 256, 96, 4
     bits = np.random.default_rng(5003).choice([2, 3, 4, 6], e_count)
     gu_blob, dn_blob = _moe_case(e_count, h, f, bits, seed=5001)
@@ -283,5 +282,50 @@ def test_records_of_many_cohorts(cohorts, tokens):
     names = _kernels(lambda: moe.moe_ffn(gu, dn, x, ids, wts))
     assert sum("tile_tc_kernel" in name for name in names) == 2, names
     assert ((moe.moe_ffn(gu, dn, x, ids, wts).double() - want).norm() / want.norm()).item() <= REL_L2
+    gu.free()
+    dn.free()
+
+
+def _ffn_reference(gu, dn, x, ids, wts):
+    e_count, f = gu.info.n_experts, dn.info.k
+    gw, dw = (torch.stack([w.dequantize_expert(e) for e in range(e_count)]).double() for w in (gu, dn))
+    every = torch.einsum("th,eoh->teo", x.double(), gw)
+    act = every[..., f:] * every[..., :f] / (1 + torch.exp(-every[..., :f]))
+    out = torch.gather(torch.einsum("tef,ehf->teh", act, dw), 1, ids.long()[:, :, None].expand(-1, -1, dn.info.out_per_expert))
+    return (out * wts.double()[:, :, None]).sum(1)
+
+
+@pytest.mark.parametrize("tokens", [40, 300, 700])
+@pytest.mark.parametrize("bits", [[4, 6], [5, 3]])
+def test_hot_experts_take_several_token_tiles(tokens, bits):
+    """One expert draws half of all routes: more pairs than a tile holds, so its later tiles start inside its rows."""
+    e_count, h, f, k = 16, 200, 72, 2
+    gu_blob, dn_blob = _moe_case(e_count, h, f, bits * 8, seed=61)
+    gu, dn = moe.MoeWeight(gu_blob), moe.MoeWeight(dn_blob)
+    gen = torch.Generator("cuda").manual_seed(tokens)
+    x = torch.randn(tokens, h, device="cuda", generator=gen).to(torch.bfloat16)
+    z = torch.randn(tokens, e_count, device="cuda", generator=gen)
+    z[:, 5] += 20.0
+    ids, wts = moe.moe_topk(z, k)
+    want = _ffn_reference(gu, dn, x, ids, wts)
+    got = moe.moe_ffn(gu, dn, x, ids, wts).double()
+    assert ((got - want).norm() / want.norm()).item() <= REL_L2
+    assert ((got[-8:] - want[-8:]).norm() / want[-8:].norm()).item() <= REL_L2
+    gu.free()
+    dn.free()
+
+
+def test_integer_tiles_of_four_pairs():
+    """Between one and a half and two pairs per expert."""
+    e_count, h, f, k, tokens = 16, 200, 72, 4, 7
+    gu_blob, dn_blob = _moe_case(e_count, h, f, [3, 4, 6, 8] * 4, seed=71)
+    gu, dn = moe.MoeWeight(gu_blob), moe.MoeWeight(dn_blob)
+    gen = torch.Generator("cuda").manual_seed(72)
+    x = torch.randn(tokens, h, device="cuda", generator=gen).to(torch.bfloat16)
+    ids, wts = moe.moe_topk(torch.randn(tokens, e_count, device="cuda", generator=gen), k)
+    want = _ffn_reference(gu, dn, x, ids, wts)
+    names = _kernels(lambda: moe.moe_ffn(gu, dn, x, ids, wts))
+    assert any("moe_hetero_tiles_kernel" in name for name in names) and not any("tile_tc_kernel" in name for name in names), names
+    assert ((moe.moe_ffn(gu, dn, x, ids, wts).double() - want).norm() / want.norm()).item() <= 2e-4   # 16-bit float32 activations
     gu.free()
     dn.free()
