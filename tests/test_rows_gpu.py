@@ -1,0 +1,91 @@
+"""The few-rows kernel (two to sixteen activation rows) against the decoded weights in float64, at the edges of its tiles, slices, passes and formats."""
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from tyloquant_b200 import QuantWeight, encode  # noqa: E402
+from test_gemm_gpu import _status  # noqa: E402
+
+# bits, group size, sub-scale bits; bound on the error over what the products add up to without cancellation.  Exact weights leave the float32 sums (some tens of roundings of 2^-24, and the two
+# terms of the group sums, 2^-22, which uncentred widths subtract from sums a few times as large); width six takes one f16 rounding of the integers above 2^11, at most 2^-12 of each (rows of one group have
+# the largest sub-scale in every place; 1.3e-4 in the mean square of long rows).
+EXACT, ROUNDED = 5e-6, 2.0 ** -12
+PROFILES = [((2, 16, 5), EXACT), ((3, 24, 5), EXACT), ((4, 24, 6), EXACT), ((4, 32, 6), EXACT), ((4, 48, 7), EXACT), ((5, 28, 7), EXACT), ((5, 32, 7), EXACT), ((5, 64, 6), EXACT),
+            ((6, 24, 7), ROUNDED), ((6, 40, 7), ROUNDED), ((6, 64, 7), ROUNDED)]
+
+
+def _x(m, k, seed, offset=0):
+    gen = torch.Generator("cuda").manual_seed(seed)
+    flat = torch.randn(m * k + offset, device="cuda", generator=gen).to(torch.bfloat16)
+    return flat[offset:].view(m, k)
+
+
+def _check(w, x, bound, **kw):
+    got = w.matmul(x, out_dtype=torch.float32, **kw)
+    ref = w.dequantize().double()
+    err, size = got.double() - x.double() @ ref.T, (x.double().square() @ ref.T.square()).sqrt()
+    assert (err.norm() / size.norm()).item() <= bound, (x.shape, ref.shape, (err.norm() / size.norm()).item())
+    assert torch.equal(got, w.matmul(x, out_dtype=torch.float32, **kw))   # the same bits in every call
+    return got
+
+
+@pytest.mark.parametrize("profile,bound", PROFILES)
+def test_scalar_weights(profile, bound):
+    bits, gs, sub = profile
+    # rows: less than a row-block, ragged, more than one per CTA; columns: one group and less, ragged, odd, more than a slice
+    for n, k in ((1, gs), (17, gs - 3), (100, 1000), (333, 777), (2400, 1030), (48, 12000)):
+        w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(n, k, bits, gs, sub, seed=n + k, device="cuda"))
+        for m in (5, 8, 9, 16) if bits == 6 else (2, 3, 8, 9, 16):
+            _check(w, _x(m, k, m), bound)
+        w.free()
+    assert _status() == 0
+
+
+def test_many_row_blocks_per_cta():
+    """More row-blocks than a CTA adds up at a time."""
+    w = QuantWeight.from_blob("NINT3", encode.random_nint_blob(148 * 16 * 30 + 5, 200, 3, 24, 5, seed=3, device="cuda"))
+    for m in (3, 16):
+        _check(w, _x(m, 200, m), EXACT)
+    w.free()
+
+
+@pytest.mark.parametrize("dtype,entries", [("NVQ3", 256), ("NVQ3J-512", 512)])
+def test_lattice_weights(dtype, entries):
+    for n, k in ((9, 20), (300, 2399), (640, 5120)):
+        wt = np.random.default_rng(n).standard_normal((n, k), dtype=np.float32) * np.float32(0.02)
+        banks = encode.d4_256_codebook()[None] if dtype == "NVQ3" else encode.synthetic_d4_banks(entries, 2, seed=9)
+        w = QuantWeight.from_blob(dtype, encode.nvq_blob(encode.quantize_nvq3(wt, banks, jsc=dtype != "NVQ3", device="cuda")))
+        for m in (2, 5, 8):
+            _check(w, _x(m, k, m), EXACT)
+        w.free()
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+def test_unaligned_rows(offset):
+    """Activation rows that start on 2, 4 and 8 bytes."""
+    for k, gs in ((1000, 24), (1004, 28), (1001, 24)):
+        bits = 5 if gs == 28 else 4
+        w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(130, k, bits, gs, 6, seed=k, device="cuda"))
+        _check(w, _x(11, k, 1, offset), EXACT)
+        w.free()
+
+
+def test_gated_epilogue_and_non_finite_rows():
+    n, k = 32 * 37, 1500
+    w = QuantWeight.from_blob("NINT4", encode.random_nint_blob(n, k, 4, 24, 6, seed=8, device="cuda"))
+    for m in (2, 7, 16):
+        x = _x(m, k, m)
+        p = (x.double() @ w.dequantize().double().T).view(m, n // 32, 2, 16)
+        want = (p[:, :, 1] * p[:, :, 0] / (1 + torch.exp(-p[:, :, 0]))).reshape(m, n // 2)
+        got = w.matmul_glu(x, out_dtype=torch.float32).double()
+        assert ((got - want).norm() / want.norm()).item() <= 2e-5
+        bad = x.clone()
+        bad[0, 3], bad[1, k - 1] = float("inf"), float("nan")
+        y = w.matmul(bad, out_dtype=torch.float32)
+        assert not torch.isfinite(y[:2]).any() and torch.isfinite(y[2:]).all()
+    assert _status() == 0
+    w.free()

@@ -21,6 +21,7 @@
 #include <cmath>
 
 #include "cuda_util.h"
+#include "rows_mma.h"
 #include "tile_tc.h"
 
 namespace mfqb {
@@ -604,7 +605,8 @@ static const float* rank_sum(mfqb_decoder* d, const float* in, float* out, size_
 static bool norm_mul_mat(mfqb_decoder* d, const mfqb_weight* w, const float* delta, const void* gamma, int rows, void* y, int y_dtype, bool glu, cudaStream_t s) {
     if (rows < 5) return false;
     const TileNorm norm{static_cast<float*>(d->h.p), delta, static_cast<const float*>(gamma), d->cfg.rms_eps};
-    return launch_tile_product(weight_device_layout(w), nullptr, rows, y, y_dtype, d->device, s, glu, &norm);
+    return launch_rows_product(weight_device_layout(w), nullptr, rows, y, y_dtype, d->device, s, glu, &norm) ||
+           launch_tile_product(weight_device_layout(w), nullptr, rows, y, y_dtype, d->device, s, glu, &norm);
 }
 
 static void mul_mat(const mfqb_weight* w, const void* x, int m, void* y, cudaStream_t s) {

@@ -1,0 +1,5 @@
+#include "rows_mma_launch.cuh"
+
+namespace mfqb {
+MFQB_ROWS_INSTANTIATE(2)
+}  // namespace mfqb

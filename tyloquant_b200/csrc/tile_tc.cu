@@ -361,10 +361,10 @@ static int lattice_shift(const float* lut) {
     return 8 - e;
 }
 // f16 state scales of a lattice record, normalised so that code x scale stays below 2^15.
-static void lattice_scales(const NintDevB& w, TileArgs& a) {
+void tile_lattice_scales(const NintDevB& w, uint16_t (&lut16)[16], float& undo) {
     const int shift = w.jsc ? lattice_shift(w.lut) : 0;
-    for (int i = 0; i < 16; ++i) a.lut16[i] = __half_as_ushort(__float2half(std::ldexp(w.jsc ? w.lut[i] : (float)i, shift)));
-    a.lut_undo = std::ldexp(1.f, -shift);
+    for (int i = 0; i < 16; ++i) lut16[i] = __half_as_ushort(__float2half(std::ldexp(w.jsc ? w.lut[i] : (float)i, shift)));
+    undo = std::ldexp(1.f, -shift);
 }
 int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes) {
     bool used[128] = {};
@@ -406,7 +406,7 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     if (units * (sms + 1) >= (1ll << 31) * 1ll * sms || units >= (1ll << 31)) return false;
     a.pools[0] = w;
     a.lut_undo = 1.f;
-    if (w.table) lattice_scales(w, a);
+    if (w.table) tile_lattice_scales(w, a.lut16, a.lut_undo);
     a.m = m;
     a.ntok = (m + n - 1) / n;
     a.x_rows = n;

@@ -50,6 +50,9 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
 // apart to be f16 numbers side by side (no tile kernel then).
 int lattice_terms(const float* lut, const int8_t* codes, size_t n_codes);
 
+// f16 state scales of a lattice record, normalised so that code x scale stays below 2^15, and what undoes that.
+void tile_lattice_scales(const NintDevB& w, uint16_t (&lut16)[16], float& undo);
+
 // A route plan whose tiles hold up to tile_rows pairs, and where each expert lives.
 struct TileRoutes {
     const int *expert_bounds, *tile_bounds, *pair_order, *expert_pool, *expert_local;

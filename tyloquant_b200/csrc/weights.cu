@@ -14,6 +14,7 @@
 #include "load.h"
 #include "nvq.h"
 #include "nvq_blayout.h"
+#include "rows_mma.h"
 #include "tile_tc.h"
 
 namespace mfqb {
@@ -266,9 +267,11 @@ int mfqb_mul_mat(const mfqb_weight* w, const void* x, int m, void* y, int y_dtyp
         const int64_t n = w->info.n, k = w->info.k;
         const size_t ysz = y_dtype == MFQB_F32 ? 4 : 2;
         if (w->family == MFQB_FAMILY_NINT) {
-            if (m >= 5) {
-                reserve_planes(w->nint, w->device, stream);   // a call with fewer rows may follow inside a capture
-                if (launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
+            if (m >= 2) {
+                if (m >= 5) reserve_planes(w->nint, w->device, stream);   // a call with fewer rows may follow inside a capture
+                if (launch_rows_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
+                if (m >= 5) reserve_rows(w->nint, w->device, stream);
+                if (m >= 5 && launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
             }
             if (m == 1 && gemv1_use_streamed(w->nint) &&
                 launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->dev.extra_at(), w->status, stream))
@@ -330,9 +333,13 @@ int mfqb_mul_mat_glu(const mfqb_weight* w, const void* x, int m, void* y, int y_
         const NintDevB& dev = weight_device_layout(w);
         const int tile_from = w->family == MFQB_FAMILY_NINT ? 5 : 2;
         static GrowOnlyScratch pool;
-        if (m >= tile_from) {
-            pool.reserve(w->device, (size_t)(tile_from - 1) * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)");   // as in mfqb_mul_mat
+        if (m >= tile_from) {   // as in mfqb_mul_mat
+            pool.reserve(w->device, (size_t)(tile_from - 1) * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)");
             if (w->family == MFQB_FAMILY_NINT) reserve_planes(dev, w->device, stream);
+        }
+        if (m >= 2 && launch_rows_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
+        if (m >= tile_from) {
+            reserve_rows(dev, w->device, stream);
             if (launch_tile_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
         }
         float* prod = static_cast<float*>(pool.get(w->device, (size_t)m * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)"));
