@@ -556,13 +556,12 @@ __device__ __forceinline__ bool tile_issue(const TileArgs& a, TileShared& sh, Ti
     auto run = [&](auto first_c, auto len_c, bool x_done) {   // slabs [first, first + len) of the chunk, all in half first / 2T
         constexpr int FIRST = decltype(first_c)::value, LEN = decltype(len_c)::value, H0 = FIRST % (2 * T);
         const uint32_t at = __shfl_sync(0xffffffffu, tmem_a + (uint32_t)(ar.stage * a.a_cols), 0);
-        const uint32_t xb = __shfl_sync(0xffffffffu, smem_u32(x_ring) + (uint32_t)(xr.stage * a.x_stage_bytes), 0);
+        const uint64_t bdesc = smem_desc_sw128(__shfl_sync(0xffffffffu, smem_u32(x_ring) + (uint32_t)(xr.stage * a.x_stage_bytes), 0));
         if (elect_one()) {
 #pragma unroll
             for (int i = 0; i < LEN; ++i) {
                 const int sl = FIRST + i;
-                const uint64_t bdesc = smem_desc_sw128(xb) + (uint64_t)(2 * (sl & 3));
-                tile_mma<TERMS, XTERMS>(td, at + (uint32_t)(8 * (H0 + i)), 16u * T, bdesc, x_pitch, idesc, sl > 0 || acc);
+                tile_mma<TERMS, XTERMS>(td, at + (uint32_t)(8 * (H0 + i)), 16u * T, bdesc + (uint64_t)(2 * (sl & 3)), x_pitch, idesc, sl > 0 || acc);
             }
             if (x_done) tc_commit(&sh.x_empty[xr.stage]);
             if (H0 + LEN == 2 * T) tc_commit(&sh.a_empty[ar.stage]);
@@ -795,24 +794,25 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
             const int t8 = a.pools[s.pool].t8;
             if (!tile_wait(&sh.d_empty[dr.stage], dr.phase ^ 1u)) { ok = false; break; }
             tc_fence_after_sync();
-            const uint32_t td = __shfl_sync(0xffffffffu, tmem_d + (uint32_t)(dr.stage * a.d_cols), 0);
-            const uint32_t x_pitch = (uint32_t)((s.ncols + 7) & ~7) * 128u;
-            bool acc = false;
-            for (int ch = s.ch0; ch < s.ch1 && ok; ch += a.step, acc = true) {
-                const int n = min(a.step, s.ch1 - ch);
-                auto issue = [&](auto t_c) {
-                    constexpr int T = decltype(t_c)::value;
-                    ok = a.x_whole ? tile_issue_step<Sets::TERMS, Sets::XTERMS, T>(a, sh, ar, xr, x_ring, x_pitch, tmem_a, td, idesc, acc, n)
-                                   : tile_issue<Sets::TERMS, Sets::XTERMS, T>(a, sh, ar, xr, x_ring, x_pitch, tmem_a, td, idesc, acc);
-                };
-                switch (t8) {
-                    case 2: issue(std::integral_constant<int, 2>{}); break;
-                    case 3: issue(std::integral_constant<int, 3>{}); break;
-                    case 4: issue(std::integral_constant<int, 4>{}); break;
-                    case 5: issue(std::integral_constant<int, 5>{}); break;
-                    case 6: issue(std::integral_constant<int, 6>{}); break;
-                    default: issue(std::integral_constant<int, 8>{}); break;
-                }
+            // Everything that the products' operands are made of is made warp-uniform here, and the loop over chunks runs inside the choice of T: beside busy decoders an instruction of this warp
+            // takes some ten clocks (NINT4 in groups of 32 14336 x 4096, 512 rows: 68.3 us, 66 with this form).
+            const int n = __shfl_sync(0xffffffffu, s.ch1 - s.ch0, 0);
+            const uint32_t td = __shfl_sync(0xffffffffu, tmem_d + (uint32_t)(dr.stage * a.d_cols), 0), ta = __shfl_sync(0xffffffffu, tmem_a, 0);
+            const uint32_t x_pitch = __shfl_sync(0xffffffffu, (uint32_t)((s.ncols + 7) & ~7) * 128u, 0);
+            auto issue = [&](auto t_c) {
+                constexpr int T = decltype(t_c)::value;
+                if (a.x_whole)
+                    for (int c = 0; c < n && ok; c += a.step) ok = tile_issue_step<Sets::TERMS, Sets::XTERMS, T>(a, sh, ar, xr, x_ring, x_pitch, ta, td, idesc, c > 0, min(a.step, n - c));
+                else
+                    for (int c = 0; c < n && ok; ++c) ok = tile_issue<Sets::TERMS, Sets::XTERMS, T>(a, sh, ar, xr, x_ring, x_pitch, ta, td, idesc, c > 0);
+            };
+            switch (t8) {
+                case 2: issue(std::integral_constant<int, 2>{}); break;
+                case 3: issue(std::integral_constant<int, 3>{}); break;
+                case 4: issue(std::integral_constant<int, 4>{}); break;
+                case 5: issue(std::integral_constant<int, 5>{}); break;
+                case 6: issue(std::integral_constant<int, 6>{}); break;
+                default: issue(std::integral_constant<int, 8>{}); break;
             }
             if (ok && elect_one()) tc_commit(&sh.d_full[dr.stage]);
             __syncwarp();
