@@ -86,6 +86,28 @@ def test_one_block_matches_the_float32_restatement():
     dec.free()
 
 
+@pytest.mark.parametrize("ctx", [0, 15, 16, 63, 64, 255, 256, 600, 1023])
+def test_new_key_and_value_take_their_place_in_the_scan(ctx):
+    """The step's own key and value never come out of the cache: they are put into the scan's ring, here in its first and
+    later rounds, at both ends of a 16-token round and alone in their slice (32 sequences leave slices of up to 256 tokens).
+    Tolerance as for the block above."""
+    cfg = dict(CFG, layers=1, max_ctx=1024, max_batch=32)
+    dec, blobs = D.random_decoder(**cfg, seed=12, keep_blobs=True)
+    dec.fill_cache(ctx, seed=4)
+    h_in = np.random.default_rng(5).standard_normal((32, cfg["hidden"])).astype(np.float32)
+    w = {k: O.dequant_nint(O.unpack_nint(b)) for k, b in blobs[0].items()}
+    rows = (0, 31)
+    none = np.zeros((cfg["n_kv_heads"], 0, 128), dtype=np.float32)
+    before = {r: [dec.read_cache(0, r, i, ctx).float().cpu().numpy() if ctx else none for i in (0, 1)] for r in rows}
+    got = dec.layer(0, torch.from_numpy(h_in).cuda()).cpu().numpy()
+    for r in rows:
+        want, k_new, v_new = _block_oracle(h_in[r], w, *before[r], ctx, cfg["n_q_heads"], cfg["n_kv_heads"])
+        assert rel_l2(got[r], want) <= 1e-3, (r, rel_l2(got[r], want))
+        assert rel_l2(dec.read_cache(0, r, 0, ctx + 1).float().cpu().numpy()[:, ctx], k_new) <= 4e-3
+        assert rel_l2(dec.read_cache(0, r, 1, ctx + 1).float().cpu().numpy()[:, ctx], v_new) <= 4e-3
+    dec.free()
+
+
 def test_greedy_steps_and_graph_replay_agree():
     """Three greedy steps launched directly equal the same three replayed from a captured graph."""
     outs = []
