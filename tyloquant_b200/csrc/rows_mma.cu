@@ -18,10 +18,11 @@ static bool rows_exact(const NintDevB& w) {
 }
 static bool rows_takes(const NintDevB& w, int m) {
     if (m < 2 || m > kRowsMax) return false;
-    if (w.table) return w.tile_terms == 1 && m <= 8;   // a look-up per four weights and the table's bank conflicts: 16 rows through NVQ3 17408 x 5120 26.0 us, tile kernel 23.7
-    if (w.bits == 8) return false;                     // a record is 26 to 66 registers: NINT8-48 14336 x 4096 32 us for 8 rows, tile kernel 20
-    // Two to four rows, and padded group sizes, have integer kernels (4e-6) or two-term weights as their other path: exact widths only.  Widths up to four bits are not centred and
-    // would lose accuracy where they are rounded.
+    // A look-up per four weights and the table's bank conflicts: NVQ3 17408 x 5120 8 rows 21.1 us, 16 rows 26.0; tile kernel 23.6.
+    if (w.table) return w.tile_terms == 1 && m <= 8;
+    if (w.bits == 8) return false;   // a record would be 26 to 66 registers: NINT8-48 14336 x 4096 32 us for 8 rows, tile kernel 17
+    // Two to four rows, and padded group sizes, have integer kernels (4e-6) or two-term weights as their other path: exact widths
+    // only.  Widths up to four bits are not centred and would lose accuracy where they are rounded.
     if (m < 5 || w.gs % 8 || w.bits < 5) return rows_exact(w);
     return true;
 }
@@ -31,8 +32,9 @@ struct RowsPlan {
     size_t x_bytes = 0, smem = 0;
 };
 
-// Split of the work: slices of K times tiles of row-blocks, one CTA each, at most one per SM.  More slices than one where shared memory does not hold all of K, or where rows are few; only as many
-// as divide the SMs evenly: a grid that leaves one to four of them free costs the chain up to 3 us (NINT4 4096 x 4096, 16 rows: 148 tiles 9.0 us, 147 11.8, 144 10.8, 128 9.3).
+// Split of the work: slices of K times tiles of row-blocks, one CTA each, at most one per SM.  More slices than one where shared
+// memory does not hold all of K, or where rows are few; only as many as divide the SMs evenly: a grid that leaves one to four of
+// them free costs the chain up to 3 us (NINT4 4096 x 4096, 16 rows: 148 tiles 9.0 us, 147 11.8, 144 10.8, 128 9.3).
 static bool rows_plan(const NintDevB& w, int m, bool glu, int sms, RowsPlan& best) {
     const int nt = m <= 8 ? 1 : 2, unit = glu ? 2 : 1, units = w.nrb / unit;
     const size_t chunk = (size_t)rows_chunk_bytes(w.t8, nt), slot = (size_t)8 * nt * kRowsSlot * 4, ctx = w.table ? (size_t)w.table_words * 4 + 64 : 0;
@@ -120,9 +122,11 @@ bool launch_rows_product(const NintDevB& w, const void* x, int m, void* y, int y
     if (!rows_takes(w, m) || (norm && (w.k % 4 || w.k > 20480))) return false;   // the row as bf16 in a CTA's 48 KB
     RowsPlan p;
     if (!rows_plan(w, m, glu, device_sm_count(device), p)) return false;
-    // Long lists of records: nine and more rows of six-bit codes are faster on the tile kernel (28672 x 4096: 15 rounds, 31.7 us against 32.3; 57344 x 4096: 29, 60.6 against 52.5).  Four bits: level
-    // at 29 rounds (47.7 and 47.8).
-    if (m > 8 && p.rounds > (w.bits == 6 ? 20 : 30) && w.gs % 8 == 0) return false;
+    // Long lists of records, nine and more rows: the tile kernel's steps cost less than the second activation tile here.
+    // Six bits, 16 rows, this kernel and the tile kernel: 28672 x 4096 (15 rounds) 31.7 and 32.1 us, 36864 (18) 37.4 and 37.4,
+    // 45056 (22) 44.4 and 43.6, 57344 (29) 62.3 and 53.9.  Four bits: 36864 29.4 and 33.3, 45056 35.7 and 38.7, 57344 47.7 and 45.8.
+    // A padded group size doubles the tile kernel's steps (NINT5-28 28672 x 4096: 33.1 and 72.1).
+    if (m > 8 && p.rounds > (w.bits == 6 ? 20 : 25) && w.gs % 8 == 0) return false;
     const int nt = m <= 8 ? 1 : 2;
     RowsArgs a{};
     a.w = w;
@@ -166,7 +170,6 @@ bool launch_rows_product(const NintDevB& w, const void* x, int m, void* y, int y
         case 4: e = launch_rows_bits<4>(a, p.smem, s); break;
         case 5: e = launch_rows_bits<5>(a, p.smem, s); break;
         case 6: e = launch_rows_bits<6>(a, p.smem, s); break;
-        case 8: e = launch_rows_bits<8>(a, p.smem, s); break;
         default: break;
     }
     if (e != cudaSuccess)

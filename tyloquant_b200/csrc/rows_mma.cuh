@@ -2,24 +2,31 @@
 //
 //   y[token, n] = sum_k x[token, k] * W[n, k]
 //
-// For a handful of tokens the tensor-memory tile kernel (tile_tc.cuh) spends its time on its pipeline: its roles pass every chunk on through barriers whose round trips take
-// 100 to 300 clocks each, and a tile of 128 rows is shared by several CTAs that add their sums up through L2.  Here a warp does everything for a 16-row record by itself: it
-// loads the record's words into registers one record ahead (asked into L2 four ahead: NINT6 28672 x 4096, 8 rows 26.6 us; not at all 28.9, eight 28.9), turns them into A operands -- in byte-lane fragment order two registers ARE
-// rows q, q + 8 of a 16 x 16 operand -- and multiplies on mma.m16n8k16.  There is no barrier between the first and the last record of a CTA.
-//   * rows_x_kernel writes the activations once as B operands (f16, group sums beside them); a CTA brings its slice of K into shared memory with bulk copies.
-//   * A CTA has a slice of K (mostly all of it) and some row-blocks; their records are one list that its 20 warps share out evenly, in the order of K, so a row-block's
-//     partial sums are few and added in a fixed order: a product has the same bits in every call.  20 warps of 96 registers leave 4096 registers, room for a CTA of
-//     rows_x_kernel, which is there when the predecessor ends.
+// For a handful of tokens the tensor-memory tile kernel (tile_tc.cuh) spends its time on its pipeline: its roles pass every chunk
+// on through barriers whose round trips take 100 to 300 clocks each, and a tile of 128 rows is shared by several CTAs that add
+// their sums up through L2.  Here a warp does everything for a 16-row record by itself: it loads the record's words into
+// registers one record ahead (asked into L2 four ahead: NINT6 28672 x 4096, 8 rows 26.6 us; not at all 28.9, eight 28.9), turns
+// them into A operands -- in byte-lane fragment order two registers ARE rows q, q + 8 of a 16 x 16 operand -- and multiplies on
+// mma.m16n8k16.  There is no barrier between the first and the last record of a CTA.
+//   * rows_x_kernel writes the activations once as B operands (f16, group sums beside them); a CTA brings its slice of K into
+//     shared memory with bulk copies.
+//   * A CTA has a slice of K (mostly all of it) and some row-blocks; their records are one list that its 20 warps share out
+//     evenly, in the order of K, so a row-block's partial sums are few and added in a fixed order: a product has the same bits in
+//     every call.  20 warps of 96 registers leave 4096 registers, room for a CTA of rows_x_kernel, which is there when the
+//     predecessor ends.
 //
-// Arithmetic.  An integer below 2048 in the low bits of a half IS the f16 number n 2^-24, so a masked field needs no conversion: one multiplication (centred widths: one
-// fused multiply-add) gives (q - mid) ss 2^-20, exact below 2^11: widths 2 to 5 with the usual sub-scales are exact throughout (1e-6 on the product, float32 sums), 6 and 8 are rounded once
-// (1.3e-4 and 2.0e-4; the tile kernel's two roundings 2.4e-4).  What the offsets add, -nm sm X_g and for centred widths ns mid ss X_g with the group sums X_g of the
-// activations in two f16 terms, is one more k-step whose A operand are the record's scale bytes as they lie.
+// Arithmetic.  An integer below 2048 in the low bits of a half IS the f16 number n 2^-24, so a masked field needs no conversion:
+// one multiplication (centred widths: one fused multiply-add) gives (q - mid) ss 2^-20, exact below 2^11: widths 2 to 5 with the
+// usual sub-scales are exact throughout (1e-6 on the product, float32 sums), six are rounded once (1.3e-4; the tile
+// kernel's two roundings 2.4e-4).  What the offsets add, -nm sm X_g and for centred widths ns mid ss X_g with the group sums
+// X_g of the activations in two f16 terms, is one more k-step whose A operand are the record's scale bytes as they lie.
 //
-// Measured (us, 16 / 8 rows; in brackets the tile kernel): NINT4 4096 x 4096 9.2 / 7.7 (13.1 / 12.8), 6144 x 4096 10.6 / 9.0 (14.4), 28672 x 4096 25.2 / 21.0 (29.0), NINT6 28672 x 4096 31.7 / 26.6
-// (32.3), 4096 x 14336 19.6 / 16.9 (20.7), NINT3 14336 x 4096 16.0 / 13.9 (20.1), NINT5 in groups of 28 5000 x 2888 10.2 / 9.1 (17.0), 28672 x 4096 33 / 28 (72), NVQ3 17408 x 5120 8 rows 21.0 (23.8);
-// 3 rows (in brackets the integer kernel): NINT4 6144 x 4096 8.9 (16.4), NINT3 14336 x 4096 13.8 (21.9).  Bound by instruction issue: some 390 a record (16 rows x 192 columns x 16 tokens) at 2.1
-// to 2.5 a clock, half of them on pipes that take one every other clock.
+// Measured (us, 16 / 8 rows; in brackets the tile kernel): NINT4 4096 x 4096 9.2 / 7.7 (13.1 / 12.8), 6144 x 4096 10.6 / 9.0
+// (14.4), 28672 x 4096 25.2 / 21.0 (28.3), NINT6 28672 x 4096 31.7 / 26.6 (32.1), 4096 x 14336 19.6 / 16.9 (20.7), NINT3 14336 x
+// 4096 16.0 / 13.9 (20.1), NINT5 in groups of 28 5000 x 2888 10.2 / 9.1 (17.0), 28672 x 4096 33 / 28 (72), NVQ3 17408 x 5120 8
+// rows 21.0 (23.6), 5120 x 5120 12.1 (20.1); 3 rows (in brackets the integer kernel): NINT4 6144 x 4096 8.9 (16.4), NINT3 14336 x
+// 4096 13.8 (21.9).  Bound by instruction issue: some 390 a record (16 rows x 192 columns x 16 tokens) at 2.1 to 2.5 a clock,
+// half of them on pipes that take one every other clock.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -100,9 +107,10 @@ __device__ __forceinline__ void rows_static_for(Fn&& f) {
     }
 }
 
-// Scalar codes.  An integer n < 2048 in the low bits of a half IS the f16 number n 2^-24, so a masked field needs no conversion: field q at bit pos is
-// q 2^(pos - 24), times d = ss 2^(4 - pos) gives q ss 2^-20 with one rounding (none below 2^11).  Widths from five bits on are centred, (q - mid) ss 2^-20, by the
-// addend of the same instruction; mid ss X_g comes back through one more k-step (S1).
+// Scalar codes.  An integer n < 2048 in the low bits of a half IS the f16 number n 2^-24, so a masked field needs no conversion:
+// field q at bit pos is q 2^(pos - 24), times d = ss 2^(4 - pos) gives q ss 2^-20 with one rounding (none below 2^11).  Widths
+// from five bits on are centred, (q - mid) ss 2^-20, by the addend of the same instruction; mid ss X_g comes back through one
+// more k-step (S1).
 template <int BITS, int T_>
 struct RowsNint {
     static constexpr int T = T_, MID = BITS >= 5 ? 1 << (BITS - 1) : 0;
@@ -171,8 +179,9 @@ struct RowsNint {
 };
 
 
-// Lattice vectors: a field is a look-up in the signed table (shared memory, codes biased by 128).  Plain records: (code + 128) 2^-24 times 16 ss less 128 of it,
-// integers below 2048, exact.  Joint-codebook records: code times the state's f16 scale, for records whose products are f16 numbers (tile_terms 1).
+// Lattice vectors: a field is a look-up in the signed table (shared memory, codes biased by 128).  Plain records: (code + 128)
+// 2^-24 times 16 ss less 128 of it, integers below 2048, exact.  Joint-codebook records: code times the state's f16 scale, for
+// records whose products are f16 numbers (tile_terms 1).
 template <int IB, bool JSC>
 struct RowsNvq {
     static constexpr int T = 3, FB = IB + 4, WC = (24 * FB + 31) / 32, SW = 1;
@@ -285,10 +294,11 @@ struct RowsGroup {
     }
 };
 
-// One group of a token's activations as B operands, by eight neighbouring lanes for the eight groups of a chunk: values scaled by a power of two per token and chunk (largest
-// magnitude next to 2^15; exact for bf16 values within 2^-28 of it), the group's sum as two f16 terms, the factor's inverse.
-// Slab 2 (f T + t) + h of a chunk holds octet t of groups 4 f + 2 h and the next: lane 4 q + c (token q of a tile of eight) reads quad c & 1 of group c >> 1, slots 0, 2
-// and 1, 3 in its two registers -- the order in which the decoders' byte pairs come.  Lanes are XORed with 4 h + f, which spreads a token's groups over the banks.
+// One group of a token's activations as B operands, by eight neighbouring lanes for the eight groups of a chunk: values scaled by
+// a power of two per token and chunk (largest magnitude next to 2^15; exact for bf16 values within 2^-28 of it), the group's sum
+// as two f16 terms, the factor's inverse. Slab 2 (f T + t) + h of a chunk holds octet t of groups 4 f + 2 h and the next: lane 4
+// q + c (token q of a tile of eight) reads quad c & 1 of group c >> 1, slots 0, 2 and 1, 3 in its two registers -- the order in
+// which the decoders' byte pairs come.  Lanes are XORed with 4 h + f, which spreads a token's groups over the banks.
 template <int T>
 __device__ __forceinline__ void rows_x_group(const RowsGroup<T>& v, unsigned char* chunk, int t, int g, int nt, float factor, bool live) {
     uint32_t mx = v.absmax(0u);
@@ -317,9 +327,10 @@ __device__ __forceinline__ void rows_x_group(const RowsGroup<T>& v, unsigned cha
     if (g == 0) *reinterpret_cast<float*>(chunk + (size_t)(4 * T + 1) * slab + 4 * t) = sc.y;
 }
 
-// At most 32 registers: a CTA of it then fits beside the 20 warps of 96 registers of the kernel before it, and waits there for its end (with more it is launched after that end: 16 rows through
-// NINT4 4096 x 4096 14.7 us instead of 9.2).
-// A CTA per chunk, a thread per (token, group): 1.3 us of a product's chain (a factor per whole row, as the tile kernel has it, needs a pass for the maxima before: 2.8).
+// At most 32 registers: a CTA of it then fits beside the 20 warps of 96 registers of the kernel before it, and waits there for
+// its end (with more it is launched after that end: 16 rows through NINT4 4096 x 4096 14.7 us instead of 9.2). A CTA per chunk, a
+// thread per (token, group): 1.3 us of a product's chain (a factor per whole row, as the tile kernel has it, needs a pass for the
+// maxima before: 2.8).
 template <int T>
 __global__ void __launch_bounds__(128, T <= 4 ? 16 : 8) rows_x_kernel(const __grid_constant__ RowsXArgs a) {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -334,7 +345,8 @@ __global__ void __launch_bounds__(128, T <= 4 ? 16 : 8) rows_x_kernel(const __gr
     rows_x_group<T>(v, a.out + (size_t)blockIdx.x * rows_chunk_bytes(T, a.nt), t, g, a.nt, a.factor, t < a.m);
 }
 
-// The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the scaling, and in shared memory as bf16 after it.
+// The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the
+// scaling, and in shared memory as bf16 after it.
 template <int T>
 __global__ void __launch_bounds__(1024) rows_norm_kernel(const __grid_constant__ RowsXArgs a, const __grid_constant__ TileNorm nm) {
     constexpr int KEEP = 2;
