@@ -520,8 +520,9 @@ __global__ void embed_rows_kernel(const int* __restrict__ ids, const __nv_bfloat
     }
 }
 
-// Seeded synthetic cache contents (a stand-in for the prefill pass): values of unit scale.  Buffer blockIdx.y takes seed + blockIdx.y.  One launch for up to 64 buffers: a launch each was 6 us for
-// the 4 us of one sequence's buffer (64 of them 0.47 ms).  Bound by integer instructions, twelve a value, two in three at half rate.
+// Seeded synthetic cache contents (a stand-in for the prefill pass): values of unit scale.  Buffer blockIdx.y takes seed +
+// blockIdx.y.  One launch for up to 64 buffers: a launch each was 6 us for the 4 us of one sequence's buffer (64 of them 0.47
+// ms).  Bound by integer instructions, twelve a value, two in three at half rate.
 constexpr int kFillMax = 64;
 struct FillArgs {
     uint4* p[kFillMax];
@@ -622,8 +623,8 @@ static const float* rank_sum(mfqb_decoder* d, const float* in, float* out, size_
     return out;
 }
 
-// Batched steps: residual add, RMSNorm and product with the normalised row going straight into the tile kernel's activation
-// layout.  False when this weight or batch has no tile kernel: the caller normalises, then multiplies.
+// Batched steps: residual add, RMSNorm and product with the normalised row going straight into the batched kernel's activation
+// layout.  False when this weight or batch has neither of the two kernels: the caller normalises, then multiplies.
 static bool norm_mul_mat(mfqb_decoder* d, const mfqb_weight* w, const float* delta, const void* gamma, int rows, void* y, int y_dtype, bool glu, cudaStream_t s) {
     if (rows < 5) return false;
     const TileNorm norm{static_cast<float*>(d->h.p), delta, static_cast<const float*>(gamma), d->cfg.rms_eps};

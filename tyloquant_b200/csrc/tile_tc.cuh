@@ -794,8 +794,9 @@ __global__ void __launch_bounds__(1024, 1) tile_tc_kernel(const __grid_constant_
             const int t8 = a.pools[s.pool].t8;
             if (!tile_wait(&sh.d_empty[dr.stage], dr.phase ^ 1u)) { ok = false; break; }
             tc_fence_after_sync();
-            // Everything that the products' operands are made of is made warp-uniform here, and the loop over chunks runs inside the choice of T: beside busy decoders an instruction of this warp
-            // takes some ten clocks (NINT4 in groups of 32 14336 x 4096, 512 rows: 68.3 us, 66 with this form).
+            // Everything that the products' operands are made of is made warp-uniform here, and the loop over chunks runs inside the
+            // choice of T: beside busy decoders an instruction of this warp takes some ten clocks (NINT4 in groups of 32
+            // 14336 x 4096, 512 rows: 68.3 us, 64.2 with this form; NINT6 28672 x 4096, 64 rows: 41.6, 38.8).
             const int n = __shfl_sync(0xffffffffu, s.ch1 - s.ch0, 0);
             const uint32_t td = __shfl_sync(0xffffffffu, tmem_d + (uint32_t)(dr.stage * a.d_cols), 0), ta = __shfl_sync(0xffffffffu, tmem_a, 0);
             const uint32_t x_pitch = __shfl_sync(0xffffffffu, (uint32_t)((s.ncols + 7) & ~7) * 128u, 0);
