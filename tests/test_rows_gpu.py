@@ -89,3 +89,24 @@ def test_gated_epilogue_and_non_finite_rows():
         assert not torch.isfinite(y[:2]).any() and torch.isfinite(y[2:]).all()
     assert _status() == 0
     w.free()
+
+
+@pytest.mark.parametrize("dtype", ["NINT4", "NINT5", "NINT6", "NVQ3", "NVQ3J-512"])
+def test_non_finite_values_make_all_outputs_of_their_row_nan(dtype):
+    n, k = 200, 1500
+    if dtype.startswith("NINT"):
+        blob = encode.random_nint_blob(n, k, int(dtype[4]), 24, 6, seed=4, device="cuda")
+    else:
+        wt = np.random.default_rng(3).standard_normal((n, k), dtype=np.float32) * np.float32(0.02)
+        banks = encode.d4_256_codebook()[None] if dtype == "NVQ3" else encode.synthetic_d4_banks(512, 2, seed=9)
+        blob = encode.nvq_blob(encode.quantize_nvq3(wt, banks, jsc=dtype != "NVQ3", device="cuda"))
+    w = QuantWeight.from_blob(dtype, blob)
+    for m in (5, 8, 16) if dtype == "NINT6" else (2, 5, 8) if dtype.startswith("NVQ") else (2, 5, 8, 16):
+        for at in (0, 700, k - 1):
+            for value in (float("inf"), -float("inf"), float("nan")):
+                x = _x(m, k, m)
+                x[m - 1, at] = value
+                y = w.matmul(x, out_dtype=torch.float32)
+                assert torch.isnan(y[m - 1]).all() and torch.isfinite(y[:m - 1]).all(), (dtype, m, at, value)
+    assert _status() == 0
+    w.free()

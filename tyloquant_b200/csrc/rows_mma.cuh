@@ -246,10 +246,13 @@ struct RowsNvq {
     }
 };
 
-// (2^e, 2^-e) with 2^e * max in [2^14, 2^15); (1, 1) for a zero, subnormal or non-finite maximum.
+// (2^e, 2^-e) with 2^e * max in [2^14, 2^15); (1, 1) for a zero or subnormal maximum.  A chunk with an infinity or NaN is scaled by
+// NaN: every product with it is one, so all outputs of the token are (an infinity left as it is gives infinities: lattice records
+// have no products with the sums, which would make NaN of it).
 __device__ __forceinline__ float2 rows_x_scale(uint32_t absmax_bits) {
     int eb = (int)(absmax_bits >> 23);
-    if (eb == 0 || eb == 255) return make_float2(1.f, 1.f);
+    if (eb == 0) return make_float2(1.f, 1.f);
+    if (eb == 255) return make_float2(__uint_as_float(0x7FC00000u), 1.f);
     eb = max(eb, 15);
     return make_float2(__uint_as_float((uint32_t)(268 - eb) << 23), __uint_as_float((uint32_t)(eb - 14) << 23));
 }
@@ -315,7 +318,7 @@ __device__ __forceinline__ void rows_x_group(const RowsGroup<T>& v, unsigned cha
             const uint32_t u0 = v.v[4 * i + 2 * e], u1 = v.v[4 * i + 2 * e + 1];
             const float x0 = __uint_as_float(u0 << 16) * sc.x, x1 = __uint_as_float(u0 & 0xFFFF0000u) * sc.x;
             const float x2 = __uint_as_float(u1 << 16) * sc.x, x3 = __uint_as_float(u1 & 0xFFFF0000u) * sc.x;
-            sum += (x0 + x1) + (x2 + x3);   // (an infinity or NaN goes through the sums' two terms into every output of the token)
+            sum += (x0 + x1) + (x2 + x3);
             *reinterpret_cast<uint2*>(at(2 * (f * T + i) + h, (4 * q + 2 * b + e) ^ (4 * h + f))) =
                 make_uint2(rows_u32(__floats2half2_rn(x0, x2)), rows_u32(__floats2half2_rn(x1, x3)));
         }
