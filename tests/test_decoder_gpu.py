@@ -6,6 +6,10 @@ The block's intermediates pass through bf16 three times (normalised input, atten
 activation), as in the reference runtime where they are fp16 (cpp_runtime/mfq_decode.cpp:12210-12400);
 the float32 restatement applies the same roundings, and the bound is then the path's 1e-3."""
 
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -148,3 +152,42 @@ def test_greedy_steps_and_graph_replay_agree():
         assert ((outs[-1] >= 0) & (outs[-1] < CFG["vocab"])).all()
         dec.free()
     assert np.array_equal(outs[0], outs[1])
+
+
+SMALLER_STEPS = """
+import sys, torch
+sys.path.insert(0, %r)
+from tyloquant_b200 import QuantWeight, decoder, encode
+hidden, ffn, vocab, first, later, profiles = %r
+dec = decoder.Decoder(hidden=hidden, n_q_heads=hidden // 128, n_kv_heads=hidden // 512, ffn=ffn, vocab=vocab, layers=1, max_ctx=64, max_batch=32)
+shapes = ((hidden + hidden // 2, hidden), (hidden, hidden), (2 * ffn, hidden), (hidden, ffn), (vocab, hidden))
+ws = [QuantWeight.from_blob(f"NINT{p[0]}", encode.random_nint_blob(*shape, *p, seed=i, device="cuda")) for i, (shape, p) in enumerate(zip(shapes, profiles))]
+dec.set_layer(0, *ws[:4])
+dec.set_head(ws[4], torch.randn(vocab, hidden, device="cuda").to(torch.bfloat16))
+ids = torch.arange(32, dtype=torch.int32, device="cuda")
+dec.fill_cache(20, seed=1)
+dec.step(ids[:first])
+torch.cuda.synchronize()
+for batch in later:
+    out = torch.empty_like(ids[:batch])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        dec.step(ids[:batch], out)
+    dec.fill_cache(20, seed=1)
+    graph.replay()
+    dec.fill_cache(20, seed=1)
+    again = dec.step(ids[:batch])
+    torch.cuda.synchronize()
+    assert torch.equal(out, again), batch
+"""
+
+
+@pytest.mark.parametrize("form", [
+    # the output projections have a kernel of their own and leave the few rows' scratch to the products behind a normalisation
+    (512, 768, 1000, 32, (16, 9, 8, 5, 4, 3, 2, 1), ((4, 24, 6), (8, 48, 7), (6, 24, 7), (8, 48, 7), (6, 24, 7))),
+    # a long head: the tile kernel's for the first batch, the few-rows kernel's for the smaller one
+    (2048, 768, 128256, 16, (8, 3), ((8, 48, 7), (8, 48, 7), (8, 48, 7), (8, 48, 7), (6, 24, 7)))])
+def test_one_step_makes_room_for_captured_steps_of_smaller_batches(form):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", SMALLER_STEPS % (root, form)], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr[-2000:]

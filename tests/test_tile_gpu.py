@@ -185,10 +185,11 @@ import sys, torch
 sys.path.insert(0, %r)
 from tyloquant_b200 import QuantWeight, encode
 ws = [QuantWeight.from_blob("NINT4", encode.random_nint_blob(14336, 4096, 4, 32, 6, seed=1, device="cuda")),
+      QuantWeight.from_blob("NINT6", encode.random_nint_blob(14336, 4096, 6, 24, 7, seed=1, device="cuda")),
       QuantWeight.from_blob("NVQ3", encode.nvq_blob(encode.quantize_nvq3(torch.randn(640, 4096).numpy(), encode.d4_256_codebook()[None], jsc=False, device="cuda")))]
 x = torch.randn(600, 4096, device="cuda").to(torch.bfloat16)
 for w in ws:
-    for warm, later in ((8, (2, 3, 5)), (257, (256, 40, 16, 3)), (512, (300, 8, 1))):
+    for warm, later in %s:
         for fn in (lambda m, w=w: w.matmul(x[:m]), lambda m, w=w: w.matmul_glu(x[:m])):
             fn(warm)
             torch.cuda.synchronize()
@@ -202,9 +203,11 @@ for w in ws:
 """
 
 
-def test_one_call_makes_room_for_captures_of_smaller_batches():
+@pytest.mark.parametrize("calls", [((8, (2, 3, 5)), (257, (256, 40, 16, 3)), (512, (300, 8, 1))),
+                                   ((257, (256, 40, 16, 9, 8, 5, 4, 3, 2, 1)),)])   # the second: nothing but the tile kernel has run before the captures
+def test_one_call_makes_room_for_captures_of_smaller_batches(calls):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    r = subprocess.run([sys.executable, "-c", WARM_CALL % root], capture_output=True, text=True, timeout=300)
+    r = subprocess.run([sys.executable, "-c", WARM_CALL % (root, calls)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr[-2000:]
 
 

@@ -27,6 +27,7 @@
 namespace mfqb {
 
 const NintDevB& weight_device_layout(const mfqb_weight* w);
+void reserve_fewer_rows(const mfqb_weight* w, int m, bool glu, cudaStream_t s);
 
 constexpr int kHeadDim = 128;
 
@@ -627,6 +628,7 @@ static const float* rank_sum(mfqb_decoder* d, const float* in, float* out, size_
 // layout.  False when this weight or batch has neither of the two kernels: the caller normalises, then multiplies.
 static bool norm_mul_mat(mfqb_decoder* d, const mfqb_weight* w, const float* delta, const void* gamma, int rows, void* y, int y_dtype, bool glu, cudaStream_t s) {
     if (rows < 5) return false;
+    reserve_fewer_rows(w, rows, glu, s);
     const TileNorm norm{static_cast<float*>(d->h.p), delta, static_cast<const float*>(gamma), d->cfg.rms_eps};
     return launch_rows_product(weight_device_layout(w), nullptr, rows, y, y_dtype, d->device, s, glu, &norm) ||
            launch_tile_product(weight_device_layout(w), nullptr, rows, y, y_dtype, d->device, s, glu, &norm);

@@ -108,7 +108,6 @@ void nvq_dequant(const NvqDevice& w, void* out, int out_dtype, cudaStream_t stre
 
 void nvq_mul_mat(const NvqDevice& w, const void* x_bf16, int m, void* y, int y_dtype, cudaStream_t stream) {
     if (m >= 2 && launch_rows_product(w.d, x_bf16, m, y, y_dtype, w.device, stream)) return;
-    if (m >= 2) reserve_rows(w.d, w.device, stream);
     if (m >= 2 && launch_tile_product(w.d, x_bf16, m, y, y_dtype, w.device, stream)) return;
     const size_t ysz = y_dtype == MFQB_F32 ? 4 : 2;
     for (int m0 = 0; m0 < m; m0 += 8) {   // batch rows one launch covers

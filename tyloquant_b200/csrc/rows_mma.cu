@@ -100,22 +100,16 @@ static void launch_rows_x(const RowsXArgs& a, int t8, const TileNorm* norm, cuda
     }
 }
 
-static GrowOnlyScratch g_frags, g_parts, g_counts;
-static unsigned char* rows_frags(const NintDevB& w, int device, cudaStream_t s) {
-    return static_cast<unsigned char*>(g_frags.get(device, (size_t)w.nchunks * rows_chunk_bytes(w.t8, 2), s, "mfqb_mul_mat (activation fragments)"));
-}
-static float* rows_parts(int device, cudaStream_t s) {   // any plan's: slices > 1 have one pass
-    return static_cast<float*>(g_parts.get(device, (size_t)device_sm_count(device) * kRowsPass * 16 * kRowsMax * 4, s, "mfqb_mul_mat (parts of shared rows)", true));
-}
-static unsigned* rows_counts(int device, cudaStream_t s) {
-    return static_cast<unsigned*>(g_counts.get(device, (size_t)device_sm_count(device) * 4, s, "mfqb_mul_mat (row counters)", true));
-}
+static GrowOnlyScratch g_frags, g_shared;
+static size_t rows_frag_bytes(const NintDevB& w) { return (size_t)w.nchunks * rows_chunk_bytes(w.t8, 2); }
+// Parts and arrival counts of any plan (slices > 1 have one pass).
+static size_t rows_part_bytes(int device) { return (size_t)device_sm_count(device) * kRowsPass * 16 * kRowsMax * 4; }
+static size_t rows_shared_bytes(int device) { return rows_part_bytes(device) + (size_t)device_sm_count(device) * 4; }
+static const char *kRowsFrags = "mfqb_mul_mat (activation fragments)", *kRowsShared = "mfqb_mul_mat (parts of shared rows)";
 void reserve_rows(const NintDevB& w, int device, cudaStream_t s) {
     if (!rows_takes(w, 2) && !rows_takes(w, 5)) return;
-    const size_t sms = (size_t)device_sm_count(device);
-    g_frags.reserve(device, (size_t)w.nchunks * rows_chunk_bytes(w.t8, 2), s, "mfqb_mul_mat (activation fragments)");
-    g_parts.reserve(device, sms * kRowsPass * 16 * kRowsMax * 4, s, "mfqb_mul_mat (parts of shared rows)");
-    g_counts.reserve(device, sms * 4, s, "mfqb_mul_mat (row counters)");
+    g_frags.reserve(device, rows_frag_bytes(w), s, kRowsFrags);
+    g_shared.reserve(device, rows_shared_bytes(device), s, kRowsShared);
 }
 
 bool launch_rows_product(const NintDevB& w, const void* x, int m, void* y, int y_dtype, int device, cudaStream_t s, bool glu, const TileNorm* norm) {
@@ -144,12 +138,12 @@ bool launch_rows_product(const NintDevB& w, const void* x, int m, void* y, int y
     a.error = device_status_word(device);
     static std::mutex launches[64];   // the two launches belong together: another thread's on the same stream would take the scratch between them
     std::lock_guard<std::mutex> lock(launches[device]);
-    unsigned char* frags = rows_frags(w, device, s);
+    // One call with this weight makes room for every smaller batch of it: fragments of 16 rows, parts of any plan.
+    unsigned char* frags = static_cast<unsigned char*>(g_frags.get(device, rows_frag_bytes(w), s, kRowsFrags));
+    unsigned char* shared = static_cast<unsigned char*>(g_shared.get(device, rows_shared_bytes(device), s, kRowsShared, true));
     a.x = frags;
-    if (p.slices > 1) {
-        a.parts = rows_parts(device, s);
-        a.counters = rows_counts(device, s);
-    }
+    a.parts = reinterpret_cast<float*>(shared);
+    a.counters = reinterpret_cast<unsigned*>(shared + rows_part_bytes(device));
     RowsXArgs xa{};
     xa.x = static_cast<const __nv_bfloat16*>(x);
     xa.m = m;

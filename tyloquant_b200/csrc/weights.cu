@@ -163,6 +163,21 @@ static mfqb_weight* make_nint_weight(const NintView& t, const SliceRange& r, int
 }
 
 const NintDevB& weight_device_layout(const mfqb_weight* w) { return w->family == MFQB_FAMILY_NINT ? w->nint : nvq_device_layout(*w->nvq); }
+
+// Rows from which the tile kernel is tried.
+static int tile_from(const mfqb_weight* w) { return w->family == MFQB_FAMILY_NINT ? 5 : 2; }
+static GrowOnlyScratch g_glu_rows;   // the products of gated rows that no kernel with the gate in its epilogue takes
+constexpr const char* kGluRows = "mfqb_mul_mat_glu (gate and up products)";
+// A call of m rows makes room for captured calls of fewer, which may take other kernels with scratch of their own: the integer
+// one below tile_from rows, the few-rows kernel below the tile kernel.  (Every kernel's own block holds all that it takes.)
+void reserve_fewer_rows(const mfqb_weight* w, int m, bool glu, cudaStream_t s) {
+    const int from = tile_from(w);
+    if (m < from) return;
+    const NintDevB& dev = weight_device_layout(w);
+    if (w->family == MFQB_FAMILY_NINT) reserve_planes(dev, w->device, s);
+    reserve_rows(dev, w->device, s);
+    if (glu) g_glu_rows.reserve(w->device, (size_t)(from - 1) * w->info.n * 4, s, kGluRows);
+}
 int weight_device_index(const mfqb_weight* w) { return w->device; }
 
 }  // namespace mfqb
@@ -266,13 +281,10 @@ int mfqb_mul_mat(const mfqb_weight* w, const void* x, int m, void* y, int y_dtyp
         DeviceGuard guard(w->device);
         const int64_t n = w->info.n, k = w->info.k;
         const size_t ysz = y_dtype == MFQB_F32 ? 4 : 2;
+        reserve_fewer_rows(w, m, false, stream);
         if (w->family == MFQB_FAMILY_NINT) {
-            if (m >= 2) {
-                if (m >= 5) reserve_planes(w->nint, w->device, stream);   // a call with fewer rows may follow inside a capture
-                if (launch_rows_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
-                if (m >= 5) reserve_rows(w->nint, w->device, stream);
-                if (m >= 5 && launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
-            }
+            if (m >= 2 && launch_rows_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
+            if (m >= 5 && launch_tile_product(w->nint, x, m, y, y_dtype, w->device, stream)) return;
             if (m == 1 && gemv1_use_streamed(w->nint) &&
                 launch_bl_gemvs(w->nint, x, MFQB_BF16, y, y_dtype, w->device, w->dev.extra_at(), w->status, stream))
                 return;
@@ -331,18 +343,10 @@ int mfqb_mul_mat_glu(const mfqb_weight* w, const void* x, int m, void* y, int y_
             return;
         }
         const NintDevB& dev = weight_device_layout(w);
-        const int tile_from = w->family == MFQB_FAMILY_NINT ? 5 : 2;
-        static GrowOnlyScratch pool;
-        if (m >= tile_from) {   // as in mfqb_mul_mat
-            pool.reserve(w->device, (size_t)(tile_from - 1) * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)");
-            if (w->family == MFQB_FAMILY_NINT) reserve_planes(dev, w->device, stream);
-        }
+        reserve_fewer_rows(w, m, true, stream);
         if (m >= 2 && launch_rows_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
-        if (m >= tile_from) {
-            reserve_rows(dev, w->device, stream);
-            if (launch_tile_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
-        }
-        float* prod = static_cast<float*>(pool.get(w->device, (size_t)m * w->info.n * 4, stream, "mfqb_mul_mat_glu (gate and up products)"));
+        if (m >= tile_from(w) && launch_tile_product(dev, x, m, y, y_dtype, w->device, stream, true)) return;
+        float* prod = static_cast<float*>(g_glu_rows.get(w->device, (size_t)m * w->info.n * 4, stream, kGluRows));
         const int rc = mfqb_mul_mat(w, x, m, prod, MFQB_F32, stream);
         if (rc != MFQB_OK) throw Error(rc, mfqb_last_error());
         const size_t total = (size_t)m * (w->info.n / 2);
