@@ -1,5 +1,7 @@
 """The few-rows kernel (two to sixteen activation rows) against the decoded weights in float64, at the edges of its tiles, slices, passes and formats."""
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -9,11 +11,12 @@ torch = pytest.importorskip("torch")
 
 from tyloquant_b200 import QuantWeight, encode  # noqa: E402
 from test_gemm_gpu import _status  # noqa: E402
+from test_tile_gpu import _kernel_nodes  # noqa: E402
 
 # bits, group size, sub-scale bits; bound on the error over what the products add up to without cancellation.  Exact weights leave the float32 sums (some tens of roundings of 2^-24, and the two
-# terms of the group sums, 2^-22, which uncentred widths subtract from sums a few times as large); width six takes one f16 rounding of the integers above 2^11, at most 2^-12 of each (rows of one group have
-# the largest sub-scale in every place; 1.3e-4 in the mean square of long rows).
-EXACT, ROUNDED = 5e-6, 2.0 ** -12
+# terms of the group sums, 2^-22, which uncentred widths subtract from sums a few times as large); width six takes one f16 rounding of the integers above 2^11, at most 2^-11 of each and
+# 1.3e-4 in the mean square of many groups; a row of one group has the largest sub-scale in every place, where all odd codes beyond 16 are off by the whole 1 of 2048 to 4064.
+EXACT, ROUNDED, ONE_GROUP = 5e-6, 2.0 ** -12, 2.0 ** -11
 PROFILES = [((2, 16, 5), EXACT), ((3, 24, 5), EXACT), ((4, 24, 6), EXACT), ((4, 32, 6), EXACT), ((4, 48, 7), EXACT), ((5, 28, 7), EXACT), ((5, 32, 7), EXACT), ((5, 64, 6), EXACT),
             ((6, 24, 7), ROUNDED), ((6, 40, 7), ROUNDED), ((6, 64, 7), ROUNDED)]
 
@@ -109,4 +112,46 @@ def test_non_finite_values_make_all_outputs_of_their_row_nan(dtype):
                 y = w.matmul(x, out_dtype=torch.float32)
                 assert torch.isnan(y[m - 1]).all() and torch.isfinite(y[:m - 1]).all(), (dtype, m, at, value)
     assert _status() == 0
+    w.free()
+
+
+WIDE = [((4, 48, 6), EXACT), ((5, 48, 6), EXACT), ((6, 32, 7), ROUNDED), ((6, 48, 7), ROUNDED), ((4, 44, 6), EXACT), ((5, 44, 6), EXACT), ((5, 60, 6), EXACT)]
+
+
+@pytest.mark.parametrize("profile,bound", WIDE)
+def test_wide_records(profile, bound):
+    """Records that come into registers by halves, groups that two threads write; rows that start on 2, 4, 8 and 16 bytes."""
+    bits, gs, sub = profile
+    for n, k in ((1, gs), (100, 1000), (333, 777), (2400, 1032), (48, 12000)):
+        w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(n, k, bits, gs, sub, seed=n + k, device="cuda"))
+        for m, offset in ((5, 0), (8, 1), (9, 2), (15, 4), (16, 8)):
+            _check(w, _x(m, k, m, offset), ONE_GROUP if bound == ROUNDED and n == 1 else bound)
+        w.free()
+    assert _status() == 0
+
+
+class _FuncAttributes(ctypes.Structure):   # cudaFuncAttributes, its first members
+    _fields_ = [("shared", ctypes.c_size_t), ("const", ctypes.c_size_t), ("local", ctypes.c_size_t), ("max_threads", ctypes.c_int), ("regs", ctypes.c_int),
+                ("rest", ctypes.c_byte * 256)]
+
+
+@pytest.mark.parametrize("profile", [p for p, _ in PROFILES + WIDE])
+def test_the_next_products_activations_fit_beside_a_product(profile):
+    """Each of an SM's four schedulers has 16,384 registers.  What a product's warps leave of them holds the CTA that writes the
+    next product's activations, which is then there when the product ends; and no product keeps more than a few words of a
+    thread in local memory."""
+    bits, gs, sub = profile
+    w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(64, 3 * gs, bits, gs, sub, seed=1, device="cuda"))
+    rt = ctypes.CDLL("libcudart.so.12")
+    for m in (8, 16):
+        x, kernels = _x(m, 3 * gs, 1), {}
+        for name, params in _kernel_nodes(lambda: w.matmul(x)):
+            attr = _FuncAttributes()
+            assert rt.cudaFuncGetAttributes(ctypes.byref(attr), ctypes.c_void_p(params.func)) == 0
+            kernels["x" if "rows_x" in name else "product" if "rows_mma" in name else name] = (attr, params.block[0])
+        (write, write_threads), (product, threads) = kernels["x"], kernels["product"]
+        rounded = lambda regs: (regs + 7) // 8 * 8   # noqa: E731
+        left = 16384 - rounded(product.regs) * threads // 4
+        assert rounded(write.regs) * 32 * -(-write_threads // 128) <= left, (m, write.regs, write_threads, product.regs, threads)
+        assert product.local <= 128, (m, product.local)
     w.free()

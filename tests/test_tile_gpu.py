@@ -267,8 +267,8 @@ class _NodeParams(ctypes.Structure):   # cudaKernelNodeParams
                 ("extra", ctypes.c_void_p)]
 
 
-def _kernels(fn):
-    """Names of the kernels that a call launches: those of its captured graph."""
+def _kernel_nodes(fn):
+    """Name and parameters of the kernels that a call launches: those of its captured graph."""
     rt = ctypes.CDLL("libcudart.so.12")
     fn()
     torch.cuda.synchronize()
@@ -279,15 +279,17 @@ def _kernels(fn):
     assert rt.cudaGraphGetNodes(raw, None, ctypes.byref(count)) == 0
     nodes = (ctypes.c_void_p * count.value)()
     assert rt.cudaGraphGetNodes(raw, nodes, ctypes.byref(count)) == 0
-    names = []
     for node in nodes:
         kind, params, name = ctypes.c_int(-1), _NodeParams(), ctypes.c_char_p()
         assert rt.cudaGraphNodeGetType(ctypes.c_void_p(node), ctypes.byref(kind)) == 0
         if kind.value == 0:   # a kernel
             assert rt.cudaGraphKernelNodeGetParams(ctypes.c_void_p(node), ctypes.byref(params)) == 0
             assert rt.cudaFuncGetName(ctypes.byref(name), ctypes.c_void_p(params.func)) == 0
-            names.append(name.value.decode())
-    return names
+            yield name.value.decode(), params
+
+
+def _kernels(fn):
+    return [name for name, _ in _kernel_nodes(fn)]
 
 
 @pytest.mark.parametrize("dtype,entries,banks", [("NVQ3J-512", 512, 4), ("NVQ3J-L", 1024, 2)])

@@ -67,8 +67,9 @@ static bool rows_plan(const NintDevB& w, int m, bool glu, int sms, RowsPlan& bes
 
 static void launch_rows_x(const RowsXArgs& a, int t8, const TileNorm* norm, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(norm ? a.m : a.nchunks));
-    cfg.blockDim = dim3(norm ? 1024u : (unsigned)((a.m * 8 + 31) / 32 * 32));
+    const int lanes = 8 * rows_x_parts(t8), tokens = 128 / lanes;
+    cfg.gridDim = norm ? dim3((unsigned)a.m) : dim3((unsigned)a.nchunks, (unsigned)((a.m + tokens - 1) / tokens));
+    cfg.blockDim = dim3(norm ? 1024u : (unsigned)((std::min(a.m, tokens) * lanes + 31) / 32 * 32));
     if (norm) cfg.dynamicSmemBytes = (size_t)(a.k + 7) / 8 * 16;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];

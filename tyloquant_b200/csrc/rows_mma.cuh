@@ -117,10 +117,14 @@ struct RowsNint {
     static constexpr bool S1 = BITS >= 5, S2 = true, TABLE = false;
     using BU = ByteUnit<BITS>;
     static constexpr int WC = BU::words_for(8 * T), SW = 2;
+    // Wide records come into registers by halves (the second half's registers start on a word): a lane's words of a whole record
+    // beside the sums of two activation tiles spilled (16 rows 28672 x 4096, NINT6-32 34.3 us, by halves 29.6; NINT6-48 48.6 and 38.6).
+    static constexpr bool HALVES = WC >= 24 && (4 * T) % BU::NP == 0;
+    static constexpr int CW = HALVES ? WC / 2 : WC, REGS = HALVES ? 4 * T : 8 * T;   // words in registers, registers decoded from them
     // last register that reads word w: a unit's words are all read by its last register where fields are rebuilt from left-over bits
     static constexpr int last_reg(int w) {
         const int unit = w / BU::U, tt = BU::EXTRA ? BU::NP - 1 : BU::F * (w % BU::U + 1) - 1, r = unit * BU::NP + tt;
-        return r < 8 * T ? r : 8 * T - 1;
+        return r < REGS ? r : REGS - 1;
     }
     __host__ __device__ static constexpr int pos(int a) { return BITS == 2 ? 2 * a : ((BITS == 3 || BITS == 4) ? BITS * (a & 1) : 0); }
     static constexpr float X_FACTOR = rows_x_factor(BITS);
@@ -153,8 +157,8 @@ struct RowsNint {
         }
     }
     template <int R>
-    __device__ static __forceinline__ void weights(const uint32_t (&code)[WC], const Half& s, uint32_t, const unsigned char*, uint32_t& even, uint32_t& odd, uint32_t) {
-        constexpr int P = pos(R % 4), TT = R % BU::NP, UNIT = R / BU::NP, A = R & 3;
+    __device__ static __forceinline__ void weights(const uint32_t (&code)[CW], const Half& s, uint32_t, const unsigned char*, uint32_t& even, uint32_t& odd, uint32_t) {
+        constexpr int P = pos(R % 4), TT = R % REGS % BU::NP, UNIT = R % REGS / BU::NP, A = R & 3;
         constexpr uint32_t M = ((1u << BITS) - 1u) << P, MASK = M | (M << 16);
         uint32_t v;
         if constexpr (TT < BU::U * BU::F) {
@@ -184,7 +188,8 @@ struct RowsNint {
 // records whose products are f16 numbers (tile_terms 1).
 template <int IB, bool JSC>
 struct RowsNvq {
-    static constexpr int T = 3, FB = IB + 4, WC = (24 * FB + 31) / 32, SW = 1;
+    static constexpr int T = 3, FB = IB + 4, WC = (24 * FB + 31) / 32, SW = 1, CW = WC;
+    static constexpr bool HALVES = false;
     static constexpr int last_reg(int w) { return (32 * w + 31) / FB < 23 ? (32 * w + 31) / FB : 23; }
     static constexpr bool S1 = false, S2 = false, TABLE = true;
     static constexpr float OUT_MIN = 0.f;
@@ -225,7 +230,7 @@ struct RowsNvq {
         }
     }
     template <int R>
-    __device__ static __forceinline__ void weights(const uint32_t (&code)[WC], const Half& s, uint32_t own, const unsigned char* ctx, uint32_t& even, uint32_t& odd, uint32_t bank_bytes) {
+    __device__ static __forceinline__ void weights(const uint32_t (&code)[CW], const Half& s, uint32_t own, const unsigned char* ctx, uint32_t& even, uint32_t& odd, uint32_t bank_bytes) {
         constexpr int POS = R * FB, WI = POS >> 5, SH = POS & 31, A = R & 3;
         uint32_t off;
         if constexpr (SH + FB <= 32) off = (SH >= 2 ? code[WI] >> (SH >= 2 ? SH - 2 : 0) : code[WI] << (SH < 2 ? 2 - SH : 0)) & OFFMASK;
@@ -257,19 +262,20 @@ __device__ __forceinline__ float2 rows_x_scale(uint32_t absmax_bits) {
     return make_float2(__uint_as_float((uint32_t)(268 - eb) << 23), __uint_as_float((uint32_t)(eb - 14) << 23));
 }
 
-// Columns of one group as bf16 pairs, zero past the group size and past the row.
+// T octets of one group's columns as bf16 pairs, from slot s0 on (PART), zero past the group size and past the row.
 template <int T>
 struct RowsGroup {
     uint32_t v[4 * T];
     // form 2: 16-byte pieces, 1: 8-byte pieces, 0: single values (a row in shared memory is padded with zeros to whole pieces)
-    template <bool SHARED = false>
-    __device__ __forceinline__ void load(const __nv_bfloat16* row, int k, int gs, int g, int form, bool live) {
-        const int k0 = g * gs;
+    template <bool SHARED, bool PART>
+    __device__ __forceinline__ void load(const __nv_bfloat16* row, int k, int gs, int g, int form, bool live, int s0 = 0) {
+        const int k0 = g * gs + s0;
+        gs -= s0;
         if (form == 2) {
 #pragma unroll
             for (int t = 0; t < T; ++t) {
                 uint4 r = make_uint4(0u, 0u, 0u, 0u);
-                if (live && k0 + 8 * t < k) r = SHARED ? *reinterpret_cast<const uint4*>(row + k0 + 8 * t) : __ldcg(reinterpret_cast<const uint4*>(row + k0 + 8 * t));
+                if (live && (!PART || 8 * t < gs) && k0 + 8 * t < k) r = SHARED ? *reinterpret_cast<const uint4*>(row + k0 + 8 * t) : __ldcg(reinterpret_cast<const uint4*>(row + k0 + 8 * t));
                 v[4 * t] = r.x; v[4 * t + 1] = r.y; v[4 * t + 2] = r.z; v[4 * t + 3] = r.w;
             }
         } else if (form == 1) {
@@ -297,31 +303,36 @@ struct RowsGroup {
     }
 };
 
-// One group of a token's activations as B operands, by eight neighbouring lanes for the eight groups of a chunk: values scaled by
-// a power of two per token and chunk (largest magnitude next to 2^15; exact for bf16 values within 2^-28 of it), the group's sum
-// as two f16 terms, the factor's inverse. Slab 2 (f T + t) + h of a chunk holds octet t of groups 4 f + 2 h and the next: lane 4
-// q + c (token q of a tile of eight) reads quad c & 1 of group c >> 1, slots 0, 2 and 1, 3 in its two registers -- the order in
-// which the decoders' byte pairs come.  Lanes are XORed with 4 h + f, which spreads a token's groups over the banks.
-template <int T>
-__device__ __forceinline__ void rows_x_group(const RowsGroup<T>& v, unsigned char* chunk, int t, int g, int nt, float factor, bool live) {
+// One group of a token's activations as B operands, by eight neighbouring lanes for the eight groups of a chunk (PARTS 2: sixteen,
+// each with half of a group's octets): values scaled by a power of two per token and chunk (largest magnitude next to 2^15; exact
+// for bf16 values within 2^-28 of it), the group's sum as two f16 terms, the factor's inverse. Slab 2 (f T + t) + h of a chunk
+// holds octet t of groups 4 f + 2 h and the next: lane 4 q + c (token q of a tile of eight) reads quad c & 1 of group c >> 1,
+// slots 0, 2 and 1, 3 in its two registers -- the order in which the decoders' byte pairs come.  Lanes are XORed with 4 h + f,
+// which spreads a token's groups over the banks.
+template <int T, int PARTS>
+__device__ __forceinline__ void rows_x_group(const RowsGroup<(T + PARTS - 1) / PARTS>& v, unsigned char* chunk, int t, int g, int part, int nt, float factor, bool live) {
+    constexpr int TP = (T + PARTS - 1) / PARTS;
     uint32_t mx = v.absmax(0u);
-    for (int o = 1; o < 8; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if (!live) return;
+    for (int o = 1; o < 8 * PARTS; o <<= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    if (PARTS == 1 && !live) return;
     const float2 sc = rows_x_scale(mx);
     const int q = t & 7, j = t >> 3, b = g & 1, h = (g >> 1) & 1, f = g >> 2, slab = 256 * nt;
     auto at = [&](int s, int unit) { return chunk + (size_t)s * slab + (nt == 1 ? unit * 8 : unit * 16 + j * 8); };   // this token's eight bytes of a lane
     float sum = 0.f;
 #pragma unroll
-    for (int i = 0; i < T; ++i)
+    for (int i = 0; i < TP; ++i)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const uint32_t u0 = v.v[4 * i + 2 * e], u1 = v.v[4 * i + 2 * e + 1];
             const float x0 = __uint_as_float(u0 << 16) * sc.x, x1 = __uint_as_float(u0 & 0xFFFF0000u) * sc.x;
             const float x2 = __uint_as_float(u1 << 16) * sc.x, x3 = __uint_as_float(u1 & 0xFFFF0000u) * sc.x;
             sum += (x0 + x1) + (x2 + x3);
-            *reinterpret_cast<uint2*>(at(2 * (f * T + i) + h, (4 * q + 2 * b + e) ^ (4 * h + f))) =
-                make_uint2(rows_u32(__floats2half2_rn(x0, x2)), rows_u32(__floats2half2_rn(x1, x3)));
+            if (PARTS == 1 || (live && (T % PARTS == 0 || part * TP + i < T)))
+                *reinterpret_cast<uint2*>(at(2 * (f * T + part * TP + i) + h, (4 * q + 2 * b + e) ^ (4 * h + f))) =
+                    make_uint2(rows_u32(__floats2half2_rn(x0, x2)), rows_u32(__floats2half2_rn(x1, x3)));
         }
+    if constexpr (PARTS == 2) sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    if (PARTS == 2 && (!live || part != 0)) return;
     sum *= factor;   // k-slots (group) and 8 + (group) of the chunk's last slab
     const __half hi = __float2half_rn(sum), lo = __float2half_rn(sum - __half2float(hi));
     unsigned char* p = at(4 * T, 4 * q + (g >> 1)) + 2 * b;
@@ -330,22 +341,25 @@ __device__ __forceinline__ void rows_x_group(const RowsGroup<T>& v, unsigned cha
     if (g == 0) *reinterpret_cast<float*>(chunk + (size_t)(4 * T + 1) * slab + 4 * t) = sc.y;
 }
 
-// At most 32 registers: a CTA of it then fits beside the 20 warps of 96 registers of the kernel before it, and waits there for
-// its end (with more it is launched after that end: 16 rows through NINT4 4096 x 4096 14.7 us instead of 9.2). A CTA per chunk, a
-// thread per (token, group): 1.3 us of a product's chain (a factor per whole row, as the tile kernel has it, needs a pass for the
-// maxima before: 2.8).
+// At most 128 threads of 32 registers a CTA: it then fits beside the 20 warps of 96 registers of the kernel before it, which leave
+// each of the SM's four schedulers 1024, and waits there for its end (with more it is launched after that end: 16 rows through
+// NINT4 4096 x 4096 14.7 us instead of 9.2, through NINT4-48 16.2 instead of 9.3).  A CTA per chunk, a thread per (token, group)
+// or, for more than four octets, two of them: 1.3 us of a product's chain (a factor per whole row, as the tile kernel has it,
+// needs a pass for the maxima before: 2.8).
+constexpr int rows_x_parts(int t8) { return t8 <= 4 ? 1 : 2; }
 template <int T>
-__global__ void __launch_bounds__(128, T <= 4 ? 16 : 8) rows_x_kernel(const __grid_constant__ RowsXArgs a) {
+__global__ void __launch_bounds__(128, 16) rows_x_kernel(const __grid_constant__ RowsXArgs a) {
+    constexpr int PARTS = rows_x_parts(T), LANES = 8 * PARTS, TP = (T + PARTS - 1) / PARTS;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int t = threadIdx.x >> 3, g = threadIdx.x & 7;
-    if (blockIdx.x == 0)
+    const int t = (int)(blockIdx.y * (128 / LANES) + threadIdx.x / LANES), g = threadIdx.x % LANES / PARTS, part = threadIdx.x % PARTS;
+    if (blockIdx.x == 0 && blockIdx.y == 0)
         for (int i = threadIdx.x; i < a.n_counters; i += blockDim.x) a.counters[i] = 0u;
     const bool al16 = (reinterpret_cast<uintptr_t>(a.x) & 15) == 0 && (a.k & 7) == 0 && (a.gs & 7) == 0;
     const bool al8 = (reinterpret_cast<uintptr_t>(a.x) & 7) == 0 && (a.k & 3) == 0 && (a.gs & 3) == 0;
-    RowsGroup<T> v;
-    v.load(a.x + (size_t)(t < a.m ? t : 0) * a.k, a.k, a.gs, 8 * (int)blockIdx.x + g, al16 ? 2 : (al8 ? 1 : 0), t < a.m);
-    rows_x_group<T>(v, a.out + (size_t)blockIdx.x * rows_chunk_bytes(T, a.nt), t, g, a.nt, a.factor, t < a.m);
+    RowsGroup<TP> v;
+    v.template load<false, PARTS == 2>(a.x + (size_t)(t < a.m ? t : 0) * a.k, a.k, a.gs, 8 * (int)blockIdx.x + g, al16 ? 2 : (al8 ? 1 : 0), t < a.m, 8 * TP * part);
+    rows_x_group<T, PARTS>(v, a.out + (size_t)blockIdx.x * rows_chunk_bytes(T, a.nt), t, g, part, a.nt, a.factor, t < a.m);
 }
 
 // The same behind a residual add and RMSNorm, one CTA per row: the row stays in registers between the sum of squares and the
@@ -405,8 +419,8 @@ __global__ void __launch_bounds__(1024) rows_norm_kernel(const __grid_constant__
         const int g = g0 + tid;
         const bool live = g < 8 * a.nchunks;
         RowsGroup<T> w;
-        w.template load<true>(x, a.k, a.gs, g, form, live);
-        rows_x_group<T>(w, a.out + (size_t)(live ? g >> 3 : 0) * rows_chunk_bytes(T, a.nt), p, g & 7, a.nt, a.factor, live);
+        w.template load<true, false>(x, a.k, a.gs, g, form, live);
+        rows_x_group<T, 1>(w, a.out + (size_t)(live ? g >> 3 : 0) * rows_chunk_bytes(T, a.nt), p, g & 7, 0, a.nt, a.factor, live);
     }
 }
 
@@ -468,11 +482,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_mma_kernel(const __grid_
             }
         };
         for (int i = 0; i < kRowsAhead; ++i) ahead();
-        uint32_t code[C::WC];
+        uint32_t code[C::CW];
         typename C::Scales sc;
         if (it0 < it1) {
 #pragma unroll
-            for (int i = 0; i < C::WC; ++i) code[i] = rows_ldg(rec + i * 32 + lane);
+            for (int i = 0; i < C::CW; ++i) code[i] = rows_ldg(rec + i * 32 + lane);
             sc.quad = rows_ldg4(rec + C::WC * 32 + (lane & ~3));
             sc.load_late(rec, lane);
         }
@@ -528,10 +542,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) rows_mma_kernel(const __grid_
                         else rows_mma(acc[j], a0, a1, a2, a3, b.r[j][0], b.r[j][1]);
                     }
                 });
-                // words that are used up make room for the next record's
-                rows_static_for<C::WC>([&](auto i_c) {
+                // words that are used up make room for the next record's, or the second half's
+                rows_static_for<C::CW>([&](auto i_c) {
                     constexpr int I = decltype(i_c)::value;
-                    if constexpr (C::last_reg(I) / 4 == S) code[I] = rows_ldg(next + I * 32 + lane);
+                    if constexpr (C::HALVES && C::last_reg(I) / 4 == S) code[I] = rows_ldg(rec + (C::CW + I) * 32 + lane);
+                    else if constexpr (C::last_reg(I) / 4 == (C::HALVES ? S - T : S)) code[I] = rows_ldg(next + I * 32 + lane);
                 });
             });
             float s2[NT][4];
