@@ -11,7 +11,7 @@ torch = pytest.importorskip("torch")
 
 from tyloquant_b200 import QuantWeight, encode  # noqa: E402
 from test_gemm_gpu import _status  # noqa: E402
-from test_tile_gpu import _kernel_nodes  # noqa: E402
+from test_tile_gpu import _kernel_nodes, _kernels  # noqa: E402
 
 # bits, group size, sub-scale bits; bound on the error over what the products add up to without cancellation.  Exact weights leave the float32 sums (some tens of roundings of 2^-24, and the two
 # terms of the group sums, 2^-22, which uncentred widths subtract from sums a few times as large); width six takes one f16 rounding of the integers above 2^11, at most 2^-11 of each and
@@ -155,3 +155,19 @@ def test_the_next_products_activations_fit_beside_a_product(profile):
         assert rounded(write.regs) * 32 * -(-write_threads // 128) <= left, (m, write.regs, write_threads, product.regs, threads)
         assert product.local <= 128, (m, product.local)
     w.free()
+
+
+@pytest.mark.parametrize("profile,n,k,here", [((2, 16, 5), 57344, 4096, True), ((3, 24, 5), 100000, 1030, True), ((4, 24, 6), 57344, 2048, True), ((4, 24, 6), 57344, 4096, False),
+                                              ((4, 24, 6), 128256, 768, False), ((5, 24, 7), 36864, 2048, True), ((5, 32, 7), 57344, 768, True), ((5, 32, 7), 57344, 2048, False),
+                                              ((6, 24, 7), 57344, 768, True), ((6, 24, 7), 57344, 1536, False), ((5, 28, 7), 70000, 1536, True)])
+def test_long_lists(profile, n, k, here):
+    """Sixteen rows through many row-blocks, one to three passes of them, on the side of the line that is the faster one (148 SMs).
+    Bound of the tile kernel: two f16 roundings, as its own tests have it."""
+    bits, gs, sub = profile
+    w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(n, k, bits, gs, sub, seed=n, device="cuda"))
+    x = _x(16, k, 1)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert any("rows_mma_kernel" in name for name in _kernels(lambda: w.matmul(x))) == here
+    _check(w, x, 3.6e-4 if not here else ROUNDED if bits == 6 else EXACT)
+    w.free()
+    assert _status() == 0

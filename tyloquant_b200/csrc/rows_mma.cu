@@ -28,7 +28,7 @@ static bool rows_takes(const NintDevB& w, int m) {
 }
 
 struct RowsPlan {
-    int tiles = 0, slices = 0, pass_rb = 0, rounds = 0;   // rounds: records of the busiest warp
+    int tiles = 0, slices = 0, pass_rb = 0, passes = 0, rounds = 0;   // rounds: records of the busiest warp
     size_t x_bytes = 0, smem = 0;
 };
 
@@ -57,12 +57,30 @@ static bool rows_plan(const NintDevB& w, int m, bool glu, int sms, RowsPlan& bes
             best.tiles = tiles;
             best.slices = s;
             best.pass_rb = pass_rb;
+            best.passes = passes;
             best.rounds = passes * rounds;
             best.x_bytes = x;
             best.smem = fixed + pass_rb * slot;
         }
     }
     return best.tiles > 0;
+}
+
+// Long lists of records, nine to sixteen rows: the tile kernel's steps cost less than the second activation tile here, the more bits
+// the sooner, and passes over row-blocks pay for their ends.  us, 16 rows, here and on the tile kernel:
+//   two and three bits at any length: NINT2-16 57344 x 4096 50.6 and 51.9, 128256 x 4096 102.7 and 103.1, NINT3-24 57344 x 4096 47.9
+//   and 49.4, 128256 x 4096 96.3 and 96.8;
+//   four bits, up to two passes: NINT4-24 45056 x 4096 (22 records a warp) 35.9 and 39.4, 57344 (30) 48.0 and 46.8, NINT4-32 57344
+//   (22) 44.7 and 47.4; three: NINT4-24 128256 x 384 (18 octets of a group) 21.5 and 22.2, x 1536 (72) 46.3 and 41.8;
+//   five and six bits, one pass: NINT5-24 36864 x 4096 (54 octets) 36.1 and 37.5, 45056 (66) 43.8 and 44.1, NINT6-24 36864 (54) 37.9
+//   and 38.1, 45056 (66) 45.1 and 44.5, NINT6-48 28672 (42) 30.4 and 30.5, 45056 (66) 43.7 and 42.6;
+//   two: NINT6-24 96000 x 384 (18) 18.7 and 19.4, x 768 (30) 26.6 and 24.5, NINT5-32 57344 x 384 (16) 16.4 and 15.9, x 4096 54.6 and 49.0.
+// A padded group size doubles the tile kernel's steps (NINT5-28 28672 x 4096: 32.4 and 72.4).
+static bool rows_long(const NintDevB& w, const RowsPlan& p) {
+    if (w.bits <= 3 || w.gs % 8) return false;
+    const int octets = p.rounds * w.t8;
+    if (p.passes > (w.bits == 4 ? 2 : 1) && octets > 20) return true;
+    return p.rounds > 25 || (w.bits > 4 && octets > (w.bits == 5 ? 66 : 60));
 }
 
 static void launch_rows_x(const RowsXArgs& a, int t8, const TileNorm* norm, cudaStream_t s) {
@@ -117,11 +135,7 @@ bool launch_rows_product(const NintDevB& w, const void* x, int m, void* y, int y
     if (!rows_takes(w, m) || (norm && (w.k % 4 || w.k > 20480))) return false;   // the row as bf16 in a CTA's 48 KB
     RowsPlan p;
     if (!rows_plan(w, m, glu, device_sm_count(device), p)) return false;
-    // Long lists of records, nine and more rows: the tile kernel's steps cost less than the second activation tile here.
-    // Six bits, 16 rows, this kernel and the tile kernel: 28672 x 4096 (15 rounds) 31.7 and 32.1 us, 36864 (18) 37.4 and 37.4,
-    // 45056 (22) 44.4 and 43.6, 57344 (29) 62.3 and 53.9.  Four bits: 36864 29.4 and 33.3, 45056 35.7 and 38.7, 57344 47.7 and 45.8.
-    // A padded group size doubles the tile kernel's steps (NINT5-28 28672 x 4096: 33.1 and 72.1).
-    if (m > 8 && p.rounds > (w.bits == 6 ? 20 : 25) && w.gs % 8 == 0) return false;
+    if (m > 8 && rows_long(w, p)) return false;
     const int nt = m <= 8 ? 1 : 2;
     RowsArgs a{};
     a.w = w;
