@@ -141,6 +141,19 @@ def test_shared_tiles_have_the_same_bits_in_every_call(n, k, bits, gs, sb, m):
     assert _status() == 0
 
 
+@pytest.mark.parametrize("bits,n,k,m,grid", [(2, 5000, 2888, 20, 120), (2, 5000, 2888, 512, 80), (4, 4960, 2888, 40, 117), (8, 5120, 2900, 128, 120), (2, 14336, 4096, 60, 148)])
+def test_chunks_of_two_octets_are_shared_out_by_whole_parts(bits, n, k, m, grid):
+    """Their sums over CTAs weigh more than their chunks: parts of one tile per CTA, unless that makes the longest CTA much longer (148 SMs)."""
+    w = QuantWeight.from_blob(f"NINT{bits}", encode.random_nint_blob(n, k, bits, 16, 5, seed=n, device="cuda"))
+    x = torch.randn(m, k, device="cuda", generator=torch.Generator("cuda").manual_seed(m)).to(torch.bfloat16)
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert [params.grid[0] for name, params in _kernel_nodes(lambda: w.matmul(x)) if "tile_tc_kernel" in name] == [grid]
+    got, want = w.matmul(x, out_dtype=torch.float32), x.double() @ w.dequantize().double().T
+    assert ((got.double() - want).norm() / want.norm()).item() <= 3.6e-4   # as below
+    assert torch.equal(got, w.matmul(x, out_dtype=torch.float32))
+    assert _status() == 0
+
+
 GROWING_CALL = """
 import ctypes, sys, torch
 sys.path.insert(0, %r)

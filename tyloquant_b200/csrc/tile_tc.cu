@@ -423,9 +423,13 @@ bool launch_tile_product(const NintDevB& w, const void* x, int m, void* y, int y
     // about as much as three chunks (1.5 to 2.5 us against 0.6 for a chunk of 16 tokens; both grow with the tokens), and half of
     // the second one is hidden behind the CTA's other part: with six chunks instead of three for two sums, 16 rows through NINT6
     // 4096 x 14336 took 22.4 us instead of 21.1, with none 8 rows through NVQ3 17408 x 5120 31.4 instead of 23.8.
+    // A chunk of groups of 16 is over sooner, in 0.4 us of 40 tokens and 0.8 of 250, beside 4.6 and 14 for two sums: they count six
+    // chunks, more than 128 tokens ten.  Split and equal, us: NINT2-16 5000 x 2888, 20 rows 11.9 and 15.8, 512 rows 32.3 and 39.2
+    // (three chunks chose the latter); 14336 x 4096, 60 rows 29.9 and 28.7; over 1400 shapes 4 % from one line to the other.
     // Without sharing there is no sum.  At most a dozen CTAs per tile (kTileGroup): the last one adds the others' parts.
+    const long long sums = terms == 1 && w.t8 == 2 ? (n > 128 ? 10 : 6) : 3;
     const long long split = std::min({(long long)sms / tiles, (long long)std::max(1, w.nchunks / 2), (long long)kTileGroup});
-    const long long chunks_split = split ? (w.nchunks + split - 1) / split + (split > 1 ? 3 : 0) : 0, chunks_equal = (units + sms - 1) / sms + 3;
+    const long long chunks_split = split ? (w.nchunks + split - 1) / split + (split > 1 ? 3 : 0) : 0, chunks_equal = (units + sms - 1) / sms + sums;
     a.split = split && chunks_split <= chunks_equal ? (int)split : 0;
     p.grid = a.split ? (int)(tiles * split) : (int)std::max<long long>(1, std::min<long long>(sms, (units + 1) / 2));
     // The two launches below belong together: another thread's on the same stream would take the scratch between them.
