@@ -129,7 +129,6 @@ struct RowsNint {
     __host__ __device__ static constexpr int pos(int a) { return BITS == 2 ? 2 * a : ((BITS == 3 || BITS == 4) ? BITS * (a & 1) : 0); }
     static constexpr float X_FACTOR = rows_x_factor(BITS);
     static constexpr float OUT_MIN = 16777216.f / X_FACTOR;
-    __host__ __device__ static size_t ctx_bytes(const NintDevB&) { return 0; }
 
     struct Scales {
         uint4 quad;          // word 0 of the lanes of this quad
@@ -194,7 +193,6 @@ struct RowsNvq {
     static constexpr bool S1 = false, S2 = false, TABLE = true;
     static constexpr float OUT_MIN = 0.f;
     static constexpr uint32_t OFFMASK = ((1u << FB) - 1u) << 2;   // a field as a byte offset into the table
-    __host__ __device__ static size_t ctx_bytes(const NintDevB& w) { return (size_t)w.table_words * 4 + 64; }
     __device__ static void ctx_init(unsigned char* ctx, const RowsArgs& a, int tid) {
         const uint4* src = reinterpret_cast<const uint4*>(a.w.table);
         for (int i = tid; i < a.w.table_words / 4; i += kRowsThreads) {
