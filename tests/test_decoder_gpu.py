@@ -20,6 +20,7 @@ torch = pytest.importorskip("torch")
 from oracle import mfq_oracle as O  # noqa: E402
 from tyloquant_b200 import decoder as D  # noqa: E402
 from test_nint_gpu import rel_l2  # noqa: E402
+from test_tile_gpu import _kernels  # noqa: E402
 
 CFG = dict(hidden=512, n_q_heads=4, n_kv_heads=2, ffn=768, vocab=1000, layers=2, max_ctx=96, max_batch=3)
 
@@ -90,10 +91,11 @@ def test_one_block_matches_the_float32_restatement():
     dec.free()
 
 
-@pytest.mark.parametrize("ctx", [0, 15, 16, 63, 64, 255, 256, 600, 1023])
+@pytest.mark.parametrize("ctx", [0, 6, 15, 16, 63, 64, 67, 255, 256, 600, 1023])
 def test_new_key_and_value_take_their_place_in_the_scan(ctx):
     """The step's own key and value never come out of the cache: they are put into the scan's ring, here in its first and
-    later rounds, at both ends of a 16-token round and alone in their slice (32 sequences leave slices of up to 256 tokens).
+    later rounds of a warp, at its first (67: offset 16 of its slice) and last token, and alone in the last slice of a cache that
+    is empty (0) or not (6); 32 sequences leave four slices of up to 256 tokens.
     Tolerance as for the block above."""
     cfg = dict(CFG, layers=1, max_ctx=1024, max_batch=32)
     dec, blobs = D.random_decoder(**cfg, seed=12, keep_blobs=True)
@@ -191,3 +193,68 @@ def test_one_step_makes_room_for_captured_steps_of_smaller_batches(form):
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", SMALLER_STEPS % (root, form)], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr[-2000:]
+
+
+def _restated_logits(dec, ids, ctx, dtype):
+    """The step's logits from the decoded weights, every sequence at once, with the roundings of the float32 restatement above."""
+    cfg = dec.cfg
+    nq, nkv, layers = cfg.n_q_heads, cfg.n_kv_heads, cfg.layers
+    *blocks, head, emb = dec._keep
+
+    def bf(x):
+        return x.to(torch.bfloat16).to(dtype)
+
+    def times(x, w):
+        return x @ w.dequantize().to(dtype).T
+
+    def norm(h):
+        return bf(h * torch.rsqrt(h.square().mean(-1, keepdim=True) + cfg.rms_eps))
+
+    ang = ctx * cfg.rope_theta ** (-torch.arange(64, device="cuda", dtype=torch.float64) / 64)
+    cos, sin = ang.cos().to(dtype), ang.sin().to(dtype)
+
+    def rope(x):
+        a, b = x[..., :64], x[..., 64:]
+        return torch.cat([a * cos - b * sin, b * cos + a * sin], -1)
+
+    h, rows = emb[ids.long()].to(dtype), len(ids)
+    for li in range(layers):
+        qkv_w, o_w, gate_up_w, down_w = blocks[4 * li:4 * li + 4]
+        kc, vc = (torch.stack([dec.read_cache(li, r, i, ctx) for r in range(rows)]).to(dtype) for i in (0, 1))
+        qkv = times(norm(h), qkv_w).view(rows, nq + 2 * nkv, 128)
+        q, k, v = rope(qkv[:, :nq]).view(rows, nkv, nq // nkv, 128), bf(rope(qkv[:, nq:nq + nkv])), bf(qkv[:, nq + nkv:])
+        kc, vc = torch.cat([kc, k[:, :, None]], 2), torch.cat([vc, v[:, :, None]], 2)
+        p = torch.softmax(torch.einsum("rhgd,rhtd->rhgt", q, kc) / 128 ** 0.5, -1)
+        h = h + times(bf(torch.einsum("rhgt,rhtd->rhgd", p, vc).reshape(rows, -1)), o_w)
+        gu = times(norm(h), gate_up_w).view(rows, -1, 2, 16)
+        act = gu[:, :, 1] * gu[:, :, 0] / (1 + torch.exp(-gu[:, :, 0]))
+        h = h + times(bf(act.reshape(rows, -1)), down_w)
+    return times(norm(h), head)
+
+
+NORM_FORMS = [dict(attn_profile=(4, 24, 6), ffn_profile=(6, 24, 7)),   # 16-byte pieces of the normalised row
+              dict(attn_profile=(5, 28, 7), ffn_profile=(5, 28, 7)),   # 8-byte pieces
+              dict(attn_profile=(4, 27, 6), ffn_profile=(4, 27, 6)),   # single values
+              # more columns than the registers of a CTA hold, more groups than it has threads, rows in slices of K
+              dict(attn_profile=(2, 16, 5), ffn_profile=(2, 16, 5), hidden=17408, n_q_heads=136, n_kv_heads=17, ffn=256, layers=1)]
+
+
+@pytest.mark.parametrize("form,batch", [(form, batch) for form in range(3) for batch in (5, 8, 9, 16)] + [(3, 8), (3, 9)])
+def test_products_behind_a_normalisation(form, batch):
+    """Residual add, RMSNorm and product of the few-rows kernel (five to sixteen sequences): two blocks and the head, so that every
+    normalisation but the first has something to add.  Bound: nine roundings to bf16, all of them to the other side, are 9^1/2 x
+    2^-9 / 3^1/2 = 3.4e-3 in the mean square (seen: 1.3e-3, the six bits' own rounding decides some).  The wide form is restated
+    in float32 and its scores have 2-bit noise: 3.4e-3 seen; one of its 1088 groups lost would be 3e-2."""
+    cfg = {**CFG, "max_batch": 16, **NORM_FORMS[form]}
+    dec, _ = D.random_decoder(**cfg, seed=30 + form)
+    ids = torch.arange(3, 3 + batch, dtype=torch.int32, device="cuda") * 7
+    ctx = 21
+    dec.fill_cache(ctx, seed=batch)
+    want = _restated_logits(dec, ids, ctx, torch.float64 if form < 3 else torch.float32)
+    dec.step(ids)
+    got = dec.read_logits(batch).to(want.dtype)
+    err = ((got - want).norm(dim=1) / want.norm(dim=1)).max().item()
+    assert err <= (4e-3 if form < 3 else 1e-2), (form, batch, err)
+    names = _kernels(lambda: dec.step(ids))
+    assert sum("rows_norm_kernel" in name for name in names) == (5 if form < 3 else 2), names   # (the wide form's q|k|v has more rows than slices of K allow)
+    dec.free()

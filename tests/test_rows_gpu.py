@@ -56,15 +56,18 @@ def test_many_row_blocks_per_cta():
     w.free()
 
 
-@pytest.mark.parametrize("dtype,entries", [("NVQ3", 256), ("NVQ3J-512", 512)])
-def test_lattice_weights(dtype, entries):
+@pytest.mark.parametrize("dtype,entries,n_banks", [("NVQ3", 256, 1), ("NVQ3J", 256, 2), ("NVQ3J", 256, 4), ("NVQ3J-512", 512, 2), ("NVQ3J-512", 512, 4), ("NVQ3J-L", 1024, 1), ("NVQ3J-L", 1024, 2)])
+def test_lattice_weights(dtype, entries, n_banks):
     for n, k in ((9, 20), (300, 2399), (640, 5120)):
         wt = np.random.default_rng(n).standard_normal((n, k), dtype=np.float32) * np.float32(0.02)
-        banks = encode.d4_256_codebook()[None] if dtype == "NVQ3" else encode.synthetic_d4_banks(entries, 2, seed=9)
+        banks = encode.d4_256_codebook()[None] if dtype == "NVQ3" else encode.synthetic_d4_banks(entries, n_banks, seed=9)
         w = QuantWeight.from_blob(dtype, encode.nvq_blob(encode.quantize_nvq3(wt, banks, jsc=dtype != "NVQ3", device="cuda")))
         for m in (2, 5, 8):
-            _check(w, _x(m, k, m), EXACT)
+            x = _x(m, k, m)
+            assert any("rows_mma_kernel" in name for name in _kernels(lambda: w.matmul(x)))
+            _check(w, x, EXACT)
         w.free()
+    assert _status() == 0
 
 
 @pytest.mark.parametrize("offset", [0, 1, 2, 4])

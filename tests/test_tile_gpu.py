@@ -231,12 +231,15 @@ def test_call_that_grows_the_scratch_while_the_default_stream_is_busy():
     assert r.returncode == 0, r.stdout + r.stderr[-2000:]
 
 
-def test_overlapping_calls_spoil_no_later_ones():
-    """Calls on one device share scratch and have to be ordered by their streams.  Two that overlap all the same may be wrong, but
-    leave nothing behind: arrival counts belong to one call."""
+@pytest.mark.parametrize("rows,kernel", [((33, 40), "tile_tc_kernel"), ((16, 9), "rows_mma_kernel")])
+def test_overlapping_calls_spoil_no_later_ones(rows, kernel):
+    """Calls on one device share scratch and have to be ordered by their streams.  Two of the same kernel that overlap all the same
+    may be wrong, but leave nothing behind: arrival counts belong to one call (tiles shared by CTAs, rows in slices of K)."""
     ws = [QuantWeight.from_blob("NINT6", encode.random_nint_blob(n, k, 6, 24, 7, seed=n, device="cuda")) for n, k in ((4096, 14336), (1000, 9000))]
     gen = torch.Generator("cuda").manual_seed(1)
-    xs = [torch.randn(m, w.k, device="cuda", generator=gen).to(torch.bfloat16) for m, w in zip((16, 40), ws)]
+    xs = [torch.randn(m, w.k, device="cuda", generator=gen).to(torch.bfloat16) for m, w in zip(rows, ws)]
+    for w, x in zip(ws, xs):
+        assert any(kernel in name for name in _kernels(lambda: w.matmul(x)))
     want = [w.matmul(x, out_dtype=torch.float32) for w, x in zip(ws, xs)]
     streams = [torch.cuda.Stream(), torch.cuda.Stream()]
     torch.cuda.synchronize()
@@ -250,11 +253,13 @@ def test_overlapping_calls_spoil_no_later_ones():
             assert torch.equal(w.matmul(x, out_dtype=torch.float32), y)
 
 
-def test_two_threads_on_one_stream():
-    """A product is two launches over scratch of the device: those of two threads on the same stream do not mix."""
+@pytest.mark.parametrize("rows", [8, 16, 40])
+def test_two_threads_on_one_stream(rows):
+    """A product is two launches over scratch of the device (of the few-rows kernel, of the tile kernel): those of two threads on
+    the same stream do not mix."""
     w = QuantWeight.from_blob("NINT4", encode.random_nint_blob(256, 512, 4, 32, 6, seed=1, device="cuda"))
     gen = torch.Generator("cuda").manual_seed(1)
-    xs = [torch.randn(40, 512, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(4)]
+    xs = [torch.randn(rows, 512, device="cuda", generator=gen).to(torch.bfloat16) for _ in range(4)]
     want = [w.matmul(x) for x in xs]
     stream = torch.cuda.Stream()
     torch.cuda.synchronize()
