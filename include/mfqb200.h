@@ -113,21 +113,29 @@ int mfqb_memory_trim(int device);
 int mfqb_dequant(const mfqb_weight* w, void* out, int out_dtype, mfqb_stream_t stream);
 
 /* y[m, n] = x[m, k] . W^T.  x is row-major bf16 with exactly k columns; y is row-major [m, n] in
- * y_dtype.  Any m >= 1 is accepted.  m <= 4 (lattice weights: m = 1) runs the
- * weight-streaming kernels: the weights stay integer codes on the int8 tensor cores, x is quantised
- * inside the kernel, group by group, to 16-bit integers with a power-of-two scale (exact for a bf16
- * value unless it lies more than 2^7 below its group's largest magnitude; the product is within
- * 1e-5 relative L2 of the float32 reference), sums are exact in int32 and the scales are applied
- * in float32.  Larger m runs the tcgen05 tile kernel (f16 operands, float32 accumulation): NINT weights
- * are rounded to f16 (within 1e-3 relative L2; where the group size is no multiple of 8 they are two f16
- * terms, within 1e-5), lattice weights are exact, every row of x is scaled
- * by a power of two (exact within 2^-28 of the row's largest magnitude), and sums are taken in a fixed
- * order: the same call gives the same bits again.
+ * y_dtype.  Any m >= 1 is accepted.  By m and format one of three kinds of kernel runs:
+ *  - weight-streaming kernels: m = 1, and m <= 4 of NINT weights that the few-rows kernel does not hold
+ *    exactly (6 and 8 bits, sub-scales so wide that code x sub-scale passes 2^11).  The weights stay integer codes
+ *    on the int8 tensor cores, x is quantised inside the kernel, group by group, to 16-bit integers with a
+ *    power-of-two scale (exact for a bf16 value unless it lies more than 2^7 below its group's largest
+ *    magnitude; the product is within 1e-5 relative L2 of the float32 reference), sums are exact in int32 and
+ *    the scales are applied in float32;
+ *  - the few-rows kernel (mma on f16 operands, float32 sums in a fixed order): 2 to 16 rows of 2- to 5-bit weights
+ *    that f16 holds exactly, 5 to 16 rows of 6-bit and the other 5-bit weights where the group size is a multiple
+ *    of 8 (9 to 16 rows of 4 bits and more: up to some size of the weight), 2 to 8 rows of lattice weights whose state
+ *    scales fit f16.  Exact weights give products within 5e-6, the others are rounded to f16 once (within 5e-4);
+ *    x is scaled by a power of two per row and chunk of eight groups (exact within 2^-28 of the chunk's largest
+ *    magnitude);
+ *  - the tcgen05 tile kernel for all other m (f16 operands, float32 sums in a fixed order): NINT weights are rounded
+ *    to f16 (within 1e-3 relative L2; where the group size is no multiple of 8 they are two f16 terms, within 1e-5),
+ *    lattice weights are exact, every row of x is scaled by a power of two (exact within 2^-28 of the row's
+ *    largest magnitude).
+ * The few-rows and the tile kernel give the same bits again for the same call.
  * An infinity or NaN in x makes the outputs NaN.
- * Library scratch: m >= 2 uses a per-device buffer (quantised planes, or activation tiles and partial sums) that
- * only ever grows -- a block handed to a kernel or baked into a captured graph stays allocated.
- * Growing calls cudaMalloc, so one call with the same weight and the same or a larger m must come first,
- * outside stream capture; inside a capture it fails with MFQB_ERR_ARG instead.  The buffer holds
+ * Library scratch: m >= 2 uses per-device buffers (quantised planes, activation fragments and parts of shared rows,
+ * or activation tiles and partial sums) that only ever grow -- a block handed to a kernel or baked into a captured
+ * graph stays allocated.  Growing calls cudaMalloc, so one call with the same weight and the same or a larger m must come first,
+ * outside stream capture; inside a capture it fails with MFQB_ERR_ARG instead.  The buffers hold
  * one call's data at a time: calls with m >= 2 on one device must be ordered by their streams.
  * A single-row (m = 1) product of a NINT weight uses a few KB of scratch owned by the weight
  * handle: two such products of the SAME weight must not overlap on the GPU.
@@ -157,7 +165,7 @@ int mfqb_mul_mat_swiglu(const mfqb_weight* w, const void* gate_up_f32, int m, vo
  * packed); y [m, n / 2] = up * gate / (1 + exp(-gate)).  The same composition as
  * mfqb_mul_mat_swiglu (mfq/kernels/cuda/glu.cuh:6-17) with the activation on the producing side,
  * so the following down projection is a plain mfqb_mul_mat.  m = 1 on NINT weights runs in the
- * single-row kernel, batches of the tile kernel apply it where a tile is finished; other cases take the
+ * single-row kernel, batches of the few-rows and the tile kernel apply it where sums are finished; other cases take the
  * product into library scratch and apply the activation. */
 int mfqb_mul_mat_glu(const mfqb_weight* w, const void* x_bf16, int m, void* y, int y_dtype,
                      mfqb_stream_t stream);

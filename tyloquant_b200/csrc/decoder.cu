@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(32 * kAttnWarps, 2) attn_decode_kernel(const f
         *reinterpret_cast<uint4*>((lane < 16 ? kb : vb) + (size_t)p * kHeadDim + 8 * l16) = v;
         fresh[lane] = v;
     }
-    // the group's queries, rotated and scaled to log2 units by 1 / sqrt(128) * log2(e): their loads were issued before the copies
+    // the group's queries, rotated and scaled to log2 units by 1 / sqrt(128) * log2(e)
     float* qs = reinterpret_cast<float*>(attn_smem + (size_t)kAttnWarps * kAttnStages * kAttnStageBytes);
 #pragma unroll
     for (int j = 0; j < QPT; ++j) {

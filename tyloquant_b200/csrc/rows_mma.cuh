@@ -12,8 +12,7 @@
 //     shared memory with bulk copies.
 //   * A CTA has a slice of K (mostly all of it) and some row-blocks; their records are one list that its 20 warps share out
 //     evenly, in the order of K, so a row-block's partial sums are few and added in a fixed order: a product has the same bits in
-//     every call.  20 warps of 96 registers leave 4096 registers, room for a CTA of rows_x_kernel, which is there when the
-//     predecessor ends.
+//     every call.  20 warps of 96 registers leave room for a CTA of rows_x_kernel, which is there when the predecessor ends.
 //
 // Arithmetic.  An integer below 2048 in the low bits of a half IS the f16 number n 2^-24, so a masked field needs no conversion:
 // one multiplication (centred widths: one fused multiply-add) gives (q - mid) ss 2^-20, exact below 2^11: widths 2 to 5 with the
@@ -25,8 +24,8 @@
 // (14.4), 28672 x 4096 25.2 / 21.0 (28.3), NINT6 28672 x 4096 31.7 / 26.6 (32.1), 4096 x 14336 19.6 / 16.9 (20.7), NINT3 14336 x
 // 4096 16.0 / 13.9 (20.1), NINT5 in groups of 28 5000 x 2888 10.2 / 9.1 (17.0), 28672 x 4096 33 / 28 (72), NVQ3 17408 x 5120 8
 // rows 21.0 (23.6), 5120 x 5120 12.1 (20.1); 3 rows (in brackets the integer kernel): NINT4 6144 x 4096 8.9 (16.4), NINT3 14336 x
-// 4096 13.8 (21.9).  Bound by instruction issue: some 390 a record (16 rows x 192 columns x 16 tokens) at 2.1 to 2.5 a clock,
-// half of them on pipes that take one every other clock.
+// 4096 13.8 (21.9).  Bound by the latency of the chain inside a warp (scales, codes, products, sums): some 390 instructions a
+// record (16 rows x 192 columns x 16 tokens) at 2.2 of 4 a clock from 20 warps, no pipe above 40 %, memory at 35 %.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
